@@ -1,0 +1,23 @@
+// Whole detection calls on the host side (detect.cpp): allocation, launch, the one wait for the counts, and the ragged
+// per-image views, shared by the region operators and by the Python modules.
+#pragma once
+
+#include <ATen/ATen.h>
+
+#include <vector>
+
+namespace functs_b200 {
+
+struct Detections {  // one image
+    at::Tensor dets, labels, ids;
+};
+
+struct SsdResult {
+    at::Tensor boxes, scores_cm;  // [B, P, 4], [B, C, P]
+    std::vector<Detections> images;
+};
+// want_ids = false leaves Detections::ids undefined
+SsdResult ssdDetect(const at::Tensor& loc, const at::Tensor& conf, const at::Tensor& priors, double clamp_max, double score_thr,
+                    int64_t topk, double iou_thr, bool want_ids);
+
+}  // namespace functs_b200

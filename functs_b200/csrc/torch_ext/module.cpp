@@ -8,11 +8,20 @@
 #include <torch/csrc/jit/passes/freeze_module.h>
 #include <torch/csrc/jit/passes/shape_analysis.h>
 
+#include "detect.h"
 #include "fusion.h"
 #include "tensorssa.h"
 
 namespace py = pybind11;
 using torch::jit::Graph;
+
+namespace {
+py::list pairs(const std::vector<functs_b200::Detections>& images) {
+    py::list out(images.size());
+    for (size_t b = 0; b < images.size(); ++b) out[b] = py::make_tuple(images[b].dets, images[b].labels);
+    return out;
+}
+}  // namespace
 
 PYBIND11_MODULE(_C, m) {
     m.doc() = "functs_b200: TensorSSA functionalization passes + immut:: operator registrations (loaded as a side effect)";
@@ -108,6 +117,17 @@ PYBIND11_MODULE(_C, m) {
         visit(g->block());
         return out;
     });
+    // whole detection calls (functs_b200/workloads.py): one (dets, labels) pair per image
+    m.def("_ssd_detect",
+          [](const at::Tensor& loc, const at::Tensor& conf, const at::Tensor& priors, double clamp_max, double score_thr, int64_t topk,
+             double iou_thr) {
+              functs_b200::SsdResult r;
+              {
+                  py::gil_scoped_release release;
+                  r = functs_b200::ssdDetect(loc, conf, priors, clamp_max, score_thr, topk, iou_thr, /*want_ids=*/false);
+              }
+              return pairs(r.images);
+          });
     m.def("_count_parallel_functors", [](std::shared_ptr<Graph> g) { return functs_b200::CountParallelFunctors(g); });
     m.def("_jit_pass_freeze", [](torch::jit::Module& module) { return torch::jit::freeze_module(module); });
     m.def("_jit_pass_clone", [](torch::jit::Module& module) { return module.clone(); });

@@ -34,6 +34,7 @@
 #include <unordered_set>
 
 #include "../../../include/functs_b200.h"
+#include "detect.h"
 #include "fusion.h"
 
 namespace functs_b200 {
@@ -459,8 +460,6 @@ Operation makeSsd(const Node* node) {
                 "ssd region: unexpected prior constants");
     at::Tensor priors_cpu = at::cat({pxy, pwh}, 1).contiguous();
     auto consts = std::make_shared<DeviceConstants>();
-    const int g1 = lookupGroup("ssd{softmax(-1)->slice[:-1]->delta2bbox->slice_rev[0::2,1::2](clamp)}");
-    const int g2 = lookupGroup("pmap[c<classes]{gt(thr)->nonzero->sort(desc,stable)->slice[:k]->index->torchvision::nms->index}");
     return [=](Stack& stack) {
         at::Tensor conf = cudaF32(pop(stack).toTensor(), "conf");
         at::Tensor loc = cudaF32(pop(stack).toTensor(), "loc");
@@ -475,44 +474,15 @@ Operation makeSsd(const Node* node) {
             if (v.empty()) v.push_back(priors_cpu.to(loc.device()));
             priors = v[0];
         }
-        const int64_t B = loc.size(0), P = loc.size(1), C = conf.size(2) - 1;
-        auto f32 = loc.options();
-        at::Tensor boxes = at::empty({B, P, 4}, f32), scores_cm = at::empty({B, C, P}, f32);
-        at::Tensor dets = at::empty({B, C, topk, 5}, f32), ids = at::empty({B, C, topk}, f32.dtype(at::kLong));
-        at::Tensor counts = at::empty({B, C}, f32.dtype(at::kInt));
-        void* stream = at::cuda::getCurrentCUDAStream().stream();
-        {
-            const void* in_ptrs[] = {loc.data_ptr(), conf.data_ptr(), priors.data_ptr()};
-            const int64_t ints[] = {B, P, C};
-            const double floats[] = {clamp_max};
-            void* outs[] = {boxes.data_ptr(), scores_cm.data_ptr()};
-            checkRc(functs_b200_group_launch(g1, in_ptrs, ints, floats, outs, nullptr, nullptr, stream), "ssd softmax + decode");
-        }
-        {
-            const void* in_ptrs[] = {boxes.data_ptr(), scores_cm.data_ptr()};
-            const int64_t ints[] = {B, P, C, topk};
-            const double floats[] = {thr, iou};
-            void* outs[] = {dets.data_ptr(), ids.data_ptr(), counts.data_ptr()};
-            checkRc(functs_b200_group_launch(g2, in_ptrs, ints, floats, outs, nullptr, nullptr, stream), "ssd class NMS");
-        }
-        // ragged results: one compaction over the whole batch, then per-image views
-        at::Tensor valid = at::arange(topk, counts.options()).view({1, 1, topk}) < counts.unsqueeze(-1);  // [B, C, K]
-        at::Tensor flat_valid = valid.reshape({-1});
-        at::Tensor all_dets = dets.reshape({-1, 5}).index({flat_valid});
-        at::Tensor all_ids = ids.reshape({-1}).index({flat_valid});
-        at::Tensor all_labels = at::arange(C, ids.options()).view({1, C, 1}).expand({B, C, topk}).reshape({-1}).index({flat_valid});
-        at::Tensor per_image = counts.sum({1}, false, at::kLong).cpu();
-        const int64_t* pi = per_image.data_ptr<int64_t>();
+        SsdResult r = ssdDetect(loc, conf, priors, clamp_max, thr, topk, iou, /*want_ids=*/true);
         c10::impl::GenericList results(c10::TupleType::create({c10::TensorType::get(), c10::TensorType::get(), c10::TensorType::get()}));
-        int64_t off = 0;
-        for (int64_t b = 0; b < B; ++b) {
-            results.push_back(c10::ivalue::Tuple::create(
-                {all_dets.narrow(0, off, pi[b]), all_labels.narrow(0, off, pi[b]), all_ids.narrow(0, off, pi[b])}));
-            off += pi[b];
+        results.reserve(r.images.size());
+        for (Detections& d : r.images) {
+            results.push_back(c10::ivalue::Tuple::create({std::move(d.dets), std::move(d.labels), std::move(d.ids)}));
         }
-        push(stack, scores_cm.permute({0, 2, 1}));
+        push(stack, r.scores_cm.permute({0, 2, 1}));
         stack.emplace_back(std::move(results));
-        push(stack, std::move(boxes));
+        push(stack, std::move(r.boxes));
     };
 }
 

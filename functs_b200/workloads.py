@@ -21,6 +21,11 @@ def _dev(device) -> torch.device:
     return d
 
 
+def _native():
+    from . import _C  # built with the package; needed by whole calls only, so that the kernels import without it
+    return _C
+
+
 def get_started(a: torch.Tensor, b: torch.Tensor, n: int, device="cuda") -> torch.Tensor:
     """examples/get_started.py:10-15: b = b.clone(); for i in range(n): b[i] = b[i] + 1; return b."""
     if n > b.size(0):
@@ -98,8 +103,14 @@ class SSDBBox:
         return boxes, dets, ids, counts
 
     def __call__(self, loc: torch.Tensor, conf: torch.Tensor) -> List[Tuple[torch.Tensor, torch.Tensor]]:
-        _, dets, ids, counts = self.forward_padded(loc, conf)
-        return [(d, l) for d, l, _ in self.unpad(dets, ids, counts)]
+        # both launches, the wait for the counts and the per-image views in one native call; the kernel writes the ragged
+        # rows itself (unpad() is for callers of forward_padded)
+        loc = ops._req(loc.to(self.device, non_blocking=True), torch.float32, "loc")
+        conf = ops._req(conf.to(self.device, non_blocking=True), torch.float32, "conf")
+        before = launch_count()
+        out = _native()._ssd_detect(loc, conf, self.priors, self.clamp_max, self.score_thr, self.topk, self.iou_thr)
+        self.kernels_last_call = launch_count() - before
+        return out
 
     @staticmethod
     def unpad(dets: torch.Tensor, ids: torch.Tensor, counts: torch.Tensor):

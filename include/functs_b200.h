@@ -190,6 +190,22 @@ int functs_b200_ssd_class_nms(const float* boxes, const float* scores_cm, int32_
                               int32_t num_classes, float score_thr, int32_t topk, float iou_thr, float* dets,
                               int64_t* prior_ids, int32_t* out_counts, void* stream);
 
+/* Both groups in one call, with the ragged result the program returns: image b's kept rows of all classes, class after class,
+ * are dets / labels / prior_ids [b * C * topk, + img_counts[b]).  dets [batch * C * topk, 5]; labels, prior_ids
+ * [batch * C * topk]; img_counts [batch] and the optional status word may be pinned host memory (both are written by the
+ * kernel, so that a caller who waits for the stream needs no copy).  Two launches, no memset.
+ * scratch: functs_b200_ssd_scratch_bytes(batch, C). */
+int64_t functs_b200_ssd_scratch_bytes(int32_t batch, int32_t num_classes);
+int functs_b200_ssd_postprocess(const float* loc, const float* conf, const float* priors, int32_t batch, int32_t num_priors,
+                                int32_t num_classes, float clamp_max, float score_thr, int32_t topk, float iou_thr, float* boxes,
+                                float* scores_cm, float* dets, int64_t* labels, int64_t* prior_ids, int32_t* img_counts,
+                                int32_t* status, void* scratch, void* stream);
+/* Moves the rows [g * stride, g * stride + counts[g]) of every group g together (ids / out_ids may be NULL): for a caller
+ * that keeps a ragged result and does not want to keep the room it was written into.  counts may be pinned host memory.
+ * One launch. */
+int functs_b200_ragged_pack(const float* dets, const int64_t* labels, const int64_t* ids, const int32_t* counts, int32_t groups,
+                            int64_t stride, float* out_dets, int64_t* out_labels, int64_t* out_ids, void* stream);
+
 /* ---- C4: imperative LSTM with slice-assigned outputs ---------------------------------------- */
 /* Follows functs/benchmark/ai_model/lstm/lstm.py:79-98, 118-133 (one layer; hs[t] = h, cs[t] = c kept).
  * x [T, B, I]; w_ih [4, I, H]; w_hh [4, H, H]; b_ih, b_hh [4, H]; hs, cs [T, B, H]; gate order i, f, g, o;
