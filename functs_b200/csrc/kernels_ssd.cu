@@ -100,7 +100,6 @@ constexpr int kSsdSelCap = 256;
 constexpr int kSsdWords = kSsdSelCap / 32;
 
 constexpr size_t kSsdSelBytes = (sizeof(SelectSmem<kSsdSelCap>) + 127) / 128 * 128;
-constexpr int kSsdRowBatch = 16;  // rows of the suppression matrix one warp tests at a time (4: 419 us, 8: 378, 16: 370)
 
 // Ragged output (RAGGED = true): the kept rows of an image's classes follow one another in class order from row
 // img * num_classes * topk on, instead of every class owning topk padded rows.  A CTA publishes its own count first and
@@ -116,8 +115,8 @@ struct SsdRagged {
 };
 constexpr unsigned long long kSsdWaitCycles = 2000000000ull;  // ~1 s
 
-// dynamic smem: [SelectSmem<256>][kCandCap candidate keys]; after the selection the NMS boxes and the 256 x 8 mask words
-// live in the selection's boundary list and histogram, which are not needed any more.  The class's scores (one contiguous
+// dynamic smem: [SelectSmem<256>][kCandCap candidate keys]; after the selection the NMS boxes live in the selection's boundary
+// list and the pair tables in the candidate list, which are not needed any more.  The class's scores (one contiguous
 // run of the class-major array) are read from global memory once: a sampled score floor, one collection pass, and the
 // exact selection on the few hundred candidates (block_select_topk_sampled).
 template <bool RAGGED>
@@ -128,15 +127,13 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
                      int32_t* __restrict__ out_counts, const SsdRagged rag) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SelectSmem<kSsdSelCap>& sm = *reinterpret_cast<SelectSmem<kSsdSelCap>*>(smem_raw);
-    static_assert(sizeof(NmsBox) * kSsdSelCap <= sizeof(sm.binlist) && sizeof(uint32_t) * kSsdSelCap * kSsdWords <= sizeof(sm.hist),
-                  "the NMS work area must fit the parts of the selection state it reuses");
+    static_assert(sizeof(PairCells<kSsdWords>) <= sizeof(uint64_t) * kCandCap, "the pair tables reuse the candidate list");
     // selected boxes as corners (one 16-byte shared load) + area, in the boundary list of the finished selection
     static_assert(sizeof(float4) * kSsdSelCap + sizeof(float) * kSsdSelCap <= sizeof(sm.binlist) &&
                       offsetof(SelectSmem<kSsdSelCap>, binlist) % 16 == 0,
                   "the corner / area arrays must fit (and be 16-byte aligned in) the boundary list");
     float4* sxy = reinterpret_cast<float4*>(sm.binlist);
     float* sarea = reinterpret_cast<float*>(sxy + kSsdSelCap);
-    uint32_t* smask = reinterpret_cast<uint32_t*>(sm.hist);
     uint64_t* cand = reinterpret_cast<uint64_t*>(smem_raw + kSsdSelBytes);
     __shared__ uint32_t keep_words[kSsdWords];
     __shared__ int word_prefix[kSsdWords + 1];
@@ -152,98 +149,48 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
         cls = s_ticket - img * num_classes;
     }
     const float* src = scores_cm + (static_cast<int64_t>(img) * num_classes + cls) * num_priors;
-    const bool vec4 = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-    const int n = block_select_topk_sampled<kSsdNmsThreads, kSsdSelCap>(src, vec4, score_thr, num_priors, topk, hist_base,
-                                                                        hist_shift, sm, cand);
+    const int n = block_select_topk_sampled<kSsdNmsThreads, kSsdSelCap>(src, score_thr, num_priors, topk, hist_base, hist_shift, sm, cand);
     // (block_select_topk ends with a barrier when n > 1; make the hand-over explicit)
     __syncthreads();
 
     const float* bimg = boxes + static_cast<int64_t>(img) * num_priors * 4;
     float4 mybox = make_float4(0.f, 0.f, 0.f, 0.f);
     uint64_t mykey = 0ull;
+    float myarea = 0.0f;
     bool tame_box = true;
     if (t < n) {
         mykey = sm.sel[t];
         mybox = __ldg(reinterpret_cast<const float4*>(bimg) + key_index(mykey));
         const NmsBox nb = make_nms_box(mybox.x, mybox.y, mybox.z, mybox.w);
         tame_box = nms_box_is_tame(nb);
+        myarea = nb.area;
         sxy[t] = mybox;
-        sarea[t] = nb.area;
+        sarea[t] = myarea;
     }
     if (t < kSsdWords) keep_words[t] = 0u;
     const bool tame = __syncthreads_and(tame_box ? 1 : 0) != 0;  // also the barrier behind the box stores
 
-    // suppression bit matrix.  A task is (column word w, batch of rows): lane b holds box j = 32w + b, the rows' boxes
-    // are broadcast reads, the tests of a batch are independent and branch-free, and one ballot per row yields the
-    // word, which a single lane stores: no atomics.  Word w only needs the rows i < 32w + 31; tasks are dealt
-    // round-robin to the warps.
+    // Suppression rows, thread t = row t.  Tame boxes only test the pairs that PairCells leaves (200 x 200 all-pairs votes
+    // took 45 % of this kernel's time); a list with a wild box tests every pair behind the row.
     const int lane = t & 31, warp = t >> 5;
-    const int words = (n + 31) >> 5;
-    for (int i = t; i < n * kSsdWords; i += kSsdNmsThreads) smask[i] = 0u;
-    __syncthreads();
-    {
-        int total = 0;
-        for (int w = 0; w < words; ++w) total += (min(n, 32 * w + 31) + kSsdRowBatch - 1) / kSsdRowBatch;
-        for (int task = warp; task < total; task += kSsdNmsThreads / 32) {
-            int w = 0, rb = task;
-            for (;; ++w) {
-                const int nb = (min(n, 32 * w + 31) + kSsdRowBatch - 1) / kSsdRowBatch;
-                if (rb < nb) break;
-                rb -= nb;
-            }
-            const int j = 32 * w + lane;
-            const bool jv = j < n;
-            const float4 cj = sxy[jv ? j : 0];
-            const float aj = sarea[jv ? j : 0];
-            const NmsBox bj{cj.x, cj.y, cj.z, cj.w, aj};
-            const int i0 = rb * kSsdRowBatch;
-            if (tame) {
-                // Common case first: most pairs do not come near the threshold.  With the width clamped at zero the
-                // product w * h is positive only for a real intersection, and for tame boxes the union is positive, so
-                // "inter >= union * thr_lo" is necessary for the quotient to exceed the threshold: one vote per row on
-                // that; the few pairs that pass are settled by the exact test, and a non-empty word (rare) is stored by
-                // one lane.  The matrix was cleared above.
-                // (Measured and dropped: the centre form (hw_a + hw_b) - |cx_a - cx_b| as an add / multiply upper bound of
-                // the overlap.  It is loose when one box contains the other, which priors of one cell do all the time:
-                // the exact test ran so often that the matrix took 24 us per list instead of 15.)
-                // (Also measured and dropped: all votes of a batch first, then the rows with a candidate: 20 us.)
-                // (And: the union test as a sum of per-box terms, inter >= c * a_i + c * a_j with c = thr / (1 + thr), plus a
-                // row mask on the vote instead of the per-lane i < j test: two instructions fewer per pair on paper, 299 us
-                // against 292 for the kernel.)
+    uint32_t row[kSsdWords];
+    if (tame) {
+        suppression_row<kSsdWords>(sxy, sarea, mybox, myarea, n, iou_thr, thr_lo, thr_hi, *reinterpret_cast<PairCells<kSsdWords>*>(cand), row);
+    } else {
+        const NmsBox bi{mybox.x, mybox.y, mybox.z, mybox.w, myarea};
 #pragma unroll
-                for (int u = 0; u < kSsdRowBatch; ++u) {
-                    const int i = i0 + u;
-                    const int ii = i < n ? i : 0;
-                    const float4 ci = sxy[ii];
-                    const float ai = sarea[ii];
-                    const float iw = fmaxf(0.0f, __fsub_rn(fminf(ci.z, cj.z), fmaxf(ci.x, cj.x)));
-                    const float ih = __fsub_rn(fminf(ci.w, cj.w), fmaxf(ci.y, cj.y));
-                    const float inter = __fmul_rn(iw, ih);
-                    const float uni = __fsub_rn(__fadd_rn(ai, aj), inter);
-                    const bool maybe = jv && i < j && !(inter < __fmul_rn(uni, thr_lo));  // i < j implies i < n
-                    uint32_t bits = __ballot_sync(kFullMask, maybe);
-                    if (bits != 0u) {
-                        const NmsBox bi{ci.x, ci.y, ci.z, ci.w, ai};
-                        bits = __ballot_sync(kFullMask, maybe && iou_exceeds(bi, bj, iou_thr, thr_lo, thr_hi));
-                        if (lane == 0 && bits != 0u) smask[i * kSsdWords + w] = bits;
-                    }
-                }
-            } else {
-#pragma unroll 1
-                for (int u = 0; u < kSsdRowBatch; ++u) {
-                    const int i = i0 + u;
-                    const int ii = i < n ? i : 0;
-                    const float4 ci = sxy[ii];
-                    const NmsBox bi{ci.x, ci.y, ci.z, ci.w, sarea[ii]};
-                    const bool hit = jv && i < j && iou_exceeds(bi, bj, iou_thr, thr_lo, thr_hi);
-                    const uint32_t bits = __ballot_sync(kFullMask, hit);
-                    if (lane == 0 && bits != 0u) smask[i * kSsdWords + w] = bits;
-                }
+        for (int w = 0; w < kSsdWords; ++w) {
+            row[w] = 0u;
+            if (t >= n) continue;
+            for (int j = max(32 * w, t + 1); j < min(32 * w + 32, n); ++j) {
+                const float4 cj = sxy[j];
+                const NmsBox bj{cj.x, cj.y, cj.z, cj.w, sarea[j]};
+                if (iou_exceeds(bi, bj, iou_thr, thr_lo, thr_hi)) row[w] |= 1u << (j & 31);
             }
         }
     }
     __syncthreads();
-    block_nms_resolve<kSsdNmsThreads, kSsdWords>(smask, n, keep_words, or_words);
+    block_nms_resolve<kSsdNmsThreads, kSsdWords>(row, n, keep_words, or_words);
     __syncthreads();
     if (t == 0) {
         int acc = 0;

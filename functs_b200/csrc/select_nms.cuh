@@ -66,31 +66,6 @@ __device__ __forceinline__ void bitonic_sort_desc(uint64_t* s, int n) {
     }
 }
 
-// Rank sort, descending, of n <= NT distinct keys: thread t counts the keys larger than s[t] (broadcast reads) and
-// drops its key at that rank.  Cheaper than the bitonic network for a few hundred keys (no barrier per step).
-// tmp: n more keys of shared memory; s must be 16-byte aligned.  Ends with a barrier; the sorted keys are back in s.
-template <int NT>
-__device__ __forceinline__ void rank_sort_desc(uint64_t* s, int n, uint64_t* tmp) {
-    const int t = threadIdx.x;
-    uint64_t mine = 0ull;
-    int rank = 0;
-    if (t < n) {
-        mine = s[t];
-        const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(s);  // two keys per (broadcast) load
-#pragma unroll 4
-        for (int j = 0; j < (n >> 1); ++j) {
-            const ulonglong2 k = s2[j];
-            rank += (k.x > mine) ? 1 : 0;
-            rank += (k.y > mine) ? 1 : 0;
-        }
-        if (n & 1) rank += (s[n - 1] > mine) ? 1 : 0;
-        tmp[rank] = mine;
-    }
-    __syncthreads();
-    if (t < n) s[t] = tmp[t];
-    __syncthreads();
-}
-
 __device__ __forceinline__ int next_pow2(int v) {
     int p = 1;
     while (p < v) p <<= 1;
@@ -554,54 +529,6 @@ struct ListKeys {
 
 constexpr int kCandCap = 1024;  // candidate keys block_select_topk_sampled may collect before it gives up
 
-// The largest digit d with (entries of hist in buckets >= d) >= target, or -1 when the histogram holds fewer.
-// hist is left as it is.  All NT threads must call it.
-template <int NT>
-__device__ int block_hist_rank_bucket(const int* hist, int* red_cnt, int* slot, int target) {
-    static_assert(kHistBins % NT == 0, "the histogram must split evenly over the block");
-    constexpr int per = kHistBins / NT;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int h[per];
-    int s = 0;
-#pragma unroll
-    for (int k = 0; k < per; ++k) {
-        h[k] = hist[tid * per + k];
-        s += h[k];
-    }
-    int incl = s;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_down_sync(kFullMask, incl, o);
-        if (lane + o < 32) incl += t;
-    }
-    if (lane == 0) red_cnt[warp] = incl;
-    if (tid == 0) *slot = -1;
-    __syncthreads();
-    int higher = 0;
-#pragma unroll
-    for (int w = 0; w < NT / 32; ++w) higher += (w > warp) ? red_cnt[w] : 0;
-    incl += higher;
-    const int suf = incl - s;
-    if (suf < target && incl >= target) {
-        int cum = suf, d = 0;
-        bool found = false;
-#pragma unroll
-        for (int k = per - 1; k >= 0; --k) {
-            if (!found) {
-                if (cum + h[k] >= target) {
-                    found = true;
-                    d = k;
-                } else {
-                    cum += h[k];
-                }
-            }
-        }
-        *slot = tid * per + d;
-    }
-    __syncthreads();
-    return *slot;
-}
-
 // the two-pass selection over a whole score array, out of line (the sampled selection's rare way out)
 template <int NT, int SELCAP>
 __device__ __noinline__ int block_select_dense_outlined(const float* s, bool vec4, float thr, int n, int topk, uint32_t hist_base,
@@ -612,91 +539,100 @@ __device__ __noinline__ int block_select_dense_outlined(const float* s, bool vec
 // Same result as block_select_topk_binned for a plain fp32 score array in GLOBAL memory (key = score above thr, index),
 // reading the array once: a spread sample of the scores (one 16-byte chunk per thread) gives a score floor that should
 // leave a few hundred candidates; one pass collects every key at or above the floor into `cand` (kCandCap keys of
-// shared memory, appended with one atomic per warp and round); the exact selection then runs on that list.  The floor
-// is only a guess, the count decides: with fewer than topk candidates (while keys below the floor exist) or more than
-// kCandCap, the two-pass selection over the whole array runs instead, so the result never depends on the sample.
+// shared memory); the exact selection then runs on that list.  The floor is only a guess, the count decides: with fewer
+// than topk candidates (while keys below the floor exist) or more than kCandCap, the two-pass selection over the whole
+// array runs instead, so the result never depends on the sample.
+// The pass is bound by issue, not by memory: twelve scores per lane cost one compare and one mask bit each, lanes without a
+// hit (about half of them) stop there, and a lane with hits reserves its places with one shared-memory atomic and reads the
+// few scores again (L1).  A warp prefix sum per 16-byte chunk instead took half as long again.
 template <int NT, int SELCAP>
-__device__ int block_select_topk_sampled(const float* __restrict__ s, bool vec4, float thr, int n, int topk,
-                                         uint32_t hist_base, int hist_shift, SelectSmem<SELCAP>& sm, uint64_t* cand) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n4 = vec4 ? (n >> 2) : 0;
-    const float4* s4 = reinterpret_cast<const float4*>(s);
-    uint32_t lo_bits = 0u;  // 0: every score above thr is a candidate
+__device__ int block_select_topk_sampled(const float* __restrict__ s, float thr, int n, int topk, uint32_t hist_base,
+                                         int hist_shift, SelectSmem<SELCAP>& sm, uint64_t* cand) {
+    const int tid = threadIdx.x;
+    // an array that starts off a 16-byte boundary has up to three scores in front of its first whole chunk
+    const int head = min(n, static_cast<int>(((16u - static_cast<uint32_t>(reinterpret_cast<uintptr_t>(s) & 15u)) & 15u) >> 2));
+    const int n4 = (n - head) >> 2;
+    const float4* s4 = reinterpret_cast<const float4*>(s + head);
+    float floor_score = __uint_as_float(__float_as_uint(thr) + 1u);  // (thr > 0) "above thr" as a >=
+    bool floored = false;
     if (n > kCandCap && n4 >= NT) {
-        for (int i = tid; i < kHistBins; i += NT) sm.hist[i] = 0;
+        // a coarse histogram will do: NT buckets, one per thread
+        constexpr int kCoarse = kHistBins / NT;
+        static_assert(kHistBins % NT == 0, "whole buckets per thread");
+        sm.hist[tid] = 0;
         __syncthreads();
         const float4 q = __ldg(s4 + static_cast<int>((static_cast<int64_t>(tid) * n4) / NT));
         auto add = [&](float v) {
-            if (v > thr) atomicAdd(&sm.hist[hist_digit(static_cast<uint64_t>(__float_as_uint(v)) << 32, hist_base, hist_shift)], 1);
+            if (v > thr)
+                atomicAdd(&sm.hist[hist_digit(static_cast<uint64_t>(__float_as_uint(v)) << 32, hist_base, hist_shift) / kCoarse], 1);
         };
         add(q.x);
         add(q.y);
         add(q.z);
         add(q.w);
+        if (tid == 0) sm.digit = 0;
         __syncthreads();
         // rank in the sample that corresponds to 1.8 * topk in the whole array (the spread of a count of a few dozen
         // sample hits is about a sixth of it: falling short of topk takes three standard deviations)
         const int target = static_cast<int>((static_cast<int64_t>(topk) * (4 * NT) * 9) / (static_cast<int64_t>(n) * 5)) + 4;
-        const int d = block_hist_rank_bucket<NT>(sm.hist, sm.red_cnt, &sm.digit, target);
-        if (d > 0) lo_bits = hist_base + (static_cast<uint32_t>(d) << hist_shift);
+        const int lane = tid & 31, warp = tid >> 5;
+        const int mine = sm.hist[tid];
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_down_sync(kFullMask, incl, o);
+            if (lane + o < 32) incl += t;
+        }
+        if (lane == 0) sm.red_cnt[warp] = incl;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < NT / 32; ++w) incl += (w > warp) ? sm.red_cnt[w] : 0;
+        if (incl >= target && incl - mine < target) sm.digit = tid * kCoarse;
     }
     if (tid == 0) sm.bin_cnt = 0;
     __syncthreads();
-    // collection: lane-local hit counts, a warp prefix sum, one atomic per warp and round
-    auto append = [&](const uint64_t (&k)[4], int cnt) {
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(kFullMask, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int total = __shfl_sync(kFullMask, incl, 31);
-        if (total != 0) {
-            int base = 0;
-            if (lane == 31) base = atomicAdd(&sm.bin_cnt, total);
-            base = __shfl_sync(kFullMask, base, 31);
-            int pos = base + incl - cnt;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (k[e] != 0ull) {
-                    if (pos < kCandCap) cand[pos] = k[e];
-                    ++pos;
-                }
-            }
-        }
-    };
-    auto key_of = [&](float v, int i) -> uint64_t {
-        return (v > thr && __float_as_uint(v) >= lo_bits) ? make_key(v, static_cast<uint32_t>(i)) : 0ull;
+    if (n > kCandCap && n4 >= NT && sm.digit > 0) {
+        floor_score = __uint_as_float(hist_base + (static_cast<uint32_t>(sm.digit) << hist_shift));
+        floored = true;
+    }
+    auto put = [&](float v, int i) {
+        const int pos = atomicAdd(&sm.bin_cnt, 1);
+        if (pos < kCandCap) cand[pos] = make_key(v, static_cast<uint32_t>(i));
     };
     constexpr int UN = 3;
-    for (int c0 = warp * 32 + lane; __any_sync(kFullMask, c0 < n4); c0 += NT * UN) {
-        float4 q[UN];
+    for (int c0 = tid; c0 < n4; c0 += NT * UN) {
+        uint32_t hits = 0u;
 #pragma unroll
         for (int u = 0; u < UN; ++u) {
             const int c = c0 + u * NT;
-            q[u] = c < n4 ? __ldg(s4 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 q = c < n4 ? __ldg(s4 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            hits |= (q.x >= floor_score ? 1u : 0u) << (4 * u);
+            hits |= (q.y >= floor_score ? 2u : 0u) << (4 * u);
+            hits |= (q.z >= floor_score ? 4u : 0u) << (4 * u);
+            hits |= (q.w >= floor_score ? 8u : 0u) << (4 * u);
         }
-#pragma unroll
-        for (int u = 0; u < UN; ++u) {
-            const int c = c0 + u * NT;
-            uint64_t k[4];
-            k[0] = key_of(q[u].x, 4 * c);
-            k[1] = key_of(q[u].y, 4 * c + 1);
-            k[2] = key_of(q[u].z, 4 * c + 2);
-            k[3] = key_of(q[u].w, 4 * c + 3);
-            append(k, (k[0] != 0ull) + (k[1] != 0ull) + (k[2] != 0ull) + (k[3] != 0ull));
+        if (hits != 0u) {
+            int pos = atomicAdd(&sm.bin_cnt, __popc(hits));
+            while (hits != 0u) {
+                const int k = __ffs(hits) - 1;
+                hits &= hits - 1u;
+                const int i = head + 4 * (c0 + (k >> 2) * NT) + (k & 3);
+                if (pos < kCandCap) cand[pos] = make_key(__ldg(s + i), static_cast<uint32_t>(i));
+                ++pos;
+            }
         }
     }
-    for (int i0 = 4 * n4 + warp * 32; i0 < n; i0 += NT) {  // scalar tail (or the whole array when it is not 16-byte aligned)
-        const int i = i0 + lane;
-        uint64_t k[4] = {i < n ? key_of(__ldg(s + i), i) : 0ull, 0ull, 0ull, 0ull};
-        append(k, k[0] != 0ull ? 1 : 0);
+    const int tail0 = head + 4 * n4;
+    if (tid < head + n - tail0) {  // the scores in front of and behind the whole chunks: at most six
+        const int i = tid < head ? tid : tail0 + tid - head;
+        const float v = __ldg(s + i);
+        if (v >= floor_score) put(v, i);
     }
     __syncthreads();
     const int c = sm.bin_cnt;
     __syncthreads();  // (the selections below reset the counter)
-    if (c > kCandCap || (lo_bits != 0u && c < topk)) {
-        return block_select_dense_outlined<NT, SELCAP>(s, vec4, thr, n, topk, hist_base, hist_shift, &sm);
+    if (c > kCandCap || (floored && c < topk)) {
+        return block_select_dense_outlined<NT, SELCAP>(s, head == 0, thr, n, topk, hist_base, hist_shift, &sm);
     }
     return block_select_topk_binned<NT, SELCAP, 2>(ListKeys{cand}, c, topk, hist_base, hist_shift, sm);
 }
@@ -734,122 +670,136 @@ __device__ __forceinline__ bool iou_exceeds(const NmsBox& a, const NmsBox& b, fl
     return __fdiv_rn(inter, uni) > thr;
 }
 
-// The same decision without branches, for callers that run several independent tests at once: verdict 0 = not above,
-// 1 = above, 2 = inside the bracket (the caller forms the correctly rounded quotient inter / uni and compares it
-// with thr, as iou_exceeds does).
-struct IouQuick {
-    float inter, uni;
-    int verdict;
-};
-__device__ __forceinline__ IouQuick iou_quick(const NmsBox& a, const NmsBox& b, float thr_lo, float thr_hi) {
-    IouQuick q;
-    const float w = fmaxf(0.0f, __fsub_rn(fminf(a.x2, b.x2), fmaxf(a.x1, b.x1)));
-    const float h = fmaxf(0.0f, __fsub_rn(fminf(a.y2, b.y2), fmaxf(a.y1, b.y1)));
-    q.inter = __fmul_rn(w, h);
-    q.uni = __fsub_rn(__fadd_rn(a.area, b.area), q.inter);
-    const bool pos = (w > 0.0f) && (q.inter > 0.0f);
-    const bool safe = q.uni > 0.0f && q.uni < 3.0e38f && q.inter < 3.0e38f;
-    const bool yes = pos && safe && q.inter > __fmul_rn(q.uni, thr_hi);
-    const bool no = !pos || (safe && q.inter < __fmul_rn(q.uni, thr_lo));
-    q.verdict = yes ? 1 : (no ? 0 : 2);
-    return q;
-}
-
-// For boxes with finite coordinates and areas below 1e37 (nms_box_is_tame) the guards of iou_exceeds are implied by a
-// positive intersection: inter <= min(area) and max(area) <= union <= 2e37.  yes / unsure as in iou_quick.
+// Finite coordinates and an area below 1e37: the guards of iou_exceeds are then implied by a positive intersection
+// (inter <= min(area) and max(area) <= union <= 2e37).
 __device__ __forceinline__ bool nms_box_is_tame(const NmsBox& b) {
     return fabsf(b.x1) < 1.0e18f && fabsf(b.y1) < 1.0e18f && fabsf(b.x2) < 1.0e18f && fabsf(b.y2) < 1.0e18f && b.area < 1.0e37f;
 }
-__device__ __forceinline__ void iou_quick_tame(const NmsBox& a, const NmsBox& b, float thr_lo, float thr_hi, bool& yes,
-                                               bool& unsure) {
-    const float w = __fsub_rn(fminf(a.x2, b.x2), fmaxf(a.x1, b.x1));
-    const float h = __fsub_rn(fminf(a.y2, b.y2), fmaxf(a.y1, b.y1));
-    const float inter = __fmul_rn(w, h);
-    const float uni = __fsub_rn(__fadd_rn(a.area, b.area), inter);
-    const bool pos = w > 0.0f && h > 0.0f && inter > 0.0f;
-    yes = pos && inter > __fmul_rn(uni, thr_hi);
-    unsure = pos && !yes && !(inter < __fmul_rn(uni, thr_lo));
+// Candidate pairs for the suppression test of up to 256 boxes, as bit sets: box j can only suppress or be suppressed by box i
+// if their x ranges and their y ranges overlap and their areas are within a factor of thr of one another (IoU <= smaller /
+// larger area).  Every one of the three is a range condition on a monotone cell number, so six tables of cumulative sets
+// answer it: lo tables hold the boxes whose cell is <= c, hi tables those whose cell is >= c, and the candidates of box i are
+// the AND of six look-ups per 32 boxes.  On SSD priors this leaves a few per cent of the pairs, where sorted windows along
+// one axis left most of them.
+constexpr int kCells = 32;  // one lane per cell in the cumulation
+template <int WORDS>
+struct PairCells {
+    uint32_t t[6][WORDS][kCells];  // x1 <=, x2 >=, y1 <=, y2 >=, area <=, area >=
+    float lo, hi;
+    uint32_t ordered_lo, ordered_hi, area_base;
+};
+// an fp32 value as an unsigned number of the same order
+__device__ __forceinline__ uint32_t ordered_bits(float v) {
+    const uint32_t b = __float_as_uint(v);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
+__device__ __forceinline__ float from_ordered_bits(uint32_t o) { return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o); }
 
-// One word of a row of the suppression matrix: lane b tests box j = 32w + b against box i (valid = j > i && j < n).
-// The x extents are compared first for the whole warp; only if some lane overlaps in x is the full test run.
-// Must be called by all 32 lanes.
-__device__ __forceinline__ uint32_t nms_row_word(const NmsBox& bi, const NmsBox* sb, int j, bool valid, float thr,
-                                                 float thr_lo, float thr_hi) {
-    bool cand = false;
-    if (valid) cand = fminf(bi.x2, sb[j].x2) > fmaxf(bi.x1, sb[j].x1);  // positive overlap in x
-    if (__ballot_sync(kFullMask, cand) == 0u) return 0u;
-    bool pred = false;
-    if (cand) pred = iou_exceeds(bi, sb[j], thr, thr_lo, thr_hi);
-    return __ballot_sync(kFullMask, pred);
-}
-
-// Serial part of greedy NMS over a precomputed suppression bit matrix, run by ONE warp.
-// mask: row i has `words` 32-bit words (row stride `row_stride` words); bit j of row i set iff j > i and box i
-// suppresses box j.  keep_words[w] receives the keep bits of boxes 32w..32w+31.  words <= 32.
-__device__ __forceinline__ void warp_nms_scan(const uint32_t* mask, int row_stride, int n, int words,
-                                              uint32_t* keep_words) {
-    const int lane = threadIdx.x & 31;
-    uint32_t removed = 0u;  // lane l tracks word l
-    for (int w = 0; w < words; ++w) {
-        uint32_t r = __shfl_sync(kFullMask, removed, w);
-        const int base = w * 32;
-        const int rows = min(32, n - base);
-        // loads first (none depends on a decision): the diagonal 32x32 block (broadcast reads, identical on every
-        // lane) and this lane's column word of the 32 rows
-        uint32_t diag[32], col[32];
-#pragma unroll
-        for (int b = 0; b < 32; ++b) {
-            const bool in = b < rows;
-            diag[b] = in ? mask[(base + b) * row_stride + w] : 0u;
-            col[b] = (in && lane < words) ? mask[(base + b) * row_stride + lane] : 0u;
+// All 32 * WORDS threads; thread t owns box t (valid = t < n; all boxes tame).  Fills row[w] with the bits of the boxes
+// 32w .. 32w + 31 behind box t that box t suppresses.
+template <int WORDS>
+__device__ __forceinline__ void suppression_row(const float4* sxy, const float* sarea, const float4 me, float area, int n, float thr,
+                                                float thr_lo, float thr_hi, PairCells<WORDS>& pc, uint32_t (&row)[WORDS]) {
+    constexpr int NT = 32 * WORDS;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const bool real = t < n && me.z > me.x && me.w > me.y && area > 0.0f;  // others intersect nothing
+    for (int i = t; i < 6 * WORDS * kCells; i += NT) (&pc.t[0][0][0])[i] = 0u;
+    if (t == 0) {
+        pc.ordered_lo = 0xffffffffu;
+        pc.ordered_hi = 0u;
+        pc.area_base = 0u;
+    }
+    __syncthreads();
+    {
+        const uint32_t l = __reduce_min_sync(kFullMask, real ? ordered_bits(fminf(me.x, me.y)) : 0xffffffffu);
+        const uint32_t h = __reduce_max_sync(kFullMask, real ? ordered_bits(fmaxf(me.z, me.w)) : 0u);
+        const uint32_t a = __reduce_max_sync(kFullMask, real ? __float_as_uint(area) >> 22 : 0u);
+        if (lane == 0) {
+            atomicMin(&pc.ordered_lo, l);
+            atomicMax(&pc.ordered_hi, h);
+            atomicMax(&pc.area_base, a);
         }
-        // Serial part.  Row b can only set bits above b, so bit b of r is final once the rows before b are done and
-        // keepw = ~r (valid rows) at the end.  Only rows with a non-empty diagonal word can change r: when there
-        // are few of them they are walked in order (re-read from shared memory by index), otherwise all 32 rows go
-        // through the unrolled register chain.
-        uint32_t nz = 0u;
+    }
+    __syncthreads();
+    const float lo = from_ordered_bits(pc.ordered_lo), hi = from_ordered_bits(pc.ordered_hi);
+    const float scale = hi > lo ? __fdividef(static_cast<float>(kCells), hi - lo) : 0.0f;
+    const int abase = static_cast<int>(pc.area_base) - (kCells - 1);  // the largest area sits in the last cell; two cells per octave
+    // monotone in v whatever the rounding of `scale`: a subtraction, a product and a conversion, each monotone
+    auto cell = [&](float v) { return min(max(__float2int_rd(__fmul_rn(__fsub_rn(v, lo), scale)), 0), kCells - 1); };
+    auto area_cell = [&](float a) { return min(max(static_cast<int>(__float_as_uint(a) >> 22) - abase, 0), kCells - 1); };
+    int cx1 = 0, cx2 = 0, cy1 = 0, cy2 = 0;
+    if (real) {
+        cx1 = cell(me.x);
+        cy1 = cell(me.y);
+        cx2 = cell(me.z);
+        cy2 = cell(me.w);
+        const int ca = area_cell(area);
+        const uint32_t bit = 1u << lane;
+        atomicOr(&pc.t[0][warp][cx1], bit);
+        atomicOr(&pc.t[1][warp][cx2], bit);
+        atomicOr(&pc.t[2][warp][cy1], bit);
+        atomicOr(&pc.t[3][warp][cy2], bit);
+        atomicOr(&pc.t[4][warp][ca], bit);
+        atomicOr(&pc.t[5][warp][ca], bit);
+    }
+    __syncthreads();
+    for (int col = warp; col < 6 * WORDS; col += WORDS) {  // one (table, word) per warp: lane = cell
+        uint32_t* p = &pc.t[col / WORDS][col % WORDS][0];
+        uint32_t v = p[lane];
+        if (((col / WORDS) & 1) == 0) {
 #pragma unroll
-        for (int b = 0; b < 32; ++b) nz |= (diag[b] != 0u) ? (1u << b) : 0u;
-        if (__popc(nz) <= 10) {
-            while (nz) {
-                const int b = __ffs(nz) - 1;
-                nz &= nz - 1u;
-                if (!(r & (1u << b))) r |= mask[(base + b) * row_stride + w];
+            for (int o = 1; o < kCells; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(kFullMask, v, o);
+                v |= lane >= o ? u : 0u;
             }
         } else {
 #pragma unroll
-            for (int b = 0; b < 32; ++b) {
-                const uint32_t alive = (r & (1u << b)) ? 0u : 0xffffffffu;
-                r |= diag[b] & alive;
+            for (int o = 1; o < kCells; o <<= 1) {
+                const uint32_t u = __shfl_down_sync(kFullMask, v, o);
+                v |= lane + o < kCells ? u : 0u;
             }
         }
-        const uint32_t valid_rows = rows >= 32 ? 0xffffffffu : ((1u << rows) - 1u);
-        const uint32_t keepw = ~r & valid_rows;
-        // kept rows of this block remove columns in the later words
+        p[lane] = v;
+    }
+    __syncthreads();
+    // the area window, a relative 1e-5 wider than the bound so that no rounding of areas or of the quotient matters
+    const int a_hi = real ? area_cell(__fdividef(area, thr * (1.0f - 1.0e-5f)) * (1.0f + 1.0e-5f)) : 0;
+    const int a_lo = real ? area_cell(area * (thr * (1.0f - 2.0e-5f))) : 0;
+    const NmsBox bi{me.x, me.y, me.z, me.w, area};
+    const int words = (n + 31) >> 5;
 #pragma unroll
-        for (int b = 0; b < 32; ++b) removed |= (keepw & (1u << b)) ? col[b] : 0u;
-        if (lane == 0) keep_words[w] = keepw;
+    for (int w = 0; w < WORDS; ++w) {
+        row[w] = 0u;
+        if (w < warp || w >= words) continue;  // warp-uniform
+        uint32_t bits = pc.t[0][w][cx2] & pc.t[1][w][cx1] & pc.t[2][w][cy2] & pc.t[3][w][cy1] & pc.t[4][w][a_hi] & pc.t[5][w][a_lo];
+        if (w == warp) bits &= lane == 31 ? 0u : (0xffffffffu << (lane + 1));
+        if (!real) bits = 0u;
+        while (__any_sync(kFullMask, bits != 0u)) {
+            if (bits != 0u) {
+                const int b = __ffs(bits) - 1;
+                bits &= bits - 1u;
+                const int j = 32 * w + b;
+                const float4 cj = sxy[j];
+                const NmsBox bj{cj.x, cj.y, cj.z, cj.w, sarea[j]};
+                if (iou_exceeds(bi, bj, thr, thr_lo, thr_hi)) row[w] |= 1u << b;
+            }
+        }
     }
 }
 
-// Greedy NMS over a precomputed suppression bit matrix, resolved by the whole block in parallel rounds instead of a
-// serial walk.  Thread i owns row i (NT == 32 * WORDS, n <= NT).  A box is certainly kept once every box that could
+// Greedy NMS over the suppression rows, resolved by the whole block in parallel rounds instead of a serial walk.  Thread i
+// owns row i (NT == 32 * WORDS, n <= NT).  A box is certainly kept once every box that could
 // suppress it is certainly removed, and certainly removed once a certainly kept box suppresses it; both sets only
 // grow, every round settles at least the first undecided box, and the fixed point is the greedy result.  Random boxes
 // need a handful of rounds.  or_words: 2 * WORDS words of shared memory.  keep_words[w] receives the keep bits.
 template <int NT, int WORDS>
-__device__ __forceinline__ void block_nms_resolve(const uint32_t* mask, int n, uint32_t* keep_words, uint32_t* or_words) {
+__device__ __forceinline__ void block_nms_resolve(const uint32_t (&row)[WORDS], int n, uint32_t* keep_words, uint32_t* or_words) {
     static_assert(NT == 32 * WORDS, "one thread per row, one warp per word");
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const bool valid = t < n;
-    uint32_t row[WORDS];
     uint32_t any = 0u;
 #pragma unroll
-    for (int w = 0; w < WORDS; ++w) {
-        row[w] = valid ? mask[t * WORDS + w] : 0u;
-        any |= row[w];
-    }
+    for (int w = 0; w < WORDS; ++w) any |= row[w];
     uint32_t* maybe = or_words;            // boxes that a not-yet-removed box suppresses
     uint32_t* gone = or_words + WORDS;     // boxes that a kept box suppresses
     bool kept = false, removed = false;
