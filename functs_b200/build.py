@@ -15,6 +15,7 @@ SOURCES = [
     "kernels_basic.cu",
     "kernels_select_nms.cu",
     "kernels_yolo.cu",
+    "kernels_yolo_post.cu",
     "kernels_ssd.cu",
     "kernels_yolact.cu",
     "kernels_lstm.cu",

@@ -114,8 +114,7 @@ constexpr int kScanChunk = 256;       // non-empty matrix rows staged in shared 
 // buckets within K of its own label; every pair that can intersect is still tested with the exact IoU expression, so
 // the matrix is the same as the one an all-pairs loop produces.
 //
-// nms_prepare_block (run by the CTA that finishes a group's top-k selection, or by nms_prepare_kernel when the selected
-// keys come from elsewhere) gathers the selected boxes, applies the class offsets, and leaves the boxes, their buckets
+// nms_prepare_kernel gathers the selected boxes, applies the class offsets, and leaves the boxes, their buckets
 // and the bucket order in scratch; nms_mask_scan_kernel (up to kMaskCtasMax CTAs per group) copies that into shared memory and
 // computes its share of the rows; the CTA of a group that finishes last then runs the greedy scan.
 struct NmsPrepHeader {
@@ -276,7 +275,7 @@ __device__ __forceinline__ void nms_prepare_block(const float* __restrict__ boxe
     }
 }
 
-// grid = groups; block = 256.  For selected keys that did not come from select_binned_kernel.
+// grid = groups; block = 256.
 __global__ void __launch_bounds__(kMaskThreads)
 nms_prepare_kernel(const float* __restrict__ boxes, int64_t num_boxes, int num_classes, const uint64_t* __restrict__ sel_keys,
                    const int32_t* __restrict__ sel_counts, int topk, int class_offset, unsigned char* __restrict__ prep_g,
@@ -299,7 +298,7 @@ nms_prepare_kernel(const float* __restrict__ boxes, int64_t num_boxes, int num_c
 // appends keys above d* to the group's `sel` list and keys inside d* to its `bin` list.  CTAs then take a ticket;
 // the one that draws the last ticket sorts the bin list, tops `sel` up from it and writes the sorted result (if the
 // lists turn out not to fit the histogram, or the boundary bucket is too crowded, it runs the exact generic selection
-// over the whole candidate list instead), and, when asked to, prepares the group's NMS input (nms_prepare_block).
+// over the whole candidate list instead).
 // No CTA ever waits for another one.
 constexpr int kBinThreads = 512;
 constexpr int kBinSplit = 4;         // CTAs per group
@@ -320,11 +319,8 @@ __global__ void __launch_bounds__(kBinThreads, 2)
 select_binned_kernel(const uint64_t* __restrict__ in_keys, const int32_t* __restrict__ in_counts, int64_t capacity,
                      const int32_t* __restrict__ hist, uint32_t hist_base, int hist_shift, int32_t topk,
                      SelectCtr* ctr, uint64_t* sel_tmp, uint64_t* bin_tmp, uint64_t* __restrict__ out_keys,
-                     int32_t* __restrict__ out_counts, const float* __restrict__ nms_boxes, int64_t num_boxes,
-                     int num_classes, int class_offset, unsigned char* __restrict__ prep_g, int32_t* __restrict__ ticket_g,
-                     int32_t* status) {
+                     int32_t* __restrict__ out_counts) {
     constexpr size_t kRaw = sizeof(BinnedSmem) > sizeof(SelectSmem<kSelCap>) ? sizeof(BinnedSmem) : sizeof(SelectSmem<kSelCap>);
-    static_assert(sizeof(uint64_t) * kSelCap + sizeof(NmsPrepSmem<kBinThreads>) <= kRaw, "NMS preparation reuses the buffer");
     __shared__ __align__(16) unsigned char raw[kRaw];
     BinnedSmem& sm = *reinterpret_cast<BinnedSmem*>(raw);  // .sel is the first member of both views
     __shared__ int s_dstar, s_above, s_inbin, s_last;
@@ -542,13 +538,6 @@ select_binned_kernel(const uint64_t* __restrict__ in_keys, const int32_t* __rest
     }
     for (int i = tid; i < topk; i += kBinThreads) out_keys[static_cast<int64_t>(g) * topk + i] = (i < result) ? sm.sel[i] : 0ull;
     if (tid == 0) out_counts[g] = result;
-    if (prep_g != nullptr) {
-        __syncthreads();
-        NmsPrepSmem<kBinThreads>& ps = *reinterpret_cast<NmsPrepSmem<kBinThreads>*>(raw + sizeof(uint64_t) * kSelCap);
-        nms_prepare_block<kBinThreads>(nms_boxes + static_cast<int64_t>(g) * num_boxes * 4, num_boxes, num_classes,
-                                       class_offset, sm.sel, result, prep_g + static_cast<int64_t>(g) * kPrepBytes,
-                                       ticket_g + g, status, ps);
-    }
 }
 
 // grid = (CTAs per group, groups); block = 256.  Rows are interleaved over the CTAs of a group (i = k * gridDim.x +
@@ -579,7 +568,7 @@ nms_mask_scan_kernel(const unsigned char* __restrict__ prep_g, float thr, float 
                      const float* __restrict__ boxes, int64_t num_boxes, int num_classes,
                      const uint64_t* __restrict__ sel_keys, int topk, float* __restrict__ dets,
                      int64_t* __restrict__ labels, int64_t* __restrict__ flat_ids, int64_t* __restrict__ keep,
-                     int32_t* __restrict__ out_counts, int4* __restrict__ records) {
+                     int32_t* __restrict__ out_counts) {
     constexpr size_t kRaw = sizeof(NmsRowsSmem) > sizeof(NmsScanSmem) ? sizeof(NmsRowsSmem) : sizeof(NmsScanSmem);
     __shared__ __align__(16) unsigned char raw[kRaw];
     __shared__ int s_last;
@@ -757,13 +746,6 @@ nms_mask_scan_kernel(const unsigned char* __restrict__ prep_g, float thr, float 
             labels[obase + rank] = static_cast<int64_t>(flat - box * static_cast<uint32_t>(num_classes));
             flat_ids[obase + rank] = static_cast<int64_t>(flat);
             if (keep != nullptr) keep[obase + rank] = c;
-            if (records != nullptr) {  // the 32-byte record of the multi-GPU gather (layout of pack_detections_kernel)
-                records[2 * (obase + rank)] = make_int4(__float_as_int(bx.x), __float_as_int(bx.y), __float_as_int(bx.z),
-                                                        __float_as_int(bx.w));
-                records[2 * (obase + rank) + 1] = make_int4(__float_as_int(key_score(k)),
-                                                            static_cast<int>(flat - box * static_cast<uint32_t>(num_classes)),
-                                                            static_cast<int>(flat), 1);
-            }
         }
     }
     // zero the tail so that the padded outputs are deterministic
@@ -774,14 +756,10 @@ nms_mask_scan_kernel(const unsigned char* __restrict__ prep_g, float thr, float 
         labels[obase + i] = -1;
         flat_ids[obase + i] = -1;
         if (keep != nullptr) keep[obase + i] = -1;
-        if (records != nullptr) {
-            records[2 * (obase + i)] = make_int4(0, 0, 0, 0);
-            records[2 * (obase + i) + 1] = make_int4(0, -1, -1, 0);
-        }
     }
 }
 
-// ---- host launchers (internal C++ API, used by the C ABI and by the YOLO pipeline) ----------------
+// ---- host launchers (internal C++ API) ----------------
 int launch_threshold_compact(const float* scores, int groups, int64_t n, float thr, uint64_t* keys, int32_t* counts,
                              int64_t capacity, int zero_counts, int32_t* hist, int32_t* status, cudaStream_t st) {
     FB_REQUIRE(scores && keys && counts, "threshold_compact: null pointer");
@@ -847,42 +825,29 @@ int64_t nms_scratch_bytes(int groups, int topk) {
     return nms_mask_bytes(groups);
 }
 
-// ctr must be zero when the kernel starts (zero_ctr != 0 makes this call clear it).  With nms_scratch != nullptr the
-// CTA that finishes a group also prepares the group's NMS input there (boxes [groups, num_boxes, 4], flat index =
-// box * num_classes + label), so that launch_batched_nms(..., prepared = 1) can follow directly.
 int launch_select_binned(const uint64_t* in_keys, const int32_t* in_counts, int64_t capacity, const int32_t* hist,
                          float thr, int groups, int topk, uint64_t* out_keys, int32_t* out_counts, void* ctr,
-                         void* lists, int zero_ctr, const float* nms_boxes, int64_t num_boxes, int num_classes,
-                         int class_offset, void* nms_scratch, int32_t* status, cudaStream_t st) {
+                         void* lists, cudaStream_t st) {
     FB_REQUIRE(in_keys && in_counts && hist && out_keys && out_counts && ctr && lists, "select_topk_binned: null pointer");
     FB_REQUIRE(groups > 0 && groups <= 65535 && topk > 0 && topk <= kSelCap && capacity > 0 && capacity < (1ll << 31),
                "select_topk_binned: bad sizes (topk must be in [1, %d])", kSelCap);
     FB_REQUIRE(thr > 0.0f, "select_topk_binned: the threshold must be positive");
     FB_REQUIRE((reinterpret_cast<uintptr_t>(hist) & 15) == 0, "select_topk_binned: the histogram must be 16-byte aligned");
-    FB_REQUIRE(nms_scratch == nullptr || (nms_boxes != nullptr && num_boxes > 0 && num_classes > 0 &&
-                                          (reinterpret_cast<uintptr_t>(nms_boxes) & 15) == 0),
-               "select_topk_binned: NMS preparation needs 16-byte aligned boxes");
-    if (zero_ctr) FB_TRY(check_cuda(cudaMemsetAsync(ctr, 0, select_binned_ctr_bytes(groups), st), "memset select counters"));
+    FB_TRY(check_cuda(cudaMemsetAsync(ctr, 0, select_binned_ctr_bytes(groups), st), "memset select counters"));
     const HistParams hp = hist_params_for(thr);
     uint64_t* sel_tmp = static_cast<uint64_t*>(lists);
     uint64_t* bin_tmp = sel_tmp + static_cast<int64_t>(groups) * kSelCap;
-    NmsScratch v{nullptr, nullptr, nullptr, nullptr};
-    if (nms_scratch != nullptr) v = nms_scratch_views(nms_scratch, groups);
     dim3 grid(kBinSplit, groups);
     select_binned_kernel<<<grid, kBinThreads, 0, st>>>(in_keys, in_counts, capacity, hist, hp.base, hp.shift, topk,
-                                                       static_cast<SelectCtr*>(ctr), sel_tmp, bin_tmp, out_keys, out_counts,
-                                                       nms_boxes, num_boxes, num_classes, class_offset, v.prep, v.ticket,
-                                                       status);
+                                                       static_cast<SelectCtr*>(ctr), sel_tmp, bin_tmp, out_keys, out_counts);
     count_launch();
     return check_launch("select_binned_kernel");
 }
 
-// prepared != 0: the group's NMS input is in the scratch already (launch_select_binned with the same scratch).
 int launch_batched_nms(const float* boxes, int64_t num_boxes, int num_classes, const uint64_t* sel_keys,
                        const int32_t* sel_counts, int groups, int topk, float iou_thr, int class_offset, float* dets,
-                       int64_t* labels, int64_t* flat_ids, int64_t* keep, int32_t* out_counts, void* mask, int prepared,
-                       int32_t* status, cudaStream_t st, int32_t* records) {
-    FB_REQUIRE(records == nullptr || (reinterpret_cast<uintptr_t>(records) & 15) == 0, "batched_nms: records must be 16-byte aligned");
+                       int64_t* labels, int64_t* flat_ids, int64_t* keep, int32_t* out_counts, void* mask,
+                       int32_t* status, cudaStream_t st) {
     FB_REQUIRE(boxes && sel_keys && sel_counts && dets && labels && flat_ids && out_counts && mask,
                "batched_nms: null pointer");
     FB_REQUIRE(groups > 0 && groups <= 65535 && topk > 0 && topk <= kNmsMaxN && num_classes > 0 && num_boxes > 0,
@@ -892,12 +857,10 @@ int launch_batched_nms(const float* boxes, int64_t num_boxes, int num_classes, c
                "batched_nms: boxes and scratch must be 16-byte aligned");
     const float thr_lo = iou_thr * (1.0f - 1.0e-6f), thr_hi = iou_thr * (1.0f + 1.0e-6f);
     const NmsScratch v = nms_scratch_views(mask, groups);
-    if (!prepared) {
-        nms_prepare_kernel<<<groups, kMaskThreads, 0, st>>>(boxes, num_boxes, num_classes, sel_keys, sel_counts, topk,
-                                                            class_offset, v.prep, v.ticket, status);
-        count_launch();
-        FB_TRY(check_launch("nms_prepare_kernel"));
-    }
+    nms_prepare_kernel<<<groups, kMaskThreads, 0, st>>>(boxes, num_boxes, num_classes, sel_keys, sel_counts, topk, class_offset,
+                                                        v.prep, v.ticket, status);
+    count_launch();
+    FB_TRY(check_launch("nms_prepare_kernel"));
     // one wave: a second, partly filled wave costs more than longer row loops per warp
     static std::atomic<int> wave_cache[64];  // resident CTAs of this kernel per device: asked once (0 = not yet)
     int dev = 0;
@@ -916,7 +879,7 @@ int launch_batched_nms(const float* boxes, int64_t num_boxes, int num_classes, c
     dim3 grid(ctas, groups);
     nms_mask_scan_kernel<<<grid, kMaskThreads, 0, st>>>(v.prep, iou_thr, thr_lo, thr_hi, v.mask, v.rowflag, v.ticket, boxes,
                                                         num_boxes, num_classes, sel_keys, topk, dets, labels, flat_ids, keep,
-                                                        out_counts, reinterpret_cast<int4*>(records));
+                                                        out_counts);
     count_launch();
     return check_launch("nms_mask_scan_kernel");
 }
@@ -955,8 +918,7 @@ int functs_b200_select_topk_binned(const uint64_t* in_keys, const int32_t* in_co
     }
     unsigned char* base = static_cast<unsigned char*>(scratch);
     return fb::launch_select_binned(in_keys, in_counts, capacity, hist, thr, groups, topk, out_keys, out_counts, base,
-                                    base + fb::select_binned_ctr_bytes(groups > 0 ? groups : 1), 1, nullptr, 0, 0, 0, nullptr,
-                                    nullptr, fb::as_stream(stream));
+                                    base + fb::select_binned_ctr_bytes(groups > 0 ? groups : 1), fb::as_stream(stream));
 }
 
 int64_t functs_b200_nms_scratch_bytes(int32_t groups, int32_t topk) {
@@ -973,8 +935,8 @@ int functs_b200_batched_nms(const float* boxes, int64_t num_boxes, int32_t num_c
         return FB_ERR_INVALID_ARGUMENT;
     }
     return fb::launch_batched_nms(boxes, num_boxes, num_classes, sel_keys, sel_counts, groups, topk, iou_thr,
-                                  class_offset, dets, labels, flat_ids, keep, out_counts, scratch, 0, status,
-                                  fb::as_stream(stream), nullptr);
+                                  class_offset, dets, labels, flat_ids, keep, out_counts, scratch, status,
+                                  fb::as_stream(stream));
 }
 
 }  // extern "C"

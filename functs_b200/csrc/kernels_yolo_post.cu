@@ -1,0 +1,415 @@
+// C2, second half: one CTA per image turns the candidate list into detections: top-k in "score descending, index ascending"
+// order (functs/benchmark/ai_model/yolov3/yolov3_bbox.py:128-134), class-wise greedy NMS through the coordinate offsets of
+// :144-146 and :177, and the compacted outputs.
+//
+// What bounds it: a chain of short dependent phases on some 2000 keys and 1000 boxes, i.e. latency.  One CTA keeps all of it in
+// shared memory; with the work in one launch there is no second kernel to start, no ticket and no round trip through global
+// memory between the phases (two kernels of up to sixteen CTAs per image took 22 + 24 us for 64 images and 22 + 16 for one).
+//   select     counting sort on 2048 score buckets that start at the image's floor (a bucket holds a key or two) + rank
+//              inside the bucket;
+//   boxes      decoded here for the selected candidates only, from the logits (four scattered loads each), so that nobody
+//              has to write and read all boxes;
+//   pairs      boxes are laid out by class; a box looks at its own class and at the classes within reach of the offsets
+//              (boxes with negative coordinates reach into the next class), skipping a class whose smallest corner lies
+//              behind its own largest one.  What overlaps enough goes into a list of (suppressor, suppressed) pairs;
+//   greedy     parallel rounds over the pair list: a box is kept once every box that could suppress it is removed.
+// Slow exact ways for the rare inputs: the floor was too high (fewer than topk candidates in the list: the image's scores are
+// formed again without one), more candidates than fit (generic selection from global memory), a crowded score bucket (bitonic
+// sort), more pairs than fit (bit matrix in global memory, walked row by row).
+#include "yolo.cuh"
+
+namespace fb {
+
+constexpr int kPostThreads = 1024;
+constexpr int kPostKeys = 4096;    // candidates the shared-memory selection takes
+constexpr int kPostTop = 1024;     // largest topk
+constexpr int kPostPairs = 8192;
+constexpr int kPostCrowded = 64;   // keys of one score bucket beyond which ranks are not counted
+constexpr int kPostWords = kPostTop / 32;
+
+struct PostSmem {
+    union {
+        uint64_t keys[kPostKeys];
+        struct {
+            float4 xy[kPostTop];       // NMS-space corners, by position (class order)
+            float area[kPostTop];
+            uint16_t rank[kPostTop];   // position -> place in the sorted top-k
+            uint8_t label[kPostTop];
+        } box;
+    };
+    union {
+        uint64_t sorted[kPostKeys];
+        uint32_t pairs[kPostPairs];    // suppressor << 16 | suppressed (places in the top-k)
+        uint32_t rows[32][kPostWords]; // staging of the dense matrix
+        SelectSmem<kPostTop> generic;
+    };
+    int hist[kHistBins];
+    uint64_t sel[kPostTop];
+    uint8_t removed[kPostTop], blocked[kPostTop], kept[kPostTop];
+    int cls_start[kYoloClasses + 1], cls_cursor[kYoloClasses];
+    uint32_t cls_min_x[kYoloClasses], cls_min_y[kYoloClasses];  // smallest corners of a class, as ordered bits
+    int warp_sum[32];
+    uint32_t words[kPostWords];
+    uint32_t hi, lo;  // extreme coordinates, as ordered bits
+    int npairs;
+};
+static_assert(sizeof(PostSmem) < 100 * 1024, "two CTAs per SM");
+
+// The image's candidates once more, without a floor.
+__device__ __noinline__ void post_rescan(const YoloLevels& L, const YoloPostArgs& A, int img) {
+    if (threadIdx.x == 0) A.counts[img] = 0;
+    __syncthreads();
+    for (int b = threadIdx.x; b < L.num_boxes; b += kPostThreads) {
+        const int lvl = b >= L.box_begin[2] ? 2 : (b >= L.box_begin[1] ? 1 : 0);
+        const int plane = L.plane[lvl], slot = b - L.box_begin[lvl];
+        int anchor, pos;
+        yolo_slot(plane, slot, anchor, pos);
+        const float* src = L.map[lvl] + (static_cast<int64_t>(img) * 3 + anchor) * kYoloAttrib * plane + pos;
+        const float so = sigmoid_f32(__ldg(src + 4 * plane));
+        if (!(so > A.thr)) continue;
+        const float cut = logit_cut(so, A.thr);
+        const uint32_t flat0 = static_cast<uint32_t>(L.box_begin[lvl] + pos * 3 + anchor) * kYoloClasses;
+        for (int c = 0; c < kYoloClasses; ++c) {
+            const float v = __ldg(src + (5 + c) * plane);
+            if (!(v > cut)) continue;
+            const float s = __fmul_rn(so, sigmoid_f32(v));
+            if (!(s > A.thr)) continue;
+            const int64_t at = atomicAdd(A.counts + img, 1);
+            if (at < A.capacity) A.keys[img * A.capacity + at] = make_key(s, flat0 + static_cast<uint32_t>(c));
+            else if (A.status != nullptr) atomicOr(A.status, FB_STATUS_CAND_OVERFLOW);
+        }
+    }
+    __syncthreads();
+}
+
+struct GlobalKeysView {
+    const uint64_t* p;
+    __device__ __forceinline__ uint64_t operator()(int i) const { return __ldcg(p + i); }
+};
+__device__ __noinline__ void post_select_generic(const uint64_t* keys, int n, int topk, PostSmem* sm) {
+    const int m = block_select_topk<kPostThreads, kPostTop, 4>(GlobalKeysView{keys}, n, topk, sm->generic);
+    __syncthreads();
+    if (static_cast<int>(threadIdx.x) < m) sm->sel[threadIdx.x] = sm->generic.sel[threadIdx.x];
+    __syncthreads();
+}
+
+// sel[0 .. min(n, topk)) = the largest keys, sorted; n <= kPostKeys
+__device__ __forceinline__ void post_select(const uint64_t* __restrict__ keys, int n, int topk, float bar, PostSmem& sm) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t base = __float_as_uint(bar);
+    const uint32_t span = 0x3F800000u > base ? 0x3F800000u - base : 1u;  // scores are products of probabilities: <= 1
+    const int shift = max(0, 21 - __clz(static_cast<int>(span - 1u)));   // (span - 1) >> shift < 2048
+    constexpr int kPer = kPostKeys / kPostThreads;
+    uint64_t k[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) k[q] = q * kPostThreads + t < n ? __ldcg(keys + q * kPostThreads + t) : 0ull;
+    sm.hist[t] = 0;
+    sm.hist[t + kPostThreads] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kPer; ++q)
+        if (k[q] != 0ull) atomicAdd(&sm.hist[hist_digit(k[q], base, shift)], 1);
+    __syncthreads();
+    // hist[d] becomes the place where bucket d starts: the number of keys in higher buckets
+    const int h0 = sm.hist[2 * t], h1 = sm.hist[2 * t + 1];
+    int incl = h0 + h1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_down_sync(kFullMask, incl, o);
+        if (lane + o < 32) incl += v;
+    }
+    if (lane == 0) sm.warp_sum[warp] = incl;
+    __syncthreads();
+    int higher = lane > warp ? sm.warp_sum[lane] : 0;
+    higher = __reduce_add_sync(kFullMask, higher);
+    const int above = incl - (h0 + h1) + higher;
+    sm.hist[2 * t + 1] = above;
+    sm.hist[2 * t] = above + h1;
+    const bool crowded = above < topk && (h0 > kPostCrowded || h1 > kPostCrowded);
+    if (__syncthreads_or(crowded ? 1 : 0) != 0) {
+        const int sn = next_pow2(n);
+#pragma unroll
+        for (int q = 0; q < kPer; ++q)
+            if (q * kPostThreads + t < sn) sm.keys[q * kPostThreads + t] = k[q];
+        __syncthreads();
+        bitonic_sort_desc<kPostThreads>(sm.keys, sn);
+        if (t < min(n, topk)) sm.sel[t] = sm.keys[t];
+        __syncthreads();
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; ++q)
+        if (k[q] != 0ull) sm.sorted[atomicAdd(&sm.hist[hist_digit(k[q], base, shift)], 1)] = k[q];
+    __syncthreads();
+    // now hist[d] is where bucket d ends and hist[d + 1] where it starts; a key counts the larger keys of its bucket
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        if (k[q] != 0ull) {
+            const int d = hist_digit(k[q], base, shift);
+            int r = d + 1 < kHistBins ? sm.hist[d + 1] : 0;
+            const int end = sm.hist[d];
+            if (r < topk) {
+                for (int j = r, j1 = end; j < j1; ++j) r += sm.sorted[j] > k[q] ? 1 : 0;
+                if (r < topk) sm.sel[r] = k[q];
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// Calls pair(i, j) for every pair of positions (this thread's p, a later q) whose boxes overlap by more than the threshold.
+template <class F>
+__device__ __forceinline__ void post_pairs(const PostSmem& sm, int m, int reach, float thr, float thr_lo, float thr_hi, F pair) {
+    const int p = threadIdx.x;
+    if (p >= m) return;
+    const float4 me = sm.box.xy[p];
+    const NmsBox bi{me.x, me.y, me.z, me.w, sm.box.area[p]};
+    const int label = sm.box.label[p], rank = sm.box.rank[p];
+    const uint32_t end_x = ordered_bits(me.z), end_y = ordered_bits(me.w);
+    for (int b = label; b <= min(label + reach, kYoloClasses - 1); ++b) {
+        int q = sm.cls_start[b];
+        const int q1 = sm.cls_start[b + 1];
+        if (b == label) q = p + 1;
+        else if (end_x <= sm.cls_min_x[b] || end_y <= sm.cls_min_y[b]) continue;
+        for (; q < q1; ++q) {
+            const float4 c = sm.box.xy[q];
+            if (!(fminf(me.z, c.z) > fmaxf(me.x, c.x))) continue;
+            const NmsBox bj{c.x, c.y, c.z, c.w, sm.box.area[q]};
+            if (iou_exceeds(bi, bj, thr, thr_lo, thr_hi)) {
+                const int other = sm.box.rank[q];
+                pair(min(rank, other), max(rank, other));
+            }
+        }
+    }
+}
+
+// Greedy NMS when the pair list overflowed: the bit matrix in global memory, rows walked in order, 32 staged at a time.
+__device__ __noinline__ void post_dense(PostSmem* smp, uint32_t* mask, int m, int reach, float thr, float thr_lo, float thr_hi) {
+    PostSmem& sm = *smp;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (int i = t; i < m * kPostWords; i += kPostThreads) mask[i] = 0u;
+    __threadfence_block();
+    __syncthreads();
+    post_pairs(sm, m, reach, thr, thr_lo, thr_hi, [&](int i, int j) { atomicOr(mask + i * kPostWords + (j >> 5), 1u << (j & 31)); });
+    __threadfence();
+    uint32_t gone = 0u;  // warp 0, lane w: removed bits of the boxes 32w .. 32w + 31
+    for (int r0 = 0; r0 < m; r0 += 32) {
+        __syncthreads();
+        sm.rows[warp][lane] = r0 + warp < m ? __ldcg(mask + (r0 + warp) * kPostWords + lane) : 0u;
+        __syncthreads();
+        if (warp == 0) {
+            for (int r = 0; r < 32; ++r) {
+                const uint32_t word = __shfl_sync(kFullMask, gone, r0 >> 5);
+                if (!((word >> r) & 1u)) gone |= sm.rows[r][lane];
+            }
+        }
+    }
+    if (warp == 0) sm.words[lane] = gone;
+    __syncthreads();
+    sm.removed[t] = (sm.words[warp] >> lane) & 1u;
+    sm.kept[t] = t < m && sm.removed[t] == 0;
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kPostThreads, 1)
+yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ YoloPostArgs A, float thr_lo, float thr_hi) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    PostSmem& sm = *reinterpret_cast<PostSmem*>(smem_raw);
+    const int img = blockIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    sm.removed[t] = 0;
+    if (t < kYoloClasses) {
+        sm.cls_cursor[t] = 0;
+        sm.cls_min_x[t] = 0xffffffffu;
+        sm.cls_min_y[t] = 0xffffffffu;
+    }
+    if (t == 0) {
+        sm.hi = 0u;
+        sm.lo = 0xffffffffu;
+        sm.npairs = 0;
+    }
+    pdl_wait();  // the candidates
+
+    // ---- top-k ----
+    float floor = __ldcg(A.floor + img);
+    int64_t n64 = *reinterpret_cast<volatile int32_t*>(A.counts + img);
+    const bool short_list = floor > 0.0f && n64 < A.topk;
+    if (short_list) {
+        post_rescan(L, A, img);
+        floor = 0.0f;
+        n64 = *reinterpret_cast<volatile int32_t*>(A.counts + img);
+    }
+    const int n = static_cast<int>(n64 < 0 ? 0 : (n64 > A.capacity ? A.capacity : n64));
+    const uint64_t* keys = A.keys + img * A.capacity;
+    if (n <= kPostKeys) post_select(keys, n, A.topk, fmaxf(A.thr, floor), sm);
+    else post_select_generic(keys, n, A.topk, &sm);
+    if (t == 0 && (short_list || n > kPostKeys)) A.fallback[img] = 1;
+    const int m = min(n, A.topk);
+
+    // ---- boxes of the selected candidates ----
+    uint64_t key = 0ull;
+    uint32_t flat = 0u;
+    int label = 0;
+    float4 bx = make_float4(0.f, 0.f, 0.f, 0.f);
+    float top = -INFINITY, bottom = INFINITY;
+    if (t < m) {
+        key = sm.sel[t];
+        flat = key_index(key);
+        const int box = static_cast<int>(flat / kYoloClasses);
+        label = static_cast<int>(flat) - box * kYoloClasses;
+        const int lvl = box >= L.box_begin[2] ? 2 : (box >= L.box_begin[1] ? 1 : 0);
+        const int plane = L.plane[lvl], local = box - L.box_begin[lvl];
+        const int pos = local / 3, anchor = local - pos * 3;
+        const float* src = L.map[lvl] + (static_cast<int64_t>(img) * 3 + anchor) * kYoloAttrib * plane + pos;
+        bx = yolo_box(L, lvl, anchor, pos, __ldg(src), __ldg(src + plane), __ldg(src + 2 * plane), __ldg(src + 3 * plane));
+        top = fmaxf(top, fmaxf(fmaxf(bx.x, bx.y), fmaxf(bx.z, bx.w)));
+        bottom = fminf(bottom, fminf(fminf(bx.x, bx.y), fminf(bx.z, bx.w)));
+        atomicAdd(&sm.cls_cursor[label], 1);
+    }
+    {
+        const uint32_t h = __reduce_max_sync(kFullMask, ordered_bits(top)), l = __reduce_min_sync(kFullMask, ordered_bits(bottom));
+        if (lane == 0) {
+            atomicMax(&sm.hi, h);
+            atomicMin(&sm.lo, l);
+        }
+    }
+    __syncthreads();
+    const float hi = from_ordered_bits(sm.hi), lo = from_ordered_bits(sm.lo);
+    const float scale = __fadd_rn(hi, 1.0f);
+    // With class offsets, class c occupies the coordinates [c * M + lo, c * M + hi] (M = hi + 1), so boxes whose labels differ
+    // by more than floor((hi - lo) / M) + 1 cannot intersect (one class more than exact: the fp32 rounding of the shifts).
+    int reach = kYoloClasses;
+    if (scale > 0.0f) {
+        const float r = floorf((hi - lo) / scale) + 1.0f;
+        if (r < static_cast<float>(kYoloClasses)) reach = static_cast<int>(r);
+    }
+    if (warp == 0) {  // class starts: an exclusive prefix over 80 counts, three per lane
+        int c[3], s = 0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            c[q] = 3 * lane + q < kYoloClasses ? sm.cls_cursor[3 * lane + q] : 0;
+            s += c[q];
+        }
+        int incl = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFullMask, incl, o);
+            if (lane >= o) incl += v;
+        }
+        int run = incl - s;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            if (3 * lane + q < kYoloClasses) {
+                sm.cls_start[3 * lane + q] = run;
+                sm.cls_cursor[3 * lane + q] = run;
+            }
+            run += c[q];
+        }
+        if (lane == 31) sm.cls_start[kYoloClasses] = incl;
+    }
+    __syncthreads();
+    if (t < m) {
+        const float off = __fmul_rn(static_cast<float>(label), scale);
+        const NmsBox b = make_nms_box(__fadd_rn(bx.x, off), __fadd_rn(bx.y, off), __fadd_rn(bx.z, off), __fadd_rn(bx.w, off));
+        const int p = atomicAdd(&sm.cls_cursor[label], 1);
+        sm.box.xy[p] = make_float4(b.x1, b.y1, b.x2, b.y2);
+        sm.box.area[p] = b.area;
+        sm.box.rank[p] = static_cast<uint16_t>(t);
+        sm.box.label[p] = static_cast<uint8_t>(label);
+        atomicMin(&sm.cls_min_x[label], ordered_bits(b.x1));
+        atomicMin(&sm.cls_min_y[label], ordered_bits(b.y1));
+    }
+    __syncthreads();
+
+    // ---- greedy NMS ----
+    post_pairs(sm, m, reach, A.iou_thr, thr_lo, thr_hi, [&](int i, int j) {
+        const int at = atomicAdd(&sm.npairs, 1);
+        if (at < kPostPairs) sm.pairs[at] = static_cast<uint32_t>(i) << 16 | static_cast<uint32_t>(j);
+    });
+    __syncthreads();
+    const int np = sm.npairs;
+    if (np > kPostPairs) {
+        post_dense(&sm, A.mask + static_cast<int64_t>(img) * kPostTop * kPostWords, m, reach, A.iou_thr, thr_lo, thr_hi);
+    } else {
+        for (int round = 0; round <= m; ++round) {
+            sm.blocked[t] = 0;
+            __syncthreads();
+            for (int i = t; i < np; i += kPostThreads) {
+                const uint32_t pr = sm.pairs[i];
+                if (sm.removed[pr >> 16] == 0) sm.blocked[pr & 0xffffu] = 1;
+            }
+            __syncthreads();
+            const bool kept = t < m && sm.removed[t] == 0 && sm.blocked[t] == 0;
+            sm.kept[t] = kept ? 1 : 0;
+            __syncthreads();
+            for (int i = t; i < np; i += kPostThreads) {
+                const uint32_t pr = sm.pairs[i];
+                if (sm.kept[pr >> 16] != 0) sm.removed[pr & 0xffffu] = 1;
+            }
+            __syncthreads();
+            if (__syncthreads_or(t < m && !kept && sm.removed[t] == 0 ? 1 : 0) == 0) break;
+        }
+    }
+
+    // ---- outputs ----
+    const bool kept = t < m && sm.kept[t] != 0;
+    const unsigned word = __ballot_sync(kFullMask, kept);
+    if (lane == 0) sm.warp_sum[warp] = __popc(word);
+    __syncthreads();
+    const int mine = sm.warp_sum[lane];
+    const int before = __reduce_add_sync(kFullMask, lane < warp ? mine : 0), total = __reduce_add_sync(kFullMask, mine);
+    const int64_t obase = static_cast<int64_t>(img) * A.topk;
+    int4* records = reinterpret_cast<int4*>(A.records);
+    if (kept) {
+        const int64_t row = obase + before + __popc(word & ((1u << lane) - 1u));
+        float* d = A.dets + row * 5;
+        d[0] = bx.x;
+        d[1] = bx.y;
+        d[2] = bx.z;
+        d[3] = bx.w;
+        d[4] = key_score(key);
+        A.labels[row] = label;
+        if (A.flat_ids != nullptr) A.flat_ids[row] = static_cast<int64_t>(flat);
+        if (records != nullptr) {  // the 32-byte record of the multi-GPU gather (layout of pack_detections_kernel)
+            records[2 * row] = make_int4(__float_as_int(bx.x), __float_as_int(bx.y), __float_as_int(bx.z), __float_as_int(bx.w));
+            records[2 * row + 1] = make_int4(__float_as_int(key_score(key)), label, static_cast<int>(flat), 1);
+        }
+    }
+    for (int i = total + t; i < A.topk; i += kPostThreads) {  // padded rows are deterministic
+        const int64_t row = obase + i;
+        float* d = A.dets + row * 5;
+        d[0] = d[1] = d[2] = d[3] = d[4] = 0.0f;
+        A.labels[row] = -1;
+        if (A.flat_ids != nullptr) A.flat_ids[row] = -1;
+        if (records != nullptr) {
+            records[2 * row] = make_int4(0, 0, 0, 0);
+            records[2 * row + 1] = make_int4(0, -1, -1, 0);
+        }
+    }
+    if (t == 0) {
+        A.out_counts[img] = total;
+        if (A.host_counts != nullptr) A.host_counts[img] = total;
+    }
+}
+
+int64_t yolo_post_mask_bytes(int batch) { return static_cast<int64_t>(batch) * kPostTop * kPostWords * 4; }
+
+int check_yolo_post(int batch, const YoloPostArgs& a) {
+    FB_REQUIRE(a.dets && a.labels && a.out_counts && a.keys && a.counts, "yolo_postprocess: null pointer");
+    FB_REQUIRE(batch > 0 && a.topk > 0 && a.topk <= kPostTop, "yolo_postprocess: bad sizes (topk must be in [1, %d])", kPostTop);
+    FB_REQUIRE(a.thr > 0.0f, "yolo_postprocess: the score threshold must be positive");
+    FB_REQUIRE(a.iou_thr > 0.0f && a.iou_thr < 1.0f, "yolo_postprocess: iou threshold must be in (0, 1)");
+    FB_REQUIRE(a.records == nullptr || (reinterpret_cast<uintptr_t>(a.records) & 15) == 0, "yolo_postprocess: records must be 16-byte aligned");
+    return FB_OK;
+}
+
+int launch_yolo_post(const YoloLevels& L, int batch, const YoloPostArgs& a, cudaStream_t st) {
+    const size_t smem = sizeof(PostSmem);
+    FB_TRY(check_cuda(cudaFuncSetAttribute(yolo_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+                      "yolo_post attr"));
+    const float thr_lo = a.iou_thr * (1.0f - 1.0e-6f), thr_hi = a.iou_thr * (1.0f + 1.0e-6f);
+    return launch_pdl(yolo_post_kernel, dim3(static_cast<unsigned>(batch)), dim3(kPostThreads), smem, st, "yolo_post_kernel", L, a, thr_lo,
+                      thr_hi);
+}
+
+}  // namespace fb

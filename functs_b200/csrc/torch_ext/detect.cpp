@@ -94,4 +94,53 @@ SsdResult ssdDetect(const at::Tensor& loc, const at::Tensor& conf, const at::Ten
     return r;
 }
 
+YoloResult yoloDetect(const std::vector<at::Tensor>& maps, double score_thr, int64_t topk, double iou_thr, bool dense, bool want_ids) {
+    TORCH_CHECK(maps.size() == 3, "yolov3: expected three prediction maps");
+    int64_t S[3], N = 0;
+    const int64_t B = maps[0].size(0);
+    for (int l = 0; l < 3; ++l) {
+        TORCH_CHECK(maps[l].dim() == 4 && maps[l].size(0) == B && maps[l].size(1) == 255 && maps[l].size(2) == maps[l].size(3),
+                    "yolov3: expected three [B, 255, S, S] maps");
+        S[l] = maps[l].size(2);
+        N += 3 * S[l] * S[l];
+    }
+    c10::cuda::CUDAGuard guard(maps[0].device());
+    const int64_t capacity = N * 80;
+    const auto f32 = maps[0].options();
+    const auto i64 = f32.dtype(at::kLong);
+    YoloResult r;
+    if (dense) {
+        r.boxes = at::empty({B, N, 4}, f32);
+        r.obj = at::empty({B, N}, f32);
+        r.cls = at::empty({B, N, 80}, f32);
+    }
+    at::Tensor dets = at::empty({B, topk, 5}, f32), labels = at::empty({B, topk}, i64);
+    at::Tensor ids = want_ids ? at::empty({B, topk}, i64) : at::Tensor();
+    const int64_t bytes = functs_b200_yolo_scratch_bytes(static_cast<int32_t>(B), static_cast<int32_t>(S[0]), static_cast<int32_t>(S[1]),
+                                                         static_cast<int32_t>(S[2]), capacity, static_cast<int32_t>(topk));
+    at::Tensor scratch = at::empty({bytes + B * 4}, f32.dtype(at::kByte));  // and the device's copy of the counts
+    int32_t* counts = reinterpret_cast<int32_t*>(static_cast<char*>(scratch.data_ptr()) + bytes);
+    at::Tensor host = pinnedWords(B + 1);
+    int32_t* words = host.data_ptr<int32_t>();
+    words[B] = 0;
+    const auto stream = at::cuda::getCurrentCUDAStream();
+    checkRc(functs_b200_yolo_detect(maps[0].data_ptr<float>(), maps[1].data_ptr<float>(), maps[2].data_ptr<float>(),
+                                    static_cast<int32_t>(B), static_cast<int32_t>(S[0]), static_cast<int32_t>(S[1]),
+                                    static_cast<int32_t>(S[2]), static_cast<float>(score_thr), static_cast<int32_t>(topk),
+                                    static_cast<float>(iou_thr), capacity, dense ? r.boxes.data_ptr<float>() : nullptr,
+                                    dense ? r.obj.data_ptr<float>() : nullptr, dense ? r.cls.data_ptr<float>() : nullptr,
+                                    dets.data_ptr<float>(), labels.data_ptr<int64_t>(), want_ids ? ids.data_ptr<int64_t>() : nullptr,
+                                    counts, nullptr, words, words + B, scratch.data_ptr(), stream.stream()),
+            "yolov3 post-process");
+    C10_CUDA_CHECK(cudaStreamSynchronize(stream.stream()));
+    raiseOnStatus(words[B], "yolov3 post-process");
+    r.images.reserve(static_cast<size_t>(B));
+    for (int64_t b = 0; b < B; ++b) {
+        const int64_t n = words[b];
+        r.images.push_back({viewAt(dets, b * topk * 5, {n, 5}), viewAt(labels, b * topk, {n}),
+                            want_ids ? viewAt(ids, b * topk, {n}) : at::Tensor()});
+    }
+    return r;
+}
+
 }  // namespace functs_b200

@@ -20,4 +20,10 @@ struct SsdResult {
 SsdResult ssdDetect(const at::Tensor& loc, const at::Tensor& conf, const at::Tensor& priors, double clamp_max, double score_thr,
                     int64_t topk, double iou_thr, bool want_ids);
 
+struct YoloResult {
+    at::Tensor boxes, obj, cls;  // [B, N, 4], [B, N], [B, N, 80]; dense = true only
+    std::vector<Detections> images;
+};
+YoloResult yoloDetect(const std::vector<at::Tensor>& maps, double score_thr, int64_t topk, double iou_thr, bool dense, bool want_ids);
+
 }  // namespace functs_b200

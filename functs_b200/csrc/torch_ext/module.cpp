@@ -128,6 +128,14 @@ PYBIND11_MODULE(_C, m) {
               }
               return pairs(r.images);
           });
+    m.def("_yolo_detect", [](const std::vector<at::Tensor>& maps, double score_thr, int64_t topk, double iou_thr) {
+        functs_b200::YoloResult r;
+        {
+            py::gil_scoped_release release;
+            r = functs_b200::yoloDetect(maps, score_thr, topk, iou_thr, /*dense=*/false, /*want_ids=*/false);
+        }
+        return pairs(r.images);
+    });
     m.def("_count_parallel_functors", [](std::shared_ptr<Graph> g) { return functs_b200::CountParallelFunctors(g); });
     m.def("_jit_pass_freeze", [](torch::jit::Module& module) { return torch::jit::freeze_module(module); });
     m.def("_jit_pass_clone", [](torch::jit::Module& module) { return module.clone(); });

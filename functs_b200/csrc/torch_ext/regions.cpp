@@ -391,8 +391,6 @@ Operation makeYolo(const Node* node, bool dense) {
                         "yolov3 region: grid / anchor constants differ from the table the kernels hold");
         }
     }
-    const int gid = lookupGroup(
-        "yolov3{decode->loop[b<B]{mul(obj,cls)->gt(thr)->nonzero->sort(desc,stable)->slice[:k]->class-offset nms}}");
     return [=](Stack& stack) {
         c10::List<at::Tensor> list = pop(stack).toTensorList();
         TORCH_CHECK(list.size() == 3, "yolov3 region: expected three prediction maps");
@@ -403,43 +401,14 @@ Operation makeYolo(const Node* node, bool dense) {
                         "yolov3 region: map ", l, " must be [B, 255, ", sizes[l], ", ", sizes[l], "]");
             maps.push_back(m);
         }
-        c10::cuda::CUDAGuard guard(maps[0].device());
-        const int64_t B = maps[0].size(0);
-        const int64_t N = 3 * (sizes[0] * sizes[0] + sizes[1] * sizes[1] + sizes[2] * sizes[2]);
-        const int64_t capacity = N * 80;
-        auto f32 = maps[0].options();
-        auto i64 = f32.dtype(at::kLong);
-        at::Tensor boxes = at::empty({B, N, 4}, f32);
-        at::Tensor obj, cls;
-        if (dense) {
-            obj = at::empty({B, N}, f32);
-            cls = at::empty({B, N, 80}, f32);
-        }
-        at::Tensor dets = at::empty({B, topk, 5}, f32), labels = at::empty({B, topk}, i64), ids = at::empty({B, topk}, i64);
-        at::Tensor counts = at::empty({B}, f32.dtype(at::kInt)), status = at::zeros({1}, f32.dtype(at::kInt));
-        at::Tensor scratch = at::empty(
-            {functs_b200_yolo_scratch_bytes(static_cast<int32_t>(B), static_cast<int32_t>(sizes[0]), static_cast<int32_t>(sizes[1]),
-                                            static_cast<int32_t>(sizes[2]), capacity, static_cast<int32_t>(topk))},
-            f32.dtype(at::kByte));
-        const void* in_ptrs[] = {maps[0].data_ptr(), maps[1].data_ptr(), maps[2].data_ptr()};
-        const int64_t ints[] = {B, sizes[0], sizes[1], sizes[2], topk, capacity};
-        const double floats[] = {thr, iou};
-        void* outs[] = {boxes.data_ptr(), dense ? obj.data_ptr() : nullptr, dense ? cls.data_ptr() : nullptr,
-                        dets.data_ptr(), labels.data_ptr(), ids.data_ptr(), counts.data_ptr(), nullptr};
-        checkRc(functs_b200_group_launch(gid, in_ptrs, ints, floats, outs, scratch.data_ptr(), status.data_ptr<int>(),
-                                         at::cuda::getCurrentCUDAStream().stream()),
-                "yolov3 post-process");
-        // the only synchronisation: counts (and the status word) come back, the padded outputs are narrowed
-        at::Tensor host = at::cat({counts, status}).cpu();
-        raiseOnStatus(host[B], "yolov3 post-process");
-        const int* cnt = host.data_ptr<int>();
+        YoloResult r = yoloDetect(maps, thr, topk, iou, dense, /*want_ids=*/true);
         c10::impl::GenericList results(c10::TupleType::create({c10::TensorType::get(), c10::TensorType::get(), c10::TensorType::get()}));
-        for (int64_t b = 0; b < B; ++b) {
-            results.push_back(c10::ivalue::Tuple::create(
-                {dets[b].narrow(0, 0, cnt[b]), labels[b].narrow(0, 0, cnt[b]), ids[b].narrow(0, 0, cnt[b])}));
+        results.reserve(r.images.size());
+        for (Detections& d : r.images) {
+            results.push_back(c10::ivalue::Tuple::create({std::move(d.dets), std::move(d.labels), std::move(d.ids)}));
         }
         if (dense) {
-            push(stack, std::move(boxes), std::move(obj), std::move(cls));
+            push(stack, std::move(r.boxes), std::move(r.obj), std::move(r.cls));
         }
         stack.emplace_back(std::move(results));
     };

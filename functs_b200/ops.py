@@ -173,22 +173,22 @@ class YoloPostprocessPlan:
         self.scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
 
     def select_fallbacks(self) -> int:
-        """Number of images of the last call whose top-k was finished by the generic (slow, exact) selection."""
-        counts_bytes = (self.batch * 4 + 255) // 256 * 256
-        hist_bytes = (self.batch * int(lib.functs_b200_hist_bins()) * 4 + 255) // 256 * 256
-        ctr = self.scratch[counts_bytes + hist_bytes: counts_bytes + hist_bytes + self.batch * 16].view(torch.int32)
-        return int(ctr.reshape(self.batch, 4)[:, 3].sum())
+        """Number of images of the last call whose top-k took one of the slow exact ways (their score floor was too high, or
+        more candidates reached it than the selection holds)."""
+        words = (self.batch * 4 + 255) // 256 * 256  # scratch: candidate counts, fallback flags, floors, ...
+        return int(self.scratch[words: words + self.batch * 4].view(torch.int32).sum())
 
     def run(self, maps: List[torch.Tensor], score_thr: float = 0.5, iou_thr: float = 0.45,
-            records: Optional[torch.Tensor] = None) -> None:
-        """records (optional, int32 [batch, topk, 8]): the NMS kernel also writes the gather records (no pack launch)."""
+            records: Optional[torch.Tensor] = None, all_boxes: bool = True) -> None:
+        """records (optional, int32 [batch, topk, 8]): the last kernel also writes the gather records (no pack launch).
+        all_boxes = False leaves self.boxes as it is (the detections do not need it)."""
         s = self.sizes
         if records is not None and (records.dtype != torch.int32 or not records.is_contiguous()
                                     or records.numel() != self.batch * self.topk * 8):
             raise ValueError("records must be a contiguous int32 [batch, topk, 8] tensor")
         check(lib.functs_b200_yolo_postprocess_dense(maps[0].data_ptr(), maps[1].data_ptr(), maps[2].data_ptr(), self.batch,
                                                      s[0], s[1], s[2], float(score_thr), self.topk, float(iou_thr),
-                                                     self.capacity, _ptr(self.boxes), None, None, _ptr(self.dets),
+                                                     self.capacity, _ptr(self.boxes) if all_boxes else None, None, None, _ptr(self.dets),
                                                      _ptr(self.labels), _ptr(self.flat_ids), _ptr(self.counts),
                                                      _ptr(records), _ptr(self.status), _ptr(self.scratch), _stream()),
               "yolo_postprocess")

@@ -34,7 +34,7 @@ def get_started(a: torch.Tensor, b: torch.Tensor, n: int, device="cuda") -> torc
 
 
 class YOLOV3BBox:
-    """Decode three [B, 255, S, S] maps, score mask, top-k, class-wise NMS.  3 kernel launches (+1 memset) per call."""
+    """Decode three [B, 255, S, S] maps, score mask, top-k, class-wise NMS.  3 kernel launches per call."""
 
     def __init__(self, sizes=(13, 26, 52), score_thr: float = 0.5, topk: int = 1000, iou_thr: float = 0.45,
                  device="cuda"):
@@ -48,25 +48,31 @@ class YOLOV3BBox:
             self._plan = ops.YoloPostprocessPlan(batch, self.sizes, self.topk, device=self.device)
         return self._plan
 
-    def forward_padded(self, pred_maps: List[torch.Tensor]):
-        """-> (dets [B,K,5], labels [B,K], flat_ids [B,K], counts [B]) on the device, rows past counts[b] are padding.
-        The tensors belong to the module and are overwritten by the next call."""
+    def _checked(self, pred_maps: List[torch.Tensor]) -> List[torch.Tensor]:
         maps = [m.to(self.device, non_blocking=True).contiguous() for m in pred_maps]
         if len(maps) != 3 or any(m.dim() != 4 or m.size(1) != 255 for m in maps):
             raise ValueError("expected three [B, 255, S, S] maps")
         if tuple(m.size(2) for m in maps) != self.sizes:
             raise ValueError(f"map sizes {[m.size(2) for m in maps]} differ from the configured {self.sizes}")
+        return maps
+
+    def forward_padded(self, pred_maps: List[torch.Tensor]):
+        """-> (dets [B,K,5], labels [B,K], flat_ids [B,K], counts [B]) on the device, rows past counts[b] are padding.
+        The tensors belong to the module and are overwritten by the next call."""
+        maps = self._checked(pred_maps)
         plan = self._plan_for(maps[0].size(0))
         before = launch_count()
-        plan.run(maps, self.score_thr, self.iou_thr)
+        plan.run(maps, self.score_thr, self.iou_thr, all_boxes=False)
         self.kernels_last_call = launch_count() - before
         return plan.dets, plan.labels, plan.flat_ids, plan.counts
 
     def __call__(self, pred_maps: List[torch.Tensor]) -> List[Tuple[torch.Tensor, torch.Tensor]]:
-        dets, labels, _, counts = self.forward_padded(pred_maps)
-        cnt = counts.tolist()
-        ops.raise_on_status(self._plan.status, "YOLOV3BBox")
-        return [(dets[b, :cnt[b]].clone(), labels[b, :cnt[b]].clone()) for b in range(len(cnt))]
+        # launches, the wait for the counts and the per-image views in one native call
+        maps = self._checked(pred_maps)
+        before = launch_count()
+        out = _native()._yolo_detect(maps, self.score_thr, self.topk, self.iou_thr)
+        self.kernels_last_call = launch_count() - before
+        return out
 
 
 class SSDBBox:

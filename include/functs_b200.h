@@ -151,9 +151,8 @@ int functs_b200_yolo_decode(const float* map0, const float* map1, const float* m
                             uint64_t* cand_keys, int32_t* cand_counts, int64_t capacity, int32_t* hist,
                             int32_t* status, void* stream);
 
-/* Whole post-process: one memset + decode -> select_topk_binned -> batched_nms(class_offset=1): 3 kernel launches
- * (decode + mask + compaction; top-k selection, which also lays out the NMS input; NMS bit matrix + greedy scan).
- * Outputs as in batched_nms.
+/* Whole post-process, 3 kernel launches: a score floor per image from a sample of its boxes; decode + mask + compaction of
+ * the candidates that reach it; top-k, class-offset NMS and outputs, one CTA per image.  Outputs as in batched_nms.
  * scratch: functs_b200_yolo_scratch_bytes(batch, s0, s1, s2, capacity, topk). */
 int64_t functs_b200_yolo_scratch_bytes(int32_t batch, int32_t s0, int32_t s1, int32_t s2, int64_t capacity,
                                        int32_t topk);
@@ -164,15 +163,23 @@ int functs_b200_yolo_postprocess(const float* map0, const float* map1, const flo
 
 /* The same with the dense per-box outputs of the decode group kept: obj_out [batch, N] and cls_out [batch, N, 80]
  * (sigmoid of the objectness / class logits), as a program that returns them needs (the slices flat[..., 4] and
- * flat[..., 5:] of yolov3_bbox.py:217-219).  Every score is formed in that case, so the decode launch is the
- * thread-per-box kernel and nothing is pruned; still 3 launches.  NULL for both = functs_b200_yolo_postprocess.
- * records (optional, [batch, topk, 8] int32, 16-byte aligned): the NMS kernel also writes every output row as the
+ * flat[..., 5:] of yolov3_bbox.py:217-219).  Still 3 launches.  NULL for both = functs_b200_yolo_postprocess.
+ * records (optional, [batch, topk, 8] int32, 16-byte aligned): the last kernel also writes every output row as the
  * 32-byte record of functs_b200_pack_detections, so that a sharded caller can gather right away (no pack launch). */
 int functs_b200_yolo_postprocess_dense(const float* map0, const float* map1, const float* map2, int32_t batch,
                                        int32_t s0, int32_t s1, int32_t s2, float score_thr, int32_t topk,
                                        float iou_thr, int64_t capacity, float* boxes, float* obj_out, float* cls_out,
                                        float* dets, int64_t* labels, int64_t* flat_ids, int32_t* out_counts,
                                        int32_t* records, int32_t* status, void* scratch, void* stream);
+
+/* The general form.  boxes may be NULL (the boxes of the detections are decoded from the logits either way), flat_ids may be
+ * NULL.  host_counts (optional, [batch]) receives the counts once more; it and the status word may be pinned host memory,
+ * so that a caller who waits for the stream needs no copy. */
+int functs_b200_yolo_detect(const float* map0, const float* map1, const float* map2, int32_t batch, int32_t s0, int32_t s1,
+                            int32_t s2, float score_thr, int32_t topk, float iou_thr, int64_t capacity, float* boxes,
+                            float* obj_out, float* cls_out, float* dets, int64_t* labels, int64_t* flat_ids,
+                            int32_t* out_counts, int32_t* records, int32_t* host_counts, int32_t* status, void* scratch,
+                            void* stream);
 
 /* ---- C3: SSD-style post-process ----------------------------------------------------------- */
 /* Follows functs/benchmark/ai_model/ssd/ssd_bbox.py:121-154 (decode with the strided clamp), :268 (softmax, last
@@ -227,8 +234,7 @@ int functs_b200_lstm_forward_mode(const float* x, const float* w_ih, const float
 
 /* Debugging switches (name -> value); returns FB_ERR_NOT_FOUND for an unknown name.
  *   "yolo_prune": 0 makes functs_b200_yolo_postprocess keep every candidate above the score threshold instead of
- *                 dropping, inside the decode kernel, those that can no longer reach the top-k (default 1; the
- *                 outputs are the same either way). */
+ *                 those that reach the image's score floor (default 1; the outputs are the same either way). */
 int functs_b200_debug_set(const char* name, int32_t value);
 
 /* ---- C5: YOLACT-style mask assembly ------------------------------------------------------------ */
