@@ -4,18 +4,20 @@
 // What bounds it: reading the 80 class planes and the objectness plane of every level (81 of the 85 channels; the box channels
 // are only read for callers that want every box).  Everything else is kept off that stream:
 //   - the score floor.  The program keeps the topk best candidates of an image, but with logits near N(0, 1) one score in
-//     thirteen passes the threshold: 65 000 per image.  yolo_floor_kernel takes the scores of one box in sixteen (eight
-//     neighbouring slots of every tile, one 32-byte sector per plane) and picks the score that about 2 * topk candidates
+//     thirteen passes the threshold: 65 000 per image.  yolo_floor_kernel takes the scores of one box in sixteen (32
+//     neighbouring slots of every 512, one 128-byte line per plane) and picks the score that about 2 * topk candidates
 //     should reach.  The floor is a guess: whoever uses the list has to see that it holds at least topk candidates, and
 //     takes the exact way otherwise (yolo_post_kernel does).
 //   - with the floor known before the first class logit is read, a box whose objectness lies below it is never walked, and
-//     a class logit costs a compare against its box's cut.  Hits (about two in a thousand) are queued in shared memory and
-//     evaluated exactly, together, at the end of the tile.
+//     a class logit costs a compare against its box's cut.  Hits (about two in a hundred of those) are queued in shared
+//     memory and evaluated exactly, together, at the end of the tile.
 // Before, the floor was found while the kernel ran, from a histogram in global memory that every candidate incremented: the
 // first wave of CTAs had none, and 12 000 candidates per image reached the selection.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <atomic>
+#include <utility>
 
 #include "yolo.cuh"
 
@@ -25,7 +27,10 @@ namespace cg = cooperative_groups;
 
 // ---- score floor ------------------------------------------------------------------------------------------------------
 constexpr int kFloorCtas = 8;        // one cluster per image
-constexpr int kFloorThreads = 384;   // 8 x 12 warps: one tile per warp up to 96 tiles (84 at 13 / 26 / 52)
+constexpr int kFloorThreads = 384;   // 8 x 3 runs of 32 slots, four warps each (21 runs at 13 / 26 / 52)
+constexpr int kFloorBlock = 512;     // one run of 32 slots per 512: a whole 128-byte line per plane, because that is what DRAM is read
+                                     // in (runs of eight slots, four times as many, moved 58 MB instead of 15: 26 us for 64 images)
+constexpr int kFloorBins = 256;      // score buckets (a guess needs no finer ones; one thread each)
 constexpr int kFloorMinSample = 256; // sampled boxes below which a floor is not worth the risk (small pyramids)
 
 struct YoloFloorArgs {
@@ -41,44 +46,54 @@ struct YoloFloorArgs {
 };
 
 // Also clears the image's counters.  The scores of the sample may be approximate: they only pick a bucket.
-__global__ void __cluster_dims__(kFloorCtas, 1, 1) __launch_bounds__(kFloorThreads)
+__global__ void __cluster_dims__(kFloorCtas, 1, 1) __launch_bounds__(kFloorThreads, 4)
 yolo_floor_kernel(const YoloFloorArgs A) {
-    __shared__ __align__(16) int hist[kHistBins];
+    __shared__ int hist[kFloorBins];    // this CTA's scores
+    __shared__ int merged[kFloorBins];  // rank 0: the cluster's
     __shared__ int s_valid, s_bucket;
-    __shared__ int s_warp[8];
+    __shared__ int s_warp[kFloorBins / 32];
     pdl_launch_dependents();
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = static_cast<int>(cluster.block_rank());
     const int img = blockIdx.x / kFloorCtas;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if (A.sample) {
-        if (rank == 0) {
-            for (int i = t; i < kHistBins; i += kFloorThreads) hist[i] = 0;
-            if (t == 0) {
-                s_valid = 0;
-                s_bucket = 0;
-            }
+        if (t < kFloorBins) {
+            hist[t] = 0;
+            merged[t] = 0;
         }
-        cluster.sync();
-        int* hist0 = cluster.map_shared_rank(hist, 0);
-        int* valid0 = cluster.map_shared_rank(&s_valid, 0);
+        if (t == 0) {
+            s_valid = 0;
+            s_bucket = 0;
+        }
+        __syncthreads();
+        auto cleared = cluster.barrier_arrive();  // (waited for before anybody adds to rank 0's words)
         const YoloLevels& L = A.L;
         int nvalid = 0;
-        for (int tile = rank * (kFloorThreads / 32) + warp; tile < L.tile_begin[3]; tile += kFloorCtas * (kFloorThreads / 32)) {
-            const int lvl = tile >= L.tile_begin[2] ? 2 : (tile >= L.tile_begin[1] ? 1 : 0);
-            const int plane = L.plane[lvl];
-            const int s0 = (tile - L.tile_begin[lvl]) * kYoloTile;
-            const int groups = max(1, min(kYoloTile, 3 * plane - s0) >> 3);
-            const int slot = s0 + 8 * ((tile * 5 + img * 3) % groups) + (lane & 7);
+        const int quarter = warp & 3;  // twenty of the eighty classes
+        for (int block = rank * (kFloorThreads / 128) + (warp >> 2);; block += kFloorCtas * (kFloorThreads / 128)) {
+            int lvl = 0, local = block;  // level and number of the 512-slot block inside it
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                const int nb = (3 * L.plane[l] + kFloorBlock - 1) / kFloorBlock;
+                if (lvl == l && local >= nb) {
+                    local -= nb;
+                    ++lvl;
+                }
+            }
+            if (lvl > 2) break;  // warp-uniform
+            const int plane = L.plane[lvl], s0 = local * kFloorBlock;
+            const int runs = max(1, min(kFloorBlock, 3 * plane - s0) >> 5);
+            const int slot = s0 + 32 * ((block * 5 + img * 3) % runs) + lane;
             const bool valid = slot < 3 * plane;
             int anchor, pos;
             yolo_slot(plane, valid ? slot : s0, anchor, pos);
             const float* src = L.map[lvl] + (static_cast<int64_t>(img) * 3 + anchor) * kYoloAttrib * plane + pos;
             const float tobj = __ldg(src + 4 * plane);
-            const float* csrc = src + (5 + (lane >> 3)) * plane;
+            const float* csrc = src + (5 + quarter * (kYoloClasses / 4)) * plane;
             float v[kYoloClasses / 4];
 #pragma unroll
-            for (int u = 0; u < kYoloClasses / 4; ++u) v[u] = __ldg(csrc + u * 4 * plane);
+            for (int u = 0; u < kYoloClasses / 4; ++u) v[u] = __ldg(csrc + u * plane);
             const float so = __fdividef(1.0f, 1.0f + __expf(-tobj));
             const bool alive = valid && so > A.thr;
             const float cut = alive ? logit_cut(so, A.thr) : INFINITY;
@@ -87,46 +102,33 @@ yolo_floor_kernel(const YoloFloorArgs A) {
                 if (v[u] > cut) {
                     const float s = so * __fdividef(1.0f, 1.0f + __expf(-v[u]));
                     if (s > A.thr)
-                        atomicAdd(hist0 + hist_digit(static_cast<uint64_t>(__float_as_uint(s)) << 32, A.hist_base, A.hist_shift), 1);
+                        atomicAdd(&hist[hist_digit(static_cast<uint64_t>(__float_as_uint(s)) << 32, A.hist_base, A.hist_shift) /
+                                        (kHistBins / kFloorBins)], 1);
                 }
             }
-            nvalid += __popc(__ballot_sync(kFullMask, valid)) >> 2;  // four lanes per box
+            if (quarter == 0) nvalid += __popc(__ballot_sync(kFullMask, valid));
         }
-        if (lane == 0 && nvalid > 0) atomicAdd(valid0, nvalid);
+        __syncthreads();
+        cluster.barrier_wait(std::move(cleared));
+        if (lane == 0 && nvalid > 0) atomicAdd(cluster.map_shared_rank(&s_valid, 0), nvalid);
+        if (t < kFloorBins && hist[t] != 0) atomicAdd(cluster.map_shared_rank(merged, 0) + t, hist[t]);
         cluster.sync();
         if (rank != 0) return;
         // the largest bucket d with (sampled candidates in buckets >= d) >= target
         const int total_valid = s_valid;
         const int target = static_cast<int>(2ll * A.topk * total_valid / L.num_boxes) + 8;
-        int h[8], mine = 0, incl = 0;
-        if (t < 256) {
-            const int4 a = reinterpret_cast<const int4*>(hist)[2 * t], b = reinterpret_cast<const int4*>(hist)[2 * t + 1];
-            h[0] = a.x; h[1] = a.y; h[2] = a.z; h[3] = a.w;
-            h[4] = b.x; h[5] = b.y; h[6] = b.z; h[7] = b.w;
+        const int mine = t < kFloorBins ? merged[t] : 0;
+        int incl = mine;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) mine += h[k];
-            incl = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int x = __shfl_down_sync(kFullMask, incl, o);
-                if (lane + o < 32) incl += x;
-            }
-            if (lane == 0) s_warp[warp] = incl;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_down_sync(kFullMask, incl, o);
+            if (lane + o < 32) incl += x;
         }
+        if (t < kFloorBins && lane == 0) s_warp[warp] = incl;
         __syncthreads();
-        if (t < 256) {
-            for (int w = warp + 1; w < 8; ++w) incl += s_warp[w];
-            if (incl >= target && incl - mine < target) {
-                int cum = incl - mine, d = 7;
-#pragma unroll
-                for (int k = 7; k >= 0; --k) {
-                    if (cum < target) {
-                        cum += h[k];
-                        d = k;
-                    }
-                }
-                s_bucket = 8 * t + d;
-            }
+        if (t < kFloorBins) {
+            for (int w = warp + 1; w < kFloorBins / 32; ++w) incl += s_warp[w];
+            if (incl >= target && incl - mine < target) s_bucket = t * (kHistBins / kFloorBins);
         }
         __syncthreads();
         if (t == 0) {
@@ -143,10 +145,10 @@ yolo_floor_kernel(const YoloFloorArgs A) {
 }
 
 // ---- decode -----------------------------------------------------------------------------------------------------------
-constexpr int kDecQueue = 512;                    // queued hits of a tile (a floored tile has some twenty); more are evaluated on the spot
-constexpr int kDecWarps = kYoloTile / 32;
+constexpr int kDecThreads = 128;
+constexpr int kDecWarps = kDecThreads / 32;
 constexpr int kDecClasses = kYoloClasses / kDecWarps;  // classes per warp
-constexpr int kDecStep = 10;                      // class planes of a warp in flight: 5 KB
+constexpr int kDecStep = 10;                           // of which loaded at a time
 
 struct YoloDecodeArgs {
     YoloLevels L;
@@ -164,18 +166,35 @@ struct YoloDecodeArgs {
     int hist_shift;
 };
 
+struct __align__(16) YoloLive {  // a slot that can yield candidates
+    float so;      // objectness score
+    float cut;     // class logits at or below this cannot reach the bar
+    int off;       // first class logit, from the start of the image's level
+    uint32_t box;  // box index inside the image
+};
 struct __align__(8) YoloHit {
     float v;        // class logit (dense form: the finished score)
-    uint32_t meta;  // slot << 7 | class
+    uint32_t meta;  // live slot << 7 | class
 };
 
-struct YoloTileSmem {
-    float cut[kYoloTile];     // class logits at or below this cannot reach the bar; +inf: the slot is dead
-    float so[kYoloTile];      // objectness score
-    uint32_t box[kYoloTile];  // box index inside the image
-    YoloHit queue[kDecQueue];
-    int queued;
+// Slots [first, first + count) of a level of an image.
+struct YoloTile {
+    int img, lvl, s0;
 };
+__device__ __forceinline__ YoloTile yolo_tile(const YoloLevels& L, int index, int slots) {
+    YoloTile T;
+    int per_image = 0, begin[3];
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+        begin[l] = per_image;
+        per_image += (3 * L.plane[l] + slots - 1) / slots;
+    }
+    T.img = index / per_image;
+    const int tile = index - T.img * per_image;
+    T.lvl = tile >= begin[2] ? 2 : (tile >= begin[1] ? 1 : 0);
+    T.s0 = (tile - (T.lvl == 2 ? begin[2] : (T.lvl == 1 ? begin[1] : 0))) * slots;
+    return T;
+}
 
 // Whole warps: appends the keys of the lanes with `pass` to the image's list.
 __device__ __forceinline__ void yolo_append(const YoloDecodeArgs& A, int img, bool pass, float s, uint32_t flat) {
@@ -194,208 +213,232 @@ __device__ __forceinline__ void yolo_append(const YoloDecodeArgs& A, int img, bo
                           hist_digit(static_cast<uint64_t>(__float_as_uint(s)) << 32, A.hist_base, A.hist_shift), 1);
     }
 }
-// One lane on its own (the queue is full).
-__device__ __noinline__ void yolo_append_one(const YoloDecodeArgs* A, int img, float s, uint32_t flat) {
-    const int64_t at = atomicAdd(A->counts + img, 1);
-    if (at < A->capacity) A->keys[img * A->capacity + at] = make_key(s, flat);
-    else if (A->status != nullptr) atomicOr(A->status, FB_STATUS_CAND_OVERFLOW);
-    if (A->hist != nullptr)
-        atomicAdd(A->hist + static_cast<int64_t>(img) * kHistBins +
-                      hist_digit(static_cast<uint64_t>(__float_as_uint(s)) << 32, A->hist_base, A->hist_shift), 1);
-}
 
-// The slot of lane `lane`, element e of a tile: four neighbours per lane where the planes are 16-byte aligned (a group of four
-// then lies inside one anchor), else a warp-wide run per element.
-template <bool VEC>
-__device__ __forceinline__ int tile_slot(int lane, int e) {
-    return VEC ? 4 * lane + e : 32 * e + lane;
-}
-
-// Warp `warp` of a tile walks its twenty class planes: four slots per lane, ten planes in flight.
-template <bool VEC>
-__device__ __forceinline__ void yolo_walk(const YoloDecodeArgs& A, YoloTileSmem& sm, const float* __restrict__ img_map, int plane, int s0,
-                                          int nslots, int img, float bar) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float cut[4];
-    int off[4];
-    if (VEC) {
-        const float4 c = reinterpret_cast<const float4*>(sm.cut)[lane];
-        cut[0] = c.x; cut[1] = c.y; cut[2] = c.z; cut[3] = c.w;
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        if (!VEC) cut[e] = sm.cut[32 * e + lane];
-        int anchor, pos;
-        yolo_slot(plane, min(s0 + tile_slot<VEC>(lane, e), nslots - 1), anchor, pos);
-        off[e] = (anchor * kYoloAttrib + 5 + warp * kDecClasses) * plane + pos;
-    }
-    const bool on = cut[0] < INFINITY || cut[1] < INFINITY || cut[2] < INFINITY || cut[3] < INFINITY;
-#pragma unroll 1
-    for (int k0 = 0; k0 < kDecClasses; k0 += kDecStep) {
-        uint32_t hits[2] = {0u, 0u};
-        if (on) {
-            float4 v[kDecStep];
-            if (VEC) {
-                const float* p = img_map + off[0] + k0 * plane;
-#pragma unroll
-                for (int u = 0; u < kDecStep; ++u) v[u] = __ldg(reinterpret_cast<const float4*>(p + u * plane));
-            } else {
-#pragma unroll
-                for (int u = 0; u < kDecStep; ++u) {
-                    const float* p = img_map + (k0 + u) * plane;
-                    v[u] = make_float4(__ldg(p + off[0]), __ldg(p + off[1]), __ldg(p + off[2]), __ldg(p + off[3]));
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kDecStep; ++u) {
-                const int sh = 4 * (u % 5);
-                uint32_t& h = hits[u / 5];
-                h |= v[u].x > cut[0] ? 1u << sh : 0u;
-                h |= v[u].y > cut[1] ? 2u << sh : 0u;
-                h |= v[u].z > cut[2] ? 4u << sh : 0u;
-                h |= v[u].w > cut[3] ? 8u << sh : 0u;
-            }
-        }
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            uint32_t h = hits[half];
-            if (h == 0u) continue;
-            int at = atomicAdd(&sm.queued, __popc(h));
-            while (h != 0u) {
-                const int k = __ffs(h) - 1;
-                h &= h - 1u;
-                const int e = k & 3, c = k0 + 5 * half + (k >> 2);
-                const int o = e == 0 ? off[0] : (e == 1 ? off[1] : (e == 2 ? off[2] : off[3]));
-                const float v = __ldg(img_map + o + c * plane);  // (read again: a hit's register cannot be named at run time)
-                const int slot = tile_slot<VEC>(lane, e), cls = warp * kDecClasses + c;
-                if (at < kDecQueue) {
-                    sm.queue[at].v = v;
-                    sm.queue[at].meta = static_cast<uint32_t>(slot << 7 | cls);
-                } else {
-                    const float s = __fmul_rn(sm.so[slot], sigmoid_f32(v));
-                    if (s > A.thr && s >= bar) yolo_append_one(&A, img, s, sm.box[slot] * kYoloClasses + static_cast<uint32_t>(cls));
-                }
-                ++at;
-            }
+// A tile whose hits did not fit the queue is walked once more, one live slot per thread.
+__device__ __noinline__ void yolo_crowded_tile(const YoloDecodeArgs* A, const float* img_map, int plane, int img, const YoloLive* live, int n,
+                                               float bar) {
+    for (int i0 = 0; i0 < n; i0 += kDecThreads) {
+        const int i = i0 + static_cast<int>(threadIdx.x);
+        YoloLive o{0.0f, INFINITY, 0, 0u};
+        if (i < n) o = live[i];
+        const float cut = i < n ? logit_cut(o.so, bar) : INFINITY;
+        for (int c = 0; c < kYoloClasses; ++c) {
+            const float v = i < n ? __ldg(img_map + o.off + c * plane) : 0.0f;
+            float s = 0.0f;
+            if (v > cut) s = __fmul_rn(o.so, sigmoid_f32(v));
+            yolo_append(*A, img, s > A->thr && s >= bar, s, o.box * kYoloClasses + static_cast<uint32_t>(c));
         }
     }
 }
 
-constexpr int kDenseRow = kYoloClasses + 1;  // odd: a warp that stores one class of 32 slots hits 32 banks
-
-// grid = batch * tiles per image.  DENSE: the objectness and class scores are outputs too; every score is formed, staged in
-// shared memory and written as whole 320-byte rows (written straight from the threads, every store instruction touched 32
-// rows: 145 us for 8 images of 608 x 608 against 19 us of traffic).
+// The queued hits of a tile, evaluated together.
 template <bool DENSE>
-__global__ void __launch_bounds__(kYoloTile, DENSE ? 5 : 7)
-yolo_decode_kernel(const __grid_constant__ YoloDecodeArgs A) {
-    __shared__ YoloTileSmem sm;
-    extern __shared__ float s_cls[];  // DENSE: [kYoloTile][kDenseRow]
-    pdl_launch_dependents();
-    const YoloLevels& L = A.L;
-    const int img = blockIdx.x / L.tile_begin[3], tile = blockIdx.x - img * L.tile_begin[3], t = threadIdx.x;
-    const int lvl = tile >= L.tile_begin[2] ? 2 : (tile >= L.tile_begin[1] ? 1 : 0);
-    const int plane = L.plane[lvl], nslots = 3 * plane;
-    const int s0 = (tile - L.tile_begin[lvl]) * kYoloTile;
-    const float* __restrict__ img_map = L.map[lvl] + static_cast<int64_t>(img) * 3 * kYoloAttrib * plane;
-
-    // one slot per thread: objectness, cut, and the box where it is wanted
-    const bool valid = s0 + t < nslots;
-    int anchor, pos;
-    yolo_slot(plane, valid ? s0 + t : s0, anchor, pos);
-    const float* src = img_map + anchor * kYoloAttrib * plane + pos;
-    const float tobj = __ldg(src + 4 * plane);
-    const uint32_t box = static_cast<uint32_t>(L.box_begin[lvl] + pos * 3 + anchor);
-    const int64_t gbox = static_cast<int64_t>(img) * L.num_boxes + box;
-    if (A.boxes != nullptr && valid) {
-        reinterpret_cast<float4*>(A.boxes)[gbox] =
-            yolo_box(L, lvl, anchor, pos, __ldg(src), __ldg(src + plane), __ldg(src + 2 * plane), __ldg(src + 3 * plane));
-    }
-    const float so = sigmoid_f32(tobj);
-    sm.so[t] = so;
-    sm.box[t] = box;
-    if (t == 0) sm.queued = 0;
-    if (DENSE && valid && A.obj_out != nullptr) A.obj_out[gbox] = so;
-    pdl_wait();  // the floor, and the counters that the floor kernel cleared
-    const float bar = fmaxf(A.thr, A.floor != nullptr ? __ldcg(A.floor + img) : 0.0f);
-    // a score is so * sigmoid(v) <= so: the box can only yield candidates if so itself clears both bars
-    const bool alive = valid && so > A.thr && so >= bar;
-    if (!DENSE) {
-        sm.cut[t] = alive ? logit_cut(so, bar) : INFINITY;
-        if (__syncthreads_or(alive ? 1 : 0) == 0) return;
-        if (L.vec4[lvl]) yolo_walk<true>(A, sm, img_map, plane, s0, nslots, img, bar);
-        else yolo_walk<false>(A, sm, img_map, plane, s0, nslots, img, bar);
-    } else {
-        sm.cut[t] = alive ? 0.0f : INFINITY;  // only tells the dead slots
-        __syncthreads();
-        const int lane = t & 31, warp = t >> 5;
-        int off[4];
-        float so4[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            int a, p;
-            yolo_slot(plane, min(s0 + 32 * e + lane, nslots - 1), a, p);
-            off[e] = (a * kYoloAttrib + 5 + warp * kDecClasses) * plane + p;
-            so4[e] = sm.cut[32 * e + lane] < INFINITY ? sm.so[32 * e + lane] : 0.0f;
-        }
-#pragma unroll 1
-        for (int k0 = 0; k0 < kDecClasses; k0 += 5) {
-            float v[5][4];
-#pragma unroll
-            for (int u = 0; u < 5; ++u)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) v[u][e] = __ldg(img_map + off[e] + (k0 + u) * plane);
-#pragma unroll
-            for (int u = 0; u < 5; ++u)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int slot = 32 * e + lane, cls = warp * kDecClasses + k0 + u;
-                    const float c = sigmoid_f32(v[u][e]);
-                    s_cls[slot * kDenseRow + cls] = c;
-                    const float s = __fmul_rn(so4[e], c);
-                    if (s > A.thr && s >= bar) {
-                        const int at = atomicAdd(&sm.queued, 1);
-                        if (at < kDecQueue) {
-                            sm.queue[at].v = s;
-                            sm.queue[at].meta = static_cast<uint32_t>(slot << 7 | cls);
-                        } else {
-                            yolo_append_one(&A, img, s, sm.box[slot] * kYoloClasses + static_cast<uint32_t>(cls));
-                        }
-                    }
-                }
-        }
-    }
-    __syncthreads();
-    if (DENSE && A.cls_out != nullptr) {
-        const int total = min(kYoloTile, nslots - s0) * kYoloClasses;
-        float* out = A.cls_out + static_cast<int64_t>(img) * L.num_boxes * kYoloClasses;
-        int slot = t / kYoloClasses, c = t - slot * kYoloClasses;
-        for (int i = t; i < total; i += kYoloTile) {
-            out[static_cast<int64_t>(sm.box[slot]) * kYoloClasses + c] = s_cls[slot * kDenseRow + c];
-            slot += kYoloTile / kYoloClasses;
-            c += kYoloTile % kYoloClasses;
-            if (c >= kYoloClasses) {
-                c -= kYoloClasses;
-                ++slot;
-            }
-        }
-    }
-    // the queued hits, evaluated together
-    const int n = min(sm.queued, kDecQueue);
-    for (int i0 = 0; i0 < n; i0 += kYoloTile) {
-        const int i = i0 + t;
+__device__ __forceinline__ void yolo_eval_queue(const YoloDecodeArgs& A, const YoloLive* live, const YoloHit* queue, int img, int n, float bar) {
+    for (int i0 = 0; i0 < n; i0 += kDecThreads) {
+        const int i = i0 + static_cast<int>(threadIdx.x);
         bool pass = i < n;
         float s = 0.0f;
         uint32_t flat = 0u;
         if (pass) {
-            const YoloHit h = sm.queue[i];
-            const uint32_t slot = h.meta >> 7;
-            s = DENSE ? h.v : __fmul_rn(sm.so[slot], sigmoid_f32(h.v));
-            flat = sm.box[slot] * kYoloClasses + (h.meta & 127u);
+            const YoloHit h = queue[i];
+            const YoloLive o = live[h.meta >> 7];
+            s = DENSE ? h.v : __fmul_rn(o.so, sigmoid_f32(h.v));
+            flat = o.box * kYoloClasses + (h.meta & 127u);
             pass = s > A.thr && s >= bar;
         }
         yolo_append(A, img, pass, s, flat);
     }
+}
+
+// One CTA per tile of 128 * E slots.  First the objectness of its slots, E per thread; the slots that clear the bar (one in seven
+// at N(0, 1), a few per cent behind a trained head) are listed in shared memory; then lane k of every warp takes live slot k
+// through the warp's twenty class planes.  The planes are streamed from DRAM almost whole either way (a 128-byte line rarely
+// holds no live slot), so what the list saves is instructions: forms in which every lane kept four neighbouring slots, dead
+// ones included, executed 17 to 22 million warp instructions for 64 images and took 42 to 53 us whatever the loads looked
+// like (registers, ten planes at a time; asynchronous copies, fifteen at a time, next tile prefetched).
+// E = 4 fills the lanes (70 live slots in 512); E = 1 makes more CTAs where there are few tiles.
+template <int E, bool BOXES>
+__global__ void __launch_bounds__(kDecThreads, 8)
+yolo_decode_kernel(const __grid_constant__ YoloDecodeArgs A) {
+    constexpr int kSlots = kDecThreads * E;
+    constexpr int kQueue = 2 * kSlots;  // hits: some 1.5 per live slot with a floor
+    __shared__ YoloLive live[kSlots];
+    __shared__ YoloHit queue[kQueue];
+    __shared__ int s_live, s_queued;
+    pdl_launch_dependents();
+    const YoloLevels& L = A.L;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const YoloTile T = yolo_tile(L, blockIdx.x, kSlots);
+    const int plane = L.plane[T.lvl], nslots = 3 * plane;
+    const float* __restrict__ img_map = L.map[T.lvl] + static_cast<int64_t>(T.img) * 3 * kYoloAttrib * plane;
+    float so[E];
+    int off[E];
+    uint32_t box[E];
+    bool valid[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int slot = T.s0 + e * kDecThreads + t;
+        valid[e] = slot < nslots;
+        int anchor, pos;
+        yolo_slot(plane, valid[e] ? slot : T.s0, anchor, pos);
+        off[e] = anchor * kYoloAttrib * plane + pos;
+        box[e] = static_cast<uint32_t>(L.box_begin[T.lvl] + pos * 3 + anchor);
+        so[e] = __ldg(img_map + off[e] + 4 * plane);
+    }
+    if (t == 0) {
+        s_live = 0;
+        s_queued = 0;
+    }
+    if (BOXES) {
+#pragma unroll 1
+        for (int e = 0; e < E; ++e) {
+            const int slot = T.s0 + e * kDecThreads + t;
+            if (slot >= nslots) continue;
+            int anchor, pos;
+            yolo_slot(plane, slot, anchor, pos);
+            const float* src = img_map + anchor * kYoloAttrib * plane + pos;
+            reinterpret_cast<float4*>(A.boxes)[static_cast<int64_t>(T.img) * L.num_boxes + L.box_begin[T.lvl] + pos * 3 + anchor] =
+                yolo_box(L, T.lvl, anchor, pos, __ldg(src), __ldg(src + plane), __ldg(src + 2 * plane), __ldg(src + 3 * plane));
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) so[e] = sigmoid_f32(so[e]);
+    pdl_wait();  // the floor, and the counters that the floor kernel cleared
+    const float bar = fmaxf(A.thr, A.floor != nullptr ? __ldcg(A.floor + T.img) : 0.0f);
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        // a score is so * sigmoid(v) <= so: the box can only yield candidates if so itself clears both bars
+        const bool alive = valid[e] && so[e] > A.thr && so[e] >= bar;
+        const unsigned m = __ballot_sync(kFullMask, alive);
+        int base = 0;
+        if (lane == 0 && m != 0u) base = atomicAdd(&s_live, __popc(m));
+        base = __shfl_sync(kFullMask, base, 0);
+        if (alive) live[base + __popc(m & ((1u << lane) - 1u))] = YoloLive{so[e], logit_cut(so[e], bar), off[e] + 5 * plane, box[e]};
+    }
+    __syncthreads();
+    const int n = s_live;
+    if (n == 0) return;
+#pragma unroll 1
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        const int i = i0 + lane;
+        const bool on = i < n;
+        YoloLive o{0.0f, INFINITY, 0, 0u};
+        if (on) o = live[i];
+        const float* p = img_map + o.off + warp * kDecClasses * plane;
+#pragma unroll 1
+        for (int k0 = 0; k0 < kDecClasses; k0 += kDecStep) {
+            float v[kDecStep];
+#pragma unroll
+            for (int u = 0; u < kDecStep; ++u) v[u] = on ? __ldg(p + (k0 + u) * plane) : -INFINITY;
+            uint32_t hits = 0u;
+#pragma unroll
+            for (int u = 0; u < kDecStep; ++u) hits |= v[u] > o.cut ? 1u << u : 0u;
+            if (hits != 0u) {
+                int at = atomicAdd(&s_queued, __popc(hits));
+#pragma unroll
+                for (int u = 0; u < kDecStep; ++u) {
+                    if ((hits >> u) & 1u) {
+                        if (at < kQueue) queue[at] = YoloHit{v[u], static_cast<uint32_t>(i << 7 | (warp * kDecClasses + k0 + u))};
+                        ++at;
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (s_queued > kQueue) yolo_crowded_tile(&A, img_map, plane, T.img, live, n, bar);
+    else yolo_eval_queue<false>(A, live, queue, T.img, s_queued, bar);
+}
+
+// The dense form, one CTA per tile of 128 slots: the objectness and class scores are outputs too; every score is formed, staged
+// in shared memory and written as whole 320-byte rows (written straight from the threads, every store instruction touched 32
+// rows: 145 us for 8 images of 608 x 608 against 19 us of traffic).
+// The exact sigmoid of every logit bounds it (some twenty instructions each), so everything else goes four classes at a time.
+constexpr int kDenseRow = kYoloClasses + 4;  // an odd number of 16-byte chunks: eight neighbouring slots store to different banks
+constexpr int kDenseQueue = 512;
+__global__ void __launch_bounds__(kDecThreads, 4)
+yolo_decode_dense_kernel(const __grid_constant__ YoloDecodeArgs A) {
+    __shared__ YoloLive live[kDecThreads];  // every slot of the tile; so = 0: it cannot yield candidates
+    __shared__ YoloHit queue[kDenseQueue];
+    __shared__ int s_queued;
+    extern __shared__ __align__(16) float s_cls[];  // [128][kDenseRow]
+    pdl_launch_dependents();
+    const YoloLevels& L = A.L;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const YoloTile T = yolo_tile(L, blockIdx.x, kDecThreads);
+    const int plane = L.plane[T.lvl], nslots = 3 * plane;
+    const float* __restrict__ img_map = L.map[T.lvl] + static_cast<int64_t>(T.img) * 3 * kYoloAttrib * plane;
+    const bool valid = T.s0 + t < nslots;
+    int anchor, pos;
+    yolo_slot(plane, valid ? T.s0 + t : T.s0, anchor, pos);
+    const float* src = img_map + anchor * kYoloAttrib * plane + pos;
+    const uint32_t box = static_cast<uint32_t>(L.box_begin[T.lvl] + pos * 3 + anchor);
+    const int64_t gbox = static_cast<int64_t>(T.img) * L.num_boxes + box;
+    const float so = sigmoid_f32(__ldg(src + 4 * plane));
+    if (valid) {
+        if (A.boxes != nullptr)
+            reinterpret_cast<float4*>(A.boxes)[gbox] =
+                yolo_box(L, T.lvl, anchor, pos, __ldg(src), __ldg(src + plane), __ldg(src + 2 * plane), __ldg(src + 3 * plane));
+        if (A.obj_out != nullptr) A.obj_out[gbox] = so;
+    }
+    if (t == 0) s_queued = 0;
+    pdl_wait();
+    const float bar = fmaxf(A.thr, A.floor != nullptr ? __ldcg(A.floor + T.img) : 0.0f);
+    live[t] = YoloLive{valid && so > A.thr && so >= bar ? so : 0.0f, 0.0f, static_cast<int>(src - img_map) + 5 * plane, box};
+    __syncthreads();
+    const float* p4[4];
+    float cut4[4];  // class scores below this cannot bring the product to the bar
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const YoloLive o = live[32 * e + lane];
+        p4[e] = img_map + o.off + warp * kDecClasses * plane;
+        cut4[e] = o.so > 0.0f ? __fdividef(bar, o.so) * (1.0f - 1.0e-5f) : INFINITY;
+    }
+#pragma unroll 1
+    for (int k0 = 0; k0 < kDecClasses; k0 += 4) {
+        float v[4][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[e][u] = __ldg(p4[e] + (k0 + u) * plane);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int slot = 32 * e + lane;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[e][u] = sigmoid_f32(v[e][u]);
+            *reinterpret_cast<float4*>(s_cls + slot * kDenseRow + warp * kDecClasses + k0) = make_float4(v[e][0], v[e][1], v[e][2], v[e][3]);
+            if (fmaxf(fmaxf(v[e][0], v[e][1]), fmaxf(v[e][2], v[e][3])) >= cut4[e]) {
+                const float so_e = live[slot].so;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float s = __fmul_rn(so_e, v[e][u]);
+                    if (s > A.thr && s >= bar) {
+                        const int at = atomicAdd(&s_queued, 1);
+                        if (at < kDenseQueue) queue[at] = YoloHit{s, static_cast<uint32_t>(slot << 7 | (warp * kDecClasses + k0 + u))};
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (A.cls_out != nullptr) {
+        constexpr int kQuads = kYoloClasses / 4;
+        const int total = min(kDecThreads, nslots - T.s0) * kQuads;
+        float4* out = reinterpret_cast<float4*>(A.cls_out + static_cast<int64_t>(T.img) * L.num_boxes * kYoloClasses);
+        int slot = t / kQuads, c = t - slot * kQuads;
+        for (int i = t; i < total; i += kDecThreads) {
+            out[static_cast<int64_t>(live[slot].box) * kQuads + c] = *reinterpret_cast<const float4*>(s_cls + slot * kDenseRow + 4 * c);
+            slot += kDecThreads / kQuads;
+            c += kDecThreads % kQuads;
+            if (c >= kQuads) {
+                c -= kQuads;
+                ++slot;
+            }
+        }
+    }
+    if (s_queued > kDenseQueue) yolo_crowded_tile(&A, img_map, plane, T.img, live, kDecThreads, bar);
+    else yolo_eval_queue<true>(A, live, queue, T.img, s_queued, bar);
 }
 
 // Development switch (functs_b200_debug_set "yolo_prune"): 0 keeps every candidate above the score threshold.
@@ -418,11 +461,9 @@ static int yolo_levels(const float* map0, const float* map1, const float* map2, 
         L.map[l] = maps[l];
         L.size[l] = S[l];
         L.plane[l] = S[l] * S[l];
-        L.tile_begin[l] = tiles;
-        tiles += (3 * L.plane[l] + kYoloTile - 1) / kYoloTile;
+        tiles += (3 * L.plane[l] + kDecThreads - 1) / kDecThreads;
         L.box_begin[l] = static_cast<int>(boxes);
         boxes += 3 * L.plane[l];
-        L.vec4[l] = (L.plane[l] % 4 == 0 && (reinterpret_cast<uintptr_t>(maps[l]) & 15) == 0) ? 1 : 0;
         L.stride[l] = kStrides[l];
         for (int a = 0; a < 3; ++a) {
             L.anchor_w[l][a] = kAnchors[l][a][0];
@@ -431,7 +472,6 @@ static int yolo_levels(const float* map0, const float* map1, const float* map2, 
     }
     FB_REQUIRE(boxes * kYoloClasses < (1ll << 32), "yolo_decode: flat index exceeds 32 bits");
     FB_REQUIRE(static_cast<int64_t>(tiles) * batch < (1ll << 31), "yolo_decode: too many tiles");
-    L.tile_begin[3] = tiles;
     L.num_boxes = static_cast<int>(boxes);
     return FB_OK;
 }
@@ -441,18 +481,28 @@ static int launch_yolo_decode(const YoloDecodeArgs& a, int batch, bool pdl, cuda
     FB_REQUIRE(a.keys && a.counts, "yolo_decode: null pointer");
     FB_REQUIRE(a.capacity > 0, "yolo_decode: bad sizes");
     FB_REQUIRE(a.thr > 0.0f, "yolo_decode: score threshold must be positive (keys require positive scores)");
-    FB_REQUIRE((reinterpret_cast<uintptr_t>(a.boxes) & 15) == 0, "yolo_decode: boxes must be 16-byte aligned");
-    const dim3 grid(static_cast<unsigned>(a.L.tile_begin[3]) * static_cast<unsigned>(batch));
-    const bool dense = a.obj_out != nullptr || a.cls_out != nullptr;
-    const size_t smem = dense ? sizeof(float) * kYoloTile * kDenseRow : 0;
-    if (pdl) {
-        return dense ? launch_pdl(yolo_decode_kernel<true>, grid, dim3(kYoloTile), smem, st, "yolo_decode_kernel", a)
-                     : launch_pdl(yolo_decode_kernel<false>, grid, dim3(kYoloTile), smem, st, "yolo_decode_kernel", a);
+    FB_REQUIRE(((reinterpret_cast<uintptr_t>(a.boxes) | reinterpret_cast<uintptr_t>(a.cls_out)) & 15) == 0,
+               "yolo_decode: boxes and class scores must be 16-byte aligned");
+    auto tiles = [&](int slots) {
+        int n = 0;
+        for (int l = 0; l < 3; ++l) n += (3 * a.L.plane[l] + slots - 1) / slots;
+        return n * batch;
+    };
+    if (a.obj_out != nullptr || a.cls_out != nullptr) {
+        const size_t smem = sizeof(float) * kDecThreads * kDenseRow;
+        FB_TRY(check_cuda(cudaFuncSetAttribute(yolo_decode_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+                          "yolo_decode attr"));
+        return launch_after(yolo_decode_dense_kernel, dim3(static_cast<unsigned>(tiles(kDecThreads))), dim3(kDecThreads), smem, st, pdl,
+                            "yolo_decode_dense_kernel", a);
     }
-    if (dense) yolo_decode_kernel<true><<<grid, kYoloTile, smem, st>>>(a);
-    else yolo_decode_kernel<false><<<grid, kYoloTile, smem, st>>>(a);
-    count_launch();
-    return check_launch("yolo_decode_kernel");
+    // large tiles once they make four CTAs per SM
+    const int large = tiles(4 * kDecThreads);
+    auto run = [&](auto kernel, int n) {
+        return launch_after(kernel, dim3(static_cast<unsigned>(n)), dim3(kDecThreads), 0, st, pdl, "yolo_decode_kernel", a);
+    };
+    if (large >= 4 * kNumSMs) return a.boxes != nullptr ? run(yolo_decode_kernel<4, true>, large) : run(yolo_decode_kernel<4, false>, large);
+    const int small = tiles(kDecThreads);
+    return a.boxes != nullptr ? run(yolo_decode_kernel<1, true>, small) : run(yolo_decode_kernel<1, false>, small);
 }
 
 static inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }

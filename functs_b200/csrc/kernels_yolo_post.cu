@@ -171,13 +171,28 @@ __device__ __forceinline__ void post_pairs(const PostSmem& sm, int m, int reach,
         const int q1 = sm.cls_start[b + 1];
         if (b == label) q = p + 1;
         else if (end_x <= sm.cls_min_x[b] || end_y <= sm.cls_min_y[b]) continue;
-        for (; q < q1; ++q) {
-            const float4 c = sm.box.xy[q];
-            if (!(fminf(me.z, c.z) > fmaxf(me.x, c.x))) continue;
-            const NmsBox bj{c.x, c.y, c.z, c.w, sm.box.area[q]};
-            if (iou_exceeds(bi, bj, thr, thr_lo, thr_hi)) {
-                const int other = sm.box.rank[q];
-                pair(min(rank, other), max(rank, other));
+        // four tests at a time without branches: a pair can only exceed the threshold if its intersection reaches
+        // union * thr_lo (or a guard of iou_exceeds may be involved: wild values, which compare as "maybe")
+        for (; q < q1; q += 4) {
+            bool maybe[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int at = min(q + u, q1 - 1);
+                const float4 c = sm.box.xy[at];
+                const float w = __fsub_rn(fminf(me.z, c.z), fmaxf(me.x, c.x)), h = __fsub_rn(fminf(me.w, c.w), fmaxf(me.y, c.y));
+                const float inter = __fmul_rn(w, h), uni = __fsub_rn(__fadd_rn(bi.area, sm.box.area[at]), inter);
+                maybe[u] = q + u < q1 && w > 0.0f && h > 0.0f && !(inter < __fmul_rn(uni, thr_lo));
+            }
+            if (!(maybe[0] || maybe[1] || maybe[2] || maybe[3])) continue;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (!maybe[u]) continue;
+                const float4 c = sm.box.xy[q + u];
+                const NmsBox bj{c.x, c.y, c.z, c.w, sm.box.area[q + u]};
+                if (iou_exceeds(bi, bj, thr, thr_lo, thr_hi)) {
+                    const int other = sm.box.rank[q + u];
+                    pair(min(rank, other), max(rank, other));
+                }
             }
         }
     }
@@ -408,7 +423,7 @@ int launch_yolo_post(const YoloLevels& L, int batch, const YoloPostArgs& a, cuda
     FB_TRY(check_cuda(cudaFuncSetAttribute(yolo_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
                       "yolo_post attr"));
     const float thr_lo = a.iou_thr * (1.0f - 1.0e-6f), thr_hi = a.iou_thr * (1.0f + 1.0e-6f);
-    return launch_pdl(yolo_post_kernel, dim3(static_cast<unsigned>(batch)), dim3(kPostThreads), smem, st, "yolo_post_kernel", L, a, thr_lo,
+    return launch_after(yolo_post_kernel, dim3(static_cast<unsigned>(batch)), dim3(kPostThreads), smem, st, true, "yolo_post_kernel", L, a, thr_lo,
                       thr_hi);
 }
 

@@ -128,10 +128,20 @@ PYBIND11_MODULE(_C, m) {
               }
               return pairs(r.images);
           });
-    m.def("_yolo_detect", [](const std::vector<at::Tensor>& maps, double score_thr, int64_t topk, double iou_thr) {
+    m.def("_yolo_detect", [](std::vector<at::Tensor> maps, const std::vector<int64_t>& sizes, at::Device device, double score_thr,
+                             int64_t topk, double iou_thr) {
         functs_b200::YoloResult r;
         {
             py::gil_scoped_release release;
+            TORCH_CHECK_VALUE(maps.size() == 3 && sizes.size() == 3, "expected three [B, 255, S, S] maps");
+            for (size_t l = 0; l < 3; ++l) {
+                at::Tensor& t = maps[l];
+                TORCH_CHECK_VALUE(t.dim() == 4 && t.size(1) == 255, "expected three [B, 255, S, S] maps");
+                TORCH_CHECK_VALUE(t.size(2) == sizes[l] && t.size(3) == sizes[l], "map ", l, " is not of the configured size ", sizes[l]);
+                TORCH_CHECK_TYPE(t.scalar_type() == at::kFloat, "pred map must be float32");
+                if (t.device() != device) t = t.to(device, t.scalar_type(), /*non_blocking=*/true);
+                t = t.contiguous();
+            }
             r = functs_b200::yoloDetect(maps, score_thr, topk, iou_thr, /*dense=*/false, /*want_ids=*/false);
         }
         return pairs(r.images);

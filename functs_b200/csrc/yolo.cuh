@@ -12,15 +12,12 @@ namespace fb {
 
 constexpr int kYoloClasses = 80;
 constexpr int kYoloAttrib = 85;
-constexpr int kYoloTile = 128;  // (anchor, position) slots per tile: one per thread of a decode CTA
 
 struct YoloLevels {
     const float* map[3];  // [batch, 255, S, S]
     int size[3];          // S
     int plane[3];         // S * S
-    int tile_begin[4];    // first tile of every level inside an image, [3] = tiles per image
     int box_begin[3];     // first box index of every level inside an image
-    int vec4[3];          // the level's planes are 16-byte aligned: four slots per load
     float stride[3];
     float anchor_w[3][3];
     float anchor_h[3][3];
@@ -64,9 +61,9 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 #endif  // __CUDACC__
 
-// Host side: launch with the programmatic-serialization attribute.
+// Host side: a launch that may overlap the end of the kernel before it (pdl) or not.
 template <class... KP, class... A>
-inline int launch_pdl(void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const char* what, A... args) {
+inline int launch_after(void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const char* what, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -76,7 +73,7 @@ inline int launch_pdl(void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem,
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl ? 1 : 0;
     FB_TRY(check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<KP>(args)...), what));
     count_launch();
     return FB_OK;

@@ -21,6 +21,11 @@ def _dev(device) -> torch.device:
     return d
 
 
+def _index(d: torch.device) -> torch.device:
+    """The device that `d` means in this call ("cuda" follows the current one)."""
+    return d if d.index is not None else torch.device("cuda", torch.cuda.current_device())
+
+
 def _native():
     from . import _C  # built with the package; needed by whole calls only, so that the kernels import without it
     return _C
@@ -67,10 +72,9 @@ class YOLOV3BBox:
         return plan.dets, plan.labels, plan.flat_ids, plan.counts
 
     def __call__(self, pred_maps: List[torch.Tensor]) -> List[Tuple[torch.Tensor, torch.Tensor]]:
-        # launches, the wait for the counts and the per-image views in one native call
-        maps = self._checked(pred_maps)
+        # checks, launches, the wait for the counts and the per-image views in one native call
         before = launch_count()
-        out = _native()._yolo_detect(maps, self.score_thr, self.topk, self.iou_thr)
+        out = _native()._yolo_detect(pred_maps, self.sizes, _index(self.device), self.score_thr, self.topk, self.iou_thr)
         self.kernels_last_call = launch_count() - before
         return out
 
