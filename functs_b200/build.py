@@ -20,6 +20,7 @@ SOURCES = [
     "kernels_yolact.cu",
     "kernels_lstm.cu",
     "kernels_lstm_tc.cu",
+    "kernels_lstm_rec.cu",
     "no_alloc.cu",
     "kernels_generic.cu",
 ]

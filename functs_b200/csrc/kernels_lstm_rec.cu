@@ -1,0 +1,421 @@
+// C4, the recurrence: one thread-block cluster of 16 CTAs owns a few batch rows and runs all time steps on its own.
+//
+// The rows of a batch are independent, so nothing but the 16 CTAs that share a row's hidden state has to meet between steps: a
+// cluster barrier and stores into each other's shared memory replace a device-wide counter and a round trip of h through
+// global memory.  (One bulk copy per receiver with completion on its mbarrier instead of the stores and the barrier: 1.6 us per
+// step against 1.26 at one row of H = 256, the same at ten.)  Every cluster holds all of w_hh: a CTA owns H / 16 hidden units,
+// four gate columns each, 64 KB (H = 256) or 256 KB (H = 512) of weights, in registers as far as they go (32 or 64 per thread),
+// the rest in shared memory.
+// What bounds it at 64 rows is fp32 multiply-add issue: seven clusters fit the chip, ten rows each, 2.6 us of 128 FMA per
+// cycle and step; at one row the latency of a step: read the weights in shared memory, reduce, exchange.
+//
+// Thread layout: a thread multiplies two gate columns of one unit with KT consecutive k of every row, two k per packed instruction
+// (fma.rn.f32x2: one issue slot for two multiply-adds); a warp is 8 units x 2 gate pairs x 2 k-slices, the two slices are
+// summed by a shuffle that leaves one gate per lane, the warps' sums meet in shared memory, and one thread per (row, unit)
+// applies the gates, assigns hs[t] / cs[t] and stores h into the sixteen CTAs' next buffer.  (Four gate columns and half the k
+// per thread needs two passes over the rows, and the weights in shared memory are then read twice: 6.5 us per step at ten
+// rows of H = 512.  A register spill here goes to L2, shared memory being full: 14 us.)
+#include "common.cuh"
+
+namespace fb {
+
+constexpr int kRecCluster = 16;
+constexpr int kRecThreads = 512;
+constexpr int kRecUnitsPerWarp = 8;
+constexpr int kRecSlices = 2;  // k-slices inside a warp
+
+template <int H, int R>
+struct RecLayout {
+    static constexpr int U = H / kRecCluster;                       // units per CTA
+    static constexpr int WG = U / kRecUnitsPerWarp;                 // warps across the units
+    static constexpr int KQ = kRecThreads / 32 / WG;                // k-ranges across the warps
+    static constexpr int KT = H / KQ / kRecSlices;                  // k per thread
+    static constexpr int BP = R * U + 4;                            // a CTA's part of h, [R][U], and four floats (banks)
+    static constexpr int Quads = KT / 4;
+    static constexpr int RegQuads = Quads < 8 ? Quads : 8;          // k-quads whose weights live in registers
+    static constexpr int SmemQuads = Quads - RegQuads;
+    static constexpr size_t h_floats = 2ull * kRecCluster * BP;
+    static constexpr size_t part_floats = static_cast<size_t>(KQ) * R * 4 * U;
+    static constexpr size_t w_bytes = static_cast<size_t>(SmemQuads) * 2 * kRecThreads * 16;
+    static constexpr size_t bytes = w_bytes + (h_floats + part_floats) * 4;
+    static_assert(KT % U == 0, "a k-slice is whole parts of h");
+};
+
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float sum2(unsigned long long v) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    return __fadd_rn(lo, hi);
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void store_remote(uint32_t local_addr, uint32_t rank, float v) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// RP rows per pass (what the accumulators allow), NP passes: R = RP * NP rows per cluster.
+template <int H, int R>
+__global__ void __launch_bounds__(kRecThreads, 1)
+lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,
+                      float* __restrict__ cs) {
+    using Y = RecLayout<H, R>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemQuads][2][kRecThreads]
+    float* h_s = reinterpret_cast<float*>(smem_raw + Y::w_bytes);               // [2][16][BP]
+    float* part = h_s + Y::h_floats;                                            // [KQ][R][4][U]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = static_cast<int>(cluster_rank());
+    const int b0 = static_cast<int>(blockIdx.x / kRecCluster) * R;
+    const int unit = (warp % Y::WG) * kRecUnitsPerWarp + (lane & 7);            // of this CTA
+    const int gates = (lane >> 2) & 2;                                          // first of this thread's two gates
+    const int kq = warp / Y::WG, slice = kq * kRecSlices + (lane >> 4);         // k = slice * KT ...
+    const int j0 = rank * Y::U;
+
+    // resident weights: gate c, k -> w_hh[c][k][j0 + unit]
+    unsigned long long w_r[Y::RegQuads][2][2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const float* src = w_hh + (static_cast<int64_t>(gates + c) * H + slice * Y::KT) * H + j0 + unit;
+#pragma unroll
+        for (int q = 0; q < Y::Quads; ++q) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = __ldg(src + static_cast<int64_t>(4 * q + i) * H);
+            if (q < Y::RegQuads) {
+                w_r[q < Y::RegQuads ? q : 0][c][0] = pack2(v[0], v[1]);
+                w_r[q < Y::RegQuads ? q : 0][c][1] = pack2(v[2], v[3]);
+            } else {
+                w_s[((q - Y::RegQuads) * 2 + c) * kRecThreads + tid] = make_ulonglong2(pack2(v[0], v[1]), pack2(v[2], v[3]));
+            }
+        }
+    }
+    // one thread per (row, unit) of the CTA: gates, cell state, outputs
+    constexpr int kItems = R * Y::U;
+    static_assert(kItems <= kRecThreads, "one thread per item");
+    const bool item = tid < kItems;
+    const int ir = item ? tid / Y::U : 0, iu = tid % Y::U;
+    const int row = b0 + ir;
+    const bool live = item && row < B;
+    const int k_own = j0 + iu;                                                  // this item's place in a row of h
+    const uint32_t h_own = smem_u32(h_s + rank * Y::BP + ir * Y::U + iu);
+    float c_state = 0.0f;
+    float pre_g[4] = {0.f, 0.f, 0.f, 0.f};
+    if (live) {
+        const float* p = pre + static_cast<int64_t>(row) * (4 * H) + k_own;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) pre_g[g] = __ldg(p + g * H);
+    }
+    cluster_arrive();  // every CTA of the cluster runs before anybody stores into another one
+    cluster_wait();
+    for (int t = 0; t < T; ++t) {
+        float gate[4] = {pre_g[0], pre_g[1], pre_g[2], pre_g[3]};
+        if (t > 0) {
+            const float* h_t = h_s + ((t & 1) * kRecCluster + slice * (Y::KT / Y::U)) * Y::BP;
+            unsigned long long acc[2][R];
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[c][r] = 0ull;
+            auto quad = [&](const float* hq, const ulonglong2& w0, const ulonglong2& w1) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const ulonglong2 hv = *reinterpret_cast<const ulonglong2*>(hq + r * Y::U);
+                    acc[0][r] = fma2(hv.x, w0.x, acc[0][r]);
+                    acc[1][r] = fma2(hv.x, w1.x, acc[1][r]);
+                    acc[0][r] = fma2(hv.y, w0.y, acc[0][r]);
+                    acc[1][r] = fma2(hv.y, w1.y, acc[1][r]);
+                }
+            };
+#pragma unroll
+            for (int q = 0; q < Y::RegQuads; ++q)
+                quad(h_t + (4 * q / Y::U) * Y::BP + 4 * q % Y::U, make_ulonglong2(w_r[q][0][0], w_r[q][0][1]),
+                     make_ulonglong2(w_r[q][1][0], w_r[q][1][1]));
+#pragma unroll 2
+            for (int q = 0; q < Y::SmemQuads; ++q) {
+                const int k = 4 * (Y::RegQuads + q);
+                quad(h_t + (k / Y::U) * Y::BP + k % Y::U, w_s[(q * 2) * kRecThreads + tid], w_s[(q * 2 + 1) * kRecThreads + tid]);
+            }
+            // sum of the warp's two k-slices: afterwards a lane of the upper half holds its second gate, of the lower its first
+            const bool up = (lane & 16) != 0;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float v0 = sum2(acc[0][r]), v1 = sum2(acc[1][r]);
+                const float b = __fadd_rn(up ? v1 : v0, __shfl_xor_sync(kFullMask, up ? v0 : v1, 16));
+                part[((kq * R + r) * 4 + gates + (lane >> 4)) * Y::U + unit] = b;
+            }
+            __syncthreads();
+            if (item) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    float s = part[(ir * 4 + g) * Y::U + iu];
+#pragma unroll
+                    for (int k = 1; k < Y::KQ; ++k) s = __fadd_rn(s, part[((k * R + ir) * 4 + g) * Y::U + iu]);
+                    gate[g] = __fadd_rn(gate[g], s);
+                }
+            }
+        }
+        float hval = 0.0f;
+        if (item) {
+            const float ig = sigmoid_f32(gate[0]);
+            const float fg = sigmoid_f32(gate[1]);
+            const float gg = tanhf(gate[2]);
+            const float og = sigmoid_f32(gate[3]);
+            c_state = __fadd_rn(__fmul_rn(fg, c_state), __fmul_rn(ig, gg));
+            hval = __fmul_rn(og, tanhf(c_state));
+            if (t + 1 < T) {
+                const uint32_t dst = h_own + static_cast<uint32_t>(((t + 1) & 1) * (kRecCluster * Y::BP) * 4);
+#pragma unroll
+                for (int k = 0; k < kRecCluster; ++k) store_remote(dst, static_cast<uint32_t>(k), hval);
+            }
+        }
+        if (t + 1 < T) cluster_arrive();
+        if (live) {
+            const int64_t o = (static_cast<int64_t>(t) * B + row) * H + k_own;
+            hs[o] = hval;
+            cs[o] = c_state;
+            if (t + 1 < T) {
+                const float* p = pre + (static_cast<int64_t>(t + 1) * B + row) * (4 * H) + k_own;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) pre_g[g] = __ldg(p + g * H);
+            }
+        }
+        if (t + 1 < T) cluster_wait();
+    }
+}
+
+// ---- many rows per cluster ----
+// With more than a few rows the loads of h bound the kernel above: a 16-byte shared load fills 512 bytes of registers whatever
+// its lanes share, four cycles, and feeds two gate columns only (ten rows of H = 512: 6.7 us per step, 5.7 here).  Here 256 threads of
+// twice the registers take eight columns each, the four gates of two neighbouring units, packed by unit (a weight pair is
+// adjacent in memory; h is the same in both halves), so that a loaded word feeds eight multiply-adds.
+constexpr int kWideThreads = 256;
+
+template <int H, int R>
+struct WideLayout {
+    static constexpr int U = H / kRecCluster;                       // units per CTA
+    static constexpr int WG = U / 16;                               // warps across the units: 8 pairs per warp
+    static constexpr int KQ = kWideThreads / 32 / WG;               // k-ranges across the warps
+    static constexpr int KT = H / KQ / 4;                           // k per thread: four slices inside a warp
+    static constexpr int BP = R * U + 4;
+    static constexpr int RegK = KT <= 12 ? KT : 12;                 // k whose weights live in registers
+    static constexpr int SmemK = KT - RegK;
+    static constexpr size_t h_floats = 2ull * kRecCluster * BP;
+    static constexpr size_t part_floats = static_cast<size_t>(KQ) * R * 4 * U;
+    static constexpr size_t w_bytes = static_cast<size_t>(SmemK) * 2 * kWideThreads * 16;
+    static constexpr size_t bytes = w_bytes + (h_floats + part_floats) * 4;
+    static_assert(U % KT == 0 && RegK % 2 == 0 && SmemK % 2 == 0, "a k-slice lies inside one part of h");
+};
+
+template <int H, int R>
+__global__ void __launch_bounds__(kWideThreads, 1)
+lstm_recurrent_wide_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,
+                           float* __restrict__ cs) {
+    using Y = WideLayout<H, R>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemK][2][kWideThreads]
+    float* h_s = reinterpret_cast<float*>(smem_raw + Y::w_bytes);               // [2][16][BP]
+    float* part = h_s + Y::h_floats;                                            // [KQ][R][4][U]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = static_cast<int>(cluster_rank());
+    const int b0 = static_cast<int>(blockIdx.x / kRecCluster) * R;
+    const int unit = (warp % Y::WG) * 16 + 2 * (lane & 7);                      // first of this thread's two units
+    const int kq = warp / Y::WG, slice = kq * 4 + (lane >> 3);                  // k = slice * KT ...
+    const int j0 = rank * Y::U;
+
+    unsigned long long w_r[Y::RegK][4];
+#pragma unroll
+    for (int k = 0; k < Y::KT; ++k) {
+        unsigned long long v[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            v[c] = __ldg(reinterpret_cast<const unsigned long long*>(w_hh + (static_cast<int64_t>(c) * H + slice * Y::KT + k) * H + j0 + unit));
+        if (k < Y::RegK) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) w_r[k < Y::RegK ? k : 0][c] = v[c];
+        } else {
+            w_s[((k - Y::RegK) * 2) * kWideThreads + tid] = make_ulonglong2(v[0], v[1]);
+            w_s[((k - Y::RegK) * 2 + 1) * kWideThreads + tid] = make_ulonglong2(v[2], v[3]);
+        }
+    }
+    constexpr int kItems = R * Y::U;                                            // (row, unit) pairs of the CTA
+    constexpr int kPer = (kItems + kWideThreads - 1) / kWideThreads;
+    float c_state[kPer], pre_g[kPer][4];
+    auto fetch = [&](int t) {
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int i = q * kWideThreads + tid, row = b0 + i / Y::U;
+            if (i < kItems && row < B) {
+                const float* p = pre + (static_cast<int64_t>(t) * B + row) * (4 * H) + j0 + i % Y::U;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) pre_g[q][g] = __ldg(p + g * H);
+            }
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        c_state[q] = 0.0f;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) pre_g[q][g] = 0.0f;
+    }
+    fetch(0);
+    cluster_arrive();  // every CTA of the cluster runs before anybody stores into another one
+    cluster_wait();
+    for (int t = 0; t < T; ++t) {
+        if (t > 0) {
+            // slice s lies in the part of CTA s * KT / U
+            const float* h_t = h_s + ((t & 1) * kRecCluster + slice * Y::KT / Y::U) * Y::BP + slice * Y::KT % Y::U;
+            unsigned long long acc[4][R];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[c][r] = 0ull;
+            auto pair = [&](const float* hk, const unsigned long long (&w0)[4], const unsigned long long (&w1)[4]) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const float2 hv = *reinterpret_cast<const float2*>(hk + r * Y::U);
+                    const unsigned long long x = pack2(hv.x, hv.x), y = pack2(hv.y, hv.y);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[c][r] = fma2(x, w0[c], acc[c][r]);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[c][r] = fma2(y, w1[c], acc[c][r]);
+                }
+            };
+#pragma unroll
+            for (int k = 0; k < Y::RegK; k += 2) pair(h_t + k, w_r[k], w_r[k + 1 < Y::RegK ? k + 1 : k]);
+#pragma unroll 1
+            for (int k = 0; k < Y::SmemK; k += 2) {
+                const ulonglong2 a0 = w_s[(2 * k) * kWideThreads + tid], a1 = w_s[(2 * k + 1) * kWideThreads + tid];
+                const ulonglong2 b0_ = w_s[(2 * k + 2) * kWideThreads + tid], b1_ = w_s[(2 * k + 3) * kWideThreads + tid];
+                const unsigned long long w0[4] = {a0.x, a0.y, a1.x, a1.y}, w1[4] = {b0_.x, b0_.y, b1_.x, b1_.y};
+                pair(h_t + Y::RegK + k, w0, w1);
+            }
+            // sum over the warp's four k-slices: after the two exchanges lane group q holds gate q of both units
+            const bool up = (lane & 16) != 0, odd = (lane & 8) != 0;
+            auto other = [&](unsigned long long v, int mask) { return __shfl_xor_sync(kFullMask, v, mask); };
+            auto add2 = [&](unsigned long long a, unsigned long long b) {
+                unsigned long long d;
+                asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+                return d;
+            };
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                unsigned long long a[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) a[c] = add2(up ? acc[2 + c][r] : acc[c][r], other(up ? acc[c][r] : acc[2 + c][r], 16));
+                const unsigned long long s = add2(odd ? a[1] : a[0], other(odd ? a[0] : a[1], 8));
+                *reinterpret_cast<unsigned long long*>(part + ((kq * R + r) * 4 + (lane >> 3)) * Y::U + unit) = s;
+            }
+            __syncthreads();
+        }
+        float hval[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int i = q * kWideThreads + tid, ir = i / Y::U, iu = i % Y::U;
+            if (i >= kItems) continue;
+            float gate[4];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                gate[g] = pre_g[q][g];
+                if (t > 0) {
+                    float s = part[(ir * 4 + g) * Y::U + iu];
+#pragma unroll
+                    for (int k = 1; k < Y::KQ; ++k) s = __fadd_rn(s, part[((k * R + ir) * 4 + g) * Y::U + iu]);
+                    gate[g] = __fadd_rn(gate[g], s);
+                }
+            }
+            const float ig = sigmoid_f32(gate[0]);
+            const float fg = sigmoid_f32(gate[1]);
+            const float gg = tanhf(gate[2]);
+            const float og = sigmoid_f32(gate[3]);
+            c_state[q] = __fadd_rn(__fmul_rn(fg, c_state[q]), __fmul_rn(ig, gg));
+            hval[q] = __fmul_rn(og, tanhf(c_state[q]));
+            if (t + 1 < T) {
+                const uint32_t dst = smem_u32(h_s + (((t + 1) & 1) * kRecCluster + rank) * Y::BP + i);
+#pragma unroll
+                for (int k = 0; k < kRecCluster; ++k) store_remote(dst, static_cast<uint32_t>(k), hval[q]);
+            }
+        }
+        if (t + 1 < T) cluster_arrive();
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int i = q * kWideThreads + tid, row = b0 + i / Y::U;
+            if (i < kItems && row < B) {
+                const int64_t o = (static_cast<int64_t>(t) * B + row) * H + j0 + i % Y::U;
+                hs[o] = hval[q];
+                cs[o] = c_state[q];
+            }
+        }
+        if (t + 1 < T) {
+            fetch(t + 1);
+            cluster_wait();
+        }
+    }
+}
+
+template <class Kernel>
+static int launch_rec(Kernel kernel, int threads, size_t smem, int rows, const float* pre, const float* w_hh, int T, int B, float* hs,
+                      float* cs, cudaStream_t st) {
+    FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "lstm_recurrent attr"));
+    FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "lstm_recurrent attr"));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>((B + rows - 1) / rows) * kRecCluster);
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kRecCluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FB_TRY(check_cuda(cudaLaunchKernelEx(&cfg, kernel, pre, w_hh, T, B, hs, cs), "lstm_recurrent launch"));
+    count_launch();
+    return FB_OK;
+}
+template <int H, int R>
+static int launch_narrow(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, cudaStream_t st) {
+    static_assert(RecLayout<H, R>::bytes <= 227 * 1024, "shared memory of one CTA");
+    return launch_rec(lstm_recurrent_kernel<H, R>, kRecThreads, RecLayout<H, R>::bytes, R, pre, w_hh, T, B, hs, cs, st);
+}
+template <int H, int R>
+static int launch_wide(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, cudaStream_t st) {
+    static_assert(WideLayout<H, R>::bytes <= 227 * 1024, "shared memory of one CTA");
+    return launch_rec(lstm_recurrent_wide_kernel<H, R>, kWideThreads, WideLayout<H, R>::bytes, R, pre, w_hh, T, B, hs, cs, st);
+}
+
+// Rows per cluster: the fewest that let all clusters run at once (seven clusters of sixteen whole SMs fit a B200; more clusters
+// than that run one after the other).
+template <int H>
+static int launch_rec_rows(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, cudaStream_t st) {
+    constexpr int kClusters = 7;
+    if (B <= kClusters) return launch_narrow<H, 1>(pre, w_hh, T, B, hs, cs, st);
+    if (B <= 2 * kClusters) return launch_narrow<H, 2>(pre, w_hh, T, B, hs, cs, st);
+    if (B <= 4 * kClusters) return launch_wide<H, 4>(pre, w_hh, T, B, hs, cs, st);
+    if (B <= 6 * kClusters) return launch_wide<H, 6>(pre, w_hh, T, B, hs, cs, st);
+    if (B <= 8 * kClusters) return launch_wide<H, 8>(pre, w_hh, T, B, hs, cs, st);
+    return launch_wide<H, 10>(pre, w_hh, T, B, hs, cs, st);
+}
+
+int launch_lstm_recurrent(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, cudaStream_t st) {
+    FB_REQUIRE(H == 256 || H == 512, "lstm recurrence: hidden size %d not supported (256 or 512)", H);
+    return H == 512 ? launch_rec_rows<512>(pre, w_hh, T, B, hs, cs, st) : launch_rec_rows<256>(pre, w_hh, T, B, hs, cs, st);
+}
+
+}  // namespace fb

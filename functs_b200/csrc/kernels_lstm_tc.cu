@@ -1,19 +1,22 @@
 // C4, launch 1 on the tensor cores: the hoisted LSTM input projection
 //     pre[m, g*H + j] = sum_k x[m, k] * w_ih[g, k, j] + b_ih[g, j] + b_hh[g, j]          (m = t*B + b)
 // as a tcgen05 GEMM with fp32-level accuracy.  fp32 operands do not fit the tensor core's TF32 inputs (10 mantissa
-// bits), so every operand is split into hi = tf32(v) and lo = tf32(v - hi) and three products are accumulated in
-// the fp32 TMEM accumulator: lo*hi + hi*lo + hi*hi (the dropped lo*lo term is ~2^-22 relative).
+// bits), so every operand is split into hi = tf32(v) and lo = tf32(v - hi) (24 bits together) and three products are
+// accumulated in fp32: lo*hi + hi*lo + hi*hi.  The tensor core truncates when it accumulates, so the long sum is spread over
+// four TMEM accumulators: hi*hi of every third k-tile in three of them, the small cross products in the fourth; they are
+// added with rounding at the end (max |h - h64| at T = 64: see tests).
 //
-// Two kernels:
-//   lstm_tc_split_kernel  writes the split operands PRE-TILED: every [128 rows x 32 k] tile is stored contiguously
-//                         in the no-swizzle K-major core-matrix order the MMA reads from shared memory
-//                         (8 rows x 16 bytes per core matrix; K-adjacent core matrices 128 B apart, 8-row groups
-//                         1024 B apart).  A tile therefore reaches shared memory with ONE bulk (TMA, untiled) copy.
-//   lstm_tc_gemm_kernel   one CTA per 128 x 128 output tile, warp-specialised: warp 0 issues the bulk copies into a
-//                         3-stage ring, warp 1 owns TMEM and issues tcgen05.mma (one elected lane), warps 2-5 read
-//                         the accumulator back with tcgen05.ld, add the biases and store.
+// One CTA per 128 x 128 output tile, any M and K (rows and columns beyond them are zeros).  Small products: three groups of four
+// warps take k-tiles in turn: load a [128 x 32] tile of x and of w_ih into registers, split it, store hi and lo to a
+// 3-stage ring in the no-swizzle K-major core-matrix order the MMA reads (8 rows x 16 bytes per core matrix; K-adjacent core
+// matrices 128 B apart, 8-row groups 1024 B apart); the last warp owns TMEM and issues tcgen05.mma (one elected lane).
+// Large products: lstm_tc_split_kernel writes the tiles once and one thread fetches them with bulk copies.
+// What bounds the large ones: L2 -> SM operand traffic (64 KB per k-tile and CTA, 512 MB at T = B = 64, H = 512) ahead of
+// 3 x 8.6 GFLOP on the TF32 pipe (33 us at the measured 776 TFLOP/s).
 // Every mbarrier wait is bounded; a wait that runs out sets FB_STATUS_WAIT_TIMEOUT, and all roles fall through to
 // the common teardown (TMEM is always released).
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace fb {
@@ -22,7 +25,11 @@ constexpr int kTcBM = 128, kTcBN = 128, kTcBK = 32;
 constexpr int kTcTileBytes = kTcBM * kTcBK * 4;   // 16 KB: one hi or lo tile
 constexpr int kTcStageBytes = 4 * kTcTileBytes;   // A_hi, A_lo, B_hi, B_lo
 constexpr int kTcStages = 3;
-constexpr int kTcThreads = 192;
+constexpr int kTcLoaders = 128;                   // threads per loader group, one k-tile at a time
+constexpr int kTcGroups = kTcStages;              // one per stage, so that a group waits for its own stage only (in order)
+constexpr int kTcThreads = kTcGroups * kTcLoaders + 32;
+constexpr int kTcMmaWarp = kTcGroups * kTcLoaders / 32;
+constexpr int kTcAccums = 4;                      // of 128 TMEM columns
 constexpr uint32_t kTcWaitLimit = 2000000u;
 
 __device__ __forceinline__ float tf32_round(float x) {
@@ -33,50 +40,6 @@ __device__ __forceinline__ float tf32_round(float x) {
 
 // byte offset of element (r, c) inside a pre-tiled [128 x 32] fp32 tile
 __device__ __forceinline__ int tile_offset(int r, int c) { return (r >> 3) * 1024 + (c >> 2) * 128 + (r & 7) * 16 + (c & 3) * 4; }
-
-// a_tiles: [M/128][K/32][hi, lo][16 KB];  b_tiles: [4H/128][K/32][hi, lo][16 KB]
-__global__ void __launch_bounds__(256)
-lstm_tc_split_kernel(const float* __restrict__ x, const float* __restrict__ w_ih, int M, int K, int H,
-                     unsigned char* __restrict__ a_tiles, unsigned char* __restrict__ b_tiles) {
-    const int kchunks = K / 4;
-    const int64_t a_items = static_cast<int64_t>(M) * kchunks;
-    const int64_t b_items = static_cast<int64_t>(4 * H) * kchunks;
-    const int KT = K / kTcBK;
-    const int64_t gstride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < a_items + b_items; e += gstride) {
-        float v[4];
-        int r, c;
-        unsigned char* tile;
-        if (e < a_items) {
-            // consecutive threads: consecutive 16-byte chunks of one row of x (coalesced reads)
-            r = static_cast<int>(e / kchunks);
-            c = static_cast<int>(e - static_cast<int64_t>(r) * kchunks) * 4;
-            const float4 q = __ldg(reinterpret_cast<const float4*>(x + static_cast<int64_t>(r) * K + c));
-            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-            tile = a_tiles + (static_cast<int64_t>(r / kTcBM) * KT + c / kTcBK) * (2 * kTcTileBytes);
-        } else {
-            // consecutive threads: consecutive output columns n = g*H + j for one k-chunk (coalesced reads of w_ih rows)
-            const int64_t f = e - a_items;
-            const int kc = static_cast<int>(f / (4 * H));
-            r = static_cast<int>(f - static_cast<int64_t>(kc) * (4 * H));  // n
-            c = kc * 4;
-            const int g = r / H, j = r - g * H;
-            const float* src = w_ih + (static_cast<int64_t>(g) * K + c) * H + j;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] = __ldg(src + static_cast<int64_t>(i) * H);
-            tile = b_tiles + (static_cast<int64_t>(r / kTcBN) * KT + c / kTcBK) * (2 * kTcTileBytes);
-        }
-        float hi[4], lo[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            hi[i] = tf32_round(v[i]);
-            lo[i] = tf32_round(__fsub_rn(v[i], hi[i]));
-        }
-        const int off = tile_offset(r % kTcBM, c % kTcBK);
-        *reinterpret_cast<float4*>(tile + off) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<float4*>(tile + kTcTileBytes + off) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-    }
-}
 
 // ---- tcgen05 helpers ----------------------------------------------------------------------------------------
 // Shared-memory matrix descriptor, no swizzle, K-major: start address, leading-dimension byte offset (between core
@@ -131,30 +94,91 @@ struct TcShared {
     volatile int abort_flag;
 };
 
-// grid = (4H / 128, M / 128).  dynamic smem: kTcStages * 64 KB of operand tiles (1024-byte aligned) + TcShared.
+// fp32 -> nearest TF32 value, ties away from zero, as cvt.rna.tf32 rounds, in two integer operations (the conversion unit takes
+// a quarter of the rate, and a k-tile has 16384 of them)
+__device__ __forceinline__ float tf32_nearest(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+
+// Four fp32 values -> their hi and lo parts, stored at `off` of the hi tile and of the lo tile behind it.
+__device__ __forceinline__ void tc_store_split(unsigned char* tile, int off, const float (&v)[4]) {
+    float hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        hi[i] = tf32_nearest(v[i]);
+        lo[i] = tf32_nearest(__fsub_rn(v[i], hi[i]));
+    }
+    *reinterpret_cast<float4*>(tile + off) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<float4*>(tile + kTcTileBytes + off) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+}
+
+// The operands split once for all CTAs, tiles in the order the MMA reads, so that a tile reaches shared memory with one bulk
+// copy.  a_tiles: [ceil(M/128)][ceil(K/32)][hi, lo][16 KB];  b_tiles: [4H/128][ceil(K/32)][hi, lo][16 KB].
+// Rows beyond M and columns beyond K are zeros.
+__global__ void __launch_bounds__(256)
+lstm_tc_split_kernel(const float* __restrict__ x, const float* __restrict__ w_ih, int M, int K, int H, int vec_x,
+                     unsigned char* __restrict__ a_tiles, unsigned char* __restrict__ b_tiles) {
+    const int KT = (K + kTcBK - 1) / kTcBK, kchunks = KT * (kTcBK / 4);
+    const int rows = (M + kTcBM - 1) / kTcBM * kTcBM;
+    const int64_t a_items = static_cast<int64_t>(rows) * kchunks;
+    const int64_t b_items = static_cast<int64_t>(4 * H) * kchunks;
+    const int64_t gstride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < a_items + b_items; e += gstride) {
+        float v[4];
+        int r, c;
+        unsigned char* tile;
+        if (e < a_items) {
+            // consecutive threads: consecutive 16-byte chunks of one row of x (coalesced reads)
+            r = static_cast<int>(e / kchunks);
+            c = static_cast<int>(e - static_cast<int64_t>(r) * kchunks) * 4;
+            const float* src = x + static_cast<int64_t>(r) * K + c;
+            if (vec_x && r < M && c + 4 <= K) {
+                const float4 q = __ldg(reinterpret_cast<const float4*>(src));
+                v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = r < M && c + i < K ? __ldg(src + i) : 0.0f;
+            }
+            tile = a_tiles + (static_cast<int64_t>(r / kTcBM) * KT + c / kTcBK) * (2 * kTcTileBytes);
+        } else {
+            // consecutive threads: consecutive output columns n = g*H + j for one k-chunk (coalesced reads of w_ih rows)
+            const int64_t f = e - a_items;
+            const int kc = static_cast<int>(f / (4 * H));
+            r = static_cast<int>(f - static_cast<int64_t>(kc) * (4 * H));  // n
+            c = kc * 4;
+            const int g = r / H, j = r - g * H;
+            const float* src = w_ih + (static_cast<int64_t>(g) * K + c) * H + j;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = c + i < K ? __ldg(src + static_cast<int64_t>(i) * H) : 0.0f;
+            tile = b_tiles + (static_cast<int64_t>(r / kTcBN) * KT + c / kTcBK) * (2 * kTcTileBytes);
+        }
+        tc_store_split(tile, tile_offset(r % kTcBM, c % kTcBK), v);
+    }
+}
+
+// grid = (4H / 128, ceil(M / 128)).  dynamic smem: kTcStages * 64 KB of operand tiles (1024-byte aligned) + TcShared.
+// PRESPLIT: x and w_ih are the tiles of lstm_tc_split_kernel.
+template <bool PRESPLIT>
 __global__ void __launch_bounds__(kTcThreads, 1)
-lstm_tc_gemm_kernel(const unsigned char* __restrict__ a_tiles, const unsigned char* __restrict__ b_tiles,
-                    const float* __restrict__ b_ih, const float* __restrict__ b_hh, int K, int H, float* __restrict__ pre,
-                    int32_t* status) {
+lstm_tc_gemm_kernel(const float* __restrict__ x, const float* __restrict__ w_ih, const float* __restrict__ b_ih,
+                    const float* __restrict__ b_hh, int M, int K, int H, int vec_x, float* __restrict__ pre, int32_t* status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* tiles = smem_raw;
     TcShared& sh = *reinterpret_cast<TcShared*>(smem_raw + kTcStages * kTcStageBytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int KT = K / kTcBK;
+    const int KT = (K + kTcBK - 1) / kTcBK;
     const int nt = blockIdx.x, mt = blockIdx.y;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kTcStages; ++s) {
-            mbar_init(&sh.full[s], 1);
+            mbar_init(&sh.full[s], PRESPLIT ? 1 : kTcLoaders / 32);
             mbar_init(&sh.empty[s], 1);
         }
         mbar_init(&sh.accum, 1);
         sh.abort_flag = 0;
         fence_barrier_init();
     }
-    if (warp == 1) {
-        // 128 fp32 accumulator columns; the allocating warp also frees them at the end
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(128u)
+    if (warp == kTcMmaWarp) {
+        // all 512 TMEM columns: four accumulators; the allocating warp also frees them at the end
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -163,10 +187,10 @@ lstm_tc_gemm_kernel(const unsigned char* __restrict__ a_tiles, const unsigned ch
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
 
-    if (warp == 0) {
+    if (PRESPLIT && warp == 0) {
         if (lane == 0) {
-            const unsigned char* a_src = a_tiles + static_cast<int64_t>(mt) * KT * (2 * kTcTileBytes);
-            const unsigned char* b_src = b_tiles + static_cast<int64_t>(nt) * KT * (2 * kTcTileBytes);
+            const unsigned char* a_src = reinterpret_cast<const unsigned char*>(x) + static_cast<int64_t>(mt) * KT * (2 * kTcTileBytes);
+            const unsigned char* b_src = reinterpret_cast<const unsigned char*>(w_ih) + static_cast<int64_t>(nt) * KT * (2 * kTcTileBytes);
             for (int kt = 0; kt < KT; ++kt) {
                 const int s = kt % kTcStages;
                 const uint32_t par = ((kt / kTcStages) & 1) ^ 1;  // passes at once on a fresh barrier
@@ -186,47 +210,109 @@ lstm_tc_gemm_kernel(const unsigned char* __restrict__ a_tiles, const unsigned ch
                               &sh.full[s]);
             }
         }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            // descriptor strides of the pre-tiled layout (tile_offset): core matrices adjacent in K are 128 bytes apart
-            // (leading-dimension offset), 8-row groups 1024 bytes apart (stride-dimension offset)
-            constexpr uint32_t lbo = 128u, sbo = 1024u;
-            uint32_t accumulate = 0;
-            bool failed = false;
-            for (int kt = 0; kt < KT && !failed; ++kt) {
-                const int s = kt % kTcStages;
-                const uint32_t par = (kt / kTcStages) & 1;
-                bool ok = false;
-                for (uint32_t it = 0; it < kTcWaitLimit && !sh.abort_flag; ++it) {
-                    if (mbar_try_wait(&sh.full[s], par)) { ok = true; break; }
-                }
-                if (!ok) {
-                    sh.abort_flag = 1;
-                    if (status != nullptr) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
-                    failed = true;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t a_hi = smem_u32(tiles + s * kTcStageBytes);
-                const uint32_t a_lo = a_hi + kTcTileBytes;
-                const uint32_t b_hi = a_hi + 2 * kTcTileBytes;
-                const uint32_t b_lo = a_hi + 3 * kTcTileBytes;
+    } else if (!PRESPLIT && warp < kTcMmaWarp) {
+        // ---- loaders: group g takes the k-tiles g, g + kTcGroups, ... ----
+        const int group = warp >> 2, gw = warp & 3;
+        const int g = nt * kTcBN / H, j0 = nt * kTcBN - g * H;  // a tile lies inside one gate because H % 128 == 0
+        const float* __restrict__ wg = w_ih + static_cast<int64_t>(g) * K * H + j0;
+        float a[8][4], b[8][4];
+        // x: a warp covers 8 rows x 4 chunks of 16 bytes (whole sectors; the eight lanes of a store phase share a chunk column
+        // and write 128 contiguous bytes); w_ih: 32 neighbouring columns, four k each
+        const float* xq = x + static_cast<int64_t>(mt * kTcBM + gw * 32 + (lane & 7)) * K + (lane >> 3) * 4;
+        const float* wq = wg + static_cast<int64_t>(gw * 8) * H + lane;
+        const bool inner = vec_x && (mt + 1) * kTcBM <= M;
+        auto load = [&](int kt) {
+            if (inner && (kt + 1) * kTcBK <= K) {  // a whole tile: no bounds to check
 #pragma unroll
-                for (int kk = 0; kk < kTcBK / 8; ++kk) {
-                    const uint32_t ko = kk * 256;  // 8 k-elements = two core matrices of 128 bytes
-                    const uint64_t dah = make_smem_desc(a_hi + ko, lbo, sbo), dal = make_smem_desc(a_lo + ko, lbo, sbo);
-                    const uint64_t dbh = make_smem_desc(b_hi + ko, lbo, sbo), dbl = make_smem_desc(b_lo + ko, lbo, sbo);
-                    tc_mma_tf32(tmem, dal, dbh, accumulate);
-                    accumulate = 1;
-                    tc_mma_tf32(tmem, dah, dbl, 1);
-                    tc_mma_tf32(tmem, dah, dbh, 1);
+                for (int q = 0; q < 8; ++q) {
+                    const float4 v = __ldg(reinterpret_cast<const float4*>(xq + kt * kTcBK + (q >> 1) * 8 * K + (q & 1) * 16));
+                    a[q][0] = v.x; a[q][1] = v.y; a[q][2] = v.z; a[q][3] = v.w;
                 }
-                tc_commit(&sh.empty[s]);  // the stage is free once these MMAs have read it
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) b[q][i] = __ldg(wq + (kt * kTcBK + (q & 1) * 4 + i) * H + (q >> 1) * 32);
+                return;
             }
-            if (!failed) tc_commit(&sh.accum);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int r = mt * kTcBM + gw * 32 + (q >> 1) * 8 + (lane & 7), c = kt * kTcBK + ((q & 1) * 4 + (lane >> 3)) * 4;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[q][i] = r < M && c + i < K ? __ldg(x + static_cast<int64_t>(r) * K + c + i) : 0.0f;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int c = kt * kTcBK + (gw * 2 + (q & 1)) * 4;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) b[q][i] = c + i < K ? __ldg(wg + static_cast<int64_t>(c + i) * H + (q >> 1) * 32 + lane) : 0.0f;
+            }
+        };
+        if (group < KT) load(group);
+        for (int kt = group; kt < KT; kt += kTcGroups) {
+            const int s = kt % kTcStages;
+            const uint32_t par = ((kt / kTcStages) & 1) ^ 1;  // passes at once on a fresh barrier
+            bool ok = false;
+            for (uint32_t it = 0; it < kTcWaitLimit && !sh.abort_flag; ++it) {
+                if (mbar_try_wait(&sh.empty[s], par)) { ok = true; break; }
+            }
+            if (!__all_sync(kFullMask, ok)) {
+                sh.abort_flag = 1;
+                if (lane == 0 && status != nullptr) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
+                break;
+            }
+            unsigned char* stage = tiles + s * kTcStageBytes;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                tc_store_split(stage, tile_offset(gw * 32 + (q >> 1) * 8 + (lane & 7), ((q & 1) * 4 + (lane >> 3)) * 4), a[q]);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                tc_store_split(stage + 2 * kTcTileBytes, tile_offset((q >> 1) * 32 + lane, (gw * 2 + (q & 1)) * 4), b[q]);
+            fence_proxy_async();  // the tensor core reads the tiles through the async proxy
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.full[s]);
+            if (kt + kTcGroups < KT) load(kt + kTcGroups);
         }
-    } else {
-        // epilogue warps 2..5: TMEM lane quadrant = warp % 4
+    } else if (warp == kTcMmaWarp && lane == 0) {
+        // ---- MMA issue ----
+        // descriptor strides of the tile layout (tile_offset): core matrices adjacent in K are 128 bytes apart
+        // (leading-dimension offset), 8-row groups 1024 bytes apart (stride-dimension offset)
+        constexpr uint32_t lbo = 128u, sbo = 1024u;
+        bool failed = false;
+        for (int kt = 0; kt < KT && !failed; ++kt) {
+            const int s = kt % kTcStages;
+            const uint32_t par = (kt / kTcStages) & 1;
+            bool ok = false;
+            for (uint32_t it = 0; it < kTcWaitLimit && !sh.abort_flag; ++it) {
+                if (mbar_try_wait(&sh.full[s], par)) { ok = true; break; }
+            }
+            if (!ok) {
+                sh.abort_flag = 1;
+                if (status != nullptr) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
+                failed = true;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t a_hi = smem_u32(tiles + s * kTcStageBytes);
+            const uint32_t a_lo = a_hi + kTcTileBytes;
+            const uint32_t b_hi = a_hi + 2 * kTcTileBytes;
+            const uint32_t b_lo = a_hi + 3 * kTcTileBytes;
+            const uint32_t d_main = tmem + static_cast<uint32_t>(kt % (kTcAccums - 1)) * kTcBN, d_cross = tmem + (kTcAccums - 1) * kTcBN;
+#pragma unroll
+            for (int kk = 0; kk < kTcBK / 8; ++kk) {
+                const uint32_t ko = kk * 256;  // 8 k-elements = two core matrices of 128 bytes
+                const uint64_t dah = make_smem_desc(a_hi + ko, lbo, sbo), dal = make_smem_desc(a_lo + ko, lbo, sbo);
+                const uint64_t dbh = make_smem_desc(b_hi + ko, lbo, sbo), dbl = make_smem_desc(b_lo + ko, lbo, sbo);
+                tc_mma_tf32(d_cross, dal, dbh, kt > 0 || kk > 0 ? 1u : 0u);
+                tc_mma_tf32(d_cross, dah, dbl, 1);
+                tc_mma_tf32(d_main, dah, dbh, kt >= kTcAccums - 1 || kk > 0 ? 1u : 0u);
+            }
+            tc_commit(&sh.empty[s]);  // the stage is free once these MMAs have read it
+        }
+        if (!failed) tc_commit(&sh.accum);
+    }
+    if (warp < kTcMmaWarp) {
+        // ---- epilogue: TMEM lane quadrant = warp % 4, 32 columns at a time ----
+        __syncwarp();
         bool ok = false;
         for (uint32_t it = 0; it < kTcWaitLimit && !sh.abort_flag; ++it) {
             if (mbar_try_wait(&sh.accum, 0)) { ok = true; break; }
@@ -236,23 +322,32 @@ lstm_tc_gemm_kernel(const unsigned char* __restrict__ a_tiles, const unsigned ch
             tc_fence_after();
             const int q = warp & 3;
             const int m = mt * kTcBM + q * 32 + lane;
-            const int n0 = nt * kTcBN;  // column in [0, 4H); a tile lies inside one gate because H % 128 == 0
+            const int n0 = nt * kTcBN;  // column in [0, 4H)
+            const uint32_t lanes = tmem + (static_cast<uint32_t>(q * 32) << 16);
+            const int mains = KT < kTcAccums - 1 ? KT : kTcAccums - 1;
             float* orow = pre + static_cast<int64_t>(m) * (4 * H) + n0;
 #pragma unroll 1
-            for (int cb = 0; cb < kTcBN / 32; ++cb) {
-                float acc[32];
-                tc_ld_32cols(tmem + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(cb * 32), acc);
+            for (int cb = warp >> 2; cb < kTcBN / 32; cb += kTcGroups) {
+                float acc[32], more[32];
+                tc_ld_32cols(lanes + static_cast<uint32_t>((kTcAccums - 1) * kTcBN + cb * 32), acc);
+                for (int d = mains - 1; d >= 0; --d) {
+                    tc_ld_32cols(lanes + static_cast<uint32_t>(d * kTcBN + cb * 32), more);
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    const int n = n0 + cb * 32 + i;
-                    const float4 bi = __ldg(reinterpret_cast<const float4*>(b_ih + n));
-                    const float4 bh = __ldg(reinterpret_cast<const float4*>(b_hh + n));
-                    float4 o;
-                    o.x = __fadd_rn(acc[i + 0], __fadd_rn(bi.x, bh.x));
-                    o.y = __fadd_rn(acc[i + 1], __fadd_rn(bi.y, bh.y));
-                    o.z = __fadd_rn(acc[i + 2], __fadd_rn(bi.z, bh.z));
-                    o.w = __fadd_rn(acc[i + 3], __fadd_rn(bi.w, bh.w));
-                    *reinterpret_cast<float4*>(orow + cb * 32 + i) = o;
+                    for (int i = 0; i < 32; ++i) acc[i] = __fadd_rn(acc[i], more[i]);
+                }
+                if (m < M) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) {
+                        const int n = n0 + cb * 32 + i;
+                        const float4 bi = __ldg(reinterpret_cast<const float4*>(b_ih + n));
+                        const float4 bh = __ldg(reinterpret_cast<const float4*>(b_hh + n));
+                        float4 o;
+                        o.x = __fadd_rn(acc[i + 0], __fadd_rn(bi.x, bh.x));
+                        o.y = __fadd_rn(acc[i + 1], __fadd_rn(bi.y, bh.y));
+                        o.z = __fadd_rn(acc[i + 2], __fadd_rn(bi.z, bh.z));
+                        o.w = __fadd_rn(acc[i + 3], __fadd_rn(bi.w, bh.w));
+                        *reinterpret_cast<float4*>(orow + cb * 32 + i) = o;
+                    }
                 }
             }
         } else if (lane == 0 && status != nullptr) {
@@ -262,16 +357,17 @@ lstm_tc_gemm_kernel(const unsigned char* __restrict__ a_tiles, const unsigned ch
     // ---- teardown: everybody meets, then the allocating warp frees TMEM ----
     tc_fence_before();
     __syncthreads();
-    if (sh.abort_flag && threadIdx.x == 0) {
+    if (PRESPLIT && sh.abort_flag && threadIdx.x == 0) {
         // give bulk copies that are still in flight time to land before the CTA's shared memory is released
         const unsigned long long t0 = clock64();
         while (clock64() - t0 < 400000ull) {
         }
     }
     __syncthreads();
-    if (warp == 1) {
+    if (warp == kTcMmaWarp) {
+        __syncwarp();
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
 }
 
@@ -590,38 +686,44 @@ int launch_lstm_recurrent_tc(const float* pre, const float* w_hh, int T, int B, 
     return check_launch("lstm_recurrent_tc_kernel");
 }
 
-bool lstm_tc_supported(int M, int K, int H) {
-    return M > 0 && K > 0 && H > 0 && (M % kTcBM) == 0 && (K % kTcBK) == 0 && (H % kTcBN) == 0;
-}
+bool lstm_tc_supported(int M, int K, int H) { return M > 0 && K > 0 && H > 0 && (H % kTcBN) == 0; }
+
+// More output tiles than SMs: split the operands once (every x tile is read by 4H / 128 CTAs, every w_ih tile by M / 128).  At
+// T = B = 64, H = 512 that is 10 + 64 us against 105 us with the split inside; with one wave of CTAs or less the extra launch
+// and the trip through memory cost more than they save (20 us against 27 at M = 64, H = 256).
+static bool tc_presplit(int M, int H) { return static_cast<int64_t>(4 * H / kTcBN) * ((M + kTcBM - 1) / kTcBM) > kNumSMs; }
 
 int64_t lstm_tc_scratch_bytes(int M, int K, int H) {
-    if (!lstm_tc_supported(M, K, H)) return 0;
-    const int64_t a = static_cast<int64_t>(M / kTcBM) * (K / kTcBK) * 2 * kTcTileBytes;
-    const int64_t b = static_cast<int64_t>(4 * H / kTcBN) * (K / kTcBK) * 2 * kTcTileBytes;
-    return a + b;
+    if (!lstm_tc_supported(M, K, H) || !tc_presplit(M, H)) return 0;
+    const int64_t KT = (K + kTcBK - 1) / kTcBK;
+    return ((M + kTcBM - 1) / kTcBM + 4 * H / kTcBN) * KT * 2 * kTcTileBytes;
 }
 
 int launch_lstm_input_proj_tc(const float* x, const float* w_ih, const float* b_ih, const float* b_hh, int M, int K,
                               int H, float* pre, void* tc_scratch, int32_t* status, cudaStream_t st) {
     FB_REQUIRE(lstm_tc_supported(M, K, H), "lstm tensor-core projection: shape not supported");
-    FB_REQUIRE(tc_scratch != nullptr && (reinterpret_cast<uintptr_t>(tc_scratch) & 255) == 0 &&
-                   (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(b_ih) & 15) == 0 &&
-                   (reinterpret_cast<uintptr_t>(b_hh) & 15) == 0 && (reinterpret_cast<uintptr_t>(pre) & 15) == 0,
+    FB_REQUIRE((reinterpret_cast<uintptr_t>(b_ih) & 15) == 0 && (reinterpret_cast<uintptr_t>(b_hh) & 15) == 0 &&
+                   (reinterpret_cast<uintptr_t>(pre) & 15) == 0 && (reinterpret_cast<uintptr_t>(tc_scratch) & 255) == 0,
                "lstm tensor-core projection: misaligned pointer");
-    unsigned char* a_tiles = static_cast<unsigned char*>(tc_scratch);
-    unsigned char* b_tiles = a_tiles + static_cast<int64_t>(M / kTcBM) * (K / kTcBK) * 2 * kTcTileBytes;
-    const int64_t items = (static_cast<int64_t>(M) + 4 * H) * (K / 4);
-    int blocks = static_cast<int>((items + 255) / 256);
-    if (blocks > kNumSMs * 8) blocks = kNumSMs * 8;
-    lstm_tc_split_kernel<<<blocks, 256, 0, st>>>(x, w_ih, M, K, H, a_tiles, b_tiles);
-    count_launch();
-    FB_TRY(check_launch("lstm_tc_split_kernel"));
     const size_t smem = static_cast<size_t>(kTcStages) * kTcStageBytes + sizeof(TcShared) + 1024;
-    FB_TRY(check_cuda(cudaFuncSetAttribute(lstm_tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(smem)),
-                      "lstm_tc_gemm attr"));
-    dim3 grid(4 * H / kTcBN, M / kTcBM);
-    lstm_tc_gemm_kernel<<<grid, kTcThreads, smem, st>>>(a_tiles, b_tiles, b_ih, b_hh, K, H, pre, status);
+    const int vec_x = K % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? 1 : 0;
+    dim3 grid(4 * H / kTcBN, (M + kTcBM - 1) / kTcBM);
+    const bool presplit = tc_presplit(M, H);
+    auto kernel = presplit ? lstm_tc_gemm_kernel<true> : lstm_tc_gemm_kernel<false>;
+    if (presplit) {
+        const int KT = (K + kTcBK - 1) / kTcBK;
+        unsigned char* a_tiles = static_cast<unsigned char*>(tc_scratch);
+        unsigned char* b_tiles = a_tiles + static_cast<int64_t>(grid.y) * KT * 2 * kTcTileBytes;
+        const int64_t items = (static_cast<int64_t>(grid.y) * kTcBM + 4 * H) * KT * (kTcBK / 4);
+        const int blocks = static_cast<int>(std::min<int64_t>((items + 255) / 256, kNumSMs * 8));
+        lstm_tc_split_kernel<<<blocks, 256, 0, st>>>(x, w_ih, M, K, H, vec_x, a_tiles, b_tiles);
+        count_launch();
+        FB_TRY(check_launch("lstm_tc_split_kernel"));
+        x = reinterpret_cast<const float*>(a_tiles);
+        w_ih = reinterpret_cast<const float*>(b_tiles);
+    }
+    FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "lstm_tc_gemm attr"));
+    kernel<<<grid, kTcThreads, smem, st>>>(x, w_ih, b_ih, b_hh, M, K, H, vec_x, pre, status);
     count_launch();
     return check_launch("lstm_tc_gemm_kernel");
 }

@@ -136,7 +136,7 @@ class SSDBBox:
 
 
 class LSTM:
-    """One-layer LSTM with per-step outputs written by slice assignment (hs[t] = h, cs[t] = c).  2 launches (3 when the tensor-core projection runs: operand split, GEMM, recurrence)."""
+    """One-layer LSTM with per-step outputs written by slice assignment (hs[t] = h, cs[t] = c).  2 or 3 launches."""
 
     def __init__(self, w_ih: torch.Tensor, w_hh: torch.Tensor, b_ih: torch.Tensor, b_hh: torch.Tensor, device="cuda"):
         self.device = _dev(device)
@@ -151,10 +151,10 @@ class LSTM:
 
     @staticmethod
     def expected_launches(seq_len: int, batch: int, hidden: int, mode: int = 0) -> int:
-        """Kernel launches of one call: operand split + tensor-core projection + recurrence, or (mode 1, or a shape the
-        tensor-core projection does not take) CUDA-core projection + recurrence.  The recurrence is one launch in every
-        mode."""
-        return 3 if (mode != 1 and (seq_len * batch) % 128 == 0 and hidden % 128 == 0) else 2
+        """Kernel launches of one call: the input projection of all steps and the recurrence; a projection of more 128 x 128
+        tiles than the GPU has SMs splits its operands first (not in mode 1, which does not use the tensor cores for it)."""
+        tiles = -(-seq_len * batch // 128) * (4 * hidden // 128)
+        return 3 if mode != 1 and tiles > 148 else 2
 
     def forward_device(self, x: torch.Tensor, mode: int = 0):
         """x on the device; outputs and scratch are reused across calls; no synchronisation."""

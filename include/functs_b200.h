@@ -217,8 +217,8 @@ int functs_b200_ragged_pack(const float* dets, const int64_t* labels, const int6
 /* Follows functs/benchmark/ai_model/lstm/lstm.py:79-98, 118-133 (one layer; hs[t] = h, cs[t] = c kept).
  * x [T, B, I]; w_ih [4, I, H]; w_hh [4, H, H]; b_ih, b_hh [4, H]; hs, cs [T, B, H]; gate order i, f, g, o;
  * h0 = c0 = 0.  scratch: functs_b200_lstm_scratch_bytes(T, B, I, H).
- * Three launches: operand split + pre-tiling, the hoisted input projection (tcgen05, 3xTF32), and one persistent
- * recurrent kernel. */
+ * Two launches: the hoisted input projection (tcgen05, 3xTF32; large ones split their operands in a launch of their own first)
+ * and the recurrence (clusters of 16 CTAs, a few batch rows each). */
 int64_t functs_b200_lstm_scratch_bytes(int32_t seq_len, int32_t batch, int32_t input, int32_t hidden);
 int functs_b200_lstm_forward(const float* x, const float* w_ih, const float* w_hh, const float* b_ih,
                              const float* b_hh, int32_t seq_len, int32_t batch, int32_t input, int32_t hidden,
