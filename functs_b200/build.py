@@ -18,11 +18,13 @@ SOURCES = [
     "kernels_yolo_post.cu",
     "kernels_ssd.cu",
     "kernels_yolact.cu",
+    "kernels_yolact_tc.cu",
     "kernels_lstm.cu",
     "kernels_lstm_tc.cu",
     "kernels_lstm_rec.cu",
     "no_alloc.cu",
     "kernels_generic.cu",
+    "kernels_region.cu",
 ]
 
 NVCC_FLAGS = [

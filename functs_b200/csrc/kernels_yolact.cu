@@ -10,7 +10,7 @@
 // warp broadcasts.
 #include <cmath>
 
-#include "common.cuh"
+#include "yolact.cuh"
 
 namespace fb {
 
@@ -18,16 +18,6 @@ constexpr int kYolactThreads = 128;
 constexpr int kYolactK = 32;
 constexpr int kYolactMaxDet = 256;
 constexpr int kYolactTileW = 16, kYolactTileH = 4;  // pixels per warp tile: 8 lanes x 2 pixels wide, 4 rows
-
-// sanitize_coordinates (yolact_mask.py:327-333) followed by "col >= x1 and col < x2" as integer bounds.
-__device__ __forceinline__ void crop_range(float a, float b, int size, int& lo, int& hi) {
-    float x1 = fminf(a, b);
-    float x2 = fmaxf(x1, b);
-    x1 = fmaxf(__fsub_rn(x1, 1.0f), 0.0f);
-    x2 = fminf(__fadd_rn(x2, 1.0f), static_cast<float>(size));
-    lo = static_cast<int>(ceilf(x1));
-    hi = static_cast<int>(ceilf(x2));
-}
 
 // sigmoid(v) > thr.  Outside [v_lo, v_hi] (a band around logit(thr) that is far wider than the rounding of the fp32
 // sigmoid) the answer is known from v alone; inside it the fp32 sigmoid is formed and compared, so the result is
@@ -55,8 +45,8 @@ yolact_masks_kernel(const float* __restrict__ proto, const float* __restrict__ c
         for (int d = t; d < num_det; d += kYolactThreads) {
             const float4 bx = __ldg(reinterpret_cast<const float4*>(boxes) + static_cast<int64_t>(img) * num_det + d);
             int xs, xe, ys, ye;
-            crop_range(bx.x, bx.z, width, xs, xe);
-            crop_range(bx.y, bx.w, height, ys, ye);
+            yolact_crop_range(bx.x, bx.z, width, xs, xe);
+            yolact_crop_range(bx.y, bx.w, height, ys, ye);
             s_bounds[d] = make_int4(xs, xe, ys, ye);
         }
     }

@@ -19,9 +19,12 @@
 #include <torch/csrc/jit/ir/constants.h>
 #include <torch/csrc/jit/ir/ir.h>
 
+#include <algorithm>
+#include <array>
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <numeric>
 #include <unordered_map>
 
 #include "../../../include/functs_b200.h"
@@ -829,56 +832,224 @@ struct Emitter {
     }
 };
 
+// ---- cutting a program into regions without branches ------------------------------------------------------------------
+
+struct Progression {  // coordinates start, start + step, ... of one dimension: all of them take the same path
+    int64_t start = 0, step = 1, count = 0;
+};
+
+// The coordinates of dimension `dim` as progressions on which no test of that dimension changes its outcome: the bounds of
+// the tests cut the extent into intervals, and inside an interval the strided tests repeat with the product of their
+// steps, so each residue class is a progression.
+bool cutDimension(const functs_b200_gprogram& P, const std::vector<int>& tests, int dim, std::vector<Progression>& out) {
+    const int64_t extent = P.shape[dim];
+    std::vector<int64_t> edge{0, extent};
+    for (int k : tests) {
+        const functs_b200_gpred& q = P.pred[k];
+        const int64_t mul = q.coef[dim];
+        if (mul <= 0) return false;
+        for (int64_t bound : {static_cast<int64_t>(q.lo) - q.add, static_cast<int64_t>(q.hi) - q.add}) {  // first x with mul * x >= bound
+            const int64_t x = bound <= 0 ? 0 : (bound + mul - 1) / mul;
+            if (x > 0 && x < extent) edge.push_back(x);
+        }
+    }
+    std::sort(edge.begin(), edge.end());
+    edge.erase(std::unique(edge.begin(), edge.end()), edge.end());
+    for (size_t e = 0; e + 1 < edge.size(); ++e) {
+        const int64_t a = edge[e], b = edge[e + 1];
+        int64_t period = 1;
+        for (int k : tests) {
+            const functs_b200_gpred& q = P.pred[k];
+            const int64_t v = static_cast<int64_t>(q.coef[dim]) * a + q.add;
+            if (q.step > 1 && v >= q.lo && v < q.hi) period = std::lcm(period, q.step / std::gcd<int64_t, int64_t>(q.step, q.coef[dim]));
+            if (period > FB_R_MAX_REGIONS) return false;
+        }
+        for (int64_t r = 0; r < period && a + r < b; ++r) out.push_back({a + r, period, (b - a - r + period - 1) / period});
+        if (out.size() > FB_R_MAX_REGIONS) return false;
+    }
+    return true;
+}
+
+// Rewrites P (dimensions in the output's order) as regions; false when it does not fit the format (the branching kernel
+// then serves it): too many regions, or a division that is not exact along a progression.
+bool cutIntoRegions(const functs_b200_gprogram& P, functs_b200_rprogram& R) {
+    const int rank = P.rank;
+    std::vector<std::vector<int>> tests(8);
+    for (int pc = 0; pc < P.ninstr; ++pc) {
+        if (P.instr[pc].op != FB_G_COND) continue;
+        const int k = P.instr[pc].arg;
+        for (int d = 0; d < rank; ++d)
+            if (P.pred[k].coef[d] != 0) tests[d].push_back(k);
+    }
+    std::vector<std::vector<Progression>> parts(rank);
+    int64_t regions = 1;
+    for (int d = 0; d < rank; ++d) {
+        if (!cutDimension(P, tests[d], d, parts[d])) return false;
+        regions *= static_cast<int64_t>(parts[d].size());
+        if (regions > FB_R_MAX_REGIONS) return false;
+    }
+    int64_t stride[8], run = 1;
+    for (int d = rank - 1; d >= 0; --d) {
+        stride[d] = run;
+        run *= P.shape[d];
+    }
+    std::memset(&R, 0, sizeof(R));
+    R.num_regions = static_cast<int32_t>(regions);
+    R.out_dtype = P.out_dtype;
+    R.numel = P.numel;
+    for (int64_t r = 0; r < regions; ++r) {
+        functs_b200_region& G = R.region[r];
+        std::vector<Progression> x(rank);
+        int64_t rest = r, base = 0, count = 1;
+        for (int d = rank - 1; d >= 0; --d) {
+            x[d] = parts[d][static_cast<size_t>(rest % static_cast<int64_t>(parts[d].size()))];
+            rest /= static_cast<int64_t>(parts[d].size());
+            base += x[d].start * stride[d];
+            count *= x[d].count;
+        }
+        G.count = static_cast<int32_t>(count);
+        G.out_base = static_cast<int32_t>(base);
+        G.first_instr = R.num_instr;
+        G.first_load = R.num_loads;
+        // the path this region takes; a load's coefficients over all output dimensions for now
+        int slot_of[FB_G_MAX_LOADS];
+        for (int& s : slot_of) s = -1;
+        std::vector<std::array<int64_t, 8>> coef;
+        for (int pc = 0;; ++pc) {
+            functs_b200_ginstr I = P.instr[pc];
+            if (I.op == FB_G_COND) {
+                const functs_b200_gpred& q = P.pred[I.arg];
+                int64_t c = q.add;
+                for (int d = 0; d < rank; ++d) c += q.coef[d] * x[d].start;
+                const bool ok = c >= q.lo && c < q.hi && (q.step <= 1 || (c - q.lo) % q.step == 0);
+                if (!ok) pc = I.imm.i - 1;
+                continue;
+            }
+            if (I.op == FB_G_JUMP) {
+                pc = I.arg - 1;
+                continue;
+            }
+            if (I.op == FB_G_LOAD) {
+                int& slot = slot_of[I.arg];
+                if (slot < 0) {
+                    const functs_b200_gload& L = P.load[I.arg];
+                    std::array<int64_t, 8> cf{};
+                    int64_t at = L.base;
+                    if (L.general == 0) {
+                        for (int d = 0; d < rank; ++d) {
+                            at += L.coef[d] * x[d].start;
+                            cf[d] = L.coef[d] * x[d].step;
+                        }
+                    } else {
+                        for (int t = 0; t < L.nterms; ++t) {
+                            const functs_b200_gterm& T = L.term[t];
+                            const int64_t first = T.add + (T.dim >= 0 ? T.mul * x[T.dim].start : 0);
+                            const int64_t step = T.dim >= 0 && x[T.dim].count > 1 ? T.mul * x[T.dim].step : 0;
+                            if (first % T.div != 0 || step % T.div != 0) return false;
+                            at += first / T.div * T.stride;
+                            if (T.dim >= 0) cf[T.dim] += step / T.div * T.stride;
+                        }
+                    }
+                    if (R.num_loads >= FB_R_MAX_LOADS || G.num_loads >= FB_R_REGION_LOADS) return false;
+                    slot = R.num_loads++;
+                    ++G.num_loads;
+                    R.load[slot].tensor = L.tensor;
+                    R.load[slot].dtype = L.dtype;
+                    R.load[slot].base = static_cast<int32_t>(at);
+                    coef.push_back(cf);
+                }
+                I.arg = static_cast<uint16_t>(slot);
+            }
+            if (R.num_instr >= FB_R_MAX_INSTR) return false;
+            R.instr[R.num_instr++] = I;
+            if (I.op == FB_G_END) break;
+        }
+        // dimensions of more than one element, neighbours merged where the output and every load walk them as one
+        int n = 0;
+        for (int d = 0; d < rank; ++d) {
+            if (x[d].count == 1) continue;
+            const int64_t oc = stride[d] * x[d].step;
+            bool merge = n > 0 && G.out_coef[n - 1] == oc * x[d].count;
+            for (int l = 0; l < G.num_loads && merge; ++l) merge = R.load[G.first_load + l].coef[n - 1] == coef[l][d] * x[d].count;
+            if (!merge) {
+                if (n == 4) return false;
+                G.shape[n++] = 1;
+            }
+            G.shape[n - 1] *= static_cast<int32_t>(x[d].count);
+            G.out_coef[n - 1] = static_cast<int32_t>(oc);
+            for (int l = 0; l < G.num_loads; ++l) R.load[G.first_load + l].coef[n - 1] = static_cast<int32_t>(coef[l][d]);
+        }
+        if (n == 0) G.shape[n++] = 1;
+        G.rank = n;
+        for (int k = 0; k < n; ++k) divisorOf(static_cast<uint32_t>(G.shape[k]), G.div_magic[k], G.div_shift[k]);
+    }
+    // do the regions interleave?
+    bool inter = regions > 1 && regions <= 8 && P.out_dtype == 0;
+    std::vector<bool> seen(static_cast<size_t>(regions), false);
+    for (int64_t r = 0; r < regions && inter; ++r) {
+        const functs_b200_region& G = R.region[r];
+        int64_t want = regions;
+        for (int k = G.rank - 1; k >= 0; --k) {
+            inter = inter && (G.shape[k] == 1 || G.out_coef[k] == want);
+            want *= G.shape[k];
+        }
+        inter = inter && G.count == R.region[0].count && G.out_base < regions && !seen[static_cast<size_t>(G.out_base)];
+        if (inter) seen[static_cast<size_t>(G.out_base)] = true;
+    }
+    R.interleave = inter ? static_cast<int32_t>(regions) : 1;
+    return true;
+}
+
 }  // namespace
 
 // What a call leaves behind for the next one: the flattened programs and, for every tensor slot of every program, where
 // the tensor came from.  key describes everything the programs depend on (shapes, dtypes, devices, scalar values).
-struct GenericPlan {
-    std::mutex mu;
-    bool valid = false;
+struct BuiltPrograms {
     std::string key;
     std::vector<functs_b200_gprogram> progs;                  // iterations x outputs (ninstr == 0: an empty output)
     std::vector<std::vector<std::pair<int, int>>> sources;    // per iteration
     std::vector<std::vector<int64_t>> out_shape;              // per program
     int32_t max_numel = 0;
+    bool regions = false;                                     // a single program without branches left: `cut` replaces it
+    functs_b200_rprogram cut;
+};
+struct GenericPlan {
+    std::mutex mu;
+    std::shared_ptr<const BuiltPrograms> built;
 };
 std::shared_ptr<GenericPlan> NewGenericPlan() { return std::make_shared<GenericPlan>(); }
 
 namespace {
 
+void put64(std::string& k, int64_t v) { k.append(reinterpret_cast<const char*>(&v), sizeof(v)); }
+
 void describe(const c10::IValue& iv, std::string& k) {
     if (iv.isTensor()) {
         const at::Tensor& t = iv.toTensor();
         k += 'T';
-        k += std::to_string(static_cast<int>(t.scalar_type()));
-        k += t.is_cuda() ? 'c' : 'h';
-        k += std::to_string(t.is_cuda() ? t.get_device() : -1);
-        for (int64_t d : t.sizes()) {
-            k += ',';
-            k += std::to_string(d);
-        }
-        k += ';';
+        k += static_cast<char>(t.scalar_type());
+        k += static_cast<char>(t.is_cuda() ? t.get_device() : -1);
+        k += static_cast<char>(t.dim());
+        for (int64_t d : t.sizes()) put64(k, d);
     } else if (iv.isDouble()) {
         const double d = iv.toDouble();
-        uint64_t bits;
+        int64_t bits;
         std::memcpy(&bits, &d, 8);
         k += 'D';
-        k += std::to_string(bits);
-        k += ';';
+        put64(k, bits);
     } else if (iv.isInt()) {
         k += 'I';
-        k += std::to_string(iv.toInt());
-        k += ';';
+        put64(k, iv.toInt());
     } else if (iv.isBool()) {
-        k += iv.toBool() ? "B1;" : "B0;";
+        k += iv.toBool() ? 'B' : 'b';
     } else if (iv.isNone()) {
-        k += "N;";
+        k += 'N';
     } else if (iv.isList()) {
         k += '[';
+        put64(k, static_cast<int64_t>(iv.toListRef().size()));
         for (const c10::IValue& e : iv.toListRef()) describe(e, k);
-        k += ']';
     } else {
-        k += "?;";  // the builder refuses such an input anyway
+        k += '?';  // the builder refuses such an input anyway
     }
 }
 
@@ -888,10 +1059,32 @@ at::Tensor sourceTensor(const std::vector<c10::IValue>& inputs, const std::pair<
     return iv.toListRef().at(static_cast<size_t>(src.second)).toTensor();
 }
 
+// one program cut into regions: allocates the output, points the program at this call's tensors and launches
+void launchRegions(const BuiltPrograms& built, const std::vector<c10::IValue>& inputs, std::vector<c10::IValue>& outputs) {
+    functs_b200_rprogram R = built.cut;
+    at::Tensor ins[FB_G_MAX_INPUTS];
+    const auto& src = built.sources[0];
+    for (size_t k = 0; k < src.size(); ++k) {
+        ins[k] = sourceTensor(inputs, src[k]).contiguous();
+        R.in_ptr[k] = ins[k].data_ptr();
+    }
+    c10::cuda::CUDAGuard guard(ins[0].device());
+    at::Tensor out = at::empty(built.out_shape[0], ins[0].options().dtype(R.out_dtype == 1 ? at::kBool : at::kFloat));
+    R.out_ptr = out.data_ptr();
+    const int rc = functs_b200_region_group_launch(&R, at::cuda::getCurrentCUDAStream().stream());
+    TORCH_CHECK(rc == FB_OK, "functs_b200 generic group: ", functs_b200_last_error());
+    outputs.clear();
+    outputs.emplace_back(std::move(out));
+}
+
 // allocates the outputs, points the programs at this call's tensors and launches
-void launchPrograms(std::vector<functs_b200_gprogram> progs, const std::vector<std::vector<std::pair<int, int>>>& sources,
-                    const std::vector<std::vector<int64_t>>& out_shape, int32_t max_numel, size_t n_out, bool is_map,
-                    const std::vector<c10::IValue>& inputs, std::vector<c10::IValue>& outputs) {
+void launchPrograms(const BuiltPrograms& built, size_t n_out, bool is_map, const std::vector<c10::IValue>& inputs,
+                    std::vector<c10::IValue>& outputs) {
+    if (built.regions) return launchRegions(built, inputs, outputs);
+    std::vector<functs_b200_gprogram> progs = built.progs;
+    const auto& sources = built.sources;
+    const auto& out_shape = built.out_shape;
+    const int32_t max_numel = built.max_numel;
     const size_t iters = progs.size() / n_out;
     std::vector<std::vector<at::Tensor>> results(n_out);
     std::vector<at::Tensor> keep_alive;
@@ -960,27 +1153,29 @@ bool RunGenericGroup(const std::shared_ptr<Graph>& sub, bool is_map, int64_t deg
     std::string key;
     if (plan != nullptr) {
         key.reserve(256);
-        key += std::to_string(degree);
-        key += '|';
+        put64(key, degree);
         for (const c10::IValue& iv : inputs) describe(iv, key);
-        std::unique_lock<std::mutex> lock(plan->mu);
-        if (plan->valid && plan->key == key) {
+        std::shared_ptr<const BuiltPrograms> built;
+        {
+            std::lock_guard<std::mutex> lock(plan->mu);
+            built = plan->built;
+        }
+        if (built && built->key == key) {
             // same shapes, dtypes, devices and scalars as the call that built the programs: only the pointers change
-            auto progs = plan->progs;
-            auto sources = plan->sources;
-            auto out_shape = plan->out_shape;
-            const int32_t max_numel = plan->max_numel;
-            lock.unlock();
-            launchPrograms(std::move(progs), sources, out_shape, max_numel, n_out, is_map, inputs, outputs);
+            launchPrograms(*built, n_out, is_map, inputs, outputs);
             return true;
         }
     }
     try {
         const int64_t iters = is_map ? degree : 1;
         G_REQUIRE(iters >= 1 && iters * static_cast<int64_t>(n_out) <= 4096, "too many programs");
-        std::vector<functs_b200_gprogram> progs(static_cast<size_t>(iters) * n_out);
-        std::vector<std::vector<std::pair<int, int>>> sources(static_cast<size_t>(iters));
-        std::vector<std::vector<int64_t>> out_shape(progs.size());
+        auto fresh = std::make_shared<BuiltPrograms>();
+        auto& progs = fresh->progs;
+        auto& sources = fresh->sources;
+        auto& out_shape = fresh->out_shape;
+        progs.resize(static_cast<size_t>(iters) * n_out);
+        sources.resize(static_cast<size_t>(iters));
+        out_shape.resize(progs.size());
         c10::Device device(c10::kCPU);
         bool have_device = false;
         int32_t max_numel = 0;
@@ -1043,21 +1238,22 @@ bool RunGenericGroup(const std::shared_ptr<Graph>& sub, bool is_map, int64_t deg
                 }
                 em.emit(e, id);
                 em.push(FB_G_END);
+                if (progs.size() == 1 && !is_map && cutIntoRegions(P, fresh->cut)) {
+                    fresh->regions = true;
+                    continue;
+                }
                 orderDimensionsForLanes(P);
                 max_numel = std::max(max_numel, P.work);
             }
             sources[static_cast<size_t>(it)] = b.sources;
         }
+        fresh->key = key;
+        fresh->max_numel = max_numel;
+        launchPrograms(*fresh, n_out, is_map, inputs, outputs);
         if (plan != nullptr) {
             std::lock_guard<std::mutex> lock(plan->mu);
-            plan->key = key;
-            plan->progs = progs;
-            plan->sources = sources;
-            plan->out_shape = out_shape;
-            plan->max_numel = max_numel;
-            plan->valid = true;
+            plan->built = std::move(fresh);
         }
-        launchPrograms(std::move(progs), sources, out_shape, max_numel, n_out, is_map, inputs, outputs);
         return true;
     } catch (const Unsupported& u) {
         if (why != nullptr) *why = u.what();

@@ -366,6 +366,43 @@ typedef struct {
 int functs_b200_generic_group_launch(const functs_b200_gprogram* programs, int32_t count, int32_t max_work,
                                      int32_t max_rank, int32_t on_device, void* stream);
 
+/* The same for one program whose COND tests can be resolved on the host: every tested dimension of the output is cut into
+ * arithmetic progressions of coordinates that take the same path, so that the output falls apart into regions (boxes of
+ * such progressions) whose programs have no branch left and whose loads are all linear; neighbouring dimensions that
+ * every load and the output walk alike are merged.  A region's element number is decomposed over `shape` (last dimension
+ * fastest); load l reads in_ptr[tensor][base + sum_k coef[k] * y[k]], the result goes to out_base + sum_k out_coef[k] * y[k].
+ * interleave = R > 1: the R regions have the same count and element i of a region lies at out_base + R * i, so that together
+ * they tile the output with stride R: a CTA then computes all R for its elements and stores whole runs. */
+#define FB_R_MAX_REGIONS 16
+#define FB_R_MAX_INSTR 384
+#define FB_R_MAX_LOADS 96
+#define FB_R_REGION_LOADS 24
+typedef struct {
+    int32_t tensor, dtype, base;
+    int32_t coef[4];
+} functs_b200_rload;
+typedef struct {
+    int32_t rank, count; /* rank <= 4 */
+    int32_t shape[4];
+    uint32_t div_magic[4], div_shift[4];
+    int32_t out_base, out_coef[4];
+    int32_t first_instr; /* straight-line instructions (LOAD: arg = place in load[]) up to END */
+    int32_t first_load, num_loads;
+} functs_b200_region;
+typedef struct {
+    int32_t num_regions, interleave;
+    int32_t out_dtype; /* as in functs_b200_gprogram */
+    int32_t numel;     /* of the output */
+    int32_t num_instr, num_loads;
+    const void* in_ptr[FB_G_MAX_INPUTS];
+    void* out_ptr;
+    functs_b200_region region[FB_R_MAX_REGIONS];
+    functs_b200_ginstr instr[FB_R_MAX_INSTR];
+    functs_b200_rload load[FB_R_MAX_LOADS];
+} functs_b200_rprogram;
+/* program in HOST memory (it travels as a kernel parameter).  One launch. */
+int functs_b200_region_group_launch(const functs_b200_rprogram* program, void* stream);
+
 /* ---- group registry: what the tssa::ParallelFunctor operator binds to ------------------------ */
 /* The reference registers one JIT operator whose Operation runs a compiled group
  * (fait/passes/te_op.cpp:238-249).  Here a group is found by a canonical signature string and launched with

@@ -193,3 +193,33 @@ def test_four_elements_per_thread_with_divided_coordinates(env):
     x = torch.randn(4099, 96, generator=g).cuda()
     y = torch.randn(96, generator=g).cuda()
     check(env, strided_big, (x, y))
+
+
+def class_deltas(boxes: torch.Tensor, deltas: torch.Tensor):
+    w = boxes[:, 2] - boxes[:, 0]
+    out = deltas.clone()
+    out[:, 0::4] = deltas[:, 1::4] * w[:, None]
+    out[:, 1:40:4] = torch.exp(deltas[:, 0:39:4])
+    out[:, 3] = deltas[:, 2]
+    return out
+
+
+def bands(x: torch.Tensor):
+    t = x.clone()
+    for k in range(6):
+        t[:, k] = t[:, k] + float(k)
+    return t > 0.5
+
+
+@pytest.mark.parametrize("fn,shape", [
+    (scaled, (1, 1)), (scaled, (1024, 1184)), (scaled, (1025, 1185)),
+    (normalize, (1, 1, 3)), (normalize, (319, 317, 3)), (normalize, (317, 1283, 3)),
+    (class_deltas, (7, 44)), (class_deltas, (4099, 84)), (bands, (33, 40)), (bands, (5003, 64)),
+])
+def test_programs_cut_into_regions(env, fn, shape):
+    """Regions that interleave and regions that do not, on both sides of the size where a thread takes several elements, with
+    remainders of its block, one or two dimensions per region, and a bool output."""
+    g = torch.Generator().manual_seed(14)
+    x = torch.randn(*shape, generator=g).cuda()
+    args = {scaled: (x, 0.75), class_deltas: (torch.randn(shape[0], 4, generator=g).cuda(), x)}.get(fn, (x,))
+    check(env, fn, args)
