@@ -147,6 +147,11 @@ int functs_b200_yolact_masks(const float* proto, const float* coef, const float*
         v_lo = -INFINITY;
         v_hi = INFINITY;
     }
+    // without the logits the dot products go to the tensor cores, unless the threshold is so extreme that no band around its
+    // logit is known (then every logit would have to be formed twice)
+    if (logits_out == nullptr && v_lo > -INFINITY) {
+        return launch_yolact_masks_tc(proto, coef, boxes, batch, height, width, num_det, thr, masks, as_stream(stream));
+    }
     const int tiles_x = (width + kYolactTileW - 1) / kYolactTileW;
     const int tiles_y = (height + kYolactTileH - 1) / kYolactTileH;
     const int num_tiles = tiles_x * tiles_y;

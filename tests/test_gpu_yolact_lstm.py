@@ -179,3 +179,25 @@ def test_lstm_rejects_unsupported_hidden(fb):
     x, w_ih, w_hh, b_ih, b_hh = W.make_lstm_inputs(2, 2, 64)
     with pytest.raises(fb.FunctsB200Error):
         fb.workloads.LSTM(w_ih, w_hh, b_ih, b_hh)(x)
+
+
+@pytest.mark.parametrize("batch,height,width,dets,thr", [
+    (1, 1, 2, 1, 0.5), (3, 5, 6, 33, 0.5), (2, 69, 70, 100, 0.3), (1, 138, 138, 16, 0.9), (5, 37, 130, 256, 0.5),
+    (70, 33, 34, 129, 0.001), (2, 64, 64, 32, 0.9995),
+])
+def test_yolact_masks_on_the_tensor_cores(fb, batch, height, width, dets, thr):
+    """Against the variant that forms every logit in fp32, byte for byte: planes that start off a word, tiles of many rows, one
+    to 256 detections, logits at and around the threshold, and values that are not finite."""
+    g = torch.Generator().manual_seed(batch + dets)
+    proto = torch.randn(batch, height, width, 32, generator=g)
+    coef = torch.tanh(torch.randn(batch, dets, 32, generator=g))
+    xy = torch.rand(batch, dets, 4, generator=g) * torch.tensor([width, height, width, height], dtype=torch.float32)
+    coef[:, ::5] *= 1e-5
+    proto[:, ::3, :, 7] = float("inf")
+    proto[:, -1, ::4] = float("nan")
+    proto[:, 0, 1::2] = 0.0
+    if batch == 3:
+        coef[1, 0, 3] = float("nan")
+    args = (proto.cuda(), coef.cuda(), xy.cuda(), thr)
+    masks, _ = fb.ops.yolact_masks(*args, with_logits=True)
+    assert torch.equal(fb.ops.yolact_masks(*args), masks)
