@@ -16,8 +16,10 @@
 //     pixels and 100 detections, 141 us; issue was the bound.)
 //   - A CTA of four warps walks neighbouring tiles of 128 pixels of one image; four CTAs per SM (128 TMEM columns each) overlap
 //     one another's loads, products and stores.
-// B = 64, 138 x 138, 100 detections: 104 us (2.7 TB/s) against 145 for the exact kernel; 8 x 276 x 276: 57 against 78; one image: 12
-// against 25.
+//     (Two warps per 32 pixels, each with half of the detections: 115 us, what both have to do costs more than more warps bring.
+//     TF32 operands, copied to shared memory unsplit, leave 1 in 100 logits open: 105 us.)
+// B = 64, 138 x 138, 100 detections: 95 us (3.0 TB/s) against 145 for the exact kernel; 8 x 276 x 276: 51 against 78; one image: 12
+// against 25.  What bounds it is issue, 1150 instructions per 32 pixels, with the 16 warps per SM that TMEM leaves room for.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -51,13 +53,18 @@ __device__ __forceinline__ void yt_store_split(unsigned char* tile, int row, int
 }
 
 // 32 rows of 32 floats, loaded by one warp: lane -> (row = (lane / 2) % 8 of eight, 32-byte piece lane / 16 of 64 bytes, half), so
-// that a load takes whole sectors and the eight rows of a store fill all banks.
-__device__ __forceinline__ void yt_load(const float* __restrict__ base, int64_t first, int64_t rows, int lane, float4 (&v)[8]) {
-    const int r = (lane >> 1) & 7, c = (lane >> 4) * 8 + (lane & 1) * 4;
+// that a load takes whole sectors and the eight rows of a store fill all banks.  (base: the first row; rows: how many there are)
+__device__ __forceinline__ void yt_load(const float* __restrict__ base, int rows, int lane, float4 (&v)[8]) {
+    const int r = (lane >> 1) & 7;
+    base += r * kYtK + (lane >> 4) * 8 + (lane & 1) * 4;
+    if (rows >= 32) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int64_t row = first + (q >> 1) * 8 + r;
-        v[q] = row < rows ? __ldg(reinterpret_cast<const float4*>(base + row * kYtK + (q & 1) * 16 + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < 8; ++q) v[q] = __ldg(reinterpret_cast<const float4*>(base + (q >> 1) * 8 * kYtK + (q & 1) * 16));
+    } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            v[q] = (q >> 1) * 8 + r < rows ? __ldg(reinterpret_cast<const float4*>(base + (q >> 1) * 8 * kYtK + (q & 1) * 16))
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 // stores the split rows [row0, row0 + 32) of the tile; returns the sum of squares of row row0 + lane
@@ -110,8 +117,10 @@ __device__ __forceinline__ uint32_t yt_crop(const int4 b, int x, int y, int widt
     uint32_t bits = 0u;
     for (int at = 0; at < 32; ++y) {
         const int n = min(width - x, 32 - at);
-        const int lo = max(b.x - x, 0), hi = min(b.y - x, n);
-        if (y >= b.z && y < b.w && hi > lo) bits |= (0xffffffffu >> (32 - (hi - lo))) << (at + lo);
+        const int lo = max(b.x - x, 0), len = max(min(b.y - x, n) - lo, 0);
+        uint32_t run;
+        asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(run) : "r"(at + lo), "r"(len));
+        if (y >= b.z && y < b.w) bits |= run;
         at += n;
         x = 0;
     }
@@ -144,7 +153,10 @@ yolact_masks_tc_kernel(const float* __restrict__ proto, const float* __restrict_
 
     const int tile0 = blockIdx.x * tiles_per_cta, tile1 = min(tile0 + tiles_per_cta, (hw + kYtThreads - 1) / kYtThreads);
     float4 v[8];
-    yt_load(pimg, static_cast<int64_t>(tile0) * kYtThreads + warp * 32, hw, lane, v);
+    {
+        const int at = tile0 * kYtThreads + warp * 32;
+        yt_load(pimg + static_cast<int64_t>(at) * kYtK, hw - at, lane, v);
+    }
     if (t == 0) {
         mbar_init(&sh.done, 1);
         fence_barrier_init();
@@ -165,7 +177,7 @@ yolact_masks_tc_kernel(const float* __restrict__ proto, const float* __restrict_
         bool odd = false;  // a NaN does not survive a maximum
         for (int g = warp; g < groups; g += kYtThreads / 32) {
             float4 c[8];
-            yt_load(cimg, g * 32, num_det, lane, c);
+            yt_load(cimg + g * 32 * kYtK, num_det - g * 32, lane, c);
             const float s = yt_store(b_tile, g * 32, lane, c);
             odd |= !(s < INFINITY);
             most = fmaxf(most, s);
@@ -184,6 +196,9 @@ yolact_masks_tc_kernel(const float* __restrict__ proto, const float* __restrict_
     // D = F32, A = B = BF16, both K-major, M = 128
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n_mma >> 3) << 17) | ((128u >> 4) << 24);
     bool usable = true;
+    // a thread stores one 16-byte piece of every 16th detection: 16 planes on, the pieces lie on the same boundary
+    uint8_t* plane0 = masks + (static_cast<int64_t>(img) * num_det + (t >> 3)) * hw;
+    const int from = tile0 * kYtThreads, to = min(tile1 * kYtThreads, hw);
 
     for (int tile = tile0; tile < tile1; ++tile) {
         const float psq = yt_store(a_tile, warp * 32, lane, v);
@@ -203,7 +218,7 @@ yolact_masks_tc_kernel(const float* __restrict__ proto, const float* __restrict_
         }
         const int p0 = tile * kYtThreads + warp * 32;
         const int y0 = p0 / width, x0 = p0 - y0 * width;
-        if (tile + 1 < tile1) yt_load(pimg, static_cast<int64_t>(p0) + kYtThreads, hw, lane, v);
+        if (tile + 1 < tile1) yt_load(pimg + static_cast<int64_t>(p0 + kYtThreads) * kYtK, hw - p0 - kYtThreads, lane, v);
         // the crops of this warp's 32 pixels, and a list of the detections that have any
         uint32_t* bits = sh.bits + ((4 * (tile - tile0) + warp) & 7) * kYtBitsPitch;
         int touched = 0;
@@ -231,21 +246,21 @@ yolact_masks_tc_kernel(const float* __restrict__ proto, const float* __restrict_
             float s[8];
             yt_columns(taddr, list, s);
             uint32_t mine = 0u;  // lane u: the pixels of detection u of the batch that lie above the threshold
-            bool decided = true;
+            float over[8], least = INFINITY;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const float over = __fsub_rn(s[u], mid);
-                const uint32_t above = __ballot_sync(kFullMask, over > 0.0f);
+                over[u] = __fsub_rn(s[u], mid);
+                const uint32_t above = __ballot_sync(kFullMask, over[u] > 0.0f);
                 mine = lane == u ? above : mine;
-                decided = decided && fabsf(over) > reach;  // (not so for a NaN)
+                least = fminf(least, fabsf(over[u]));
             }
             const int d = sh.list[warp][i + (lane & 7)];
             uint32_t res = mine & bits[d];
-            if (!__all_sync(kFullMask, decided)) {
+            if (!__all_sync(kFullMask, least > reach)) {
                 uint32_t open = 0u;
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    const uint32_t o = __ballot_sync(kFullMask, !(fabsf(__fsub_rn(s[u], mid)) > reach));
+                    const uint32_t o = __ballot_sync(kFullMask, !(fabsf(over[u]) > reach));
                     open = lane == u ? o : open;
                 }
                 open &= bits[d];
@@ -272,33 +287,40 @@ yolact_masks_tc_kernel(const float* __restrict__ proto, const float* __restrict_
         }
         tc_fence_before();
         __syncthreads();
-        // Out in aligned pieces of 16 bytes, eight lanes to a row: the piece that covers the boundary to the tile before takes
+        // Out in aligned pieces of 16 bytes, eight threads to a row: the piece that covers the boundary to the tile before takes
         // that tile's bits along; what lies outside this CTA's run is left to its neighbours.
         const int first = tile * kYtThreads, row0 = 4 * (tile - tile0);
-        const int from = tile0 * kYtThreads, to = min(tile1 * kYtThreads, hw);
-        auto put = [&](int d, int piece) {
-            uint8_t* plane = masks + (static_cast<int64_t>(img) * num_det + d) * hw;
-            const int back = static_cast<int>(reinterpret_cast<uintptr_t>(plane + first) & 15);
-            const int at = piece * 16 - back;  // relative to the tile
-            const int r = row0 + (at >> 5);    // (arithmetic shift: at = -1 .. -15 is the row before)
-            const uint32_t w = __funnelshift_r(sh.bits[(r & 7) * kYtBitsPitch + d], sh.bits[((r + 1) & 7) * kYtBitsPitch + d], at & 31);
+        auto put = [&](uint8_t* plane, int d, int step, int piece) {
+            const int at = piece * 16 - static_cast<int>(reinterpret_cast<uintptr_t>(plane + first) & 15);  // relative to the tile
+            const int r = row0 + (at >> 5);  // (arithmetic shift: at = -1 .. -15 is the row before)
+            const uint32_t* w0 = sh.bits + (r & 7) * kYtBitsPitch;
+            const uint32_t* w1 = sh.bits + ((r + 1) & 7) * kYtBitsPitch;
             const int p = first + at;
+            plane += p;
             if (p >= from && p + 16 <= to) {
-                uint4 o;
-                o.x = ((w & 15u) * 0x00204081u) & 0x01010101u;
-                o.y = (((w >> 4) & 15u) * 0x00204081u) & 0x01010101u;
-                o.z = (((w >> 8) & 15u) * 0x00204081u) & 0x01010101u;
-                o.w = (((w >> 12) & 15u) * 0x00204081u) & 0x01010101u;
-                *reinterpret_cast<uint4*>(plane + p) = o;
+#pragma unroll 2
+                for (; d < num_det; d += step, plane += static_cast<int64_t>(step) * hw) {
+                    const uint32_t w = __funnelshift_r(w0[d], w1[d], at);
+                    uint4 o;
+                    o.x = ((w & 15u) * 0x00204081u) & 0x01010101u;
+                    o.y = (((w >> 4) & 15u) * 0x00204081u) & 0x01010101u;
+                    o.z = (((w >> 8) & 15u) * 0x00204081u) & 0x01010101u;
+                    o.w = (((w >> 12) & 15u) * 0x00204081u) & 0x01010101u;
+                    *reinterpret_cast<uint4*>(plane) = o;
+                }
             } else {  // planes and runs start at even addresses
-                for (int k = max(from - p, 0); k < min(16, to - p); k += 2)
-                    *reinterpret_cast<uint16_t*>(plane + p + k) = static_cast<uint16_t>(((w >> k) & 1u) | (((w >> k) & 2u) << 7));
+                const int k0 = max(from - p, 0), k1 = min(16, to - p);
+                if (k0 >= k1) return;
+                for (; d < num_det; d += step, plane += static_cast<int64_t>(step) * hw) {
+                    const uint32_t w = __funnelshift_r(w0[d], w1[d], at);
+                    for (int k = k0; k < k1; k += 2)
+                        *reinterpret_cast<uint16_t*>(plane + k) = static_cast<uint16_t>(((w >> k) & 1u) | (((w >> k) & 2u) << 7));
+                }
             }
         };
-#pragma unroll 2
-        for (int i = t; i < 8 * num_det; i += kYtThreads) put(i >> 3, i & 7);
+        put(plane0, t >> 3, kYtThreads / 8, t & 7);
         if (tile + 1 == tile1)
-            for (int d = t; d < num_det; d += kYtThreads) put(d, 8);
+            for (int d = t; d < num_det; d += kYtThreads) put(masks + (static_cast<int64_t>(img) * num_det + d) * hw, d, kYtMaxDet, 8);
     }
     tc_fence_before();
     __syncthreads();
