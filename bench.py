@@ -281,7 +281,7 @@ def extra_workloads(torch, fb, W, hbm_peak, peak_kind="measured"):
     by = BATCH * 4356432
     out["yolact"] = {"batch": BATCH, "latency_us": ms * 1e3, "batches_per_s": 1e3 / ms, "kernels_per_call": 1,
                      "algorithmic_gbs": by / (ms * 1e-3) / 1e9, "frac_of_hbm_peak": by / (ms * 1e-3) / 1e9 / hbm_peak,
-                     "roofline": hbm_roofline("yolact_masks_kernel", by, ms, hbm_peak, peak_kind)}
+                     "roofline": hbm_roofline("yolact_masks_tc_kernel", by, ms, hbm_peak, peak_kind)}
     del proto, ym
     # C4, T=64 B=64 H=512
     x, w_ih, w_hh, b_ih, b_hh = W.make_lstm_inputs()
@@ -378,7 +378,7 @@ def simple_ops(torch, fb, hbm_peak, peak_kind):
         i0 = J.interpreted_functor_runs()
         fused(*arg_sets[0])
         rec["one_launch"]["interpreted_functors"] = J.interpreted_functor_runs() - i0
-        rec["roofline"] = hbm_roofline("generic_group_kernel_param", alg_bytes, rec["one_launch"]["latency_us"] * 1e-3,
+        rec["roofline"] = hbm_roofline("region_group_kernel", alg_bytes, rec["one_launch"]["latency_us"] * 1e-3,
                                        hbm_peak, peak_kind,
                                        "time of the whole call on the stream (host-side program flattening included when "
                                        "the device is idle)")
@@ -506,7 +506,7 @@ def run_ours(args):
                 # the gather that used this group of record buffers n_rec groups ago is done (inside a capture the first
                 # uses have no earlier gather: a replay starts after the previous one has finished)
                 cur.wait_event(g_ev[j])
-            # memset + decode/mask/compact + binned top-k + NMS: 3 kernels; with N > 1 the NMS kernel also writes the records
+            # score floor + decode / compact + selection and NMS: 3 kernels; with N > 1 the last one also writes the records
             p.run(sets[i % n_sets], 0.5, 0.45, records=recs[j][slot] if world > 1 else None)
             if handles is not None:
                 lib.functs_b200_set_stage_events(None, 0)
@@ -614,9 +614,9 @@ def run_ours(args):
         block_ms.append(timed_block(False, in_flight > 1))
     total_ms = statistics.median(block_ms)
     fb.ops.raise_on_status(plan.status, "bench")
-    decode_ms = statistics.mean(e[0].elapsed_time(e[1]) for e in ev)
-    select_ms = statistics.mean(e[1].elapsed_time(e[2]) for e in ev)
-    nms_ms = statistics.mean(e[2].elapsed_time(e[3]) for e in ev)
+    floor_ms = statistics.mean(e[0].elapsed_time(e[1]) for e in ev)
+    decode_ms = statistics.mean(e[1].elapsed_time(e[2]) for e in ev)
+    post_ms = statistics.mean(e[2].elapsed_time(e[3]) for e in ev)
     kept = int(plan.counts.sum())
 
     # ---- e2e: public module, pinned host inputs, detections read back ----
@@ -642,10 +642,10 @@ def run_ours(args):
     clocks = sampler.stop() if rank == 0 else None
 
     # ---- max over ranks ----
-    stats = torch.tensor([total_ms, e2e_ms, decode_ms, select_ms, nms_ms, seq_ms], dtype=torch.float64, device=dev)
+    stats = torch.tensor([total_ms, e2e_ms, floor_ms, decode_ms, post_ms, seq_ms], dtype=torch.float64, device=dev)
     if world > 1:
         dist.all_reduce(stats, op=dist.ReduceOp.MAX)
-    total_ms, e2e_ms, decode_ms, select_ms, nms_ms, seq_ms = [float(v) for v in stats.tolist()]
+    total_ms, e2e_ms, floor_ms, decode_ms, post_ms, seq_ms = [float(v) for v in stats.tolist()]
 
     if rank == 0:
         ms_per_step = total_ms / args.steps
@@ -664,12 +664,12 @@ def run_ours(args):
             **({"diagnostic": "gather skipped (--no-gather): not a result"} if args.no_gather else {}),
             "latency_us": seq_ms / args.steps * 1e3, "kernels_per_call": launches / args.steps,
             "images_per_s": world * BATCH * 1e3 / ms_per_step,
-            "stage_us": {"decode_mask_compact": decode_ms * 1e3, "select_topk": select_ms * 1e3, "nms": nms_ms * 1e3},
+            "stage_us": {"score_floor": floor_ms * 1e3, "decode_compact": decode_ms * 1e3, "select_nms": post_ms * 1e3},
             "detections_kept_last_step": kept, "select_fallbacks_last_step": plan.select_fallbacks(),
             "gpu_launches": launches,
             "e2e": {"value": world * 1e3 / e2e_ms, "unit": UNIT, "h2d_bytes_per_step": bytes_in,
                     "d2h_bytes_per_step": bytes_out, "ms_per_step": e2e_ms, "steps": e2e_steps},
-            "roofline": {"bound": "hbm", "kernel": "yolo_decode_staged_kernel", "achieved": achieved, "peak": hbm_peak,
+            "roofline": {"bound": "hbm", "kernel": "yolo_decode_kernel", "achieved": achieved, "peak": hbm_peak,
                          "unit": "GB/s", "frac": achieved / hbm_peak, "peak_kind": peak_kind, "traffic": None,
                          "algorithmic_bytes_per_launch": alg_bytes, "whole_step_frac": (alg_bytes + BATCH * OUT_BYTES_PER_IMG) / (ms_per_step * 1e-3) / 1e9 / hbm_peak},
             "clocks": clocks,
