@@ -213,7 +213,7 @@ def bands(x: torch.Tensor):
 
 @pytest.mark.parametrize("fn,shape", [
     (scaled, (1, 1)), (scaled, (1024, 1184)), (scaled, (1025, 1185)),
-    (normalize, (1, 1, 3)), (normalize, (319, 317, 3)), (normalize, (317, 1283, 3)),
+    (normalize, (1, 1, 3)), (normalize, (319, 317, 3)), (normalize, (317, 1283, 3)), (normalize, (811, 753, 3)),
     (class_deltas, (7, 44)), (class_deltas, (4099, 84)), (bands, (33, 40)), (bands, (5003, 64)),
 ])
 def test_programs_cut_into_regions(env, fn, shape):
