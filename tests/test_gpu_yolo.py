@@ -240,3 +240,48 @@ def test_one_call_postprocess_replays_from_a_cuda_graph(fb):
         assert int(plan.status.item()) == 0 and int(ref.status.item()) == 0
         assert torch.equal(plan.counts, ref.counts)
         assert torch.equal(plan.dets, ref.dets) and torch.equal(plan.labels, ref.labels) and torch.equal(plan.flat_ids, ref.flat_ids)
+
+
+@pytest.mark.parametrize("batch,sizes,kind,topk", [
+    (1, (13, 26, 52), "plain", 1000), (30, (13, 26, 52), "plain", 1000), (2, (10, 20, 40), "plain", 1),  # one / four slots per thread
+    (2, (13, 26, 52), "sampled high", 1000), (2, (13, 26, 52), "sampled low", 1000),  # floor too high: rescan; too low: long lists
+    (2, (13, 26, 52), "crowded tile", 1000), (3, (4, 8, 16), "equal", 1000), (2, (13, 26, 52), "equal few", 1024),
+    (2, (13, 26, 52), "one class", 1000), (2, (19, 38, 76), "sparse", 1000), (2, (11, 22, 44), "none", 100),
+])
+def test_yolo_one_call_form_at_its_edges(fb, batch, sizes, kind, topk):
+    """Every branch of the floor, decode and post kernels: the detections of both forms are what the oracle's mask, sort, top-k and
+    NMS make of the decoded floats."""
+    g = torch.Generator().manual_seed(batch + sizes[0] + topk)
+    maps = [torch.randn(batch, 255, s, s, generator=g) for s in sizes]
+    for m in maps:
+        v = m.view(batch, 3, 85, -1)
+        slot = torch.arange(3 * v.size(3)).view(3, -1)  # (anchor, position)
+        if kind.startswith("sampled"):
+            v[:, :, 4] += torch.where((slot % 512 < 32) == (kind == "sampled high"), 3.0, -3.0)
+        elif kind == "crowded tile":
+            v[:, :, 4:] += torch.where((slot >= 40) & (slot < 200), 4.0, -6.0)[:, None]
+        elif kind == "equal":
+            v[:, :, 4:] = 2.0
+        elif kind == "equal few":
+            v[:, :, 4:] = torch.where((slot % 97 == 5) & (slot < 800), 2.0, -4.0)[:, None]
+        elif kind == "one class":
+            v[:, :, 5:] -= 8.0
+            v[:, :, 5] += 12.0
+            v[:, :, 2:4] += 2.0
+        elif kind == "sparse":
+            v[:, :, 4] -= 4.0
+        elif kind == "none":
+            v[:, :, 4] -= 30.0
+    cmaps = [m.cuda() for m in maps]
+    boxes, obj, cls, _, _ = fb.ops.yolo_decode(cmaps, 0.5, dense=True)
+    boxes, obj, cls = boxes.cpu(), obj.cpu(), cls.cpu()
+    mod = fb.workloads.YOLOV3BBox(sizes=sizes, topk=topk)
+    dets, labels, flat, cnt = [t.cpu() for t in mod.forward_padded(cmaps)]
+    fb.ops.raise_on_status(mod._plan.status, "yolo")
+    lists = mod(cmaps)
+    post = W.YOLOV3Post(sizes=sizes, topk=topk)
+    for b in range(batch):
+        wd, wl, wf = post.post_single(boxes[b], obj[b], cls[b])
+        m = int(cnt[b])
+        assert m == wf.numel() and torch.equal(flat[b, :m], wf) and torch.equal(labels[b, :m], wl) and torch.equal(dets[b, :m], wd)
+        assert torch.equal(lists[b][0].cpu(), wd) and torch.equal(lists[b][1].cpu(), wl)
