@@ -108,8 +108,9 @@ constexpr size_t kSsdSelBytes = (sizeof(SelectSmem<kSsdSelCap>) + 127) / 128 * 1
 // the compaction to some thirty ATen launches and three synchronisations per image: 8.9 ms for 64 images against 0.35.
 struct SsdRagged {
     int32_t* words;        // [batch * num_classes] kept count + 1 (0 = not known yet), then the ticket; zero at launch
+    unsigned long long* done;  // [batch] classes that have written their rows << 32 | rows; zero at launch
     int64_t* labels;       // like prior_ids
-    int32_t* img_counts;   // [batch] rows of every image (may be pinned host memory)
+    int32_t* img_counts;   // [batch] rows of every image (may be pinned host memory): written when they are all in place
     int32_t* status;       // optional; plain store (may be pinned host memory)
     int batch;
 };
@@ -213,16 +214,14 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
                 while ((v = words[c]) == 0) {
                     if (clock64() - start > kSsdWaitCycles) {
                         if (rag.status != nullptr) *reinterpret_cast<volatile int32_t*>(rag.status) = FB_STATUS_WAIT_TIMEOUT;
+                        __threadfence_system();  // before this image's count
                         break;
                     }
                 }
                 before += v > 0 ? v - 1 : 0;
             }
             before = __reduce_add_sync(kFullMask, before);
-            if (lane == 0) {
-                s_before = before;
-                if (cls == num_classes - 1) rag.img_counts[img] = before + word_prefix[kSsdWords];
-            }
+            if (lane == 0) s_before = before;
         }
         __syncthreads();
         const int64_t obase = static_cast<int64_t>(img) * num_classes * topk + s_before;
@@ -239,6 +238,17 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
                 d[4] = key_score(mykey);
                 rag.labels[row] = cls;
                 prior_ids[row] = static_cast<int64_t>(key_index(mykey));
+            }
+        }
+        __syncthreads();
+        if (t == 0) {
+            // the class that finishes last publishes the image: a host that watches the count finds the rows complete
+            __threadfence();
+            const unsigned long long mine = (1ull << 32) + static_cast<unsigned>(word_prefix[kSsdWords]);
+            const unsigned long long all = atomicAdd(rag.done + img, mine) + mine;
+            if (static_cast<int>(all >> 32) == num_classes) {
+                __threadfence_system();
+                *reinterpret_cast<volatile int32_t*>(rag.img_counts + img) = static_cast<int32_t>(all);
             }
         }
         return;
@@ -361,7 +371,7 @@ int functs_b200_ssd_class_nms(const float* boxes, const float* scores_cm, int32_
 
 int64_t functs_b200_ssd_scratch_bytes(int32_t batch, int32_t num_classes) {
     if (batch <= 0 || num_classes <= 0) return 0;
-    return (static_cast<int64_t>(batch) * num_classes + 1) * 4;
+    return static_cast<int64_t>(batch) * 8 + (static_cast<int64_t>(batch) * num_classes + 1) * 4;
 }
 
 int functs_b200_ssd_postprocess(const float* loc, const float* conf, const float* priors, int32_t batch, int32_t num_priors,
@@ -372,9 +382,11 @@ int functs_b200_ssd_postprocess(const float* loc, const float* conf, const float
     FB_REQUIRE(labels && img_counts && scratch, "ssd_postprocess: null pointer");
     const int64_t words = static_cast<int64_t>(batch) * num_classes;
     FB_REQUIRE(batch > 0 && num_classes > 0 && words < (1ll << 30), "ssd_postprocess: bad sizes");
-    SsdRagged rag{static_cast<int32_t*>(scratch), labels, img_counts, status, batch};
-    FB_TRY(launch_ssd_softmax_decode(loc, conf, priors, batch, num_priors, num_classes, clamp_max, boxes, scores_cm, rag.words,
-                                     static_cast<int>(words) + 1, as_stream(stream)));
+    FB_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 7) == 0, "ssd_postprocess: scratch must be 8-byte aligned");
+    int32_t* sync = static_cast<int32_t*>(scratch);
+    SsdRagged rag{sync + 2 * batch, static_cast<unsigned long long*>(scratch), labels, img_counts, status, batch};
+    FB_TRY(launch_ssd_softmax_decode(loc, conf, priors, batch, num_priors, num_classes, clamp_max, boxes, scores_cm, sync,
+                                     2 * batch + static_cast<int>(words) + 1, as_stream(stream)));
     return launch_ssd_class_nms(boxes, scores_cm, batch, num_priors, num_classes, score_thr, topk, iou_thr, dets, prior_ids, nullptr,
                                 &rag, as_stream(stream));
 }

@@ -401,9 +401,13 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
             records[2 * row + 1] = make_int4(0, -1, -1, 0);
         }
     }
+    if (A.host_counts != nullptr) __syncthreads();  // a host that watches the count finds the rows complete
     if (t == 0) {
         A.out_counts[img] = total;
-        if (A.host_counts != nullptr) A.host_counts[img] = total;
+        if (A.host_counts != nullptr) {
+            __threadfence_system();
+            *reinterpret_cast<volatile int32_t*>(A.host_counts + img) = total;
+        }
     }
 }
 

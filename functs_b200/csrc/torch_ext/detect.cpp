@@ -4,6 +4,9 @@
 #include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <chrono>
+#include <limits>
+
 #include "../../../include/functs_b200.h"
 
 namespace functs_b200 {
@@ -21,9 +24,51 @@ at::Tensor viewAt(const at::Tensor& base, int64_t offset, at::IntArrayRef sizes)
     return at::Tensor(std::move(impl));
 }
 
-// Host words that the kernels write themselves (pinned memory is mapped into the device's address space): waiting for the
-// stream is all a caller has to do, there is no copy and one wait.
-at::Tensor pinnedWords(int64_t n) { return at::empty({n}, at::TensorOptions().dtype(at::kInt).pinned_memory(true)); }
+// Host words that the kernels write themselves (pinned memory is mapped into the device's address space): one per image, its
+// count, written after its rows, and the status word.  The host watches the counts instead of waiting for the stream: no
+// copy, no wake-up (about 6 us), and the views of an image are made while the kernel works on later ones.  The words return to
+// their pool only when all of them have been written, or the stream is idle.
+class HostCounts {
+public:
+    HostCounts(int64_t n, cudaStream_t stream)
+        : host_(at::empty({n + 1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true))), words_(host_.data_ptr<int32_t>()), n_(n), stream_(stream) {
+        for (int64_t i = 0; i < n; ++i) words_[i] = kPending;
+        words_[n] = 0;
+    }
+    ~HostCounts() {
+        if (launched && seen_ < n_) (void)cudaStreamSynchronize(stream_);  // leaving through an exception
+    }
+    int32_t* counts() { return const_cast<int32_t*>(words_); }
+    int32_t* status() { return const_cast<int32_t*>(words_ + n_); }
+    const at::Tensor& tensor() const { return host_; }
+    // the next image's count, images in order
+    int64_t next() {
+        const auto start = std::chrono::steady_clock::now();
+        for (unsigned spin = 1; words_[seen_] == kPending; ++spin) {
+            cpuRelax();
+            if (spin % 1024 != 0) continue;
+            cudaError_t e = cudaStreamQuery(stream_);
+            if (e == cudaErrorNotReady && std::chrono::steady_clock::now() - start > std::chrono::milliseconds(5)) e = cudaStreamSynchronize(stream_);
+            if (e == cudaErrorNotReady) continue;
+            C10_CUDA_CHECK(e);
+            TORCH_CHECK(words_[seen_] != kPending, "functs_b200: the kernels ended without a count");
+        }
+        return words_[seen_++];
+    }
+    bool launched = false;
+
+private:
+    static constexpr int32_t kPending = std::numeric_limits<int32_t>::min();
+    static void cpuRelax() {
+#if defined(__x86_64__)
+        __builtin_ia32_pause();
+#endif
+    }
+    at::Tensor host_;
+    volatile int32_t* words_;
+    int64_t n_, seen_ = 0;
+    cudaStream_t stream_;
+};
 
 void raiseOnStatus(int bits, const char* what) {
     TORCH_CHECK(bits == 0, "functs_b200 ", what, ": device status ", bits,
@@ -40,7 +85,7 @@ constexpr int64_t kKeepRoomBytes = 4 << 20;
 }  // namespace
 
 SsdResult ssdDetect(const at::Tensor& loc, const at::Tensor& conf, const at::Tensor& priors, double clamp_max, double score_thr,
-                    int64_t topk, double iou_thr, bool want_ids) {
+                    int64_t topk, double iou_thr, bool want_ids, const EmitImage& emit) {
     TORCH_CHECK(loc.dim() == 3 && loc.size(2) == 4 && conf.dim() == 3 && conf.size(0) == loc.size(0) && conf.size(1) == loc.size(1) &&
                     conf.size(2) >= 2 && priors.dim() == 2 && priors.size(0) == loc.size(1) && priors.size(1) == 4,
                 "ssd: loc [B, P, 4] / conf [B, P, C+1] do not fit the prior table");
@@ -52,29 +97,40 @@ SsdResult ssdDetect(const at::Tensor& loc, const at::Tensor& conf, const at::Ten
     r.scores_cm = at::empty({B, C, P}, f32);
     at::Tensor dets = at::empty({rows, 5}, f32), labels = at::empty({rows}, f32.dtype(at::kLong)), ids = at::empty({rows}, f32.dtype(at::kLong));
     at::Tensor scratch = at::empty({functs_b200_ssd_scratch_bytes(static_cast<int32_t>(B), static_cast<int32_t>(C))}, f32.dtype(at::kByte));
-    at::Tensor host = pinnedWords(B + 1);
-    int32_t* words = host.data_ptr<int32_t>();
-    words[B] = 0;
     const auto stream = at::cuda::getCurrentCUDAStream();
+    HostCounts host(B, stream.stream());
+    host.launched = true;
     checkRc(functs_b200_ssd_postprocess(loc.data_ptr<float>(), conf.data_ptr<float>(), priors.data_ptr<float>(), static_cast<int32_t>(B),
                                         static_cast<int32_t>(P), static_cast<int32_t>(C), static_cast<float>(clamp_max),
                                         static_cast<float>(score_thr), static_cast<int32_t>(topk), static_cast<float>(iou_thr),
                                         r.boxes.data_ptr<float>(), r.scores_cm.data_ptr<float>(), dets.data_ptr<float>(),
-                                        labels.data_ptr<int64_t>(), ids.data_ptr<int64_t>(), words, words + B, scratch.data_ptr(),
+                                        labels.data_ptr<int64_t>(), ids.data_ptr<int64_t>(), host.counts(), host.status(), scratch.data_ptr(),
                                         stream.stream()),
             "ssd post-process");
-    C10_CUDA_CHECK(cudaStreamSynchronize(stream.stream()));
-    raiseOnStatus(words[B], "ssd post-process");
-    int64_t total = 0, stride = C * topk;
-    for (int64_t b = 0; b < B; ++b) total += words[b];
-    const bool packed = rows * 28 > kKeepRoomBytes && total * 4 < rows;
-    if (packed) {
+    const int64_t stride = C * topk;
+    const bool may_pack = rows * 28 > kKeepRoomBytes;
+    std::vector<int64_t> counts(static_cast<size_t>(B));
+    int64_t total = 0, emitted = 0;
+    auto emitUpTo = [&](int64_t end, bool packed) {
+        for (int64_t row = 0; emitted < end; ++emitted) {
+            const int64_t n = counts[static_cast<size_t>(emitted)], at_row = packed ? row : emitted * stride;
+            emit({viewAt(dets, at_row * 5, {n, 5}), viewAt(labels, at_row, {n}), want_ids ? viewAt(ids, at_row, {n}) : at::Tensor()});
+            row += n;
+        }
+    };
+    for (int64_t b = 0; b < B; ++b) {
+        total += counts[static_cast<size_t>(b)] = host.next();
+        raiseOnStatus(*host.status(), "ssd post-process");
+        // (once a quarter of the room is filled the results stay where they are)
+        if (!may_pack || total * 4 >= rows) emitUpTo(b + 1, false);
+    }
+    if (may_pack && total * 4 < rows) {
         at::Tensor d = at::empty({total, 5}, f32), l = at::empty({total}, labels.options());
         at::Tensor i = want_ids ? at::empty({total}, ids.options()) : at::Tensor();
         if (total > 0) {
             // (`host` goes back to its pool before the kernel runs: copy_ tells the pool when the copy is done)
             at::Tensor dev_counts = at::empty({B}, f32.dtype(at::kInt));
-            dev_counts.copy_(host.narrow(0, 0, B), /*non_blocking=*/true);
+            dev_counts.copy_(host.tensor().narrow(0, 0, B), /*non_blocking=*/true);
             checkRc(functs_b200_ragged_pack(dets.data_ptr<float>(), labels.data_ptr<int64_t>(), ids.data_ptr<int64_t>(),
                                             dev_counts.data_ptr<int32_t>(), static_cast<int32_t>(B), stride, d.data_ptr<float>(),
                                             l.data_ptr<int64_t>(), want_ids ? i.data_ptr<int64_t>() : nullptr, stream.stream()),
@@ -83,18 +139,13 @@ SsdResult ssdDetect(const at::Tensor& loc, const at::Tensor& conf, const at::Ten
         dets = d;
         labels = l;
         ids = i;
-    }
-    r.images.reserve(static_cast<size_t>(B));
-    int64_t at_row = 0;
-    for (int64_t b = 0; b < B; ++b) {
-        const int64_t n = words[b], row = packed ? at_row : b * stride;
-        r.images.push_back({viewAt(dets, row * 5, {n, 5}), viewAt(labels, row, {n}), want_ids ? viewAt(ids, row, {n}) : at::Tensor()});
-        at_row += n;
+        emitUpTo(B, true);
     }
     return r;
 }
 
-YoloResult yoloDetect(const std::vector<at::Tensor>& maps, double score_thr, int64_t topk, double iou_thr, bool dense, bool want_ids) {
+YoloResult yoloDetect(const std::vector<at::Tensor>& maps, double score_thr, int64_t topk, double iou_thr, bool dense, bool want_ids,
+                      const EmitImage& emit) {
     TORCH_CHECK(maps.size() == 3, "yolov3: expected three prediction maps");
     int64_t S[3], N = 0;
     const int64_t B = maps[0].size(0);
@@ -120,25 +171,21 @@ YoloResult yoloDetect(const std::vector<at::Tensor>& maps, double score_thr, int
                                                          static_cast<int32_t>(S[2]), capacity, static_cast<int32_t>(topk));
     at::Tensor scratch = at::empty({bytes + B * 4}, f32.dtype(at::kByte));  // and the device's copy of the counts
     int32_t* counts = reinterpret_cast<int32_t*>(static_cast<char*>(scratch.data_ptr()) + bytes);
-    at::Tensor host = pinnedWords(B + 1);
-    int32_t* words = host.data_ptr<int32_t>();
-    words[B] = 0;
     const auto stream = at::cuda::getCurrentCUDAStream();
+    HostCounts host(B, stream.stream());
+    host.launched = true;
     checkRc(functs_b200_yolo_detect(maps[0].data_ptr<float>(), maps[1].data_ptr<float>(), maps[2].data_ptr<float>(),
                                     static_cast<int32_t>(B), static_cast<int32_t>(S[0]), static_cast<int32_t>(S[1]),
                                     static_cast<int32_t>(S[2]), static_cast<float>(score_thr), static_cast<int32_t>(topk),
                                     static_cast<float>(iou_thr), capacity, dense ? r.boxes.data_ptr<float>() : nullptr,
                                     dense ? r.obj.data_ptr<float>() : nullptr, dense ? r.cls.data_ptr<float>() : nullptr,
                                     dets.data_ptr<float>(), labels.data_ptr<int64_t>(), want_ids ? ids.data_ptr<int64_t>() : nullptr,
-                                    counts, nullptr, words, words + B, scratch.data_ptr(), stream.stream()),
+                                    counts, nullptr, host.counts(), host.status(), scratch.data_ptr(), stream.stream()),
             "yolov3 post-process");
-    C10_CUDA_CHECK(cudaStreamSynchronize(stream.stream()));
-    raiseOnStatus(words[B], "yolov3 post-process");
-    r.images.reserve(static_cast<size_t>(B));
     for (int64_t b = 0; b < B; ++b) {
-        const int64_t n = words[b];
-        r.images.push_back({viewAt(dets, b * topk * 5, {n, 5}), viewAt(labels, b * topk, {n}),
-                            want_ids ? viewAt(ids, b * topk, {n}) : at::Tensor()});
+        const int64_t n = host.next();
+        raiseOnStatus(*host.status(), "yolov3 post-process");
+        emit({viewAt(dets, b * topk * 5, {n, 5}), viewAt(labels, b * topk, {n}), want_ids ? viewAt(ids, b * topk, {n}) : at::Tensor()});
     }
     return r;
 }

@@ -4,6 +4,7 @@
 
 #include <ATen/ATen.h>
 
+#include <functional>
 #include <vector>
 
 namespace functs_b200 {
@@ -12,18 +13,19 @@ struct Detections {  // one image
     at::Tensor dets, labels, ids;
 };
 
+using EmitImage = std::function<void(Detections&&)>;  // called once per image, in order
+
 struct SsdResult {
     at::Tensor boxes, scores_cm;  // [B, P, 4], [B, C, P]
-    std::vector<Detections> images;
 };
 // want_ids = false leaves Detections::ids undefined
 SsdResult ssdDetect(const at::Tensor& loc, const at::Tensor& conf, const at::Tensor& priors, double clamp_max, double score_thr,
-                    int64_t topk, double iou_thr, bool want_ids);
+                    int64_t topk, double iou_thr, bool want_ids, const EmitImage& emit);
 
 struct YoloResult {
     at::Tensor boxes, obj, cls;  // [B, N, 4], [B, N], [B, N, 80]; dense = true only
-    std::vector<Detections> images;
 };
-YoloResult yoloDetect(const std::vector<at::Tensor>& maps, double score_thr, int64_t topk, double iou_thr, bool dense, bool want_ids);
+YoloResult yoloDetect(const std::vector<at::Tensor>& maps, double score_thr, int64_t topk, double iou_thr, bool dense, bool want_ids,
+                      const EmitImage& emit);
 
 }  // namespace functs_b200

@@ -16,10 +16,12 @@ namespace py = pybind11;
 using torch::jit::Graph;
 
 namespace {
-py::list pairs(const std::vector<functs_b200::Detections>& images) {
-    py::list out(images.size());
-    for (size_t b = 0; b < images.size(); ++b) out[b] = py::make_tuple(images[b].dets, images[b].labels);
-    return out;
+// Appends (dets, labels) to a Python list, from code that runs without the interpreter lock.
+functs_b200::EmitImage appendTo(py::list& out) {
+    return [&out](functs_b200::Detections&& d) {
+        py::gil_scoped_acquire gil;
+        out.append(py::make_tuple(std::move(d.dets), std::move(d.labels)));
+    };
 }
 }  // namespace
 
@@ -121,16 +123,16 @@ PYBIND11_MODULE(_C, m) {
     m.def("_ssd_detect",
           [](const at::Tensor& loc, const at::Tensor& conf, const at::Tensor& priors, double clamp_max, double score_thr, int64_t topk,
              double iou_thr) {
-              functs_b200::SsdResult r;
+              py::list out;
               {
                   py::gil_scoped_release release;
-                  r = functs_b200::ssdDetect(loc, conf, priors, clamp_max, score_thr, topk, iou_thr, /*want_ids=*/false);
+                  functs_b200::ssdDetect(loc, conf, priors, clamp_max, score_thr, topk, iou_thr, /*want_ids=*/false, appendTo(out));
               }
-              return pairs(r.images);
+              return out;
           });
     m.def("_yolo_detect", [](std::vector<at::Tensor> maps, const std::vector<int64_t>& sizes, at::Device device, double score_thr,
                              int64_t topk, double iou_thr) {
-        functs_b200::YoloResult r;
+        py::list out;
         {
             py::gil_scoped_release release;
             TORCH_CHECK_VALUE(maps.size() == 3 && sizes.size() == 3, "expected three [B, 255, S, S] maps");
@@ -142,9 +144,9 @@ PYBIND11_MODULE(_C, m) {
                 if (t.device() != device) t = t.to(device, t.scalar_type(), /*non_blocking=*/true);
                 t = t.contiguous();
             }
-            r = functs_b200::yoloDetect(maps, score_thr, topk, iou_thr, /*dense=*/false, /*want_ids=*/false);
+            functs_b200::yoloDetect(maps, score_thr, topk, iou_thr, /*dense=*/false, /*want_ids=*/false, appendTo(out));
         }
-        return pairs(r.images);
+        return out;
     });
     m.def("_count_parallel_functors", [](std::shared_ptr<Graph> g) { return functs_b200::CountParallelFunctors(g); });
     m.def("_jit_pass_freeze", [](torch::jit::Module& module) { return torch::jit::freeze_module(module); });

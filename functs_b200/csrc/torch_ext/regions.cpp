@@ -401,12 +401,10 @@ Operation makeYolo(const Node* node, bool dense) {
                         "yolov3 region: map ", l, " must be [B, 255, ", sizes[l], ", ", sizes[l], "]");
             maps.push_back(m);
         }
-        YoloResult r = yoloDetect(maps, thr, topk, iou, dense, /*want_ids=*/true);
         c10::impl::GenericList results(c10::TupleType::create({c10::TensorType::get(), c10::TensorType::get(), c10::TensorType::get()}));
-        results.reserve(r.images.size());
-        for (Detections& d : r.images) {
+        YoloResult r = yoloDetect(maps, thr, topk, iou, dense, /*want_ids=*/true, [&](Detections&& d) {
             results.push_back(c10::ivalue::Tuple::create({std::move(d.dets), std::move(d.labels), std::move(d.ids)}));
-        }
+        });
         if (dense) {
             push(stack, std::move(r.boxes), std::move(r.obj), std::move(r.cls));
         }
@@ -443,12 +441,10 @@ Operation makeSsd(const Node* node) {
             if (v.empty()) v.push_back(priors_cpu.to(loc.device()));
             priors = v[0];
         }
-        SsdResult r = ssdDetect(loc, conf, priors, clamp_max, thr, topk, iou, /*want_ids=*/true);
         c10::impl::GenericList results(c10::TupleType::create({c10::TensorType::get(), c10::TensorType::get(), c10::TensorType::get()}));
-        results.reserve(r.images.size());
-        for (Detections& d : r.images) {
+        SsdResult r = ssdDetect(loc, conf, priors, clamp_max, thr, topk, iou, /*want_ids=*/true, [&](Detections&& d) {
             results.push_back(c10::ivalue::Tuple::create({std::move(d.dets), std::move(d.labels), std::move(d.ids)}));
-        }
+        });
         push(stack, r.scores_cm.permute({0, 2, 1}));
         stack.emplace_back(std::move(results));
         push(stack, std::move(r.boxes));

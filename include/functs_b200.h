@@ -174,7 +174,8 @@ int functs_b200_yolo_postprocess_dense(const float* map0, const float* map1, con
 
 /* The general form.  boxes may be NULL (the boxes of the detections are decoded from the logits either way), flat_ids may be
  * NULL.  host_counts (optional, [batch]) receives the counts once more; it and the status word may be pinned host memory,
- * so that a caller who waits for the stream needs no copy. */
+ * so that a caller who waits for the stream needs no copy.  An image's host count is written after its rows and after any
+ * status bit, so that a host may as well watch the counts. */
 int functs_b200_yolo_detect(const float* map0, const float* map1, const float* map2, int32_t batch, int32_t s0, int32_t s1,
                             int32_t s2, float score_thr, int32_t topk, float iou_thr, int64_t capacity, float* boxes,
                             float* obj_out, float* cls_out, float* dets, int64_t* labels, int64_t* flat_ids,
@@ -200,8 +201,9 @@ int functs_b200_ssd_class_nms(const float* boxes, const float* scores_cm, int32_
 /* Both groups in one call, with the ragged result the program returns: image b's kept rows of all classes, class after class,
  * are dets / labels / prior_ids [b * C * topk, + img_counts[b]).  dets [batch * C * topk, 5]; labels, prior_ids
  * [batch * C * topk]; img_counts [batch] and the optional status word may be pinned host memory (both are written by the
- * kernel, so that a caller who waits for the stream needs no copy).  Two launches, no memset.
- * scratch: functs_b200_ssd_scratch_bytes(batch, C). */
+ * kernel, an image's count after its rows and after any status bit, so that a caller needs no copy and may watch the counts
+ * instead of waiting for the stream).  Two launches, no memset.
+ * scratch: functs_b200_ssd_scratch_bytes(batch, C), 8-byte aligned. */
 int64_t functs_b200_ssd_scratch_bytes(int32_t batch, int32_t num_classes);
 int functs_b200_ssd_postprocess(const float* loc, const float* conf, const float* priors, int32_t batch, int32_t num_priors,
                                 int32_t num_classes, float clamp_max, float score_thr, int32_t topk, float iou_thr, float* boxes,
