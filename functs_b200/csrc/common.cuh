@@ -46,6 +46,31 @@ __device__ __forceinline__ float sigmoid_f32(float x) {
     return __frcp_rn(__fadd_rn(1.0f, expf(-x)));
 }
 
+// The same for N values at once.  __frcp_rn ends in a branch per value, which keeps the compiler from interleaving them.  From an
+// approximation within one ulp, one Newton step with a fused remainder gives the correctly rounded reciprocal (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990; equal to __frcp_rn for every float in
+// [1, 2^125], tried one by one); larger denominators, whose reciprocals leave the normal range, take the other road together.
+template <int N>
+__device__ __forceinline__ void sigmoid_f32_n(float (&v)[N]) {
+    float x[N], most = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        x[i] = __fadd_rn(1.0f, expf(-v[i]));
+        most = fmaxf(most, x[i]);
+    }
+    if (most < 0x1p125f) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            float y;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x[i]));
+            v[i] = fmaf(y, fmaf(-x[i], y, 1.0f), y);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] = __frcp_rn(x[i]);
+    }
+}
+
 // Candidate key: score bits in the high word, inverted flat index in the low word, so that
 // "larger key" == "larger score, then smaller index".  Requires score > 0.
 __device__ __forceinline__ uint64_t make_key(float score, uint32_t flat_idx) {
