@@ -116,10 +116,11 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
     const uint32_t h_own = smem_u32(h_s + rank * Y::BP + ir * Y::U + iu);
     float c_state = 0.0f;
     float pre_g[4] = {0.f, 0.f, 0.f, 0.f};
+    pdl_wait();  // the projection (read with __ldcg: a __ldg could be moved up across this); the weights are not its output
     if (live) {
         const float* p = pre + static_cast<int64_t>(row) * (4 * H) + k_own;
 #pragma unroll
-        for (int g = 0; g < 4; ++g) pre_g[g] = __ldg(p + g * H);
+        for (int g = 0; g < 4; ++g) pre_g[g] = __ldcg(p + g * H);
     }
     cluster_arrive();  // every CTA of the cluster runs before anybody stores into another one
     cluster_wait();
@@ -192,7 +193,7 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
             if (t + 1 < T) {
                 const float* p = pre + (static_cast<int64_t>(t + 1) * B + row) * (4 * H) + k_own;
 #pragma unroll
-                for (int g = 0; g < 4; ++g) pre_g[g] = __ldg(p + g * H);
+                for (int g = 0; g < 4; ++g) pre_g[g] = __ldcg(p + g * H);
             }
         }
         if (t + 1 < T) cluster_wait();
@@ -263,7 +264,7 @@ lstm_recurrent_wide_kernel(const float* __restrict__ pre, const float* __restric
             if (i < kItems && row < B) {
                 const float* p = pre + (static_cast<int64_t>(t) * B + row) * (4 * H) + j0 + i % Y::U;
 #pragma unroll
-                for (int g = 0; g < 4; ++g) pre_g[q][g] = __ldg(p + g * H);
+                for (int g = 0; g < 4; ++g) pre_g[q][g] = __ldcg(p + g * H);
             }
         }
     };
@@ -273,6 +274,7 @@ lstm_recurrent_wide_kernel(const float* __restrict__ pre, const float* __restric
 #pragma unroll
         for (int g = 0; g < 4; ++g) pre_g[q][g] = 0.0f;
     }
+    pdl_wait();  // the projection, as in the kernel above
     fetch(0);
     cluster_arrive();  // every CTA of the cluster runs before anybody stores into another one
     cluster_wait();
@@ -378,13 +380,15 @@ static int launch_rec(Kernel kernel, int threads, size_t smem, int rows, const f
     cfg.blockDim = dim3(static_cast<unsigned>(threads));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = kRecCluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the weights are fetched while the projection ends
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     FB_TRY(check_cuda(cudaLaunchKernelEx(&cfg, kernel, pre, w_hh, T, B, hs, cs), "lstm_recurrent launch"));
     count_launch();
     return FB_OK;

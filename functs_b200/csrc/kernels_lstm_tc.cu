@@ -82,6 +82,7 @@ __device__ __forceinline__ void tc_store_split(unsigned char* tile, int off, con
 __global__ void __launch_bounds__(256)
 lstm_tc_split_kernel(const float* __restrict__ x, const float* __restrict__ w_ih, int M, int K, int H, int vec_x,
                      unsigned char* __restrict__ a_tiles, unsigned char* __restrict__ b_tiles) {
+    pdl_launch_dependents();
     const int KT = (K + kTcBK - 1) / kTcBK, kchunks = KT * (kTcBK / 4);
     const int rows = (M + kTcBM - 1) / kTcBM * kTcBM;
     const int64_t a_items = static_cast<int64_t>(rows) * kchunks;
@@ -132,6 +133,7 @@ lstm_tc_gemm_kernel(const float* __restrict__ x, const float* __restrict__ w_ih,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int KT = (K + kTcBK - 1) / kTcBK;
     const int nt = blockIdx.x, mt = blockIdx.y;
+    pdl_launch_dependents();
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kTcStages; ++s) {
@@ -154,6 +156,7 @@ lstm_tc_gemm_kernel(const float* __restrict__ x, const float* __restrict__ w_ih,
     const uint32_t tmem = sh.tmem_base;
 
     if (PRESPLIT && warp == 0) {
+        pdl_wait();  // the tiles
         if (lane == 0) {
             const unsigned char* a_src = reinterpret_cast<const unsigned char*>(x) + static_cast<int64_t>(mt) * KT * (2 * kTcTileBytes);
             const unsigned char* b_src = reinterpret_cast<const unsigned char*>(w_ih) + static_cast<int64_t>(nt) * KT * (2 * kTcTileBytes);
@@ -689,9 +692,8 @@ int launch_lstm_input_proj_tc(const float* x, const float* w_ih, const float* b_
         w_ih = reinterpret_cast<const float*>(b_tiles);
     }
     FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "lstm_tc_gemm attr"));
-    kernel<<<grid, kTcThreads, smem, st>>>(x, w_ih, b_ih, b_hh, M, K, H, vec_x, pre, status);
-    count_launch();
-    return check_launch("lstm_tc_gemm_kernel");
+    return launch_after(kernel, grid, dim3(kTcThreads), smem, st, presplit, "lstm_tc_gemm_kernel", x, w_ih, b_ih, b_hh, M, K, H, vec_x, pre,
+                        status);
 }
 
 }  // namespace fb

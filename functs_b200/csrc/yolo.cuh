@@ -54,30 +54,7 @@ __device__ __forceinline__ float logit_cut(float so, float bar) {
     return __logf(__fdividef(q, 1.0f - q)) - 0.02f;
 }
 
-// Programmatic dependent launch: the next kernel of the stream may start once every CTA has said launch_dependents (or
-// ended); what it reads or overwrites of this kernel's it only touches behind its own wait, which covers all of this kernel.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 #endif  // __CUDACC__
-
-// Host side: a launch that may overlap the end of the kernel before it (pdl) or not.
-template <class... KP, class... A>
-inline int launch_after(void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const char* what, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    FB_TRY(check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<KP>(args)...), what));
-    count_launch();
-    return FB_OK;
-}
 
 // kernels_yolo_post.cu
 struct YoloPostArgs {

@@ -32,7 +32,10 @@ def new_status(device) -> torch.Tensor:
 
 
 def raise_on_status(status: torch.Tensor, what: str) -> None:
-    """Reads the device status word (synchronises) and raises if a kernel reported a problem."""
+    """Reads the status word (synchronises) and raises if a kernel reported a problem.  A word in pinned host memory is the
+    current stream's."""
+    if not status.is_cuda:
+        torch.cuda.current_stream().synchronize()
     bits = int(status.item())
     if bits == 0:
         return

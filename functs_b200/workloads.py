@@ -146,7 +146,8 @@ class LSTM:
         self.b_hh = b_hh.to(self.device, torch.float32).reshape(4, -1).contiguous()
         self._scratch = None
         self._out = None
-        self._status = ops.new_status(self.device)
+        # in host memory: the kernels write it only when something went wrong, and reading it takes no copy
+        self._status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.kernels_last_call = 0
 
     @staticmethod
