@@ -8,6 +8,10 @@
 #include <torch/csrc/jit/passes/freeze_module.h>
 #include <torch/csrc/jit/passes/shape_analysis.h>
 
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAException.h>
+
+#include "../../../include/functs_b200.h"
 #include "detect.h"
 #include "fusion.h"
 #include "tensorssa.h"
@@ -147,6 +151,29 @@ PYBIND11_MODULE(_C, m) {
             functs_b200::yoloDetect(maps, score_thr, topk, iou_thr, /*dense=*/false, /*want_ids=*/false, appendTo(out));
         }
         return out;
+    });
+    // one LSTM call on prepared weights and buffers: checks, launches and, with `wait`, the wait for the stream.  Returns the
+    // library's (negative) error code, else the status word when it has waited.
+    m.def("_lstm_forward", [](const at::Tensor& x, const at::Tensor& w_ih, const at::Tensor& w_hh, const at::Tensor& b_ih, const at::Tensor& b_hh,
+                              const at::Tensor& hs, const at::Tensor& cs, const at::Tensor& scratch, const at::Tensor& status, int64_t mode,
+                              bool wait) -> int64_t {
+        py::gil_scoped_release release;
+        TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (functs_b200 has no CPU path)");
+        TORCH_CHECK_TYPE(x.scalar_type() == at::kFloat, "x must be torch.float32");
+        const int64_t T = x.size(0), B = x.size(1), I = x.size(2), H = w_hh.size(2);
+        TORCH_CHECK_VALUE(w_ih.dim() == 3 && w_ih.size(0) == 4 && w_ih.size(1) == I && w_ih.size(2) == H && w_hh.dim() == 3 &&
+                              w_hh.size(0) == 4 && w_hh.size(1) == H,
+                          "weights must be gate-leading: w_ih [4, I, H], w_hh [4, H, H]");
+        TORCH_CHECK_VALUE(b_ih.numel() == 4 * H && b_hh.numel() == 4 * H, "biases must have 4*H elements");
+        const at::Tensor xc = x.contiguous();
+        const auto stream = at::cuda::getCurrentCUDAStream();
+        const int rc = functs_b200_lstm_forward_mode(xc.data_ptr<float>(), w_ih.data_ptr<float>(), w_hh.data_ptr<float>(), b_ih.data_ptr<float>(),
+                                                     b_hh.data_ptr<float>(), static_cast<int32_t>(T), static_cast<int32_t>(B),
+                                                     static_cast<int32_t>(I), static_cast<int32_t>(H), hs.data_ptr<float>(), cs.data_ptr<float>(),
+                                                     status.data_ptr<int32_t>(), scratch.data_ptr(), stream.stream(), static_cast<int32_t>(mode));
+        if (rc != FB_OK || !wait) return rc;
+        C10_CUDA_CHECK(cudaStreamSynchronize(stream.stream()));
+        return *static_cast<volatile int32_t*>(status.data_ptr<int32_t>());
     });
     m.def("_count_parallel_functors", [](std::shared_ptr<Graph> g) { return functs_b200::CountParallelFunctors(g); });
     m.def("_jit_pass_freeze", [](torch::jit::Module& module) { return torch::jit::freeze_module(module); });

@@ -159,6 +159,11 @@ class LSTM:
 
     def forward_device(self, x: torch.Tensor, mode: int = 0):
         """x on the device; outputs and scratch are reused across calls; no synchronisation."""
+        self._buffers(x)
+        self._run(x, mode, wait=False)
+        return self._out
+
+    def _buffers(self, x: torch.Tensor) -> None:
         t, b, i = x.shape
         h = self.w_hh.size(2)
         if self._out is None or self._out[0].shape != (t, b, h):
@@ -167,16 +172,21 @@ class LSTM:
             from ._lib import lib
             self._scratch = torch.empty(int(lib.functs_b200_lstm_scratch_bytes(t, b, i, h)), dtype=torch.uint8,
                                         device=self.device)
+
+    def _run(self, x: torch.Tensor, mode: int, wait: bool) -> None:
         before = launch_count()
-        ops.lstm_forward(x, self.w_ih, self.w_hh, self.b_ih, self.b_hh, mode=mode, scratch=self._scratch,
-                         status=self._status, out=self._out)
+        code = _native()._lstm_forward(x, self.w_ih, self.w_hh, self.b_ih, self.b_hh, *self._out, self._scratch, self._status, mode, wait)
         self.kernels_last_call = launch_count() - before
-        return self._out
+        if code < 0:
+            ops.check(code, "lstm_forward")
+        if code > 0:
+            ops.raise_on_status(self._status, "LSTM")
 
     def __call__(self, x: torch.Tensor, mode: int = 0) -> Tuple[torch.Tensor, torch.Tensor]:
-        hs, cs = self.forward_device(x.to(self.device, non_blocking=True).contiguous(), mode)
-        ops.raise_on_status(self._status, "LSTM")
-        return hs, cs
+        x = x.to(self.device, non_blocking=True)
+        self._buffers(x)
+        self._run(x, mode, wait=True)
+        return self._out
 
 
 class YolactBBoxMask:
