@@ -211,7 +211,15 @@ def bands(x: torch.Tensor):
     return t > 0.5
 
 
+def columns(x: torch.Tensor):
+    t = x.clone()
+    for k in range(5):
+        t[:, k] = t[:, k] * float(k + 1)
+    return t + 0.5
+
+
 @pytest.mark.parametrize("fn,shape", [
+    (columns, (7, 5)), (columns, (606301, 5)),  # five interleaved regions: too many loads to fetch ahead
     (scaled, (1, 1)), (scaled, (1024, 1184)), (scaled, (1025, 1185)),
     (normalize, (1, 1, 3)), (normalize, (319, 317, 3)), (normalize, (317, 1283, 3)), (normalize, (811, 753, 3)),
     (class_deltas, (7, 44)), (class_deltas, (4099, 84)), (bands, (33, 40)), (bands, (5003, 64)),
