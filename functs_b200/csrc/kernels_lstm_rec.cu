@@ -173,10 +173,9 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
         }
         float hval = 0.0f;
         if (item) {
-            const float ig = sigmoid_f32(gate[0]);
-            const float fg = sigmoid_f32(gate[1]);
-            const float gg = tanhf(gate[2]);
-            const float og = sigmoid_f32(gate[3]);
+            float sg[3] = {gate[0], gate[1], gate[3]};
+            sigmoid_f32_n(sg);
+            const float ig = sg[0], fg = sg[1], og = sg[2], gg = tanhf(gate[2]);
             c_state = __fadd_rn(__fmul_rn(fg, c_state), __fmul_rn(ig, gg));
             hval = __fmul_rn(og, tanhf(c_state));
             if (t + 1 < T) {
@@ -341,10 +340,9 @@ lstm_recurrent_wide_kernel(const float* __restrict__ pre, const float* __restric
                     gate[g] = __fadd_rn(gate[g], s);
                 }
             }
-            const float ig = sigmoid_f32(gate[0]);
-            const float fg = sigmoid_f32(gate[1]);
-            const float gg = tanhf(gate[2]);
-            const float og = sigmoid_f32(gate[3]);
+            float sg[3] = {gate[0], gate[1], gate[3]};
+            sigmoid_f32_n(sg);
+            const float ig = sg[0], fg = sg[1], og = sg[2], gg = tanhf(gate[2]);
             c_state[q] = __fadd_rn(__fmul_rn(fg, c_state[q]), __fmul_rn(ig, gg));
             hval[q] = __fmul_rn(og, tanhf(c_state[q]));
             if (t + 1 < T) {
