@@ -175,6 +175,20 @@ PYBIND11_MODULE(_C, m) {
         C10_CUDA_CHECK(cudaStreamSynchronize(stream.stream()));
         return *static_cast<volatile int32_t*>(status.data_ptr<int32_t>());
     });
+    // masks into `out` [B, N, H, W]; returns the library's error code
+    m.def("_yolact_masks", [](const at::Tensor& proto, const at::Tensor& coef, const at::Tensor& boxes, double thr, const at::Tensor& out) -> int64_t {
+        py::gil_scoped_release release;
+        auto checked = [](const at::Tensor& t, const char* name) {
+            TORCH_CHECK_VALUE(t.is_cuda(), name, " must be a CUDA tensor (functs_b200 has no CPU path)");
+            TORCH_CHECK_TYPE(t.scalar_type() == at::kFloat, name, " must be torch.float32");
+            return t.contiguous();
+        };
+        const at::Tensor p = checked(proto, "proto"), c = checked(coef, "coef"), b = checked(boxes, "boxes");
+        TORCH_CHECK_VALUE(p.dim() == 4 && p.size(3) == 32, "prototype depth must be 32");
+        return functs_b200_yolact_masks(p.data_ptr<float>(), c.data_ptr<float>(), b.data_ptr<float>(), static_cast<int32_t>(p.size(0)),
+                                        static_cast<int32_t>(p.size(1)), static_cast<int32_t>(p.size(2)), static_cast<int32_t>(c.size(1)),
+                                        static_cast<float>(thr), out.data_ptr<uint8_t>(), nullptr, at::cuda::getCurrentCUDAStream().stream());
+    });
     m.def("_count_parallel_functors", [](std::shared_ptr<Graph> g) { return functs_b200::CountParallelFunctors(g); });
     m.def("_jit_pass_freeze", [](torch::jit::Module& module) { return torch::jit::freeze_module(module); });
     m.def("_jit_pass_clone", [](torch::jit::Module& module) { return module.clone(); });

@@ -199,14 +199,14 @@ class YolactBBoxMask:
         self.kernels_last_call = 0
 
     def __call__(self, proto: torch.Tensor, coef: torch.Tensor, boxes: torch.Tensor) -> torch.Tensor:
-        proto = proto.to(self.device, non_blocking=True).contiguous()
-        coef = coef.to(self.device, non_blocking=True).contiguous()
-        boxes = boxes.to(self.device, non_blocking=True).contiguous()
+        proto = proto.to(self.device, non_blocking=True)
+        coef = coef.to(self.device, non_blocking=True)
+        boxes = boxes.to(self.device, non_blocking=True)
         b, h, w, _ = proto.shape
         n = coef.size(1)
         if self._out is None or self._out.shape != (b, n, h, w):
             self._out = torch.empty(b, n, h, w, dtype=torch.uint8, device=self.device)
         before = launch_count()
-        ops.yolact_masks(proto, coef, boxes, self.thr, out=self._out)
+        ops.check(_native()._yolact_masks(proto, coef, boxes, self.thr, self._out), "yolact_masks")
         self.kernels_last_call = launch_count() - before
         return self._out
