@@ -60,18 +60,31 @@ struct TcShared {
     volatile int abort_flag;
 };
 
-// fp32 -> nearest TF32 value, ties away from zero, as cvt.rna.tf32 rounds, in two integer operations (the conversion unit takes
-// a quarter of the rate, and a k-tile has 16384 of them)
+// Finite fp32 -> nearest TF32 value, ties away from zero, as cvt.rna.tf32 rounds, in two integer operations (the conversion unit
+// takes a quarter of the rate, and a k-tile has 16384 of them).  Not for NaN: the addition can carry into the sign.
 __device__ __forceinline__ float tf32_nearest(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
 
-// Four fp32 values -> their hi and lo parts, stored at `off` of the hi tile and of the lo tile behind it.
+// Four fp32 values -> their hi and lo parts, stored at `off` of the hi tile and of the lo tile behind it.  NaN, infinities and
+// what rounds to infinity have no such parts (v - hi is not finite for all three): they go in as a NaN, which reaches every
+// output they take part in, and the epilogue forms those outputs again from the operands themselves (tc_exact_row).
 __device__ __forceinline__ void tc_store_split(unsigned char* tile, int off, const float (&v)[4]) {
     float hi[4], lo[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         hi[i] = tf32_nearest(v[i]);
-        lo[i] = tf32_nearest(__fsub_rn(v[i], hi[i]));
+        lo[i] = __fsub_rn(v[i], hi[i]);
     }
+    // (finite remainders are below 2^117: their sum is finite)
+    if (!(fabsf(__fadd_rn(__fadd_rn(lo[0], lo[1]), __fadd_rn(lo[2], lo[3]))) < INFINITY)) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (fabsf(lo[i]) < INFINITY) continue;
+            hi[i] = __uint_as_float(0x7fc00000u);
+            lo[i] = 0.0f;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) lo[i] = tf32_nearest(lo[i]);
     *reinterpret_cast<float4*>(tile + off) = make_float4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<float4*>(tile + kTcTileBytes + off) = make_float4(lo[0], lo[1], lo[2], lo[3]);
 }
@@ -121,12 +134,29 @@ lstm_tc_split_kernel(const float* __restrict__ x, const float* __restrict__ w_ih
     }
 }
 
+// Whole warps: the outputs of row m whose bit is set in `columns`, columns n .. n + 31, lane c column n + c: fp32 products summed in
+// the order of lstm_input_proj_simt_kernel, so that NaN, infinities and overflow come out as IEEE arithmetic has them.
+__device__ __noinline__ void tc_exact_row(const float* __restrict__ x, const float* __restrict__ w_ih, const float* __restrict__ b_ih,
+                                          const float* __restrict__ b_hh, int K, int H, int m, int n, uint32_t columns, float* pre) {
+    const int lane = threadIdx.x & 31;
+    if (((columns >> lane) & 1u) == 0u) return;
+    n += lane;
+    const int g = n / H, j = n - g * H;
+    const float* xr = x + static_cast<int64_t>(m) * K;
+    const float* w = w_ih + static_cast<int64_t>(g) * K * H + j;
+    float acc = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) acc = fmaf(__ldg(xr + k), __ldg(w + static_cast<int64_t>(k) * H), acc);
+    pre[static_cast<int64_t>(m) * (4 * H) + n] = __fadd_rn(acc, __fadd_rn(__ldg(b_ih + n), __ldg(b_hh + n)));
+}
+
 // grid = (4H / 128, ceil(M / 128)).  dynamic smem: kTcStages * 64 KB of operand tiles (1024-byte aligned) + TcShared.
-// PRESPLIT: x and w_ih are the tiles of lstm_tc_split_kernel.
+// PRESPLIT: a_tiles and b_tiles are what lstm_tc_split_kernel made of x and w_ih.
 template <bool PRESPLIT>
 __global__ void __launch_bounds__(kTcThreads, 1)
-lstm_tc_gemm_kernel(const float* __restrict__ x, const float* __restrict__ w_ih, const float* __restrict__ b_ih,
-                    const float* __restrict__ b_hh, int M, int K, int H, int vec_x, float* __restrict__ pre, int32_t* status) {
+lstm_tc_gemm_kernel(const float* __restrict__ x, const float* __restrict__ w_ih, const unsigned char* __restrict__ a_tiles,
+                    const unsigned char* __restrict__ b_tiles, const float* __restrict__ b_ih, const float* __restrict__ b_hh, int M,
+                    int K, int H, int vec_x, float* __restrict__ pre, int32_t* status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* tiles = smem_raw;
     TcShared& sh = *reinterpret_cast<TcShared*>(smem_raw + kTcStages * kTcStageBytes);
@@ -158,8 +188,8 @@ lstm_tc_gemm_kernel(const float* __restrict__ x, const float* __restrict__ w_ih,
     if (PRESPLIT && warp == 0) {
         pdl_wait();  // the tiles
         if (lane == 0) {
-            const unsigned char* a_src = reinterpret_cast<const unsigned char*>(x) + static_cast<int64_t>(mt) * KT * (2 * kTcTileBytes);
-            const unsigned char* b_src = reinterpret_cast<const unsigned char*>(w_ih) + static_cast<int64_t>(nt) * KT * (2 * kTcTileBytes);
+            const unsigned char* a_src = a_tiles + static_cast<int64_t>(mt) * KT * (2 * kTcTileBytes);
+            const unsigned char* b_src = b_tiles + static_cast<int64_t>(nt) * KT * (2 * kTcTileBytes);
             for (int kt = 0; kt < KT; ++kt) {
                 const int s = kt % kTcStages;
                 const uint32_t par = ((kt / kTcStages) & 1) ^ 1;  // passes at once on a fresh barrier
@@ -304,7 +334,10 @@ lstm_tc_gemm_kernel(const float* __restrict__ x, const float* __restrict__ w_ih,
 #pragma unroll
                     for (int i = 0; i < 32; ++i) acc[i] = __fadd_rn(acc[i], more[i]);
                 }
+                uint32_t wild = 0u;  // columns of this row whose sum is not finite
                 if (m < M) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) wild |= fabsf(acc[i]) < INFINITY ? 0u : 1u << i;
 #pragma unroll
                     for (int i = 0; i < 32; i += 4) {
                         const int n = n0 + cb * 32 + i;
@@ -317,6 +350,14 @@ lstm_tc_gemm_kernel(const float* __restrict__ x, const float* __restrict__ w_ih,
                         o.w = __fadd_rn(acc[i + 3], __fadd_rn(bi.w, bh.w));
                         *reinterpret_cast<float4*>(orow + cb * 32 + i) = o;
                     }
+                }
+                uint32_t rows = __ballot_sync(kFullMask, wild != 0u);
+                __syncwarp();  // (the stores above come first)
+                while (rows != 0u) {
+                    const int r = __ffs(rows) - 1;
+                    rows &= rows - 1u;
+                    tc_exact_row(x, w_ih, b_ih, b_hh, K, H, mt * kTcBM + q * 32 + r, n0 + cb * 32, __shfl_sync(kFullMask, wild, r), pre);
+                    __syncwarp();
                 }
             }
         } else if (lane == 0 && status != nullptr) {
@@ -679,21 +720,20 @@ int launch_lstm_input_proj_tc(const float* x, const float* w_ih, const float* b_
     dim3 grid(4 * H / kTcBN, (M + kTcBM - 1) / kTcBM);
     const bool presplit = tc_presplit(M, H);
     auto kernel = presplit ? lstm_tc_gemm_kernel<true> : lstm_tc_gemm_kernel<false>;
+    unsigned char *a_tiles = nullptr, *b_tiles = nullptr;
     if (presplit) {
         const int KT = (K + kTcBK - 1) / kTcBK;
-        unsigned char* a_tiles = static_cast<unsigned char*>(tc_scratch);
-        unsigned char* b_tiles = a_tiles + static_cast<int64_t>(grid.y) * KT * 2 * kTcTileBytes;
+        a_tiles = static_cast<unsigned char*>(tc_scratch);
+        b_tiles = a_tiles + static_cast<int64_t>(grid.y) * KT * 2 * kTcTileBytes;
         const int64_t items = (static_cast<int64_t>(grid.y) * kTcBM + 4 * H) * KT * (kTcBK / 4);
         const int blocks = static_cast<int>(std::min<int64_t>((items + 255) / 256, kNumSMs * 8));
         lstm_tc_split_kernel<<<blocks, 256, 0, st>>>(x, w_ih, M, K, H, vec_x, a_tiles, b_tiles);
         count_launch();
         FB_TRY(check_launch("lstm_tc_split_kernel"));
-        x = reinterpret_cast<const float*>(a_tiles);
-        w_ih = reinterpret_cast<const float*>(b_tiles);
     }
     FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "lstm_tc_gemm attr"));
-    return launch_after(kernel, grid, dim3(kTcThreads), smem, st, presplit, "lstm_tc_gemm_kernel", x, w_ih, b_ih, b_hh, M, K, H, vec_x, pre,
-                        status);
+    return launch_after(kernel, grid, dim3(kTcThreads), smem, st, presplit, "lstm_tc_gemm_kernel", x, w_ih, a_tiles, b_tiles, b_ih, b_hh,
+                        M, K, H, vec_x, pre, status);
 }
 
 }  // namespace fb

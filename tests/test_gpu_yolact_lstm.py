@@ -175,6 +175,33 @@ def test_lstm_cell_golden(fb):
     close(cs[0].cpu(), want_c, rtol=1e-5, atol=1e-6, what="c1")
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("seq,batch,inputs,hidden", [
+    (2, 64, 512, 512),    # one whole row tile
+    (3, 5, 63, 256),      # rows and depth that fill no tile
+    (40, 33, 512, 512),   # operands split by a launch of their own
+])
+def test_lstm_inputs_that_are_not_finite(fb, seq, batch, inputs, hidden, mode):
+    """NaN of every sign and payload, infinities and the largest float pass through the projection as they do in the oracle:
+    NaN rows become NaN, the others saturate their gates.  The bound for finite values is test_gpu_ragged's, on fp64."""
+    g = torch.Generator().manual_seed(seq)
+    bound = hidden ** -0.5
+    w = [(torch.rand(*s, generator=g) * 2 - 1) * bound for s in ((4, inputs, hidden), (4, hidden, hidden), (4, 1, hidden), (4, 1, hidden))]
+    x = torch.randn(seq, batch, inputs, generator=g)
+    x[..., 3] *= 0.1  # (times the weight below: large, but no second infinity)
+    odd = torch.tensor([0x7fffffff, -1, 0x7fc00000, 0x7f800000, -0x800000], dtype=torch.int32).view(torch.float32)
+    x[0, torch.arange(5), torch.tensor([0, 31, 40, 62, 7])] = odd
+    x[-1, 3, 1] = torch.finfo(torch.float32).max
+    x[-1, 4, 61] = -torch.finfo(torch.float32).max
+    w[0][2, 3, 7] = torch.finfo(torch.float32).max
+    hs64, cs64 = W.LSTMSeq(*[t.double() for t in w])(x.double())
+    assert bool(hs64[:, :3].isnan().all()) and bool(hs64[:, 3:].isfinite().all())
+    for got, want in zip(fb.workloads.LSTM(*w)(x, mode=mode), (hs64, cs64)):
+        got = got.cpu().double()
+        assert torch.equal(got.isnan(), want.isnan())
+        assert float((got - want)[:, 3:].abs().max()) < 3e-6
+
+
 def test_lstm_rejects_unsupported_hidden(fb):
     x, w_ih, w_hh, b_ih, b_hh = W.make_lstm_inputs(2, 2, 64)
     with pytest.raises(fb.FunctsB200Error):
