@@ -6,12 +6,13 @@
 namespace fb {
 
 #ifdef __CUDACC__
-// sanitize_coordinates (yolact_mask.py:327-333) followed by "col >= x1 and col < x2" as integer bounds.
+// sanitize_coordinates (yolact_mask.py:327-333) followed by "col >= x1 and col < x2" as integer bounds, both in [0, size]: a box
+// outside the integers' range would saturate, and the differences that the kernels form with the bounds would wrap.
 __device__ __forceinline__ void yolact_crop_range(float a, float b, int size, int& lo, int& hi) {
     float x1 = fminf(a, b);
     float x2 = fmaxf(x1, b);
-    x1 = fmaxf(__fsub_rn(x1, 1.0f), 0.0f);
-    x2 = fminf(__fadd_rn(x2, 1.0f), static_cast<float>(size));
+    x1 = fminf(fmaxf(__fsub_rn(x1, 1.0f), 0.0f), static_cast<float>(size));
+    x2 = fmaxf(fminf(__fadd_rn(x2, 1.0f), static_cast<float>(size)), 0.0f);
     lo = static_cast<int>(ceilf(x1));
     hi = static_cast<int>(ceilf(x2));
 }

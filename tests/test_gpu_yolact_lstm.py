@@ -228,3 +228,18 @@ def test_yolact_masks_on_the_tensor_cores(fb, batch, height, width, dets, thr):
     args = (proto.cuda(), coef.cuda(), xy.cuda(), thr)
     masks, _ = fb.ops.yolact_masks(*args, with_logits=True)
     assert torch.equal(fb.ops.yolact_masks(*args), masks)
+
+
+@pytest.mark.parametrize("far", [3e9, 2147483648.0, float("inf")])
+@pytest.mark.parametrize("height,width", [(1, 138), (33, 10)])
+def test_yolact_boxes_outside_the_integers(fb, height, width, far):
+    """Crops of boxes whose coordinates no 32-bit integer holds: empty on the far sides, everything where the box spans the image;
+    the same from both mask kernels."""
+    proto = torch.ones(1, height, width, 32, device="cuda")
+    coef = torch.ones(1, 6, 32, device="cuda")
+    h, w = float(height), float(width)
+    boxes = torch.tensor([[[-far, 0, -far, h], [far, 0, far, h], [-far, 0, far, h], [0, -far, w, -far], [0, far, w, far],
+                           [-far, -far, far, far]]], device="cuda")
+    masks, _ = fb.ops.yolact_masks(proto, coef, boxes, with_logits=True)
+    assert masks.flatten(2).sum(2).tolist() == [[n * height * width for n in (0, 0, 1, 0, 0, 1)]]
+    assert torch.equal(fb.ops.yolact_masks(proto, coef, boxes), masks)
