@@ -65,6 +65,7 @@ SIGNATURES = {
     "functs_b200_ssd_postprocess": (c_int32, [P, P, P, c_int32, c_int32, c_int32, c_float, c_float, c_int32, c_float, P, P, P, P, P,
                                               P, P, P, P]),
     "functs_b200_ragged_pack": (c_int32, [P, P, P, P, c_int32, c_int64, P, P, P, P]),
+    "functs_b200_ragged_split": (c_int32, [P, P, P, c_int32, P]),
     "functs_b200_lstm_scratch_bytes": (c_int64, [c_int32, c_int32, c_int32, c_int32]),
     "functs_b200_lstm_forward": (c_int32, [P, P, P, P, P, c_int32, c_int32, c_int32, c_int32, P, P, P, P, P]),
     "functs_b200_lstm_forward_mode": (c_int32, [P, P, P, P, P, c_int32, c_int32, c_int32, c_int32, P, P, P, P, P, c_int32]),

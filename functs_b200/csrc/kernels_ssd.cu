@@ -9,6 +9,8 @@
 // Group 2 (ssd_class_nms_kernel): the loop over classes (ssd_bbox.py:163-172 + :212 per class) with every
 // (image, class) iteration mapped onto one CTA: mask > thr, top-k by (score desc, prior asc), gather boxes,
 // greedy NMS, write the kept rows and their count.
+#include <algorithm>
+
 #include "select_nms.cuh"
 
 namespace fb {
@@ -303,6 +305,20 @@ ragged_pack_kernel(const float* __restrict__ dets, const int64_t* __restrict__ l
     }
 }
 
+// Every part's rows into arrays of its own: grid = (chunks of rows, parts).  Latency: 64 parts of a few hundred rows are some
+// hundred KB.
+struct RaggedParts {
+    functs_b200_ragged_part part[FB_RAGGED_MAX_PARTS];
+};
+__global__ void __launch_bounds__(kPackThreads)
+ragged_split_kernel(const float* __restrict__ dets, const int64_t* __restrict__ labels, const __grid_constant__ RaggedParts P) {
+    const functs_b200_ragged_part& G = P.part[blockIdx.y];
+    const float* d = dets + 5 * G.first;
+    const int64_t at = static_cast<int64_t>(blockIdx.x) * kPackThreads + threadIdx.x, step = static_cast<int64_t>(gridDim.x) * kPackThreads;
+    for (int64_t i = at; i < 5 * G.rows; i += step) G.dets[i] = d[i];
+    for (int64_t i = at; i < G.rows; i += step) G.labels[i] = labels[G.first + i];
+}
+
 static int launch_ssd_softmax_decode(const float* loc, const float* conf, const float* priors, int batch, int num_priors,
                                      int num_classes, float clamp_max, float* boxes, float* scores_cm, int32_t* clear,
                                      int num_clear, cudaStream_t st) {
@@ -400,6 +416,25 @@ int functs_b200_ragged_pack(const float* dets, const int64_t* labels, const int6
                                                                                            out_labels, out_ids);
     count_launch();
     return check_launch("ragged_pack_kernel");
+}
+
+int functs_b200_ragged_split(const float* dets, const int64_t* labels, const functs_b200_ragged_part* parts, int32_t count, void* stream) {
+    using namespace fb;
+    FB_REQUIRE(dets && labels && parts, "ragged_split: null pointer");
+    FB_REQUIRE(count > 0 && count <= FB_RAGGED_MAX_PARTS, "ragged_split: between 1 and %d parts", FB_RAGGED_MAX_PARTS);
+    RaggedParts p{};
+    int64_t most = 0;
+    for (int k = 0; k < count; ++k) {
+        FB_REQUIRE(parts[k].first >= 0 && parts[k].rows >= 0 && (parts[k].rows == 0 || (parts[k].dets && parts[k].labels)),
+                   "ragged_split: bad part %d", k);
+        p.part[k] = parts[k];
+        most = std::max(most, parts[k].rows);
+    }
+    // two or three rows per thread, 16 CTAs to a part at most
+    const int64_t chunks = std::min<int64_t>(16, std::max<int64_t>(1, most / 512));
+    ragged_split_kernel<<<dim3(static_cast<unsigned>(chunks), static_cast<unsigned>(count)), kPackThreads, 0, as_stream(stream)>>>(dets, labels, p);
+    count_launch();
+    return check_launch("ragged_split_kernel");
 }
 
 }  // extern "C"

@@ -130,7 +130,7 @@ PYBIND11_MODULE(_C, m) {
               py::list out;
               {
                   py::gil_scoped_release release;
-                  functs_b200::ssdDetect(loc, conf, priors, clamp_max, score_thr, topk, iou_thr, /*want_ids=*/false, appendTo(out));
+                  functs_b200::ssdDetect(loc, conf, priors, clamp_max, score_thr, topk, iou_thr, functs_b200::Lists::kOwn, appendTo(out));
               }
               return out;
           });
@@ -148,7 +148,7 @@ PYBIND11_MODULE(_C, m) {
                 if (t.device() != device) t = t.to(device, t.scalar_type(), /*non_blocking=*/true);
                 t = t.contiguous();
             }
-            functs_b200::yoloDetect(maps, score_thr, topk, iou_thr, /*dense=*/false, /*want_ids=*/false, appendTo(out));
+            functs_b200::yoloDetect(maps, score_thr, topk, iou_thr, /*dense=*/false, functs_b200::Lists::kOwn, appendTo(out));
         }
         return out;
     });

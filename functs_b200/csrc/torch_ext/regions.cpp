@@ -402,7 +402,7 @@ Operation makeYolo(const Node* node, bool dense) {
             maps.push_back(m);
         }
         c10::impl::GenericList results(c10::TupleType::create({c10::TensorType::get(), c10::TensorType::get(), c10::TensorType::get()}));
-        YoloResult r = yoloDetect(maps, thr, topk, iou, dense, /*want_ids=*/true, [&](Detections&& d) {
+        YoloResult r = yoloDetect(maps, thr, topk, iou, dense, Lists::kViews, [&](Detections&& d) {
             results.push_back(c10::ivalue::Tuple::create({std::move(d.dets), std::move(d.labels), std::move(d.ids)}));
         });
         if (dense) {
@@ -442,7 +442,7 @@ Operation makeSsd(const Node* node) {
             priors = v[0];
         }
         c10::impl::GenericList results(c10::TupleType::create({c10::TensorType::get(), c10::TensorType::get(), c10::TensorType::get()}));
-        SsdResult r = ssdDetect(loc, conf, priors, clamp_max, thr, topk, iou, /*want_ids=*/true, [&](Detections&& d) {
+        SsdResult r = ssdDetect(loc, conf, priors, clamp_max, thr, topk, iou, Lists::kViews, [&](Detections&& d) {
             results.push_back(c10::ivalue::Tuple::create({std::move(d.dets), std::move(d.labels), std::move(d.ids)}));
         });
         push(stack, r.scores_cm.permute({0, 2, 1}));

@@ -214,6 +214,15 @@ int functs_b200_ssd_postprocess(const float* loc, const float* conf, const float
  * One launch. */
 int functs_b200_ragged_pack(const float* dets, const int64_t* labels, const int64_t* ids, const int32_t* counts, int32_t groups,
                             int64_t stride, float* out_dets, int64_t* out_labels, int64_t* out_ids, void* stream);
+/* Copies rows [first, first + rows) of dets / labels to arrays of their own, part by part: for a caller whose lists are kept one by
+ * one.  parts (at most FB_RAGGED_MAX_PARTS) are in HOST memory and travel as a kernel parameter.  One launch. */
+#define FB_RAGGED_MAX_PARTS 64
+typedef struct {
+    int64_t first, rows;
+    float* dets;     /* [rows, 5] */
+    int64_t* labels; /* [rows] */
+} functs_b200_ragged_part;
+int functs_b200_ragged_split(const float* dets, const int64_t* labels, const functs_b200_ragged_part* parts, int32_t count, void* stream);
 
 /* ---- C4: imperative LSTM with slice-assigned outputs ---------------------------------------- */
 /* Follows functs/benchmark/ai_model/lstm/lstm.py:79-98, 118-133 (one layer; hs[t] = h, cs[t] = c kept).
