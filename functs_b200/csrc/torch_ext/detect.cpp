@@ -25,10 +25,18 @@ at::Tensor viewAt(const at::Tensor& base, int64_t offset, at::IntArrayRef sizes)
     return at::Tensor(std::move(impl));
 }
 
+void raiseOnStatus(int bits, const char* what) {
+    TORCH_CHECK(bits == 0, "functs_b200 ", what, ": device status ", bits,
+                (bits & FB_STATUS_CAND_OVERFLOW) ? " (a candidate list overflowed)" : "",
+                (bits & FB_STATUS_WAIT_TIMEOUT) ? " (a bounded device-side wait ran out)" : "",
+                (bits & FB_STATUS_INDEX_RANGE) ? " (an index was out of range)" : "");
+}
+
 // Host words that the kernels write themselves (pinned memory is mapped into the device's address space): one per image, its
 // count, written after its rows, and the status word.  The host watches the counts instead of waiting for the stream: no
-// copy, no wake-up (about 6 us), and the views of an image are made while the kernel works on later ones.  The words return to
-// their pool only when all of them have been written, or the stream is idle.
+// copy, no wake-up (about 6 us), and the lists of an image are made while the kernel works on later ones.  The kernels write
+// the status word before the count of the image it concerns, so the host loads the count with acquire order and the status
+// behind it.  The words return to their pool only when all of them have been written, or the stream is idle.
 class HostCounts {
 public:
     HostCounts(int64_t n, cudaStream_t stream)
@@ -39,44 +47,41 @@ public:
     ~HostCounts() {
         if (launched && seen_ < n_) (void)cudaStreamSynchronize(stream_);  // leaving through an exception
     }
-    int32_t* counts() { return const_cast<int32_t*>(words_); }
-    int32_t* status() { return const_cast<int32_t*>(words_ + n_); }
+    int32_t* counts() { return words_; }  // for the kernels
+    int32_t* status() { return words_ + n_; }
     const at::Tensor& tensor() const { return host_; }
-    // the next image's count, images in order
-    int64_t next() {
+    // the next image's count, images in order; raises if a kernel reported a problem up to there
+    int64_t next(const char* what) {
         const auto start = std::chrono::steady_clock::now();
-        for (unsigned spin = 1; words_[seen_] == kPending; ++spin) {
+        int32_t count = load(seen_);
+        for (unsigned spin = 1; count == kPending; ++spin, count = load(seen_)) {
             cpuRelax();
             if (spin % 1024 != 0) continue;
             cudaError_t e = cudaStreamQuery(stream_);
             if (e == cudaErrorNotReady && std::chrono::steady_clock::now() - start > std::chrono::milliseconds(5)) e = cudaStreamSynchronize(stream_);
             if (e == cudaErrorNotReady) continue;
             C10_CUDA_CHECK(e);
-            TORCH_CHECK(words_[seen_] != kPending, "functs_b200: the kernels ended without a count");
+            TORCH_CHECK(load(seen_) != kPending, "functs_b200: the kernels ended without a count");
         }
-        return words_[seen_++];
+        ++seen_;
+        raiseOnStatus(load(n_), what);
+        return count;
     }
     bool launched = false;
 
 private:
     static constexpr int32_t kPending = std::numeric_limits<int32_t>::min();
+    int32_t load(int64_t i) const { return __atomic_load_n(words_ + i, __ATOMIC_ACQUIRE); }
     static void cpuRelax() {
 #if defined(__x86_64__)
         __builtin_ia32_pause();
 #endif
     }
     at::Tensor host_;
-    volatile int32_t* words_;
+    int32_t* words_;
     int64_t n_, seen_ = 0;
     cudaStream_t stream_;
 };
-
-void raiseOnStatus(int bits, const char* what) {
-    TORCH_CHECK(bits == 0, "functs_b200 ", what, ": device status ", bits,
-                (bits & FB_STATUS_CAND_OVERFLOW) ? " (a candidate list overflowed)" : "",
-                (bits & FB_STATUS_WAIT_TIMEOUT) ? " (a bounded device-side wait ran out)" : "",
-                (bits & FB_STATUS_INDEX_RANGE) ? " (an index was out of range)" : "");
-}
 
 // A ragged result is written into room for the largest possible one.  Views of a large room of which less than a quarter is
 // filled are made of memory of their own total size instead (one launch, nothing waits for it), so that a caller who keeps
@@ -141,8 +146,7 @@ SsdResult ssdDetect(const at::Tensor& loc, const at::Tensor& conf, const at::Ten
     if (lists == Lists::kOwn) {
         OwnLists own(dets, labels, stream.stream());
         for (int64_t b = 0; b < B; ++b) {
-            const int64_t n = host.next();
-            raiseOnStatus(*host.status(), "ssd post-process");
+            const int64_t n = host.next("ssd post-process");
             emit(own.take(b * stride, n));
         }
         own.flush();
@@ -159,8 +163,7 @@ SsdResult ssdDetect(const at::Tensor& loc, const at::Tensor& conf, const at::Ten
         }
     };
     for (int64_t b = 0; b < B; ++b) {
-        total += counts[static_cast<size_t>(b)] = host.next();
-        raiseOnStatus(*host.status(), "ssd post-process");
+        total += counts[static_cast<size_t>(b)] = host.next("ssd post-process");
         // (once a quarter of the room is filled the results stay where they are)
         if (!may_pack || total * 4 >= rows) emitUpTo(b + 1, false);
     }
@@ -223,8 +226,7 @@ YoloResult yoloDetect(const std::vector<at::Tensor>& maps, double score_thr, int
             "yolov3 post-process");
     OwnLists own(dets, labels, stream.stream());
     for (int64_t b = 0; b < B; ++b) {
-        const int64_t n = host.next();
-        raiseOnStatus(*host.status(), "yolov3 post-process");
+        const int64_t n = host.next("yolov3 post-process");
         if (lists == Lists::kOwn) emit(own.take(b * topk, n));
         else emit({viewAt(dets, b * topk * 5, {n, 5}), viewAt(labels, b * topk, {n}), viewAt(ids, b * topk, {n})});
     }
