@@ -442,7 +442,20 @@ struct RtcShared {
     float gates[kRtcBatch * kRtcGateStride];
 };
 
-__device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kRtcEpiThreads) : "memory"); }
+__device__ __forceinline__ void epi_barrier() { asm volatile("barrier.sync 1, %0;" ::"n"(kRtcEpiThreads) : "memory"); }
+// the same barrier; true for all of its threads if `value` is true for one of them
+__device__ __forceinline__ bool epi_barrier_any(bool value) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "barrier.red.or.pred q, 1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"(value ? 1u : 0u), "n"(kRtcEpiThreads)
+        : "memory");
+    return any != 0;
+}
 
 // grid = H / 4 CTAs (cooperative).  h_tiles: [2 (step parity)][H / 32][hi, lo][8 KB]; pre: [T * B, 4H].
 __global__ void __launch_bounds__(kRtcThreads, 1)
@@ -482,6 +495,7 @@ lstm_recurrent_tc_kernel(const float* __restrict__ pre, const float* __restrict_
         *reinterpret_cast<float*>(tile + kRtcBTile + off) = lo;
     }
     if (warp == 1) {
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(32u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -598,12 +612,13 @@ lstm_recurrent_tc_kernel(const float* __restrict__ pre, const float* __restrict_
                     if (mbar_try_wait(&sh.accum, static_cast<uint32_t>((t - 1) & 1))) { ok = true; break; }
                     if (clock64() - start > 2 * kRtcWaitCycles) break;
                 }
+                ok = __all_sync(kFullMask, ok);
                 if (!ok) {
                     sh.abort_flag = 1;
                     if (status != nullptr && lane == 0) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
                 }
                 // warps 4 and 5 own the TMEM lane quadrants 0 and 1 (rows 0..31, 32..63)
-                if ((warp == 4 || warp == 5) && !sh.abort_flag) {
+                if ((warp == 4 || warp == 5) && ok) {
                     tc_fence_after();
                     const int q = warp & 3;
                     float acc[16];
@@ -613,8 +628,7 @@ lstm_recurrent_tc_kernel(const float* __restrict__ pre, const float* __restrict_
                     for (int i = 0; i < 16; ++i) grow[i] = acc[i];
                     tc_fence_before();
                 }
-                epi_barrier();
-                if (sh.abort_flag) break;
+                if (epi_barrier_any(!ok)) break;  // all threads leave in the same step
 #pragma unroll
                 for (int g = 0; g < 4; ++g) s_g[g] = sh.gates[eb * kRtcGateStride + g * kRtcUnits + eu];
             }

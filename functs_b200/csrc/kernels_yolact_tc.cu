@@ -102,6 +102,7 @@ __device__ __forceinline__ void yt_mma(uint32_t d_tmem, uint64_t a_desc, uint64_
 
 // eight TMEM columns, one 32-bit value each per lane
 __device__ __forceinline__ void yt_columns(uint32_t taddr, uint2 list, float (&s)[8]) {
+    __syncwarp();
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
         const uint32_t col = ((u < 4 ? list.x : list.y) >> (8 * (u & 3))) & 255u;
@@ -162,6 +163,7 @@ yolact_masks_tc_kernel(const float* __restrict__ proto, const float* __restrict_
         fence_barrier_init();
     }
     if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
