@@ -10,6 +10,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAException.h>
+#include <c10/cuda/CUDAGuard.h>
 
 #include "../../../include/functs_b200.h"
 #include "detect.h"
@@ -20,6 +21,18 @@ namespace py = pybind11;
 using torch::jit::Graph;
 
 namespace {
+// What a kernel may be pointed at: float32 on `device`.
+void checkInput(const at::Tensor& t, const at::Device& device, const char* name) {
+    TORCH_CHECK_VALUE(t.is_cuda(), name, " must be a CUDA tensor (functs_b200 has no CPU path)");
+    TORCH_CHECK_VALUE(t.device() == device, name, " must be on ", device, ", not on ", t.device());
+    TORCH_CHECK_TYPE(t.scalar_type() == at::kFloat, name, " must be torch.float32");
+}
+// The same for memory that a kernel writes, or reads as it lies.
+void checkBuffer(const at::Tensor& t, const at::Device& device, at::ScalarType dtype, at::IntArrayRef sizes, const char* name) {
+    TORCH_CHECK_VALUE(t.device() == device && t.scalar_type() == dtype && t.is_contiguous() && t.sizes() == sizes, name, " must be a contiguous ",
+                      dtype, " tensor of sizes ", sizes, " on ", device);
+}
+
 // Appends (dets, labels) to a Python list, from code that runs without the interpreter lock.
 functs_b200::EmitImage appendTo(py::list& out) {
     return [&out](functs_b200::Detections&& d) {
@@ -158,13 +171,26 @@ PYBIND11_MODULE(_C, m) {
                               const at::Tensor& hs, const at::Tensor& cs, const at::Tensor& scratch, const at::Tensor& status, int64_t mode,
                               bool wait) -> int64_t {
         py::gil_scoped_release release;
-        TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (functs_b200 has no CPU path)");
-        TORCH_CHECK_TYPE(x.scalar_type() == at::kFloat, "x must be torch.float32");
+        checkInput(x, x.device(), "x");
+        TORCH_CHECK_VALUE(x.dim() == 3 && w_hh.dim() == 3, "x must be [T, B, I], w_hh [4, H, H]");
         const int64_t T = x.size(0), B = x.size(1), I = x.size(2), H = w_hh.size(2);
-        TORCH_CHECK_VALUE(w_ih.dim() == 3 && w_ih.size(0) == 4 && w_ih.size(1) == I && w_ih.size(2) == H && w_hh.dim() == 3 &&
-                              w_hh.size(0) == 4 && w_hh.size(1) == H,
+        TORCH_CHECK_VALUE(w_ih.dim() == 3 && w_ih.size(0) == 4 && w_ih.size(1) == I && w_ih.size(2) == H && w_hh.size(0) == 4 &&
+                              w_hh.size(1) == H,
                           "weights must be gate-leading: w_ih [4, I, H], w_hh [4, H, H]");
         TORCH_CHECK_VALUE(b_ih.numel() == 4 * H && b_hh.numel() == 4 * H, "biases must have 4*H elements");
+        checkBuffer(w_ih, x.device(), at::kFloat, w_ih.sizes(), "w_ih");
+        checkBuffer(w_hh, x.device(), at::kFloat, w_hh.sizes(), "w_hh");
+        checkBuffer(b_ih, x.device(), at::kFloat, b_ih.sizes(), "b_ih");
+        checkBuffer(b_hh, x.device(), at::kFloat, b_hh.sizes(), "b_hh");
+        checkBuffer(hs, x.device(), at::kFloat, {T, B, H}, "hs");
+        checkBuffer(cs, x.device(), at::kFloat, {T, B, H}, "cs");
+        const int64_t need = functs_b200_lstm_scratch_bytes(static_cast<int32_t>(T), static_cast<int32_t>(B), static_cast<int32_t>(I),
+                                                            static_cast<int32_t>(H));
+        TORCH_CHECK_VALUE(scratch.device() == x.device() && scratch.is_contiguous() && static_cast<int64_t>(scratch.nbytes()) >= need,
+                          "scratch must hold ", need, " bytes on ", x.device());
+        TORCH_CHECK_VALUE(status.is_cpu() && status.scalar_type() == at::kInt && status.numel() >= 1 && status.is_pinned(),
+                          "status must be an int32 tensor in pinned memory");
+        c10::cuda::CUDAGuard guard(x.device());
         const at::Tensor xc = x.contiguous();
         const auto stream = at::cuda::getCurrentCUDAStream();
         const int rc = functs_b200_lstm_forward_mode(xc.data_ptr<float>(), w_ih.data_ptr<float>(), w_hh.data_ptr<float>(), b_ih.data_ptr<float>(),
@@ -178,15 +204,19 @@ PYBIND11_MODULE(_C, m) {
     // masks into `out` [B, N, H, W]; returns the library's error code
     m.def("_yolact_masks", [](const at::Tensor& proto, const at::Tensor& coef, const at::Tensor& boxes, double thr, const at::Tensor& out) -> int64_t {
         py::gil_scoped_release release;
-        auto checked = [](const at::Tensor& t, const char* name) {
-            TORCH_CHECK_VALUE(t.is_cuda(), name, " must be a CUDA tensor (functs_b200 has no CPU path)");
-            TORCH_CHECK_TYPE(t.scalar_type() == at::kFloat, name, " must be torch.float32");
-            return t.contiguous();
-        };
-        const at::Tensor p = checked(proto, "proto"), c = checked(coef, "coef"), b = checked(boxes, "boxes");
-        TORCH_CHECK_VALUE(p.dim() == 4 && p.size(3) == 32, "prototype depth must be 32");
-        return functs_b200_yolact_masks(p.data_ptr<float>(), c.data_ptr<float>(), b.data_ptr<float>(), static_cast<int32_t>(p.size(0)),
-                                        static_cast<int32_t>(p.size(1)), static_cast<int32_t>(p.size(2)), static_cast<int32_t>(c.size(1)),
+        checkInput(proto, proto.device(), "proto");
+        checkInput(coef, proto.device(), "coef");
+        checkInput(boxes, proto.device(), "boxes");
+        TORCH_CHECK_VALUE(proto.dim() == 4 && proto.size(3) == 32, "prototype depth must be 32");
+        const int64_t B = proto.size(0), H = proto.size(1), W = proto.size(2);
+        TORCH_CHECK_VALUE(coef.dim() == 3 && coef.size(0) == B && coef.size(2) == 32 && boxes.dim() == 3 && boxes.size(0) == B &&
+                              boxes.size(1) == coef.size(1) && boxes.size(2) == 4,
+                          "proto [B, H, W, 32], coef [B, N, 32] and boxes [B, N, 4] do not fit one another");
+        checkBuffer(out, proto.device(), at::kByte, {B, coef.size(1), H, W}, "out");
+        c10::cuda::CUDAGuard guard(proto.device());
+        const at::Tensor p = proto.contiguous(), c = coef.contiguous(), b = boxes.contiguous();
+        return functs_b200_yolact_masks(p.data_ptr<float>(), c.data_ptr<float>(), b.data_ptr<float>(), static_cast<int32_t>(B),
+                                        static_cast<int32_t>(H), static_cast<int32_t>(W), static_cast<int32_t>(c.size(1)),
                                         static_cast<float>(thr), out.data_ptr<uint8_t>(), nullptr, at::cuda::getCurrentCUDAStream().stream());
     });
     m.def("_count_parallel_functors", [](std::shared_ptr<Graph> g) { return functs_b200::CountParallelFunctors(g); });

@@ -281,6 +281,10 @@ def yolact_masks(proto: torch.Tensor, coef: torch.Tensor, boxes: torch.Tensor, t
     if k != 32:
         raise ValueError("prototype depth must be 32")
     n = coef.size(1)
+    if tuple(coef.shape) != (b, n, 32) or tuple(boxes.shape) != (b, n, 4):
+        raise ValueError("proto [B, H, W, 32], coef [B, N, 32] and boxes [B, N, 4] do not fit one another")
+    if out is not None and (tuple(out.shape) != (b, n, h, w) or out.dtype != torch.uint8 or not out.is_contiguous()):
+        raise ValueError("out must be a contiguous uint8 [B, N, H, W] tensor")
     masks = out if out is not None else torch.empty(b, n, h, w, dtype=torch.uint8, device=proto.device)
     logits = torch.empty(b, n, h, w, dtype=torch.float32, device=proto.device) if with_logits else None
     check(lib.functs_b200_yolact_masks(_ptr(proto), _ptr(coef), _ptr(boxes), b, h, w, n, float(thr), _ptr(masks),

@@ -148,6 +148,7 @@ class LSTM:
         self.b_ih = b_ih.to(self.device, torch.float32).reshape(4, -1).contiguous()
         self.b_hh = b_hh.to(self.device, torch.float32).reshape(4, -1).contiguous()
         self._scratch = None
+        self._sizes = None
         self._out = None
         # in host memory: the kernels write it only when something went wrong, and reading it takes no copy
         self._status = torch.zeros(1, dtype=torch.int32).pin_memory()
@@ -169,12 +170,13 @@ class LSTM:
     def _buffers(self, x: torch.Tensor) -> None:
         t, b, i = x.shape
         h = self.w_hh.size(2)
-        if self._out is None or self._out[0].shape != (t, b, h):
+        if self._sizes != (t, b, i):
             self._out = (torch.empty(t, b, h, dtype=torch.float32, device=self.device),
                          torch.empty(t, b, h, dtype=torch.float32, device=self.device))
             from ._lib import lib
             self._scratch = torch.empty(int(lib.functs_b200_lstm_scratch_bytes(t, b, i, h)), dtype=torch.uint8,
                                         device=self.device)
+            self._sizes = (t, b, i)
 
     def _run(self, x: torch.Tensor, mode: int, wait: bool) -> None:
         before = launch_count()

@@ -243,3 +243,43 @@ def test_yolact_boxes_outside_the_integers(fb, height, width, far):
     masks, _ = fb.ops.yolact_masks(proto, coef, boxes, with_logits=True)
     assert masks.flatten(2).sum(2).tolist() == [[n * height * width for n in (0, 0, 1, 0, 0, 1)]]
     assert torch.equal(fb.ops.yolact_masks(proto, coef, boxes), masks)
+
+
+def test_yolact_rejects_shapes_that_do_not_fit(fb):
+    """Sizes come from proto and coef: anything else that the kernel would read or write beside them is refused on the host."""
+    mod = fb.workloads.YolactBBoxMask()
+    proto, coef, boxes = [t.cuda() for t in W.make_yolact_inputs(2, size=20, num_det=7)]
+    want = mod(proto, coef, boxes).clone()
+    bad = [(proto, coef[:1], boxes), (proto, coef, boxes[:1]), (proto, coef, boxes[:, :6]), (proto, coef[..., :31], boxes),
+           (proto, coef, boxes[..., :3]), (proto[..., :31], coef, boxes), (proto[0], coef, boxes)]
+    for args in bad:
+        with pytest.raises(ValueError):
+            mod(*args)
+        with pytest.raises(ValueError):
+            fb.ops.yolact_masks(*args)
+    with pytest.raises(ValueError):
+        fb.ops.yolact_masks(proto, coef, boxes, out=torch.empty(2, 7, 20, 18, dtype=torch.uint8, device="cuda"))
+    with pytest.raises(TypeError):
+        mod(proto.double(), coef, boxes)
+    assert torch.equal(mod(proto, coef, boxes), want)
+
+
+def test_lstm_rejects_buffers_that_do_not_fit(fb):
+    x, w_ih, w_hh, b_ih, b_hh = W.make_lstm_inputs(2, 3, 256)
+    mod = fb.workloads.LSTM(w_ih, w_hh, b_ih, b_hh)
+    # an input of another depth is refused, and the buffers allocated for it do not serve the next call
+    with pytest.raises(ValueError):
+        mod(x[..., :8])
+    hs, cs = mod(x)
+    want = W.LSTMSeq(w_ih, w_hh, b_ih, b_hh)(x)
+    close(hs.cpu(), want[0], rtol=1e-5, scale=1.0, what="hs")
+    native = fb.workloads._native()._lstm_forward
+    ok = [x.cuda(), mod.w_ih, mod.w_hh, mod.b_ih, mod.b_hh, hs, cs, mod._scratch, mod._status, 0, True]
+    assert native(*ok) == 0
+    for at, other in [(0, x[0].cuda()), (1, mod.w_ih.transpose(1, 2)), (1, mod.w_ih.double()), (2, mod.w_hh[:3]), (3, mod.b_ih[:, :255]),
+                      (5, hs[:1]), (6, cs[..., :255]), (7, mod._scratch[:-256]), (8, torch.zeros(1, dtype=torch.int32)),
+                      (8, torch.zeros(1, dtype=torch.int32, device="cuda")), (1, mod.w_ih.cpu())]:
+        args = list(ok)
+        args[at] = other
+        with pytest.raises(ValueError):
+            native(*args)
