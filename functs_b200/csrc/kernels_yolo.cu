@@ -437,15 +437,23 @@ yolo_decode_dense_kernel(const __grid_constant__ YoloDecodeArgs A) {
     if (A.cls_out != nullptr) {
         constexpr int kQuads = kYoloClasses / 4;
         const int total = min(kDecThreads, nslots - T.s0) * kQuads;
-        float4* out = reinterpret_cast<float4*>(A.cls_out + static_cast<int64_t>(T.img) * L.num_boxes * kYoloClasses);
-        int slot = t / kQuads, c = t - slot * kQuads;
-        for (int i = t; i < total; i += kDecThreads) {
-            out[static_cast<int64_t>(live[slot].box) * kQuads + c] = *reinterpret_cast<const float4*>(s_cls + slot * kDenseRow + 4 * c);
-            slot += kDecThreads / kQuads;
-            c += kDecThreads % kQuads;
-            if (c >= kQuads) {
-                c -= kQuads;
-                ++slot;
+        float* img_out = A.cls_out + static_cast<int64_t>(T.img) * L.num_boxes * kYoloClasses;
+        if ((reinterpret_cast<uintptr_t>(img_out) & 15) == 0) {
+            float4* out = reinterpret_cast<float4*>(img_out);
+            int slot = t / kQuads, c = t - slot * kQuads;
+            for (int i = t; i < total; i += kDecThreads) {
+                out[static_cast<int64_t>(live[slot].box) * kQuads + c] = *reinterpret_cast<const float4*>(s_cls + slot * kDenseRow + 4 * c);
+                slot += kDecThreads / kQuads;
+                c += kDecThreads % kQuads;
+                if (c >= kQuads) {
+                    c -= kQuads;
+                    ++slot;
+                }
+            }
+        } else {  // a caller's array off a 16-byte boundary
+            for (int i = t; i < 4 * total; i += kDecThreads) {
+                const int slot = i / kYoloClasses, c = i - slot * kYoloClasses;
+                img_out[static_cast<int64_t>(live[slot].box) * kYoloClasses + c] = s_cls[slot * kDenseRow + c];
             }
         }
     }
@@ -493,8 +501,7 @@ static int launch_yolo_decode(const YoloDecodeArgs& a, int batch, bool pdl, cuda
     FB_REQUIRE(a.keys && a.counts, "yolo_decode: null pointer");
     FB_REQUIRE(a.capacity > 0, "yolo_decode: bad sizes");
     FB_REQUIRE(a.thr > 0.0f, "yolo_decode: score threshold must be positive (keys require positive scores)");
-    FB_REQUIRE(((reinterpret_cast<uintptr_t>(a.boxes) | reinterpret_cast<uintptr_t>(a.cls_out)) & 15) == 0,
-               "yolo_decode: boxes and class scores must be 16-byte aligned");
+    FB_REQUIRE((reinterpret_cast<uintptr_t>(a.boxes) & 15) == 0, "yolo_decode: boxes must be 16-byte aligned");
     auto tiles = [&](int slots) {
         int n = 0;
         for (int l = 0; l < 3; ++l) n += (3 * a.L.plane[l] + slots - 1) / slots;

@@ -285,3 +285,18 @@ def test_yolo_one_call_form_at_its_edges(fb, batch, sizes, kind, topk):
         m = int(cnt[b])
         assert m == wf.numel() and torch.equal(flat[b, :m], wf) and torch.equal(labels[b, :m], wl) and torch.equal(dets[b, :m], wd)
         assert torch.equal(lists[b][0].cpu(), wd) and torch.equal(lists[b][1].cpu(), wl)
+
+
+def test_yolo_dense_class_scores_off_a_16_byte_boundary(fb):
+    """The class-score output only has to be aligned to its elements."""
+    sizes = (5, 9, 17)  # 395 boxes x 3: a ragged last tile on every level
+    maps = [torch.randn(2, 255, s, s, generator=torch.Generator().manual_seed(s)).cuda() for s in sizes]
+    boxes, obj, cls, keys, counts = fb.ops.yolo_decode(maps, 0.5, dense=True)
+    for shift in (1, 2, 3):
+        room = torch.full((cls.numel() + 4,), 7.0, device="cuda")
+        boxes2, keys2, counts2 = torch.empty_like(boxes), torch.empty_like(keys), torch.empty_like(counts)
+        fb._lib.check(fb._lib.lib.functs_b200_yolo_decode(*[m.data_ptr() for m in maps], 2, *sizes, 0.5, boxes2.data_ptr(), None,
+                                                          room.data_ptr() + 4 * shift, keys2.data_ptr(), counts2.data_ptr(), keys.size(1), None,
+                                                          None, torch.cuda.current_stream().cuda_stream), "yolo_decode")
+        assert torch.equal(room[shift:shift + cls.numel()].view_as(cls), cls) and torch.equal(counts2, counts)
+        assert bool((room[:shift] == 7.0).all()) and bool((room[shift + cls.numel():] == 7.0).all())
