@@ -596,6 +596,7 @@ int functs_b200_yolo_postprocess_dense(const float* map0, const float* map1, con
                                        float iou_thr, int64_t capacity, float* boxes, float* obj_out, float* cls_out,
                                        float* dets, int64_t* labels, int64_t* flat_ids, int32_t* out_counts,
                                        int32_t* records, int32_t* status, void* scratch, void* stream) {
+    FB_REQUIRE(boxes != nullptr && flat_ids != nullptr, "yolo_postprocess: null pointer");
     return functs_b200_yolo_detect(map0, map1, map2, batch, s0, s1, s2, score_thr, topk, iou_thr, capacity, boxes, obj_out,
                                    cls_out, dets, labels, flat_ids, out_counts, records, nullptr, status, scratch, stream);
 }

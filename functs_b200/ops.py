@@ -189,11 +189,11 @@ class YoloPostprocessPlan:
         if records is not None and (records.dtype != torch.int32 or not records.is_contiguous()
                                     or records.numel() != self.batch * self.topk * 8):
             raise ValueError("records must be a contiguous int32 [batch, topk, 8] tensor")
-        check(lib.functs_b200_yolo_postprocess_dense(maps[0].data_ptr(), maps[1].data_ptr(), maps[2].data_ptr(), self.batch,
-                                                     s[0], s[1], s[2], float(score_thr), self.topk, float(iou_thr),
-                                                     self.capacity, _ptr(self.boxes) if all_boxes else None, None, None, _ptr(self.dets),
-                                                     _ptr(self.labels), _ptr(self.flat_ids), _ptr(self.counts),
-                                                     _ptr(records), _ptr(self.status), _ptr(self.scratch), _stream()),
+        check(lib.functs_b200_yolo_detect(maps[0].data_ptr(), maps[1].data_ptr(), maps[2].data_ptr(), self.batch, s[0], s[1], s[2],
+                                          float(score_thr), self.topk, float(iou_thr), self.capacity,
+                                          _ptr(self.boxes) if all_boxes else None, None, None, _ptr(self.dets), _ptr(self.labels),
+                                          _ptr(self.flat_ids), _ptr(self.counts), _ptr(records), None, _ptr(self.status),
+                                          _ptr(self.scratch), _stream()),
               "yolo_postprocess")
 
 

@@ -40,3 +40,16 @@ def test_argument_errors_without_gpu():
         assert lib.functs_b200_group_lookup(sig) == i
     assert lib.functs_b200_yolo_scratch_bytes(64, 13, 26, 52, 10647 * 80, 1000) > 64 * 10647 * 80 * 8
     assert lib.functs_b200_lstm_scratch_bytes(64, 64, 512, 512) >= 64 * 64 * 2048 * 4
+
+
+def test_yolo_postprocess_needs_its_box_and_id_outputs():
+    """Only functs_b200_yolo_detect takes NULL for them; refused before anything is launched."""
+    from functs_b200 import _lib
+    p = 4096         # never dereferenced:
+    scratch = p + 1  # a scratch off its boundary is refused as well
+    for boxes, ids in ((None, p), (p, None)):
+        assert _lib.lib.functs_b200_yolo_postprocess(p, p, p, 1, 1, 1, 1, 0.5, 10, 0.45, 720, boxes, p, p, ids, p, p, scratch, None) == -1
+        assert "null" in _lib.last_error()
+        assert _lib.lib.functs_b200_yolo_postprocess_dense(p, p, p, 1, 1, 1, 1, 0.5, 10, 0.45, 720, boxes, None, None, p, p, ids, p, None, p,
+                                                           scratch, None) == -1
+        assert "null" in _lib.last_error()
