@@ -49,7 +49,7 @@ def test_yolo_postprocess_needs_its_box_and_id_outputs():
     scratch = p + 1  # a scratch off its boundary is refused as well
     for boxes, ids in ((None, p), (p, None)):
         assert _lib.lib.functs_b200_yolo_postprocess(p, p, p, 1, 1, 1, 1, 0.5, 10, 0.45, 720, boxes, p, p, ids, p, p, scratch, None) == -1
-        assert "null" in _lib.last_error()
+        assert "null pointer" in _lib.last_error()
         assert _lib.lib.functs_b200_yolo_postprocess_dense(p, p, p, 1, 1, 1, 1, 0.5, 10, 0.45, 720, boxes, None, None, p, p, ids, p, None, p,
                                                            scratch, None) == -1
-        assert "null" in _lib.last_error()
+        assert "null pointer" in _lib.last_error()
