@@ -231,3 +231,36 @@ def test_programs_cut_into_regions(env, fn, shape):
     x = torch.randn(*shape, generator=g).cuda()
     args = {scaled: (x, 0.75), class_deltas: (torch.randn(shape[0], 4, generator=g).cuda(), x)}.get(fn, (x,))
     check(env, fn, args)
+
+
+def bounds(x: torch.Tensor, y: torch.Tensor):
+    t = x.clone()
+    t[:, 0] = torch.relu(t[:, 0])
+    t[:, 1] = torch.clamp(t[:, 1], min=-0.5, max=0.75)
+    return torch.maximum(torch.minimum(t, y), y * 0.5 - 1.0)
+
+
+def bounds_of_scales(feats: List[torch.Tensor]):
+    outs: List[torch.Tensor] = []
+    for i in range(2):
+        x = feats[i].clone()
+        x[:, 0:2] = torch.clamp(torch.relu(x[:, 0:2]), max=0.5)
+        outs.append(x * 2.0)
+    return outs
+
+
+@pytest.mark.parametrize("rows", [5, 200003])
+def test_nan_passes_relu_clamp_maximum_and_minimum(env, rows):
+    """As in eager mode, in the kernels for small and large regions and in the one for maps."""
+    fb, J = env
+    g = torch.Generator().manual_seed(15)
+    x, y = torch.randn(rows, 3, generator=g).cuda(), torch.randn(rows, 3, generator=g).cuda()
+    x[::2], y[1::4] = float("nan"), float("nan")
+    for fn, args in ((bounds, (x, y)), (bounds_of_scales, ([x, y[:4]],))):
+        built = J.build(fn, args)
+        built(*args)
+        g0 = J.generic_group_runs()
+        got, want = built(*args), fn(*args)
+        assert J.generic_group_runs() > g0
+        for a, b in zip(got, want):
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(nan=7.0), b.nan_to_num(nan=7.0))
