@@ -71,6 +71,18 @@ __device__ __forceinline__ void sigmoid_f32_n(float (&v)[N]) {
     }
 }
 
+// The larger / smaller of two values, NaN if one of them is: what relu, clamp, maximum and minimum of ATen give.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // Candidate key: score bits in the high word, inverted flat index in the low word, so that
 // "larger key" == "larger score, then smaller index".  Requires score > 0.
 __device__ __forceinline__ uint64_t make_key(float score, uint32_t flat_idx) {

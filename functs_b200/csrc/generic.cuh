@@ -15,27 +15,15 @@ __device__ __forceinline__ float g_fetch(const void* p, int dtype, int off) {
     }
 }
 
-// The larger / smaller of two values, NaN if one of them is: what relu, clamp, maximum and minimum of ATen give.
-__device__ __forceinline__ float g_max(float a, float b) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float g_min(float a, float b) {
-    float r;
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-
 __device__ __forceinline__ float g_unary(int op, float a, float imm) {
     switch (op) {
         case FB_G_EXP: return expf(a);
         case FB_G_SIGMOID: return sigmoid_f32(a);
         case FB_G_TANH: return tanhf(a);
-        case FB_G_RELU: return g_max(a, 0.0f);
+        case FB_G_RELU: return max_nan(a, 0.0f);
         case FB_G_NEG: return -a;
-        case FB_G_CLAMP_MIN: return g_max(a, imm);
-        case FB_G_CLAMP_MAX: return g_min(a, imm);
+        case FB_G_CLAMP_MIN: return max_nan(a, imm);
+        case FB_G_CLAMP_MAX: return min_nan(a, imm);
         case FB_G_ABS: return fabsf(a);
         case FB_G_SQRT: return sqrtf(a);
         case FB_G_LOG: return logf(a);
@@ -49,8 +37,8 @@ __device__ __forceinline__ float g_binary(int op, float a, float b) {
         case FB_G_SUB: return __fsub_rn(a, b);
         case FB_G_MUL: return __fmul_rn(a, b);
         case FB_G_DIV: return __fdiv_rn(a, b);
-        case FB_G_MIN: return g_min(a, b);
-        case FB_G_MAX: return g_max(a, b);
+        case FB_G_MIN: return min_nan(a, b);
+        case FB_G_MAX: return max_nan(a, b);
         case FB_G_GT: return a > b ? 1.0f : 0.0f;
         case FB_G_GE: return a >= b ? 1.0f : 0.0f;
         case FB_G_LT: return a < b ? 1.0f : 0.0f;

@@ -80,10 +80,10 @@ ssd_softmax_decode_kernel(const float* __restrict__ loc, const float* __restrict
         const float gh = __fmul_rn(pr.w, expf(__fmul_rn(d.w, 0.2f)));
         const float hw = __fmul_rn(gw, 0.5f), hh = __fmul_rn(gh, 0.5f);
         float4 o;
-        o.x = fminf(fmaxf(__fsub_rn(gx, hw), 0.0f), clamp_max);
-        o.y = fminf(fmaxf(__fsub_rn(gy, hh), 0.0f), clamp_max);
-        o.z = fminf(fmaxf(__fadd_rn(gx, hw), 0.0f), clamp_max);
-        o.w = fminf(fmaxf(__fadd_rn(gy, hh), 0.0f), clamp_max);
+        o.x = min_nan(max_nan(__fsub_rn(gx, hw), 0.0f), clamp_max);
+        o.y = min_nan(max_nan(__fsub_rn(gy, hh), 0.0f), clamp_max);
+        o.z = min_nan(max_nan(__fadd_rn(gx, hw), 0.0f), clamp_max);
+        o.w = min_nan(max_nan(__fadd_rn(gy, hh), 0.0f), clamp_max);
         reinterpret_cast<float4*>(boxes)[static_cast<int64_t>(img) * num_priors + p] = o;
     }
     __syncthreads();

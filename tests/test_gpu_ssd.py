@@ -97,6 +97,26 @@ def test_ssd_ragged_small(fb):
     run_case(fb, loc, conf, pri, thr=0.05, topk=50)
 
 
+def test_ssd_nan_in_the_deltas_stays_in_the_boxes(fb):
+    """The strided clamp keeps a NaN, as clamp_ does; such a box suppresses nothing and nothing suppresses it."""
+    g = torch.Generator().manual_seed(10)
+    p, c = 333, 5
+    pri = torch.cat([torch.rand(p, 2, generator=g) * 300, torch.rand(p, 2, generator=g) * 80 + 4], dim=1)
+    loc = torch.randn(1, p, 4, generator=g)
+    loc[0, torch.arange(0, p, 3), torch.randint(0, 4, (111,), generator=g)] = float("nan")
+    conf = torch.randn(1, p, c + 1, generator=g) * 2
+    o = W.SSDPost(score_thr=0.05, topk=200)
+    o.priors = pri
+    mod = fb.workloads.SSDBBox(pri, score_thr=0.05, topk=200)
+    boxes, dets, ids, counts = mod.forward_padded(loc, conf)
+    boxes_c, scores_c = boxes[0].cpu(), mod._bufs[2][0].cpu().t().contiguous()
+    assert torch.equal(boxes_c.isnan(), o(loc, conf)[0][0].isnan())
+    want = o.post_single(boxes_c, scores_c)
+    got = mod.unpad(dets, ids, counts)[0]
+    assert torch.equal(got[2].cpu(), want[2]) and torch.equal(got[1].cpu(), want[1])
+    assert torch.equal(got[0].cpu().nan_to_num(nan=-7.0), want[0].nan_to_num(nan=-7.0))
+
+
 def test_ssd_golden_decode(fb):
     """Decode against the fixture written by the reference's delta2bbox (clamp 320)."""
     import os
