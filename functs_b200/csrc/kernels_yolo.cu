@@ -149,6 +149,8 @@ constexpr int kDecThreads = 128;
 constexpr int kDecWarps = kDecThreads / 32;
 constexpr int kDecClasses = kYoloClasses / kDecWarps;  // classes per warp
 constexpr int kDecStep = 10;                           // of which loaded at a time
+constexpr int kDenseRow = kYoloClasses + 4;  // floats per slot of the dense form's staging: an odd number of 16-byte chunks, so that
+                                             // eight neighbouring slots store to different banks
 
 struct YoloDecodeArgs {
     YoloLevels L;
@@ -214,23 +216,6 @@ __device__ __forceinline__ void yolo_append(const YoloDecodeArgs& A, int img, bo
     }
 }
 
-// A tile whose hits did not fit the queue is walked once more, one live slot per thread.
-__device__ __noinline__ void yolo_crowded_tile(const YoloDecodeArgs* A, const float* img_map, int plane, int img, const YoloLive* live, int n,
-                                               float bar) {
-    for (int i0 = 0; i0 < n; i0 += kDecThreads) {
-        const int i = i0 + static_cast<int>(threadIdx.x);
-        YoloLive o{0.0f, INFINITY, 0, 0u};
-        if (i < n) o = live[i];
-        const float cut = i < n ? logit_cut(o.so, bar) : INFINITY;
-        for (int c = 0; c < kYoloClasses; ++c) {
-            const float v = i < n ? __ldg(img_map + o.off + c * plane) : 0.0f;
-            float s = 0.0f;
-            if (v > cut) s = __fmul_rn(o.so, sigmoid_f32(v));
-            yolo_append(*A, img, s > A->thr && s >= bar, s, o.box * kYoloClasses + static_cast<uint32_t>(c));
-        }
-    }
-}
-
 // The queued hits of a tile, evaluated together.
 template <bool DENSE>
 __device__ __forceinline__ void yolo_eval_queue(const YoloDecodeArgs& A, const YoloLive* live, const YoloHit* queue, int img, int n, float bar) {
@@ -250,6 +235,99 @@ __device__ __forceinline__ void yolo_eval_queue(const YoloDecodeArgs& A, const Y
     }
 }
 
+// The same for a long queue: a warp evaluates its share first and makes room for all of it with one atomic (one for 32 hits
+// each waits for the one before).  The evaluated scores go back to the queue.
+template <bool DENSE>
+__device__ __forceinline__ void yolo_eval_many(const YoloDecodeArgs& A, const YoloLive* live, YoloHit* queue, int img, int n, float bar) {
+    constexpr uint32_t kNone = 0xffffffffu;
+    const int t = threadIdx.x, lane = t & 31;
+    int found = 0;
+    for (int i0 = 0; i0 < n; i0 += kDecThreads) {
+        const int i = i0 + t;
+        bool pass = false;
+        if (i < n) {
+            const YoloHit h = queue[i];
+            const YoloLive o = live[h.meta >> 7];
+            const float s = DENSE ? h.v : __fmul_rn(o.so, sigmoid_f32(h.v));
+            pass = s > A.thr && s >= bar;
+            queue[i] = YoloHit{s, pass ? o.box * kYoloClasses + (h.meta & 127u) : kNone};  // (flat indices are below 2^32 - 1)
+        }
+        found += __popc(__ballot_sync(kFullMask, pass));
+    }
+    if (found == 0) return;
+    int64_t at = 0;
+    if (lane == 0) at = atomicAdd(A.counts + img, found);
+    at = __shfl_sync(kFullMask, at, 0);
+    for (int i0 = 0; i0 < n; i0 += kDecThreads) {
+        const int i = i0 + t;
+        const YoloHit h = i < n ? queue[i] : YoloHit{0.0f, kNone};
+        const unsigned m = __ballot_sync(kFullMask, h.meta != kNone);
+        if (h.meta != kNone) {
+            const int64_t k = at + __popc(m & ((1u << lane) - 1u));
+            if (k < A.capacity) A.keys[img * A.capacity + k] = make_key(h.v, h.meta);
+            else if (A.status != nullptr) atomicOr(A.status, FB_STATUS_CAND_OVERFLOW);
+            if (A.hist != nullptr)
+                atomicAdd(A.hist + static_cast<int64_t>(img) * kHistBins +
+                              hist_digit(static_cast<uint64_t>(__float_as_uint(h.v)) << 32, A.hist_base, A.hist_shift), 1);
+        }
+        at += __popc(m);
+    }
+}
+
+// All candidates of a tile, for callers without a floor and for tiles whose hits did not fit the queue: in rounds of 32 live slots
+// and STEP classes per warp; the queue is evaluated whenever another round might not fit (room: its entries).  DENSE: the class
+// scores come from s_cls.  (One live slot per thread through all its classes with an append for every class took 375 us for 32
+// images at N(0, 1), seven candidates in a hundred: 320 global atomics a tile, most of them for a hit or two.)
+template <int STEP>
+constexpr int kRoundHits = 32 * STEP * kDecWarps;
+template <bool DENSE, int STEP>
+__device__ __noinline__ void yolo_collect_all(const YoloDecodeArgs* A, const float* img_map, int plane, int img, const YoloLive* live, int n,
+                                              float bar, YoloHit* queue, int room, int* counter, const float* s_cls) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    __syncthreads();  // whoever filled the queue before has seen how far
+    if (t == 0) *counter = 0;
+    __syncthreads();
+    constexpr int kSteps = kDecClasses / STEP;
+    static_assert(kDecClasses % STEP == 0, "whole steps");
+    const int rounds = (n + 31) / 32 * kSteps;
+    float v[STEP], cut = 0.0f;
+    uint32_t first = 0u;  // of this lane's values: live slot << 7 | class
+    auto load = [&](int round) {
+        const int i = round / kSteps * 32 + lane, k0 = warp * kDecClasses + round % kSteps * STEP;
+        const bool on = i < n;
+        YoloLive o{0.0f, INFINITY, 0, 0u};
+        if (on) o = live[i];
+        cut = o.cut;
+        first = static_cast<uint32_t>(i << 7 | k0);
+#pragma unroll
+        for (int u = 0; u < STEP; ++u) {
+            if (DENSE) v[u] = on ? __fmul_rn(o.so, s_cls[i * kDenseRow + k0 + u]) : 0.0f;
+            else v[u] = on ? __ldg(img_map + o.off + (k0 + u) * plane) : -INFINITY;
+        }
+    };
+    load(0);
+#pragma unroll 1
+    for (int round = 0; round < rounds; ++round) {
+        uint32_t hits = 0u;
+#pragma unroll
+        for (int u = 0; u < STEP; ++u) hits |= (DENSE ? v[u] > A->thr && v[u] >= bar : v[u] > cut) ? 1u << u : 0u;
+        int at = 0;
+        if (hits != 0u) {
+            at = atomicAdd(counter, __popc(hits));
+#pragma unroll
+            for (int u = 0; u < STEP; ++u)
+                if ((hits >> u) & 1u) queue[at++] = YoloHit{v[u], first + static_cast<uint32_t>(u)};
+        }
+        const bool last = round + 1 == rounds;
+        if (!last) load(round + 1);  // on its way while this round's hits are evaluated
+        if (__syncthreads_or(last || at > room - kRoundHits<STEP> ? 1 : 0) == 0) continue;
+        yolo_eval_many<DENSE>(*A, live, queue, img, *counter, bar);
+        __syncthreads();
+        if (t == 0) *counter = 0;
+        __syncthreads();
+    }
+}
+
 // One CTA per tile of 128 * E slots.  First the objectness of its slots, E per thread; the slots that clear the bar (one in seven
 // at N(0, 1), a few per cent behind a trained head) are listed in shared memory; then lane k of every warp takes live slot k
 // through the warp's twenty class planes.  The planes are streamed from DRAM almost whole either way (a 128-byte line rarely
@@ -257,11 +335,14 @@ __device__ __forceinline__ void yolo_eval_queue(const YoloDecodeArgs& A, const Y
 // ones included, executed 17 to 22 million warp instructions for 64 images and took 42 to 53 us whatever the loads looked
 // like (registers, ten planes at a time; asynchronous copies, fifteen at a time, next tile prefetched).
 // E = 4 fills the lanes (70 live slots in 512); E = 1 makes more CTAs where there are few tiles.
-template <int E, bool BOXES>
+// ALL: no floor, every candidate above the threshold is wanted (yolo_collect_all from the start, with a longer queue; in the other
+// form that queue would take the L1 cache its loads need: 64 images 76.0 us instead of 71.2).
+template <int E, bool BOXES, bool ALL>
 __global__ void __launch_bounds__(kDecThreads, 8)
 yolo_decode_kernel(const __grid_constant__ YoloDecodeArgs A) {
     constexpr int kSlots = kDecThreads * E;
-    constexpr int kQueue = 2 * kSlots;  // hits: some 1.5 per live slot with a floor
+    constexpr int kQueue = ALL ? kRoundHits<kDecStep> * 3 / 2 : kRoundHits<kDecStep>;  // hits: some 1.5 per live slot with a floor
+    static_assert(kQueue >= 2 * kSlots, "room for the usual hits of a tile");
     __shared__ YoloLive live[kSlots];
     __shared__ YoloHit queue[kQueue];
     __shared__ int s_live, s_queued;
@@ -319,35 +400,39 @@ yolo_decode_kernel(const __grid_constant__ YoloDecodeArgs A) {
     __syncthreads();
     const int n = s_live;
     if (n == 0) return;
+    bool all = ALL;
+    if (!ALL) {
 #pragma unroll 1
-    for (int i0 = 0; i0 < n; i0 += 32) {
-        const int i = i0 + lane;
-        const bool on = i < n;
-        YoloLive o{0.0f, INFINITY, 0, 0u};
-        if (on) o = live[i];
-        const float* p = img_map + o.off + warp * kDecClasses * plane;
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            const int i = i0 + lane;
+            const bool on = i < n;
+            YoloLive o{0.0f, INFINITY, 0, 0u};
+            if (on) o = live[i];
+            const float* p = img_map + o.off + warp * kDecClasses * plane;
 #pragma unroll 1
-        for (int k0 = 0; k0 < kDecClasses; k0 += kDecStep) {
-            float v[kDecStep];
+            for (int k0 = 0; k0 < kDecClasses; k0 += kDecStep) {
+                float v[kDecStep];
 #pragma unroll
-            for (int u = 0; u < kDecStep; ++u) v[u] = on ? __ldg(p + (k0 + u) * plane) : -INFINITY;
-            uint32_t hits = 0u;
+                for (int u = 0; u < kDecStep; ++u) v[u] = on ? __ldg(p + (k0 + u) * plane) : -INFINITY;
+                uint32_t hits = 0u;
 #pragma unroll
-            for (int u = 0; u < kDecStep; ++u) hits |= v[u] > o.cut ? 1u << u : 0u;
-            if (hits != 0u) {
-                int at = atomicAdd(&s_queued, __popc(hits));
+                for (int u = 0; u < kDecStep; ++u) hits |= v[u] > o.cut ? 1u << u : 0u;
+                if (hits != 0u) {
+                    int at = atomicAdd(&s_queued, __popc(hits));
 #pragma unroll
-                for (int u = 0; u < kDecStep; ++u) {
-                    if ((hits >> u) & 1u) {
-                        if (at < kQueue) queue[at] = YoloHit{v[u], static_cast<uint32_t>(i << 7 | (warp * kDecClasses + k0 + u))};
-                        ++at;
+                    for (int u = 0; u < kDecStep; ++u) {
+                        if ((hits >> u) & 1u) {
+                            if (at < kQueue) queue[at] = YoloHit{v[u], static_cast<uint32_t>(i << 7 | (warp * kDecClasses + k0 + u))};
+                            ++at;
+                        }
                     }
                 }
             }
         }
+        __syncthreads();
+        all = s_queued > kQueue;
     }
-    __syncthreads();
-    if (s_queued > kQueue) yolo_crowded_tile(&A, img_map, plane, T.img, live, n, bar);
+    if (all) yolo_collect_all<false, kDecStep>(&A, img_map, plane, T.img, live, n, bar, queue, kQueue, &s_queued, nullptr);
     else yolo_eval_queue<false>(A, live, queue, T.img, s_queued, bar);
 }
 
@@ -357,12 +442,13 @@ yolo_decode_kernel(const __grid_constant__ YoloDecodeArgs A) {
 // The exact sigmoid of every logit bounds it (some twenty instructions each), so everything else goes four classes at a time, with
 // reciprocals that the compiler can interleave; and the class loop stays a loop: unrolled, a warp passes once through 30 KB of
 // instructions and waits for most of them to arrive (49 us for 8 images of 608 x 608; 36 as it is).
-constexpr int kDenseRow = kYoloClasses + 4;  // an odd number of 16-byte chunks: eight neighbouring slots store to different banks
-constexpr int kDenseQueue = 512;
+// ALL: no floor (790 hits in a tile at N(0, 1)).
+template <bool ALL>
 __global__ void __launch_bounds__(kDecThreads, 4)
 yolo_decode_dense_kernel(const __grid_constant__ YoloDecodeArgs A) {
     __shared__ YoloLive live[kDecThreads];  // every slot of the tile; so = 0: it cannot yield candidates
-    __shared__ YoloHit queue[kDenseQueue];
+    constexpr int kStep = ALL ? 10 : 4, kQueue = kRoundHits<kStep>;
+    __shared__ YoloHit queue[kQueue];
     __shared__ int s_queued;
     extern __shared__ __align__(16) float s_cls[];  // [128][kDenseRow]
     pdl_launch_dependents();
@@ -427,7 +513,7 @@ yolo_decode_dense_kernel(const __grid_constant__ YoloDecodeArgs A) {
                     const float s = __fmul_rn(so_e, v[e][u]);
                     if (s > A.thr && s >= bar) {
                         const int at = atomicAdd(&s_queued, 1);
-                        if (at < kDenseQueue) queue[at] = YoloHit{s, static_cast<uint32_t>(slot << 7 | (warp * kDecClasses + k0 + u))};
+                        if (at < kQueue) queue[at] = YoloHit{s, static_cast<uint32_t>(slot << 7 | (warp * kDecClasses + k0 + u))};
                     }
                 }
             }
@@ -457,7 +543,8 @@ yolo_decode_dense_kernel(const __grid_constant__ YoloDecodeArgs A) {
             }
         }
     }
-    if (s_queued > kDenseQueue) yolo_crowded_tile(&A, img_map, plane, T.img, live, kDecThreads, bar);
+    if (s_queued > kQueue) yolo_collect_all<true, kStep>(&A, img_map, plane, T.img, live, kDecThreads, bar, queue, kQueue, &s_queued, s_cls);
+    else if (s_queued > kDecThreads) yolo_eval_many<true>(A, live, queue, T.img, s_queued, bar);
     else yolo_eval_queue<true>(A, live, queue, T.img, s_queued, bar);
 }
 
@@ -509,9 +596,10 @@ static int launch_yolo_decode(const YoloDecodeArgs& a, int batch, bool pdl, cuda
     };
     if (a.obj_out != nullptr || a.cls_out != nullptr) {
         const size_t smem = sizeof(float) * kDecThreads * kDenseRow;
-        FB_TRY(check_cuda(cudaFuncSetAttribute(yolo_decode_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+        auto kernel = a.floor == nullptr ? yolo_decode_dense_kernel<true> : yolo_decode_dense_kernel<false>;
+        FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
                           "yolo_decode attr"));
-        return launch_after(yolo_decode_dense_kernel, dim3(static_cast<unsigned>(tiles(kDecThreads))), dim3(kDecThreads), smem, st, pdl,
+        return launch_after(kernel, dim3(static_cast<unsigned>(tiles(kDecThreads))), dim3(kDecThreads), smem, st, pdl,
                             "yolo_decode_dense_kernel", a);
     }
     // large tiles once they make four CTAs per SM
@@ -519,9 +607,11 @@ static int launch_yolo_decode(const YoloDecodeArgs& a, int batch, bool pdl, cuda
     auto run = [&](auto kernel, int n) {
         return launch_after(kernel, dim3(static_cast<unsigned>(n)), dim3(kDecThreads), 0, st, pdl, "yolo_decode_kernel", a);
     };
-    if (large >= 4 * kNumSMs) return a.boxes != nullptr ? run(yolo_decode_kernel<4, true>, large) : run(yolo_decode_kernel<4, false>, large);
-    const int small = tiles(kDecThreads);
-    return a.boxes != nullptr ? run(yolo_decode_kernel<1, true>, small) : run(yolo_decode_kernel<1, false>, small);
+    const bool is_large = large >= 4 * kNumSMs;
+    const int n = is_large ? large : tiles(kDecThreads);
+    if (a.floor == nullptr) return is_large ? run(yolo_decode_kernel<4, true, true>, n) : run(yolo_decode_kernel<1, true, true>, n);
+    if (a.boxes != nullptr) return is_large ? run(yolo_decode_kernel<4, true, false>, n) : run(yolo_decode_kernel<1, true, false>, n);
+    return is_large ? run(yolo_decode_kernel<4, false, false>, n) : run(yolo_decode_kernel<1, false, false>, n);
 }
 
 static inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
