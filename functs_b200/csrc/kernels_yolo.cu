@@ -28,10 +28,13 @@ namespace cg = cooperative_groups;
 // ---- score floor ------------------------------------------------------------------------------------------------------
 constexpr int kFloorCtas = 8;        // one cluster per image
 constexpr int kFloorThreads = 384;   // 8 x 3 runs of 32 slots, four warps each (21 runs at 13 / 26 / 52)
-constexpr int kFloorBlock = 512;     // one run of 32 slots per 512: a whole 128-byte line per plane, because that is what DRAM is read
+constexpr int kFloorShift = 9;       // one run of 32 slots per 512: a whole 128-byte line per plane, because that is what DRAM is read
                                      // in (runs of eight slots, four times as many, moved 58 MB instead of 15: 26 us for 64 images)
+constexpr int kFloorAll = 5;         // every run
 constexpr int kFloorBins = 256;      // score buckets (a guess needs no finer ones; one thread each)
-constexpr int kFloorMinSample = 256; // sampled boxes below which a floor is not worth the risk (small pyramids)
+constexpr int kFloorMinSample = 256; // sampled boxes below which a guess is not worth the risk: such a pyramid (below some 3000 boxes)
+                                     // is sampled whole, in some 90 runs, four per warp.  Without any floor one CTA had to select from
+                                     // all candidates: 6 / 12 / 24 cells 66 us, at a threshold of 0.05 302 us
 
 struct YoloFloorArgs {
     YoloLevels L;
@@ -46,6 +49,8 @@ struct YoloFloorArgs {
 };
 
 // Also clears the image's counters.  The scores of the sample may be approximate: they only pick a bucket.
+// SHIFT: log2 of the slots that one run is taken from.
+template <int SHIFT>
 __global__ void __cluster_dims__(kFloorCtas, 1, 1) __launch_bounds__(kFloorThreads, 4)
 yolo_floor_kernel(const YoloFloorArgs A) {
     __shared__ int hist[kFloorBins];    // this CTA's scores
@@ -75,15 +80,15 @@ yolo_floor_kernel(const YoloFloorArgs A) {
             int lvl = 0, local = block;  // level and number of the 512-slot block inside it
 #pragma unroll
             for (int l = 0; l < 3; ++l) {
-                const int nb = (3 * L.plane[l] + kFloorBlock - 1) / kFloorBlock;
+                const int nb = (3 * L.plane[l] + (1 << SHIFT) - 1) >> SHIFT;
                 if (lvl == l && local >= nb) {
                     local -= nb;
                     ++lvl;
                 }
             }
             if (lvl > 2) break;  // warp-uniform
-            const int plane = L.plane[lvl], s0 = local * kFloorBlock;
-            const int runs = max(1, min(kFloorBlock, 3 * plane - s0) >> 5);
+            const int plane = L.plane[lvl], s0 = local << SHIFT;
+            const int runs = max(1, min(1 << SHIFT, 3 * plane - s0) >> 5);
             const int slot = s0 + 32 * ((block * 5 + img * 3) % runs) + lane;
             const bool valid = slot < 3 * plane;
             int anchor, pos;
@@ -132,7 +137,7 @@ yolo_floor_kernel(const YoloFloorArgs A) {
         }
         __syncthreads();
         if (t == 0) {
-            const int d = total_valid >= kFloorMinSample ? s_bucket : 0;
+            const int d = total_valid >= kFloorMinSample || total_valid == L.num_boxes ? s_bucket : 0;
             A.floor[img] = d > 0 ? __uint_as_float(A.hist_base + (static_cast<uint32_t>(d) << A.hist_shift)) : 0.0f;
             A.counts[img] = 0;
             A.fallback[img] = 0;
@@ -583,6 +588,14 @@ static int yolo_levels(const float* map0, const float* map1, const float* map2, 
     return FB_OK;
 }
 
+// A run per 512 slots, or all runs if that leaves too small a sample.
+static int yolo_floor_shift(const YoloLevels& L) {
+    int sampled = 0;
+    for (int l = 0; l < 3; ++l)
+        for (int left = 3 * L.plane[l]; left > 0 && sampled < kFloorMinSample; left -= 1 << kFloorShift) sampled += std::min(left, 32);
+    return sampled >= kFloorMinSample ? kFloorShift : kFloorAll;
+}
+
 // pdl: the launch may overlap the end of the kernel before it (the floor kernel)
 static int launch_yolo_decode(const YoloDecodeArgs& a, int batch, bool pdl, cudaStream_t st) {
     FB_REQUIRE(a.keys && a.counts, "yolo_decode: null pointer");
@@ -735,7 +748,8 @@ int functs_b200_yolo_detect(const float* map0, const float* map1, const float* m
     p.status = status;
     FB_TRY(check_yolo_post(batch, p));  // before anything is launched
     record_stage_event(0, st);
-    yolo_floor_kernel<<<static_cast<unsigned>(batch) * kFloorCtas, kFloorThreads, 0, st>>>(f);
+    auto floor_kernel = yolo_floor_shift(d.L) == kFloorShift ? yolo_floor_kernel<kFloorShift> : yolo_floor_kernel<kFloorAll>;
+    floor_kernel<<<static_cast<unsigned>(batch) * kFloorCtas, kFloorThreads, 0, st>>>(f);
     count_launch();
     FB_TRY(check_launch("yolo_floor_kernel"));
     record_stage_event(1, st);

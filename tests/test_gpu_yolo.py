@@ -300,3 +300,21 @@ def test_yolo_dense_class_scores_off_a_16_byte_boundary(fb):
                                                           None, torch.cuda.current_stream().cuda_stream), "yolo_decode")
         assert torch.equal(room[shift:shift + cls.numel()].view_as(cls), cls) and torch.equal(counts2, counts)
         assert bool((room[:shift] == 7.0).all()) and bool((room[shift + cls.numel():] == 7.0).all())
+
+
+@pytest.mark.parametrize("sizes", [(2, 4, 8), (3, 6, 12), (6, 12, 24), (7, 14, 28), (8, 15, 27)])
+def test_yolo_small_pyramids_have_a_floor(fb, sizes):
+    """Pyramids on both sides of the size below which the whole of them is sampled: no image falls back to selecting from all of
+    its candidates, and the detections are those without a floor."""
+    maps = [torch.randn(3, 255, s, s, generator=torch.Generator().manual_seed(s)).cuda() for s in sizes]
+    mod = fb.workloads.YOLOV3BBox(sizes=sizes, score_thr=0.05)
+    got = [t.clone() for t in mod.forward_padded(maps)]
+    assert mod._plan.select_fallbacks() == 0
+    fb._lib.lib.functs_b200_debug_set(b"yolo_prune", 0)
+    try:
+        want = mod.forward_padded(maps)
+        assert mod._plan.select_fallbacks() == 3  # more candidates than the selection holds
+    finally:
+        fb._lib.lib.functs_b200_debug_set(b"yolo_prune", 1)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
