@@ -31,6 +31,10 @@ constexpr int kFloorThreads = 384;   // 8 x 3 runs of 32 slots, four warps each 
 constexpr int kFloorShift = 9;       // one run of 32 slots per 512: a whole 128-byte line per plane, because that is what DRAM is read
                                      // in (runs of eight slots, four times as many, moved 58 MB instead of 15: 26 us for 64 images)
 constexpr int kFloorAll = 5;         // every run
+constexpr int kFloorSpread = 128;    // sampled boxes that can yield candidates, below which the floor aims at three times the top-k
+                                     // instead of twice.  A few clusters of boxes are met by the sample or missed: a floor that
+                                     // comes out too high costs a second look at the image by one CTA (some 50 us), one too low
+                                     // a longer selection (some 10).  Always three times: 64 images at N(0, 1) 76.6 us (71.4)
 constexpr int kFloorBins = 256;      // score buckets (a guess needs no finer ones; one thread each)
 constexpr int kFloorMinSample = 256; // sampled boxes below which a guess is not worth the risk: such a pyramid (below some 3000 boxes)
                                      // is sampled whole, in some 90 runs, four per warp.  Without any floor one CTA had to select from
@@ -55,7 +59,7 @@ __global__ void __cluster_dims__(kFloorCtas, 1, 1) __launch_bounds__(kFloorThrea
 yolo_floor_kernel(const YoloFloorArgs A) {
     __shared__ int hist[kFloorBins];    // this CTA's scores
     __shared__ int merged[kFloorBins];  // rank 0: the cluster's
-    __shared__ int s_valid, s_bucket;
+    __shared__ int s_valid, s_alive, s_bucket;
     __shared__ int s_warp[kFloorBins / 32];
     pdl_launch_dependents();
     cg::cluster_group cluster = cg::this_cluster();
@@ -69,12 +73,13 @@ yolo_floor_kernel(const YoloFloorArgs A) {
         }
         if (t == 0) {
             s_valid = 0;
+            s_alive = 0;
             s_bucket = 0;
         }
         __syncthreads();
         auto cleared = cluster.barrier_arrive();  // (waited for before anybody adds to rank 0's words)
         const YoloLevels& L = A.L;
-        int nvalid = 0;
+        int nvalid = 0, nalive = 0;
         const int quarter = warp & 3;  // twenty of the eighty classes
         for (int block = rank * (kFloorThreads / 128) + (warp >> 2);; block += kFloorCtas * (kFloorThreads / 128)) {
             int lvl = 0, local = block;  // level and number of the 512-slot block inside it
@@ -111,17 +116,24 @@ yolo_floor_kernel(const YoloFloorArgs A) {
                                         (kHistBins / kFloorBins)], 1);
                 }
             }
-            if (quarter == 0) nvalid += __popc(__ballot_sync(kFullMask, valid));
+            if (quarter == 0) {
+                nvalid += __popc(__ballot_sync(kFullMask, valid));
+                nalive += __popc(__ballot_sync(kFullMask, alive));
+            }
         }
         __syncthreads();
         cluster.barrier_wait(std::move(cleared));
-        if (lane == 0 && nvalid > 0) atomicAdd(cluster.map_shared_rank(&s_valid, 0), nvalid);
+        if (lane == 0 && nvalid > 0) {
+            atomicAdd(cluster.map_shared_rank(&s_valid, 0), nvalid);
+            atomicAdd(cluster.map_shared_rank(&s_alive, 0), nalive);
+        }
         if (t < kFloorBins && hist[t] != 0) atomicAdd(cluster.map_shared_rank(merged, 0) + t, hist[t]);
         cluster.sync();
         if (rank != 0) return;
         // the largest bucket d with (sampled candidates in buckets >= d) >= target
         const int total_valid = s_valid;
-        const int target = static_cast<int>(2ll * A.topk * total_valid / L.num_boxes) + 8;
+        const int aim = s_alive < kFloorSpread ? 3 : 2;
+        const int target = static_cast<int>(static_cast<int64_t>(aim) * A.topk * total_valid / L.num_boxes) + 8;
         const int mine = t < kFloorBins ? merged[t] : 0;
         int incl = mine;
 #pragma unroll

@@ -14,7 +14,7 @@
 //              behind its own largest one.  What overlaps enough goes into a list of (suppressor, suppressed) pairs;
 //   greedy     parallel rounds over the pair list: a box is kept once every box that could suppress it is removed.
 // Slow exact ways for the rare inputs: the floor was too high (fewer than topk candidates in the list: the image's scores are
-// formed again without one), more candidates than fit (generic selection from global memory), a crowded score bucket (bitonic
+// formed again without one), more candidates than fit (two-pass selection from global memory), a crowded score bucket (bitonic
 // sort), more pairs than fit (bit matrix in global memory, walked row by row).
 #include "yolo.cuh"
 
@@ -27,9 +27,15 @@ constexpr int kPostPairs = 8192;
 constexpr int kPostCrowded = 64;   // keys of one score bucket beyond which ranks are not counted
 constexpr int kPostWords = kPostTop / 32;
 
+struct RescanSlot {
+    float so;  // objectness score
+    int slot;  // of the level
+};
+
 struct PostSmem {
     union {
         uint64_t keys[kPostKeys];
+        RescanSlot rescan[kPostKeys];
         struct {
             float4 xy[kPostTop];       // NMS-space corners, by position (class order)
             float area[kPostTop];
@@ -52,42 +58,90 @@ struct PostSmem {
     uint32_t words[kPostWords];
     uint32_t hi, lo;  // extreme coordinates, as ordered bits
     int npairs;
+    int live, found;  // post_rescan
 };
 static_assert(sizeof(PostSmem) < 100 * 1024, "two CTAs per SM");
 
-// The image's candidates once more, without a floor.
-__device__ __noinline__ void post_rescan(const YoloLevels& L, const YoloPostArgs& A, int img) {
-    if (threadIdx.x == 0) A.counts[img] = 0;
-    __syncthreads();
-    for (int b = threadIdx.x; b < L.num_boxes; b += kPostThreads) {
-        const int lvl = b >= L.box_begin[2] ? 2 : (b >= L.box_begin[1] ? 1 : 0);
-        const int plane = L.plane[lvl], slot = b - L.box_begin[lvl];
-        int anchor, pos;
-        yolo_slot(plane, slot, anchor, pos);
-        const float* src = L.map[lvl] + (static_cast<int64_t>(img) * 3 + anchor) * kYoloAttrib * plane + pos;
-        const float so = sigmoid_f32(__ldg(src + 4 * plane));
-        if (!(so > A.thr)) continue;
-        const float cut = logit_cut(so, A.thr);
-        const uint32_t flat0 = static_cast<uint32_t>(L.box_begin[lvl] + pos * 3 + anchor) * kYoloClasses;
-        for (int c = 0; c < kYoloClasses; ++c) {
-            const float v = __ldg(src + (5 + c) * plane);
-            if (!(v > cut)) continue;
-            const float s = __fmul_rn(so, sigmoid_f32(v));
-            if (!(s > A.thr)) continue;
-            const int64_t at = atomicAdd(A.counts + img, 1);
-            if (at < A.capacity) A.keys[img * A.capacity + at] = make_key(s, flat0 + static_cast<uint32_t>(c));
-            else if (A.status != nullptr) atomicOr(A.status, FB_STATUS_CAND_OVERFLOW);
+// 2048 buckets of the scores from `bar` to 1
+__device__ __forceinline__ void post_buckets(float bar, uint32_t& base, int& shift) {
+    base = __float_as_uint(bar);
+    const uint32_t span = 0x3F800000u > base ? 0x3F800000u - base : 1u;  // scores are products of probabilities: <= 1
+    shift = max(0, 21 - __clz(static_cast<int>(span - 1u)));            // (span - 1) >> shift < 2048
+}
+
+// The image's candidates once more, without a floor.  Latency bounds it (one CTA, 3.6 MB at 416 x 416): so the boxes that can yield
+// any are listed first, 4096 slots at a time, and a thread then takes sixteen classes of one of them, loaded together.  (A thread
+// per box, one class after another: some 200 us.)
+constexpr int kRescanClasses = 16;
+__device__ __noinline__ void post_rescan(const YoloLevels& L, const YoloPostArgs& A, int img, PostSmem* smp) {
+    PostSmem& sm = *smp;
+    const int t = threadIdx.x, lane = t & 31;
+    if (t == 0) sm.found = 0;
+    for (int lvl = 0; lvl < 3; ++lvl) {
+        const int plane = L.plane[lvl];
+        const float* img_map = L.map[lvl] + static_cast<int64_t>(img) * 3 * kYoloAttrib * plane;
+        for (int s0 = 0; s0 < 3 * plane; s0 += kPostKeys) {
+            __syncthreads();  // the list of the slots before is done with
+            if (t == 0) sm.live = 0;
+            __syncthreads();
+            float so[kPostKeys / kPostThreads];
+#pragma unroll
+            for (int q = 0; q < kPostKeys / kPostThreads; ++q) {
+                const int slot = s0 + q * kPostThreads + t;
+                int anchor, pos;
+                yolo_slot(plane, min(slot, 3 * plane - 1), anchor, pos);
+                so[q] = slot < 3 * plane ? __ldg(img_map + (anchor * kYoloAttrib + 4) * plane + pos) : -INFINITY;
+            }
+#pragma unroll
+            for (int q = 0; q < kPostKeys / kPostThreads; ++q) {
+                so[q] = sigmoid_f32(so[q]);
+                const bool alive = so[q] > A.thr;
+                const unsigned m = __ballot_sync(kFullMask, alive);
+                int at = 0;
+                if (lane == 0 && m != 0u) at = atomicAdd(&sm.live, __popc(m));
+                at = __shfl_sync(kFullMask, at, 0) + __popc(m & ((1u << lane) - 1u));
+                if (alive) sm.rescan[at] = RescanSlot{so[q], s0 + q * kPostThreads + t};
+            }
+            __syncthreads();
+            const int n = sm.live, items = n * (kYoloClasses / kRescanClasses);
+            for (int i = t; i < items; i += kPostThreads) {  // neighbouring threads: neighbouring slots
+                const int group = i / n;
+                const RescanSlot o = sm.rescan[i - group * n];
+                int anchor, pos;
+                yolo_slot(plane, o.slot, anchor, pos);
+                const float* src = img_map + (anchor * kYoloAttrib + 5 + group * kRescanClasses) * plane + pos;
+                float v[kRescanClasses];
+#pragma unroll
+                for (int u = 0; u < kRescanClasses; ++u) v[u] = __ldg(src + u * plane);
+                const float cut = logit_cut(o.so, A.thr);
+                const uint32_t flat0 = static_cast<uint32_t>(L.box_begin[lvl] + pos * 3 + anchor) * kYoloClasses + group * kRescanClasses;
+#pragma unroll
+                for (int u = 0; u < kRescanClasses; ++u) {
+                    if (!(v[u] > cut)) continue;
+                    const float s = __fmul_rn(o.so, sigmoid_f32(v[u]));
+                    if (!(s > A.thr)) continue;
+                    const int64_t at = atomicAdd(&sm.found, 1);
+                    if (at < A.capacity) A.keys[img * A.capacity + at] = make_key(s, flat0 + static_cast<uint32_t>(u));
+                    else if (A.status != nullptr) atomicOr(A.status, FB_STATUS_CAND_OVERFLOW);
+                }
+            }
         }
     }
     __syncthreads();
+    if (t == 0) A.counts[img] = sm.found;
 }
 
 struct GlobalKeysView {
+    static constexpr bool kDenseScores = false;
     const uint64_t* p;
     __device__ __forceinline__ uint64_t operator()(int i) const { return __ldcg(p + i); }
 };
-__device__ __noinline__ void post_select_generic(const uint64_t* keys, int n, int topk, PostSmem* sm) {
-    const int m = block_select_topk<kPostThreads, kPostTop, 4>(GlobalKeysView{keys}, n, topk, sm->generic);
+// more keys than the shared-memory selection takes: two passes over the list (a third way stands behind a crowded bucket)
+__device__ __noinline__ void post_select_many(const uint64_t* keys, int n, int topk, float bar, PostSmem* sm) {
+    uint32_t base;
+    int shift;
+    post_buckets(bar, base, shift);
+    const int m = block_select_topk_binned<kPostThreads, kPostTop, 8>(GlobalKeysView{keys}, n, topk, base, shift, sm->generic);
     __syncthreads();
     if (static_cast<int>(threadIdx.x) < m) sm->sel[threadIdx.x] = sm->generic.sel[threadIdx.x];
     __syncthreads();
@@ -96,9 +150,9 @@ __device__ __noinline__ void post_select_generic(const uint64_t* keys, int n, in
 // sel[0 .. min(n, topk)) = the largest keys, sorted; n <= kPostKeys
 __device__ __forceinline__ void post_select(const uint64_t* __restrict__ keys, int n, int topk, float bar, PostSmem& sm) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t base = __float_as_uint(bar);
-    const uint32_t span = 0x3F800000u > base ? 0x3F800000u - base : 1u;  // scores are products of probabilities: <= 1
-    const int shift = max(0, 21 - __clz(static_cast<int>(span - 1u)));   // (span - 1) >> shift < 2048
+    uint32_t base;
+    int shift;
+    post_buckets(bar, base, shift);
     constexpr int kPer = kPostKeys / kPostThreads;
     uint64_t k[kPer];
 #pragma unroll
@@ -250,14 +304,14 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     int64_t n64 = *reinterpret_cast<volatile int32_t*>(A.counts + img);
     const bool short_list = floor > 0.0f && n64 < A.topk;
     if (short_list) {
-        post_rescan(L, A, img);
+        post_rescan(L, A, img, &sm);
         floor = 0.0f;
-        n64 = *reinterpret_cast<volatile int32_t*>(A.counts + img);
+        n64 = sm.found;
     }
     const int n = static_cast<int>(n64 < 0 ? 0 : (n64 > A.capacity ? A.capacity : n64));
     const uint64_t* keys = A.keys + img * A.capacity;
     if (n <= kPostKeys) post_select(keys, n, A.topk, fmaxf(A.thr, floor), sm);
-    else post_select_generic(keys, n, A.topk, &sm);
+    else post_select_many(keys, n, A.topk, fmaxf(A.thr, floor), &sm);
     if (t == 0 && (short_list || n > kPostKeys)) A.fallback[img] = 1;
     const int m = min(n, A.topk);
 

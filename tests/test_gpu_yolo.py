@@ -244,7 +244,7 @@ def test_one_call_postprocess_replays_from_a_cuda_graph(fb):
 
 @pytest.mark.parametrize("batch,sizes,kind,topk", [
     (1, (13, 26, 52), "plain", 1000), (30, (13, 26, 52), "plain", 1000), (2, (10, 20, 40), "plain", 1),  # one / four slots per thread
-    (2, (13, 26, 52), "sampled high", 1000), (2, (13, 26, 52), "sampled low", 1000),  # floor too high: rescan; too low: long lists
+    (2, (13, 26, 52), "sampled high", 1000), (2, (13, 26, 52), "sampled low", 1000),  # hits in one run of sixteen only / in all others
     (2, (13, 26, 52), "crowded tile", 1000), (3, (4, 8, 16), "equal", 1000), (2, (13, 26, 52), "equal few", 1024),
     (2, (13, 26, 52), "one class", 1000), (2, (19, 38, 76), "sparse", 1000), (2, (11, 22, 44), "none", 100),
 ])
@@ -318,3 +318,47 @@ def test_yolo_small_pyramids_have_a_floor(fb, sizes):
         fb._lib.lib.functs_b200_debug_set(b"yolo_prune", 1)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("sizes,others", [((13, 26, 52), 7), ((13, 26, 52), 2), ((19, 38, 76), 11)])
+def test_yolo_sample_that_misleads(fb, sizes, others):
+    """The best boxes lie exactly where the floor kernel looks, so that its floor leaves fewer than the top-k: the image is looked at
+    again.  others = 2: more candidates than the shared-memory selection holds then."""
+    batch, topk = 2, 1000
+    maps = [torch.full((batch, 255, s, s), -8.0) for s in sizes]
+    block = sampled = total = 0
+    for m in maps:
+        v = m.view(batch, 3, 85, -1)
+        n = 3 * v.size(3)
+        slot = torch.arange(n)
+        seen = torch.zeros(batch, n, dtype=torch.bool)
+        for s0 in range(0, n, 512):  # one run of 32 slots per block of 512
+            runs = max(1, min(512, n - s0) // 32)
+            for img in range(batch):
+                at = s0 + 32 * ((block * 5 + img * 3) % runs)
+                seen[img, at:min(at + 32, n)] = True
+            block += 1
+        for img in range(batch):
+            hot, other = seen[img], ~seen[img] & (slot % others == 0)
+            value = torch.where(hot, 3.0, 0.5) + slot / 1.0e5
+            cls = (slot * 7) % 80
+            for i in torch.nonzero(hot | other)[:, 0].tolist():
+                a, p = divmod(i, v.size(3))
+                v[img, a, 4, p] = 6.0
+                v[img, a, 5 + int(cls[i]), p] = float(value[i])
+            sampled += int(hot.sum())
+            total += int((hot | other).sum())
+    assert (total > batch * 4096) == (others == 2)
+    cmaps = [m.cuda() for m in maps]
+    mod = fb.workloads.YOLOV3BBox(sizes=sizes, topk=topk)
+    dets, labels, flat, cnt = [t.cpu() for t in mod.forward_padded(cmaps)]
+    fb.ops.raise_on_status(mod._plan.status, "yolo")
+    if sizes[0] == 13:  # (the larger pyramid's sample holds more than the top-k)
+        assert sampled < batch * topk
+        assert mod._plan.select_fallbacks() == batch
+    boxes, obj, cls, _, _ = fb.ops.yolo_decode(cmaps, 0.5, dense=True)
+    post = W.YOLOV3Post(sizes=sizes, topk=topk)
+    for b in range(batch):
+        wd, wl, wf = post.post_single(boxes[b].cpu(), obj[b].cpu(), cls[b].cpu())
+        m = int(cnt[b])
+        assert m == wf.numel() and torch.equal(flat[b, :m], wf) and torch.equal(labels[b, :m], wl) and torch.equal(dets[b, :m], wd)
