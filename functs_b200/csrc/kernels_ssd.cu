@@ -305,18 +305,27 @@ ragged_pack_kernel(const float* __restrict__ dets, const int64_t* __restrict__ l
     }
 }
 
-// Every part's rows into arrays of its own: grid = (chunks of rows, parts).  Latency: 64 parts of a few hundred rows are some
-// hundred KB.
+// Every part's rows into arrays of its own: grid = (256 rows, parts).  Latency bounds it, so a thread's words are on their way
+// together.
 struct RaggedParts {
     functs_b200_ragged_part part[FB_RAGGED_MAX_PARTS];
 };
 __global__ void __launch_bounds__(kPackThreads)
 ragged_split_kernel(const float* __restrict__ dets, const int64_t* __restrict__ labels, const __grid_constant__ RaggedParts P) {
     const functs_b200_ragged_part& G = P.part[blockIdx.y];
-    const float* d = dets + 5 * G.first;
-    const int64_t at = static_cast<int64_t>(blockIdx.x) * kPackThreads + threadIdx.x, step = static_cast<int64_t>(gridDim.x) * kPackThreads;
-    for (int64_t i = at; i < 5 * G.rows; i += step) G.dets[i] = d[i];
-    for (int64_t i = at; i < G.rows; i += step) G.labels[i] = labels[G.first + i];
+    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * kPackThreads;
+    if (r0 >= G.rows) return;
+    const int t = threadIdx.x, rows = static_cast<int>(min(G.rows - r0, static_cast<int64_t>(kPackThreads)));
+    const float* src = dets + 5 * (G.first + r0);
+    float* dst = G.dets + 5 * r0;
+    float v[5];
+#pragma unroll
+    for (int u = 0; u < 5; ++u) v[u] = t + u * kPackThreads < 5 * rows ? __ldg(src + t + u * kPackThreads) : 0.0f;
+    const int64_t label = t < rows ? __ldg(reinterpret_cast<const long long*>(labels) + G.first + r0 + t) : 0;
+#pragma unroll
+    for (int u = 0; u < 5; ++u)
+        if (t + u * kPackThreads < 5 * rows) dst[t + u * kPackThreads] = v[u];
+    if (t < rows) G.labels[r0 + t] = label;
 }
 
 static int launch_ssd_softmax_decode(const float* loc, const float* conf, const float* priors, int batch, int num_priors,
@@ -430,8 +439,8 @@ int functs_b200_ragged_split(const float* dets, const int64_t* labels, const fun
         p.part[k] = parts[k];
         most = std::max(most, parts[k].rows);
     }
-    // two or three rows per thread, 16 CTAs to a part at most
-    const int64_t chunks = std::min<int64_t>(16, std::max<int64_t>(1, most / 512));
+    FB_REQUIRE(most <= (1ll << 30), "ragged_split: bad sizes");
+    const int64_t chunks = std::max<int64_t>(1, (most + kPackThreads - 1) / kPackThreads);
     ragged_split_kernel<<<dim3(static_cast<unsigned>(chunks), static_cast<unsigned>(count)), kPackThreads, 0, as_stream(stream)>>>(dets, labels, p);
     count_launch();
     return check_launch("ragged_split_kernel");

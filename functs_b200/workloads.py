@@ -40,7 +40,7 @@ def get_started(a: torch.Tensor, b: torch.Tensor, n: int, device="cuda") -> torc
 
 class YOLOV3BBox:
     """Decode three [B, 255, S, S] maps, score mask, top-k, class-wise NMS.  3 kernel launches, and one that gives the lists of
-    a __call__ storages of their own; scratch and padded room of a __call__ come from the caching allocator (436 MB for 64 images
+    a __call__ on several images storages of their own; scratch and padded room of a __call__ come from the caching allocator (436 MB for 64 images
     of 416 x 416) and go back to it."""
 
     def __init__(self, sizes=(13, 26, 52), score_thr: float = 0.5, topk: int = 1000, iou_thr: float = 0.45,
@@ -82,8 +82,8 @@ class YOLOV3BBox:
 
 
 class SSDBBox:
-    """softmax + decode, then the per-class loop (mask, top-k, NMS) with one CTA per (image, class).  2 launches, and one that
-    gives the lists of a __call__ storages of their own."""
+    """softmax + decode, then the per-class loop (mask, top-k, NMS) with one CTA per (image, class).  2 launches, and mostly one
+    that gives the lists of a __call__ storages of their own."""
 
     def __init__(self, priors: torch.Tensor, score_thr: float = 0.01, topk: int = 200, iou_thr: float = 0.45,
                  clamp_max: float = 300.0, device="cuda"):

@@ -77,6 +77,11 @@ def test_lists_of_the_modules_own_their_storage(cuda_device, batch):
     for pair, expected in zip(got, want):
         for t, w in zip(pair, expected):
             assert torch.equal(t, w) and t.untyped_storage().nbytes() == t.numel() * t.element_size()
+            assert not t._is_view() and torch.cat([t, t]).size(0) == 2 * t.size(0)
+    grown = [t.clone() for t in got[0]]
+    for t in got[0]:
+        t.resize_(2000, *t.shape[1:])  # (past what lies behind the storage)
+    assert all(torch.equal(t[:len(w)], w) for t, w in zip(got[0], grown)) and got[0][0].untyped_storage().nbytes() == 40000
     assert len({t.untyped_storage().data_ptr() for pair in got for t in pair if t.numel()}) == sum(t.numel() > 0 for pair in got for t in pair)
 
 
