@@ -6,8 +6,8 @@
 // step against 1.26 at one row of H = 256, the same at ten.)  Every cluster holds all of w_hh: a CTA owns H / 16 hidden units,
 // four gate columns each, 64 KB (H = 256) or 256 KB (H = 512) of weights, in registers as far as they go (32 or 64 per thread),
 // the rest in shared memory.
-// What bounds it at 64 rows is fp32 multiply-add issue: seven clusters fit the chip, ten rows each, 2.6 us of 128 FMA per
-// cycle and step; at one row the latency of a step: read the weights in shared memory, reduce, exchange.
+// What bounds it at 64 rows: seven clusters fit the chip, ten rows each; of 5.6 us per step 2.6 are fp32 multiply-adds at 128 per
+// cycle and SM, the reduction, the gates and the exchange follow one after the other (a third of the issue slots used); at one row the latency of a step: read the weights in shared memory, reduce, exchange.
 //
 // Thread layout: a thread multiplies two gate columns of one unit with KT consecutive k of every row, two k per packed instruction
 // (fma.rn.f32x2: one issue slot for two multiply-adds); a warp is 8 units x 2 gate pairs x 2 k-slices, the two slices are
@@ -70,7 +70,7 @@ __device__ __forceinline__ void store_remote(uint32_t local_addr, uint32_t rank,
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
-// RP rows per pass (what the accumulators allow), NP passes: R = RP * NP rows per cluster.
+// R rows per cluster, multiplied in one pass.
 template <int H, int R>
 __global__ void __launch_bounds__(kRecThreads, 1)
 lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,

@@ -18,8 +18,8 @@
 //     one another's loads, products and stores.
 //     (Two warps per 32 pixels, each with half of the detections: 115 us, what both have to do costs more than more warps bring.
 //     TF32 operands, copied to shared memory unsplit, leave 1 in 100 logits open: 105 us.)
-// B = 64, 138 x 138, 100 detections: 95 us (3.0 TB/s) against 145 for the exact kernel; 8 x 276 x 276: 51 against 78; one image: 12
-// against 25.  What bounds it is issue, 1150 instructions per 32 pixels, with the 16 warps per SM that TMEM leaves room for.
+// B = 64, 138 x 138, 100 detections: 89 us (3.1 TB/s) against 129 for the exact kernel, each pass on other inputs; on the same ones
+// 75 against 112, 8 x 276 x 276 42 against 57, one image 13 against 13.  What bounds it is issue, 1150 instructions per 32 pixels, with the 16 warps per SM that TMEM leaves room for.
 #include <cuda_bf16.h>
 
 #include <algorithm>

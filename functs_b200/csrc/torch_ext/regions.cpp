@@ -16,9 +16,9 @@
 //                         top level; on equality the window is replaced by ONE tssa::ParallelFunctor node that carries
 //                         the pattern's name (attribute `region`), the free constants as named attributes, the tensor
 //                         constants (attribute `tparams`) and, as Subgraph, a copy of the window it replaced.
-//   operator              a region functor never interprets its subgraph: it allocates outputs and scratch with torch,
-//                         launches through functs_b200_group_launch on the current stream, reads the per-list counts
-//                         back and narrows the padded outputs to the ragged lists the program returns.
+//   operator              a region functor never interprets its subgraph: it allocates outputs and scratch with torch and
+//                         launches on the current stream (functs_b200_group_launch; the detection programs through
+//                         detect.cpp, which watches the images' counts in host memory and makes the ragged lists).
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
