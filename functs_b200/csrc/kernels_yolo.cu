@@ -292,15 +292,18 @@ __device__ __forceinline__ void yolo_eval_many(const YoloDecodeArgs& A, const Yo
 }
 
 // All candidates of a tile, for callers without a floor and for tiles whose hits did not fit the queue: in rounds of 32 live slots
-// and STEP classes per warp; the queue is evaluated whenever another round might not fit (room: its entries).  DENSE: the class
+// and STEP classes per warp; the queue is evaluated whenever another round might not fit (ROOM: its entries).  DENSE: the class
 // scores come from s_cls.  (One live slot per thread through all its classes with an append for every class took 375 us for 32
 // images at N(0, 1), seven candidates in a hundred: 320 global atomics a tile, most of them for a hit or two.)
 template <int STEP>
 constexpr int kRoundHits = 32 * STEP * kDecWarps;
-template <bool DENSE, int STEP>
-__device__ __noinline__ void yolo_collect_all(const YoloDecodeArgs* A, const float* img_map, int plane, int img, const YoloLive* live, int n,
-                                              float bar, YoloHit* queue, int room, int* counter, const float* s_cls) {
+template <bool DENSE, int STEP, int ROOM>
+__device__ __noinline__ void yolo_collect_all(const YoloDecodeArgs* A, int lvl, int img, const YoloLive* live, int n, float bar,
+                                              YoloHit* queue, int* counter) {
+    extern __shared__ __align__(16) float s_cls[];  // [128][kDenseRow]
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int plane = A->L.plane[lvl];
+    const float* img_map = A->L.map[lvl] + static_cast<int64_t>(img) * 3 * kYoloAttrib * plane;
     __syncthreads();  // whoever filled the queue before has seen how far
     if (t == 0) *counter = 0;
     __syncthreads();
@@ -337,7 +340,7 @@ __device__ __noinline__ void yolo_collect_all(const YoloDecodeArgs* A, const flo
         }
         const bool last = round + 1 == rounds;
         if (!last) load(round + 1);  // on its way while this round's hits are evaluated
-        if (__syncthreads_or(last || at > room - kRoundHits<STEP> ? 1 : 0) == 0) continue;
+        if (__syncthreads_or(last || at > ROOM - kRoundHits<STEP> ? 1 : 0) == 0) continue;
         yolo_eval_many<DENSE>(*A, live, queue, img, *counter, bar);
         __syncthreads();
         if (t == 0) *counter = 0;
@@ -449,7 +452,7 @@ yolo_decode_kernel(const __grid_constant__ YoloDecodeArgs A) {
         __syncthreads();
         all = s_queued > kQueue;
     }
-    if (all) yolo_collect_all<false, kDecStep>(&A, img_map, plane, T.img, live, n, bar, queue, kQueue, &s_queued, nullptr);
+    if (all) yolo_collect_all<false, kDecStep, kQueue>(&A, T.lvl, T.img, live, n, bar, queue, &s_queued);
     else yolo_eval_queue<false>(A, live, queue, T.img, s_queued, bar);
 }
 
@@ -560,7 +563,7 @@ yolo_decode_dense_kernel(const __grid_constant__ YoloDecodeArgs A) {
             }
         }
     }
-    if (s_queued > kQueue) yolo_collect_all<true, kStep>(&A, img_map, plane, T.img, live, kDecThreads, bar, queue, kQueue, &s_queued, s_cls);
+    if (s_queued > kQueue) yolo_collect_all<true, kStep, kQueue>(&A, T.lvl, T.img, live, kDecThreads, bar, queue, &s_queued);
     else if (s_queued > kDecThreads) yolo_eval_many<true>(A, live, queue, T.img, s_queued, bar);
     else yolo_eval_queue<true>(A, live, queue, T.img, s_queued, bar);
 }
