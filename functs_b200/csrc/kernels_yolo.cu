@@ -339,7 +339,7 @@ __device__ __noinline__ void yolo_collect_all(const YoloDecodeArgs* A, int lvl, 
                 if ((hits >> u) & 1u) queue[at++] = YoloHit{v[u], first + static_cast<uint32_t>(u)};
         }
         const bool last = round + 1 == rounds;
-        if (!last) load(round + 1);  // on its way while this round's hits are evaluated
+        if (!last) load(round + 1);  // on its way while these hits are evaluated
         if (__syncthreads_or(last || at > ROOM - kRoundHits<STEP> ? 1 : 0) == 0) continue;
         yolo_eval_many<DENSE>(*A, live, queue, img, *counter, bar);
         __syncthreads();
