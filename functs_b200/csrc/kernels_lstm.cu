@@ -16,7 +16,7 @@ int64_t lstm_tc_scratch_bytes(int M, int K, int H);
 bool lstm_tc_supported(int M, int K, int H);
 bool lstm_rtc_supported(int B, int H);
 int64_t lstm_rtc_scratch_bytes(int H);
-int launch_lstm_recurrent(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, cudaStream_t st);  // kernels_lstm_rec.cu
+int launch_lstm_recurrent(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, int32_t* status, cudaStream_t st);  // kernels_lstm_rec.cu
 int launch_lstm_recurrent_tc(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, void* h_tiles,
                              unsigned int* step_counter, int32_t* status, cudaStream_t st);
 
@@ -138,7 +138,7 @@ int functs_b200_lstm_forward_mode(const float* x, const float* w_ih, const float
         record_stage_event(2, st);
         return rc;
     }
-    FB_TRY(launch_lstm_recurrent(pre, w_hh, seq_len, batch, hidden, hs, cs, st));
+    FB_TRY(launch_lstm_recurrent(pre, w_hh, seq_len, batch, hidden, hs, cs, status, st));
     record_stage_event(2, st);
     return FB_OK;
 }

@@ -74,7 +74,7 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 template <int H, int R>
 __global__ void __launch_bounds__(kRecThreads, 1)
 lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,
-                      float* __restrict__ cs) {
+                      float* __restrict__ cs, int32_t* /*status*/) {
     using Y = RecLayout<H, R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemQuads][2][kRecThreads]
@@ -202,94 +202,140 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
 
 // ---- many rows per cluster ----
 // With more than a few rows the loads of h bound the kernel above: a 16-byte shared load fills 512 bytes of registers whatever
-// its lanes share, four cycles, and feeds two gate columns only (ten rows of H = 512: 6.7 us per step, 5.7 here).  Here 256 threads of
-// twice the registers take eight columns each, the four gates of two neighbouring units, packed by unit (a weight pair is
-// adjacent in memory; h is the same in both halves), so that a loaded word feeds eight multiply-adds.
-constexpr int kWideThreads = 256;
+// its lanes share, four cycles, and feeds two gate columns only.  Here 256 threads of most of the registers take eight columns
+// each, the four gates of two neighbouring units, packed by unit (a weight pair is adjacent in memory; h is the same in both
+// halves), so that a loaded word feeds eight multiply-adds.
+//
+// The rows of a cluster are two halves that take turns: while eight warps multiply one half, eight others reduce, apply the gates
+// and exchange the h of the other, so that the chain of a step (reduction, gates, exchange) lies behind multiplications instead of
+// after them.  The exchange is st.async: 16 bytes and their count on the receiver's mbarrier in one store, no fence, no cluster
+// barrier.  Nothing else orders the CTAs: a CTA can send h[t + 2] into a buffer only after it received all of h[t + 1], which every
+// CTA sends after its own multiplications of h[t] have ended; the partial sums have one buffer per half for the same reason.
+constexpr int kPairFma = 256, kPairGate = 256, kPairThreads = kPairFma + kPairGate;
+constexpr int kPairFmaRegs = 200, kPairGateRegs = 56;               // of 128 per thread at launch
+static_assert((kPairFmaRegs + kPairGateRegs) * 256 <= kPairThreads * 128, "registers of the launch");
+constexpr uint32_t kRecWaitLimit = 2000000u;
 
-template <int H, int R>
-struct WideLayout {
+template <int H, int RH>                                            // RH: rows of a half
+struct PairLayout {
     static constexpr int U = H / kRecCluster;                       // units per CTA
     static constexpr int WG = U / 16;                               // warps across the units: 8 pairs per warp
-    static constexpr int KQ = kWideThreads / 32 / WG;               // k-ranges across the warps
+    static constexpr int KQ = kPairFma / 32 / WG;                   // k-ranges across the warps
     static constexpr int KT = H / KQ / 4;                           // k per thread: four slices inside a warp
-    static constexpr int BP = R * U + 4;
-    static constexpr int RegK = KT <= 12 ? KT : 12;                 // k whose weights live in registers
+    static constexpr int BP = RH * U + 4;                           // a CTA's part of a half of h, [RH][U], and four floats (banks)
+    static constexpr int RegK = KT <= 14 ? KT : 14;                 // k whose weights live in registers
     static constexpr int SmemK = KT - RegK;
-    static constexpr size_t h_floats = 2ull * kRecCluster * BP;
-    static constexpr size_t part_floats = static_cast<size_t>(KQ) * R * 4 * U;
-    static constexpr size_t w_bytes = static_cast<size_t>(SmemK) * 2 * kWideThreads * 16;
-    static constexpr size_t bytes = w_bytes + (h_floats + part_floats) * 4;
+    static constexpr int Items = RH * U;                            // (row, unit) pairs of a half
+    static constexpr int GateWarps = (Items + 31) / 32;
+    static constexpr size_t h_floats = 4ull * kRecCluster * BP;     // [buffer][half]
+    static constexpr size_t part_floats = 2ull * KQ * RH * 4 * U;   // [half]
+    static constexpr size_t w_bytes = static_cast<size_t>(SmemK) * 2 * kPairFma * 16;
+    static constexpr size_t bytes = w_bytes + (h_floats + part_floats) * 4 + 64;
     static_assert(U % KT == 0 && RegK % 2 == 0 && SmemK % 2 == 0, "a k-slice lies inside one part of h");
+    static_assert(GateWarps * 32 <= kPairGate, "one thread per item");
 };
 
-template <int H, int R>
-__global__ void __launch_bounds__(kWideThreads, 1)
-lstm_recurrent_wide_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,
-                           float* __restrict__ cs) {
-    using Y = WideLayout<H, R>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemK][2][kWideThreads]
-    float* h_s = reinterpret_cast<float*>(smem_raw + Y::w_bytes);               // [2][16][BP]
-    float* part = h_s + Y::h_floats;                                            // [KQ][R][4][U]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int rank = static_cast<int>(cluster_rank());
-    const int b0 = static_cast<int>(blockIdx.x / kRecCluster) * R;
-    const int unit = (warp % Y::WG) * 16 + 2 * (lane & 7);                      // first of this thread's two units
-    const int kq = warp / Y::WG, slice = kq * 4 + (lane >> 3);                  // k = slice * KT ...
-    const int j0 = rank * Y::U;
-
-    unsigned long long w_r[Y::RegK][4];
-#pragma unroll
-    for (int k = 0; k < Y::KT; ++k) {
-        unsigned long long v[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            v[c] = __ldg(reinterpret_cast<const unsigned long long*>(w_hh + (static_cast<int64_t>(c) * H + slice * Y::KT + k) * H + j0 + unit));
-        if (k < Y::RegK) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) w_r[k < Y::RegK ? k : 0][c] = v[c];
-        } else {
-            w_s[((k - Y::RegK) * 2) * kWideThreads + tid] = make_ulonglong2(v[0], v[1]);
-            w_s[((k - Y::RegK) * 2 + 1) * kWideThreads + tid] = make_ulonglong2(v[2], v[3]);
-        }
+// Address of this CTA's shared-memory word in the CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_remote(uint32_t local_addr, uint32_t rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void store_async4(uint32_t remote, float a, float b, float c, float d, uint32_t remote_bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(remote), "f"(a),
+                 "f"(b), "f"(c), "f"(d), "r"(remote_bar)
+                 : "memory");
+}
+// Wait for what other CTAs of the cluster store; false when the limit runs out.
+__device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < kRecWaitLimit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
     }
-    constexpr int kItems = R * Y::U;                                            // (row, unit) pairs of the CTA
-    constexpr int kPer = (kItems + kWideThreads - 1) / kWideThreads;
-    float c_state[kPer], pre_g[kPer][4];
-    auto fetch = [&](int t) {
+    return false;
+}
+// Phase of a buffer's mbarrier that step t waits for: steps 1, 3, 5, ... use buffer 1, steps 2, 4, ... buffer 0.
+__device__ __forceinline__ uint32_t step_parity(int t) { return static_cast<uint32_t>((t - 1) >> 1) & 1u; }
+
+template <int H, int RH>
+__global__ void __launch_bounds__(kPairThreads, 1)
+lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,
+                           float* __restrict__ cs, int32_t* status) {
+    using Y = PairLayout<H, RH>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemK][2][kPairFma]
+    float* h_s = reinterpret_cast<float*>(smem_raw + Y::w_bytes);               // [buffer][half][16][BP]
+    float* part = h_s + Y::h_floats;                                            // [half][KQ][RH][4][U]
+    uint64_t* full = reinterpret_cast<uint64_t*>(part + Y::part_floats);        // [half][buffer]
+    int* late = reinterpret_cast<int*>(full + 4);                               // a wait ran out
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int rank = static_cast<int>(cluster_rank());
+    const int b0 = static_cast<int>(blockIdx.x / kRecCluster) * (2 * RH);
+    const int j0 = rank * Y::U;
+    constexpr uint32_t kPhaseBytes = RH * H * 4;                                // one half of h
+
+    if (tid == 0) {
+        *late = 0;
 #pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-            const int i = q * kWideThreads + tid, row = b0 + i / Y::U;
-            if (i < kItems && row < B) {
-                const float* p = pre + (static_cast<int64_t>(t) * B + row) * (4 * H) + j0 + i % Y::U;
+        for (int i = 0; i < 4; ++i) {
+            mbar_init(full + i, 1);
+            mbar_arrive_expect_tx(full + i, kPhaseBytes);
+        }
+        fence_barrier_init();
+    }
+    if (tid < kPairFma) {
+        // ---- multiplications ----
+        __syncwarp();
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPairFmaRegs));
+        const int warp = tid >> 5;
+        const int unit = (warp % Y::WG) * 16 + 2 * (lane & 7);                  // first of this thread's two units
+        const int kq = warp / Y::WG, slice = kq * 4 + (lane >> 3);              // k = slice * KT ...
+        unsigned long long w_r[Y::RegK][4];
 #pragma unroll
-                for (int g = 0; g < 4; ++g) pre_g[q][g] = __ldcg(p + g * H);
+        for (int k = 0; k < Y::KT; ++k) {
+            unsigned long long v[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                v[c] = __ldg(reinterpret_cast<const unsigned long long*>(w_hh + (static_cast<int64_t>(c) * H + slice * Y::KT + k) * H + j0 + unit));
+            if (k < Y::RegK) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) w_r[k < Y::RegK ? k : 0][c] = v[c];
+            } else {
+                w_s[((k - Y::RegK) * 2) * kPairFma + tid] = make_ulonglong2(v[0], v[1]);
+                w_s[((k - Y::RegK) * 2 + 1) * kPairFma + tid] = make_ulonglong2(v[2], v[3]);
             }
         }
-    };
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-        c_state[q] = 0.0f;
-#pragma unroll
-        for (int g = 0; g < 4; ++g) pre_g[q][g] = 0.0f;
-    }
-    pdl_wait();  // the projection, as in the kernel above
-    fetch(0);
-    cluster_arrive();  // every CTA of the cluster runs before anybody stores into another one
-    cluster_wait();
-    for (int t = 0; t < T; ++t) {
-        if (t > 0) {
-            // slice s lies in the part of CTA s * KT / U
-            const float* h_t = h_s + ((t & 1) * kRecCluster + slice * Y::KT / Y::U) * Y::BP + slice * Y::KT % Y::U;
-            unsigned long long acc[4][R];
+        cluster_arrive();  // every CTA of the cluster runs, its barriers set, before anybody stores into another one
+        cluster_wait();
+        bool waiting = true;
+        // slice s lies in the part of CTA s * KT / U
+        const float* h_mine = h_s + (slice * Y::KT / Y::U) * Y::BP + slice * Y::KT % Y::U;
+#pragma unroll 1
+        for (int u = 2; u < 2 * T; ++u) {                                       // (step, half)
+            const int t = u >> 1, half = u & 1;
+            uint64_t* bar = full + half * 2 + (t & 1);
+            if (waiting && !wait_cluster(smem_u32(bar), step_parity(t))) {
+                waiting = false;  // the rest is computed from what is there: every CTA goes through all steps
+                *late = 1;
+                if (status != nullptr) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
+            }
+            if (tid == 0 && t + 2 < T) mbar_arrive_expect_tx(bar, kPhaseBytes);
+            const float* h_t = h_mine + ((t & 1) * 2 + half) * (kRecCluster * Y::BP);
+            unsigned long long acc[4][RH];
 #pragma unroll
             for (int c = 0; c < 4; ++c)
 #pragma unroll
-                for (int r = 0; r < R; ++r) acc[c][r] = 0ull;
+                for (int r = 0; r < RH; ++r) acc[c][r] = 0ull;
             auto pair = [&](const float* hk, const unsigned long long (&w0)[4], const unsigned long long (&w1)[4]) {
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
+                for (int r = 0; r < RH; ++r) {
                     const float2 hv = *reinterpret_cast<const float2*>(hk + r * Y::U);
                     const unsigned long long x = pack2(hv.x, hv.x), y = pack2(hv.y, hv.y);
 #pragma unroll
@@ -300,10 +346,10 @@ lstm_recurrent_wide_kernel(const float* __restrict__ pre, const float* __restric
             };
 #pragma unroll
             for (int k = 0; k < Y::RegK; k += 2) pair(h_t + k, w_r[k], w_r[k + 1 < Y::RegK ? k + 1 : k]);
-#pragma unroll 1
+#pragma unroll
             for (int k = 0; k < Y::SmemK; k += 2) {
-                const ulonglong2 a0 = w_s[(2 * k) * kWideThreads + tid], a1 = w_s[(2 * k + 1) * kWideThreads + tid];
-                const ulonglong2 b0_ = w_s[(2 * k + 2) * kWideThreads + tid], b1_ = w_s[(2 * k + 3) * kWideThreads + tid];
+                const ulonglong2 a0 = w_s[(2 * k) * kPairFma + tid], a1 = w_s[(2 * k + 1) * kPairFma + tid];
+                const ulonglong2 b0_ = w_s[(2 * k + 2) * kPairFma + tid], b1_ = w_s[(2 * k + 3) * kPairFma + tid];
                 const unsigned long long w0[4] = {a0.x, a0.y, a1.x, a1.y}, w1[4] = {b0_.x, b0_.y, b1_.x, b1_.y};
                 pair(h_t + Y::RegK + k, w0, w1);
             }
@@ -316,62 +362,99 @@ lstm_recurrent_wide_kernel(const float* __restrict__ pre, const float* __restric
                 return d;
             };
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
+            for (int r = 0; r < RH; ++r) {
                 unsigned long long a[2];
 #pragma unroll
                 for (int c = 0; c < 2; ++c) a[c] = add2(up ? acc[2 + c][r] : acc[c][r], other(up ? acc[c][r] : acc[2 + c][r], 16));
                 const unsigned long long s = add2(odd ? a[1] : a[0], other(odd ? a[0] : a[1], 8));
-                *reinterpret_cast<unsigned long long*>(part + ((kq * R + r) * 4 + (lane >> 3)) * Y::U + unit) = s;
+                *reinterpret_cast<unsigned long long*>(part + (((half * Y::KQ + kq) * RH + r) * 4 + (lane >> 3)) * Y::U + unit) = s;
             }
-            __syncthreads();
+            asm volatile("barrier.arrive %0, %1;" ::"r"(1 + half), "n"(kPairFma + Y::GateWarps * 32) : "memory");
         }
-        float hval[kPer];
+    } else {
+        // ---- gates and exchange: one thread per (row, unit) of a half ----
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairGateRegs));
+        cluster_arrive();
+        if ((tid - kPairFma) / 32 < Y::GateWarps) {
+            const int i = tid - kPairFma, ir = i / Y::U, iu = i % Y::U;
+            const bool item = i < Y::Items;                                     // (a last half warp may have none)
+            const int irc = item ? ir : 0;
+            float c_state[2] = {0.0f, 0.0f}, pre_g[2][4] = {};
+            auto fetch = [&](int t, int half) {
+                const int row = b0 + half * RH + ir;
+                if (!item || row >= B) return;
+                const float* p = pre + (static_cast<int64_t>(t) * B + row) * (4 * H) + j0 + iu;
 #pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-            const int i = q * kWideThreads + tid, ir = i / Y::U, iu = i % Y::U;
-            if (i >= kItems) continue;
-            float gate[4];
+                for (int g = 0; g < 4; ++g) pre_g[half][g] = __ldcg(p + g * H);
+            };
+            pdl_wait();  // the projection (read with __ldcg: a __ldg could be moved up across this); the weights are not its output
+            fetch(0, 0);
+            fetch(0, 1);
+            // this lane sends its quad of units to four CTAs
+            uint32_t dst[4];
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                gate[g] = pre_g[q][g];
-                if (t > 0) {
-                    float s = part[(ir * 4 + g) * Y::U + iu];
+            for (int k = 0; k < 4; ++k) dst[k] = map_remote(smem_u32(smem_raw), static_cast<uint32_t>((lane & 3) * 4 + k));
+            const uint32_t h_off = smem_u32(h_s + rank * Y::BP + irc * Y::U + (iu & ~3)) - smem_u32(smem_raw);
+            const uint32_t bar_off = smem_u32(full) - smem_u32(smem_raw);
+            cluster_wait();
+#pragma unroll 1
+            for (int t = 0; t < T; ++t) {
 #pragma unroll
-                    for (int k = 1; k < Y::KQ; ++k) s = __fadd_rn(s, part[((k * R + ir) * 4 + g) * Y::U + iu]);
-                    gate[g] = __fadd_rn(gate[g], s);
+                for (int half = 0; half < 2; ++half) {
+                    float gate[4];
+                    if (t > 0) asm volatile("barrier.sync %0, %1;" ::"r"(1 + half), "n"(kPairFma + Y::GateWarps * 32) : "memory");
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        gate[g] = pre_g[half][g];
+                        if (t > 0) {
+                            const float* p = part + ((half * Y::KQ * RH + irc) * 4 + g) * Y::U + iu;
+                            float s = p[0];
+#pragma unroll
+                            for (int k = 1; k < Y::KQ; ++k) s = __fadd_rn(s, p[k * RH * 4 * Y::U]);
+                            gate[g] = __fadd_rn(gate[g], s);
+                        }
+                    }
+                    float sg[3] = {gate[0], gate[1], gate[3]};
+                    sigmoid_f32_n(sg);
+                    const float ig = sg[0], fg = sg[1], og = sg[2], gg = tanhf(gate[2]);
+                    c_state[half] = __fadd_rn(__fmul_rn(fg, c_state[half]), __fmul_rn(ig, gg));
+                    const float hval = __fmul_rn(og, tanhf(c_state[half]));
+                    if (t + 1 < T) {
+                        float v[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(kFullMask, hval, (lane & ~3) + k);
+                        const uint32_t to = h_off + static_cast<uint32_t>((((t + 1) & 1) * 2 + half) * (kRecCluster * Y::BP) * 4);
+                        const uint32_t bar = bar_off + static_cast<uint32_t>(half * 2 + ((t + 1) & 1)) * 8;
+                        if (item) {
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) store_async4(dst[k] + to, v[0], v[1], v[2], v[3], dst[k] + bar);
+                        }
+                    }
+                    const int row = b0 + half * RH + ir;
+                    if (item && row < B) {
+                        const int64_t o = (static_cast<int64_t>(t) * B + row) * H + j0 + iu;
+                        hs[o] = hval;
+                        cs[o] = c_state[half];
+                    }
+                    if (t + 1 < T) fetch(t + 1, half);
                 }
             }
-            float sg[3] = {gate[0], gate[1], gate[3]};
-            sigmoid_f32_n(sg);
-            const float ig = sg[0], fg = sg[1], og = sg[2], gg = tanhf(gate[2]);
-            c_state[q] = __fadd_rn(__fmul_rn(fg, c_state[q]), __fmul_rn(ig, gg));
-            hval[q] = __fmul_rn(og, tanhf(c_state[q]));
-            if (t + 1 < T) {
-                const uint32_t dst = smem_u32(h_s + (((t + 1) & 1) * kRecCluster + rank) * Y::BP + i);
-#pragma unroll
-                for (int k = 0; k < kRecCluster; ++k) store_remote(dst, static_cast<uint32_t>(k), hval[q]);
-            }
-        }
-        if (t + 1 < T) cluster_arrive();
-#pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-            const int i = q * kWideThreads + tid, row = b0 + i / Y::U;
-            if (i < kItems && row < B) {
-                const int64_t o = (static_cast<int64_t>(t) * B + row) * H + j0 + i % Y::U;
-                hs[o] = hval[q];
-                cs[o] = c_state[q];
-            }
-        }
-        if (t + 1 < T) {
-            fetch(t + 1);
+        } else {
             cluster_wait();
+        }
+    }
+    cluster_arrive();  // nobody leaves while another CTA may still store into its shared memory
+    cluster_wait();
+    if (*late) {       // (after a wait that ran out, stores may be under way)
+        const unsigned long long t0 = clock64();
+        while (clock64() - t0 < 400000ull) {
         }
     }
 }
 
 template <class Kernel>
 static int launch_rec(Kernel kernel, int threads, size_t smem, int rows, const float* pre, const float* w_hh, int T, int B, float* hs,
-                      float* cs, cudaStream_t st) {
+                      float* cs, int32_t* status, cudaStream_t st) {
     FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "lstm_recurrent attr"));
     FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "lstm_recurrent attr"));
     cudaLaunchConfig_t cfg = {};
@@ -388,37 +471,38 @@ static int launch_rec(Kernel kernel, int threads, size_t smem, int rows, const f
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    FB_TRY(check_cuda(cudaLaunchKernelEx(&cfg, kernel, pre, w_hh, T, B, hs, cs), "lstm_recurrent launch"));
+    FB_TRY(check_cuda(cudaLaunchKernelEx(&cfg, kernel, pre, w_hh, T, B, hs, cs, status), "lstm_recurrent launch"));
     count_launch();
     return FB_OK;
 }
 template <int H, int R>
-static int launch_narrow(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, cudaStream_t st) {
+static int launch_narrow(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     static_assert(RecLayout<H, R>::bytes <= 227 * 1024, "shared memory of one CTA");
-    return launch_rec(lstm_recurrent_kernel<H, R>, kRecThreads, RecLayout<H, R>::bytes, R, pre, w_hh, T, B, hs, cs, st);
+    return launch_rec(lstm_recurrent_kernel<H, R>, kRecThreads, RecLayout<H, R>::bytes, R, pre, w_hh, T, B, hs, cs, status, st);
 }
 template <int H, int R>
-static int launch_wide(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, cudaStream_t st) {
-    static_assert(WideLayout<H, R>::bytes <= 227 * 1024, "shared memory of one CTA");
-    return launch_rec(lstm_recurrent_wide_kernel<H, R>, kWideThreads, WideLayout<H, R>::bytes, R, pre, w_hh, T, B, hs, cs, st);
+static int launch_pair(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
+    using Y = PairLayout<H, R / 2>;
+    static_assert(R % 2 == 0 && Y::bytes <= 227 * 1024, "shared memory of one CTA");
+    return launch_rec(lstm_recurrent_pair_kernel<H, R / 2>, kPairThreads, Y::bytes, R, pre, w_hh, T, B, hs, cs, status, st);
 }
 
 // Rows per cluster: the fewest that let all clusters run at once (seven clusters of sixteen whole SMs fit a B200; more clusters
 // than that run one after the other).
 template <int H>
-static int launch_rec_rows(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, cudaStream_t st) {
+static int launch_rec_rows(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     constexpr int kClusters = 7;
-    if (B <= kClusters) return launch_narrow<H, 1>(pre, w_hh, T, B, hs, cs, st);
-    if (B <= 2 * kClusters) return launch_narrow<H, 2>(pre, w_hh, T, B, hs, cs, st);
-    if (B <= 4 * kClusters) return launch_wide<H, 4>(pre, w_hh, T, B, hs, cs, st);
-    if (B <= 6 * kClusters) return launch_wide<H, 6>(pre, w_hh, T, B, hs, cs, st);
-    if (B <= 8 * kClusters) return launch_wide<H, 8>(pre, w_hh, T, B, hs, cs, st);
-    return launch_wide<H, 10>(pre, w_hh, T, B, hs, cs, st);
+    if (B <= kClusters) return launch_narrow<H, 1>(pre, w_hh, T, B, hs, cs, status, st);
+    if (B <= 2 * kClusters) return launch_narrow<H, 2>(pre, w_hh, T, B, hs, cs, status, st);
+    if (B <= 4 * kClusters) return launch_pair<H, 4>(pre, w_hh, T, B, hs, cs, status, st);
+    if (B <= 6 * kClusters) return launch_pair<H, 6>(pre, w_hh, T, B, hs, cs, status, st);
+    if (B <= 8 * kClusters) return launch_pair<H, 8>(pre, w_hh, T, B, hs, cs, status, st);
+    return launch_pair<H, 10>(pre, w_hh, T, B, hs, cs, status, st);
 }
 
-int launch_lstm_recurrent(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, cudaStream_t st) {
+int launch_lstm_recurrent(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     FB_REQUIRE(H == 256 || H == 512, "lstm recurrence: hidden size %d not supported (256 or 512)", H);
-    return H == 512 ? launch_rec_rows<512>(pre, w_hh, T, B, hs, cs, st) : launch_rec_rows<256>(pre, w_hh, T, B, hs, cs, st);
+    return H == 512 ? launch_rec_rows<512>(pre, w_hh, T, B, hs, cs, status, st) : launch_rec_rows<256>(pre, w_hh, T, B, hs, cs, status, st);
 }
 
 }  // namespace fb
