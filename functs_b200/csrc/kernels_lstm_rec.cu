@@ -214,6 +214,7 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
 constexpr int kPairFma = 256, kPairGate = 256, kPairThreads = kPairFma + kPairGate;
 constexpr int kPairFmaRegs = 200, kPairGateRegs = 56;               // of 128 per thread at launch
 static_assert((kPairFmaRegs + kPairGateRegs) * 256 <= kPairThreads * 128, "registers of the launch");
+constexpr int kPairAhead = 2;                                       // steps that the projection's values are fetched ahead
 constexpr uint32_t kRecWaitLimit = 2000000u;
 
 template <int H, int RH>                                            // RH: rows of a half
@@ -230,7 +231,8 @@ struct PairLayout {
     static constexpr size_t h_floats = 4ull * kRecCluster * BP;     // [buffer][half]
     static constexpr size_t part_floats = 2ull * KQ * RH * 4 * U;   // [half]
     static constexpr size_t w_bytes = static_cast<size_t>(SmemK) * 2 * kPairFma * 16;
-    static constexpr size_t bytes = w_bytes + (h_floats + part_floats) * 4 + 64;
+    static constexpr size_t pre_floats = (kPairAhead + 1ull) * 2 * RH * 4 * U;  // [step][half][RH][4][U]
+    static constexpr size_t bytes = w_bytes + (h_floats + part_floats + pre_floats) * 4 + 64;
     static_assert(U % KT == 0 && RegK % 2 == 0 && SmemK % 2 == 0, "a k-slice lies inside one part of h");
     static_assert(GateWarps * 32 <= kPairGate, "one thread per item");
 };
@@ -272,8 +274,9 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemK][2][kPairFma]
     float* h_s = reinterpret_cast<float*>(smem_raw + Y::w_bytes);               // [buffer][half][16][BP]
-    float* part = h_s + Y::h_floats;                                            // [half][KQ][RH][4][U]
-    uint64_t* full = reinterpret_cast<uint64_t*>(part + Y::part_floats);        // [half][buffer]
+    float* part = h_s + Y::h_floats;                                            // [half][KQ][RH][U][4]
+    float* pre_s = part + Y::part_floats;                                       // [step % 3][half][RH][4][U]
+    uint64_t* full = reinterpret_cast<uint64_t*>(pre_s + Y::pre_floats);        // [half][buffer]
     int* late = reinterpret_cast<int*>(full + 4);                               // a wait ran out
     const int tid = threadIdx.x, lane = tid & 31;
     const int rank = static_cast<int>(cluster_rank());
@@ -353,21 +356,21 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
                 const unsigned long long w0[4] = {a0.x, a0.y, a1.x, a1.y}, w1[4] = {b0_.x, b0_.y, b1_.x, b1_.y};
                 pair(h_t + Y::RegK + k, w0, w1);
             }
-            // sum over the warp's four k-slices: after the two exchanges lane group q holds gate q of both units
+            // sum over the warp's four k-slices: after the two exchanges a lane holds two gates of one of its units
             const bool up = (lane & 16) != 0, odd = (lane & 8) != 0;
-            auto other = [&](unsigned long long v, int mask) { return __shfl_xor_sync(kFullMask, v, mask); };
-            auto add2 = [&](unsigned long long a, unsigned long long b) {
-                unsigned long long d;
-                asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-                return d;
-            };
 #pragma unroll
             for (int r = 0; r < RH; ++r) {
-                unsigned long long a[2];
+                float a[4];
 #pragma unroll
-                for (int c = 0; c < 2; ++c) a[c] = add2(up ? acc[2 + c][r] : acc[c][r], other(up ? acc[c][r] : acc[2 + c][r], 16));
-                const unsigned long long s = add2(odd ? a[1] : a[0], other(odd ? a[0] : a[1], 8));
-                *reinterpret_cast<unsigned long long*>(part + (((half * Y::KQ + kq) * RH + r) * 4 + (lane >> 3)) * Y::U + unit) = s;
+                for (int c = 0; c < 4; ++c) {
+                    float u0, u1;
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(u0), "=f"(u1) : "l"(acc[c][r]));
+                    a[c] = __fadd_rn(up ? u1 : u0, __shfl_xor_sync(kFullMask, up ? u0 : u1, 16));
+                }
+                const float s0 = __fadd_rn(odd ? a[2] : a[0], __shfl_xor_sync(kFullMask, odd ? a[0] : a[2], 8));
+                const float s1 = __fadd_rn(odd ? a[3] : a[1], __shfl_xor_sync(kFullMask, odd ? a[1] : a[3], 8));
+                *reinterpret_cast<float2*>(part + (((half * Y::KQ + kq) * RH + r) * Y::U + unit + (lane >> 4)) * 4 + (odd ? 2 : 0)) =
+                    make_float2(s0, s1);
             }
             asm volatile("barrier.arrive %0, %1;" ::"r"(1 + half), "n"(kPairFma + Y::GateWarps * 32) : "memory");
         }
@@ -375,68 +378,97 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
         // ---- gates and exchange: one thread per (row, unit) of a half ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairGateRegs));
         cluster_arrive();
-        if ((tid - kPairFma) / 32 < Y::GateWarps) {
-            const int i = tid - kPairFma, ir = i / Y::U, iu = i % Y::U;
-            const bool item = i < Y::Items;                                     // (a last half warp may have none)
-            const int irc = item ? ir : 0;
-            float c_state[2] = {0.0f, 0.0f}, pre_g[2][4] = {};
-            auto fetch = [&](int t, int half) {
-                const int row = b0 + half * RH + ir;
-                if (!item || row >= B) return;
-                const float* p = pre + (static_cast<int64_t>(t) * B + row) * (4 * H) + j0 + iu;
+        // The first half's items are on the first warps, the second half's on the last ones: no scheduler has the odd warp of both.
+        const int gw = (tid - kPairFma) >> 5;
+        if (gw < Y::GateWarps || gw >= kPairGate / 32 - Y::GateWarps) {
+            int item[2];                                                        // (row, unit) of each half, or -1
+            item[0] = tid - kPairFma;
+            item[1] = item[0] - (kPairGate - Y::GateWarps * 32);
+            const bool mine[2] = {gw < Y::GateWarps, item[1] >= 0};             // the warp has items of this half
 #pragma unroll
-                for (int g = 0; g < 4; ++g) pre_g[half][g] = __ldcg(p + g * H);
+            for (int half = 0; half < 2; ++half) item[half] = item[half] < Y::Items ? item[half] : -1;
+            const int iu = tid % Y::U;
+            float c_state[2] = {0.0f, 0.0f};
+            // The projection's values come through shared memory, 16 bytes a thread: a load into registers one step ahead took
+            // longer than the step (2500 cycles behind the shared-memory traffic of the multiplications), and every gate waited.
+            const int fg = iu / (Y::U / 4), fu = iu % (Y::U / 4) * 4;           // gate and first unit that this thread fetches
+            auto fetch = [&](int t, int half) {
+                if (item[half] >= 0 && t < T) {
+                    const int ir = item[half] / Y::U, row = b0 + half * RH + ir;
+                    const float* p = pre + (static_cast<int64_t>(t) * B + (row < B ? row : 0)) * (4 * H) + fg * H + j0 + fu;
+                    const uint32_t to = smem_u32(pre_s + (((t % (kPairAhead + 1)) * 2 + half) * Y::Items + item[half]) * 4);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(p) : "memory");
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
             };
-            pdl_wait();  // the projection (read with __ldcg: a __ldg could be moved up across this); the weights are not its output
-            fetch(0, 0);
-            fetch(0, 1);
+            pdl_wait();  // the projection; the weights are not its output
+#pragma unroll
+            for (int t = 0; t < kPairAhead; ++t) {
+                fetch(t, 0);
+                fetch(t, 1);
+            }
             // this lane sends its quad of units to four CTAs
             uint32_t dst[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) dst[k] = map_remote(smem_u32(smem_raw), static_cast<uint32_t>((lane & 3) * 4 + k));
-            const uint32_t h_off = smem_u32(h_s + rank * Y::BP + irc * Y::U + (iu & ~3)) - smem_u32(smem_raw);
+            const uint32_t h_off = smem_u32(h_s + rank * Y::BP) - smem_u32(smem_raw);
             const uint32_t bar_off = smem_u32(full) - smem_u32(smem_raw);
             cluster_wait();
 #pragma unroll 1
             for (int t = 0; t < T; ++t) {
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    float gate[4];
-                    if (t > 0) asm volatile("barrier.sync %0, %1;" ::"r"(1 + half), "n"(kPairFma + Y::GateWarps * 32) : "memory");
+                    asm volatile("cp.async.wait_group %0;" ::"n"(2 * kPairAhead - 1) : "memory");
+                    if (mine[half]) {
+                        const int i = item[half] >= 0 ? item[half] : 0;
+                        if (t > 0)  // the partial sums of all warps, the fetched values of all gate threads
+                            asm volatile("barrier.sync %0, %1;" ::"r"(1 + half), "n"(kPairFma + Y::GateWarps * 32) : "memory");
+                        else
+                            asm volatile("barrier.sync %0, %1;" ::"r"(3 + half), "n"(Y::GateWarps * 32) : "memory");
+                        const float* pre_t = pre_s + ((t % (kPairAhead + 1)) * 2 + half) * (Y::Items * 4) + i / Y::U * (4 * Y::U) + iu;
+                        float gate[4];
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        gate[g] = pre_g[half][g];
+                        for (int g = 0; g < 4; ++g) gate[g] = pre_t[g * Y::U];
                         if (t > 0) {
-                            const float* p = part + ((half * Y::KQ * RH + irc) * 4 + g) * Y::U + iu;
-                            float s = p[0];
+                            const float4* p = reinterpret_cast<const float4*>(part) + half * Y::KQ * Y::Items + i;
+                            float4 s = p[0];
 #pragma unroll
-                            for (int k = 1; k < Y::KQ; ++k) s = __fadd_rn(s, p[k * RH * 4 * Y::U]);
-                            gate[g] = __fadd_rn(gate[g], s);
+                            for (int k = 1; k < Y::KQ; ++k) {
+                                const float4 v = p[k * Y::Items];
+                                s.x = __fadd_rn(s.x, v.x);
+                                s.y = __fadd_rn(s.y, v.y);
+                                s.z = __fadd_rn(s.z, v.z);
+                                s.w = __fadd_rn(s.w, v.w);
+                            }
+                            gate[0] = __fadd_rn(gate[0], s.x);
+                            gate[1] = __fadd_rn(gate[1], s.y);
+                            gate[2] = __fadd_rn(gate[2], s.z);
+                            gate[3] = __fadd_rn(gate[3], s.w);
+                        }
+                        float sg[3] = {gate[0], gate[1], gate[3]};
+                        sigmoid_f32_n(sg);
+                        const float ig = sg[0], fgt = sg[1], og = sg[2], gg = tanhf(gate[2]);
+                        c_state[half] = __fadd_rn(__fmul_rn(fgt, c_state[half]), __fmul_rn(ig, gg));
+                        const float hval = __fmul_rn(og, tanhf(c_state[half]));
+                        if (t + 1 < T) {
+                            float v[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(kFullMask, hval, (lane & ~3) + k);
+                            const uint32_t to = h_off + static_cast<uint32_t>((((t + 1) & 1) * 2 + half) * (kRecCluster * Y::BP) + (i & ~3)) * 4;
+                            const uint32_t bar = bar_off + static_cast<uint32_t>(half * 2 + ((t + 1) & 1)) * 8;
+                            if (item[half] >= 0) {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) store_async4(dst[k] + to, v[0], v[1], v[2], v[3], dst[k] + bar);
+                            }
+                        }
+                        const int row = b0 + half * RH + i / Y::U;
+                        if (item[half] >= 0 && row < B) {
+                            const int64_t o = (static_cast<int64_t>(t) * B + row) * H + j0 + iu;
+                            hs[o] = hval;
+                            cs[o] = c_state[half];
                         }
                     }
-                    float sg[3] = {gate[0], gate[1], gate[3]};
-                    sigmoid_f32_n(sg);
-                    const float ig = sg[0], fg = sg[1], og = sg[2], gg = tanhf(gate[2]);
-                    c_state[half] = __fadd_rn(__fmul_rn(fg, c_state[half]), __fmul_rn(ig, gg));
-                    const float hval = __fmul_rn(og, tanhf(c_state[half]));
-                    if (t + 1 < T) {
-                        float v[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(kFullMask, hval, (lane & ~3) + k);
-                        const uint32_t to = h_off + static_cast<uint32_t>((((t + 1) & 1) * 2 + half) * (kRecCluster * Y::BP) * 4);
-                        const uint32_t bar = bar_off + static_cast<uint32_t>(half * 2 + ((t + 1) & 1)) * 8;
-                        if (item) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) store_async4(dst[k] + to, v[0], v[1], v[2], v[3], dst[k] + bar);
-                        }
-                    }
-                    const int row = b0 + half * RH + ir;
-                    if (item && row < B) {
-                        const int64_t o = (static_cast<int64_t>(t) * B + row) * H + j0 + iu;
-                        hs[o] = hval;
-                        cs[o] = c_state[half];
-                    }
-                    if (t + 1 < T) fetch(t + 1, half);
+                    fetch(t + kPairAhead, half);  // (into the place of step t - 1, which all threads have read)
                 }
             }
         } else {
