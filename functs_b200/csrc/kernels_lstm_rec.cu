@@ -23,6 +23,8 @@ constexpr int kRecCluster = 16;
 constexpr int kRecThreads = 512;
 constexpr int kRecUnitsPerWarp = 8;
 constexpr int kRecSlices = 2;  // k-slices inside a warp
+constexpr int kRecAhead = 2;   // steps that the projection's values are fetched ahead
+constexpr uint32_t kRecWaitLimit = 2000000u;
 
 template <int H, int R>
 struct RecLayout {
@@ -37,8 +39,13 @@ struct RecLayout {
     static constexpr size_t h_floats = 2ull * kRecCluster * BP;
     static constexpr size_t part_floats = static_cast<size_t>(KQ) * R * 4 * U;
     static constexpr size_t w_bytes = static_cast<size_t>(SmemQuads) * 2 * kRecThreads * 16;
-    static constexpr size_t bytes = w_bytes + (h_floats + part_floats) * 4;
+    static constexpr int Items = R * U;                             // (row, unit) pairs of the CTA
+    static constexpr int GateWarps = (Items + 31) / 32;
+    static constexpr int Sends = kRecCluster * (Items / 4) / (GateWarps * 32);  // CTAs that a gate thread sends a quad of units to
+    static constexpr size_t pre_floats = (kRecAhead + 1ull) * Items * 4;        // [step][R][4][U]
+    static constexpr size_t bytes = w_bytes + (h_floats + part_floats + pre_floats) * 4 + 32;
     static_assert(KT % U == 0, "a k-slice is whole parts of h");
+    static_assert(Items % 16 == 0 && Items / 4 * kRecCluster == Sends * GateWarps * 32, "every gate thread sends");
 };
 
 __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
@@ -61,11 +68,35 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void store_remote(uint32_t local_addr, uint32_t rank, float v) {
+// Address of this CTA's shared-memory word in the CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_remote(uint32_t local_addr, uint32_t rank) {
     uint32_t a;
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+    return a;
 }
+__device__ __forceinline__ void store_async4(uint32_t remote, float a, float b, float c, float d, uint32_t remote_bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(remote), "f"(a),
+                 "f"(b), "f"(c), "f"(d), "r"(remote_bar)
+                 : "memory");
+}
+// Wait for what other CTAs of the cluster store; false when the limit runs out.
+__device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < kRecWaitLimit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+// Phase of a buffer's mbarrier that step t waits for: steps 1, 3, 5, ... use buffer 1, steps 2, 4, ... buffer 0.
+__device__ __forceinline__ uint32_t step_parity(int t) { return static_cast<uint32_t>((t - 1) >> 1) & 1u; }
+
 // (not the .aligned forms: the lanes of a warp come here from different sides of a branch)
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
@@ -74,12 +105,15 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 template <int H, int R>
 __global__ void __launch_bounds__(kRecThreads, 1)
 lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,
-                      float* __restrict__ cs, int32_t* /*status*/) {
+                      float* __restrict__ cs, int32_t* status) {
     using Y = RecLayout<H, R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemQuads][2][kRecThreads]
     float* h_s = reinterpret_cast<float*>(smem_raw + Y::w_bytes);               // [2][16][BP]
-    float* part = h_s + Y::h_floats;                                            // [KQ][R][4][U]
+    float* part = h_s + Y::h_floats;                                            // [KQ][R][U][4]
+    float* pre_s = part + Y::part_floats;                                       // [step % 3][R][4][U]
+    uint64_t* full = reinterpret_cast<uint64_t*>(pre_s + Y::pre_floats);        // [buffer]
+    int* late = reinterpret_cast<int*>(full + 2);                               // a wait ran out
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = static_cast<int>(cluster_rank());
     const int b0 = static_cast<int>(blockIdx.x / kRecCluster) * R;
@@ -87,6 +121,16 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
     const int gates = (lane >> 2) & 2;                                          // first of this thread's two gates
     const int kq = warp / Y::WG, slice = kq * kRecSlices + (lane >> 4);         // k = slice * KT ...
     const int j0 = rank * Y::U;
+    constexpr uint32_t kPhaseBytes = R * H * 4;                                 // all of h
+    if (tid == 0) {
+        *late = 0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(full + i, 1);
+            mbar_arrive_expect_tx(full + i, kPhaseBytes);
+        }
+        fence_barrier_init();
+    }
 
     // resident weights: gate c, k -> w_hh[c][k][j0 + unit]
     unsigned long long w_r[Y::RegQuads][2][2];
@@ -106,28 +150,44 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
             }
         }
     }
-    // one thread per (row, unit) of the CTA: gates, cell state, outputs
-    constexpr int kItems = R * Y::U;
-    static_assert(kItems <= kRecThreads, "one thread per item");
-    const bool item = tid < kItems;
-    const int ir = item ? tid / Y::U : 0, iu = tid % Y::U;
-    const int row = b0 + ir;
-    const bool live = item && row < B;
-    const int k_own = j0 + iu;                                                  // this item's place in a row of h
-    const uint32_t h_own = smem_u32(h_s + rank * Y::BP + ir * Y::U + iu);
+    // the first warps: one thread per (row, unit) of the CTA applies the gates, keeps the cell state and writes the outputs
+    const bool gating = warp < Y::GateWarps, item = tid < Y::Items;
+    const int i = item ? tid : 0, iu = i % Y::U, row = b0 + i / Y::U;
     float c_state = 0.0f;
-    float pre_g[4] = {0.f, 0.f, 0.f, 0.f};
-    pdl_wait();  // the projection (read with __ldcg: a __ldg could be moved up across this); the weights are not its output
-    if (live) {
-        const float* p = pre + static_cast<int64_t>(row) * (4 * H) + k_own;
+    // 16 bytes a thread: gate (tid % U) / (U / 4), four units
+    auto fetch = [&](int t) {
+        if (item && t < T) {
+            const int g = iu / (Y::U / 4), u = iu % (Y::U / 4) * 4;
+            const float* p = pre + (static_cast<int64_t>(t) * B + (row < B ? row : 0)) * (4 * H) + g * H + j0 + u;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(pre_s + ((t % (kRecAhead + 1)) * Y::Items + i) * 4)), "l"(p)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // what this thread sends: a quad of units to Sends CTAs
+    const int per_quad = kRecCluster / Y::Sends, quad = lane / per_quad;
+    uint32_t dst[Y::Sends];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) pre_g[g] = __ldcg(p + g * H);
+    for (int k = 0; k < Y::Sends; ++k)
+        dst[k] = map_remote(smem_u32(smem_raw), static_cast<uint32_t>(lane % per_quad * Y::Sends + k));
+    const uint32_t h_off = smem_u32(h_s + rank * Y::BP + warp * 32 + quad * 4) - smem_u32(smem_raw);
+    const uint32_t bar_off = smem_u32(full) - smem_u32(smem_raw);
+    if (gating) {
+        pdl_wait();  // the projection; the weights are not its output
+#pragma unroll
+        for (int t = 0; t < kRecAhead; ++t) fetch(t);
     }
-    cluster_arrive();  // every CTA of the cluster runs before anybody stores into another one
+    cluster_arrive();  // every CTA of the cluster runs, its barriers set, before anybody stores into another one
     cluster_wait();
+    bool waiting = true;
     for (int t = 0; t < T; ++t) {
-        float gate[4] = {pre_g[0], pre_g[1], pre_g[2], pre_g[3]};
         if (t > 0) {
+            if (waiting && !wait_cluster(smem_u32(full + (t & 1)), step_parity(t))) {
+                waiting = false;  // the rest is computed from what is there: every CTA goes through all steps
+                *late = 1;
+                if (status != nullptr) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
+            }
+            if (tid == 0 && t + 2 < T) mbar_arrive_expect_tx(full + (t & 1), kPhaseBytes);
             const float* h_t = h_s + ((t & 1) * kRecCluster + slice * (Y::KT / Y::U)) * Y::BP;
             unsigned long long acc[2][R];
 #pragma unroll
@@ -159,44 +219,65 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
             for (int r = 0; r < R; ++r) {
                 const float v0 = sum2(acc[0][r]), v1 = sum2(acc[1][r]);
                 const float b = __fadd_rn(up ? v1 : v0, __shfl_xor_sync(kFullMask, up ? v0 : v1, 16));
-                part[((kq * R + r) * 4 + gates + (lane >> 4)) * Y::U + unit] = b;
-            }
-            __syncthreads();
-            if (item) {
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    float s = part[(ir * 4 + g) * Y::U + iu];
-#pragma unroll
-                    for (int k = 1; k < Y::KQ; ++k) s = __fadd_rn(s, part[((k * R + ir) * 4 + g) * Y::U + iu]);
-                    gate[g] = __fadd_rn(gate[g], s);
-                }
+                part[((kq * R + r) * Y::U + unit) * 4 + gates + (lane >> 4)] = b;
             }
         }
-        float hval = 0.0f;
-        if (item) {
-            float sg[3] = {gate[0], gate[1], gate[3]};
-            sigmoid_f32_n(sg);
-            const float ig = sg[0], fg = sg[1], og = sg[2], gg = tanhf(gate[2]);
-            c_state = __fadd_rn(__fmul_rn(fg, c_state), __fmul_rn(ig, gg));
-            hval = __fmul_rn(og, tanhf(c_state));
-            if (t + 1 < T) {
-                const uint32_t dst = h_own + static_cast<uint32_t>(((t + 1) & 1) * (kRecCluster * Y::BP) * 4);
-#pragma unroll
-                for (int k = 0; k < kRecCluster; ++k) store_remote(dst, static_cast<uint32_t>(k), hval);
-            }
+        // the partial sums of all warps, the fetched values of the gate warps; the other warps go on to the next step
+        if (!gating) {
+            __syncwarp();
+            asm volatile("barrier.arrive 1, %0;" ::"n"(kRecThreads) : "memory");
+            continue;
         }
-        if (t + 1 < T) cluster_arrive();
-        if (live) {
-            const int64_t o = (static_cast<int64_t>(t) * B + row) * H + k_own;
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRecAhead - 1) : "memory");
+        __syncwarp();
+        asm volatile("barrier.sync 1, %0;" ::"n"(kRecThreads) : "memory");
+        const float* pre_t = pre_s + (t % (kRecAhead + 1)) * (Y::Items * 4) + i / Y::U * (4 * Y::U) + iu;
+        float gate[4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) gate[g] = pre_t[g * Y::U];
+        if (t > 0) {
+            const float4* p = reinterpret_cast<const float4*>(part) + i;
+            float4 s = p[0];
+#pragma unroll
+            for (int k = 1; k < Y::KQ; ++k) {
+                const float4 v = p[k * Y::Items];
+                s.x = __fadd_rn(s.x, v.x);
+                s.y = __fadd_rn(s.y, v.y);
+                s.z = __fadd_rn(s.z, v.z);
+                s.w = __fadd_rn(s.w, v.w);
+            }
+            gate[0] = __fadd_rn(gate[0], s.x);
+            gate[1] = __fadd_rn(gate[1], s.y);
+            gate[2] = __fadd_rn(gate[2], s.z);
+            gate[3] = __fadd_rn(gate[3], s.w);
+        }
+        float sg[3] = {gate[0], gate[1], gate[3]};
+        sigmoid_f32_n(sg);
+        const float ig = sg[0], fg = sg[1], og = sg[2], gg = tanhf(gate[2]);
+        c_state = __fadd_rn(__fmul_rn(fg, c_state), __fmul_rn(ig, gg));
+        const float hval = __fmul_rn(og, tanhf(c_state));
+        if (t + 1 < T) {
+            float v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(kFullMask, hval, quad * 4 + k);
+            const uint32_t to = h_off + static_cast<uint32_t>(((t + 1) & 1) * (kRecCluster * Y::BP)) * 4;
+            const uint32_t bar = bar_off + static_cast<uint32_t>((t + 1) & 1) * 8;
+#pragma unroll
+            for (int k = 0; k < Y::Sends; ++k) store_async4(dst[k] + to, v[0], v[1], v[2], v[3], dst[k] + bar);
+        }
+        if (item && row < B) {
+            const int64_t o = (static_cast<int64_t>(t) * B + row) * H + j0 + iu;
             hs[o] = hval;
             cs[o] = c_state;
-            if (t + 1 < T) {
-                const float* p = pre + (static_cast<int64_t>(t + 1) * B + row) * (4 * H) + k_own;
-#pragma unroll
-                for (int g = 0; g < 4; ++g) pre_g[g] = __ldcg(p + g * H);
-            }
         }
-        if (t + 1 < T) cluster_wait();
+        fetch(t + kRecAhead);  // (into the place of step t - 1, which all gate threads have read)
+    }
+    cluster_arrive();  // nobody leaves while another CTA may still store into its shared memory
+    cluster_wait();
+    if (*late) {       // (after a wait that ran out, stores may be under way)
+        const unsigned long long t0 = clock64();
+        while (clock64() - t0 < 400000ull) {
+        }
     }
 }
 
@@ -214,8 +295,6 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
 constexpr int kPairFma = 256, kPairGate = 256, kPairThreads = kPairFma + kPairGate;
 constexpr int kPairFmaRegs = 200, kPairGateRegs = 56;               // of 128 per thread at launch
 static_assert((kPairFmaRegs + kPairGateRegs) * 256 <= kPairThreads * 128, "registers of the launch");
-constexpr int kPairAhead = 2;                                       // steps that the projection's values are fetched ahead
-constexpr uint32_t kRecWaitLimit = 2000000u;
 
 template <int H, int RH>                                            // RH: rows of a half
 struct PairLayout {
@@ -231,40 +310,11 @@ struct PairLayout {
     static constexpr size_t h_floats = 4ull * kRecCluster * BP;     // [buffer][half]
     static constexpr size_t part_floats = 2ull * KQ * RH * 4 * U;   // [half]
     static constexpr size_t w_bytes = static_cast<size_t>(SmemK) * 2 * kPairFma * 16;
-    static constexpr size_t pre_floats = (kPairAhead + 1ull) * 2 * RH * 4 * U;  // [step][half][RH][4][U]
+    static constexpr size_t pre_floats = (kRecAhead + 1ull) * 2 * RH * 4 * U;  // [step][half][RH][4][U]
     static constexpr size_t bytes = w_bytes + (h_floats + part_floats + pre_floats) * 4 + 64;
     static_assert(U % KT == 0 && RegK % 2 == 0 && SmemK % 2 == 0, "a k-slice lies inside one part of h");
     static_assert(GateWarps * 32 <= kPairGate, "one thread per item");
 };
-
-// Address of this CTA's shared-memory word in the CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t map_remote(uint32_t local_addr, uint32_t rank) {
-    uint32_t a;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
-    return a;
-}
-__device__ __forceinline__ void store_async4(uint32_t remote, float a, float b, float c, float d, uint32_t remote_bar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(remote), "f"(a),
-                 "f"(b), "f"(c), "f"(d), "r"(remote_bar)
-                 : "memory");
-}
-// Wait for what other CTAs of the cluster store; false when the limit runs out.
-__device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < kRecWaitLimit; ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-// Phase of a buffer's mbarrier that step t waits for: steps 1, 3, 5, ... use buffer 1, steps 2, 4, ... buffer 0.
-__device__ __forceinline__ uint32_t step_parity(int t) { return static_cast<uint32_t>((t - 1) >> 1) & 1u; }
 
 template <int H, int RH>
 __global__ void __launch_bounds__(kPairThreads, 1)
@@ -372,6 +422,7 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
                 *reinterpret_cast<float2*>(part + (((half * Y::KQ + kq) * RH + r) * Y::U + unit + (lane >> 4)) * 4 + (odd ? 2 : 0)) =
                     make_float2(s0, s1);
             }
+            __syncwarp();
             asm volatile("barrier.arrive %0, %1;" ::"r"(1 + half), "n"(kPairFma + Y::GateWarps * 32) : "memory");
         }
     } else {
@@ -396,14 +447,14 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
                 if (item[half] >= 0 && t < T) {
                     const int ir = item[half] / Y::U, row = b0 + half * RH + ir;
                     const float* p = pre + (static_cast<int64_t>(t) * B + (row < B ? row : 0)) * (4 * H) + fg * H + j0 + fu;
-                    const uint32_t to = smem_u32(pre_s + (((t % (kPairAhead + 1)) * 2 + half) * Y::Items + item[half]) * 4);
+                    const uint32_t to = smem_u32(pre_s + (((t % (kRecAhead + 1)) * 2 + half) * Y::Items + item[half]) * 4);
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(p) : "memory");
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
             };
             pdl_wait();  // the projection; the weights are not its output
 #pragma unroll
-            for (int t = 0; t < kPairAhead; ++t) {
+            for (int t = 0; t < kRecAhead; ++t) {
                 fetch(t, 0);
                 fetch(t, 1);
             }
@@ -418,14 +469,15 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
             for (int t = 0; t < T; ++t) {
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    asm volatile("cp.async.wait_group %0;" ::"n"(2 * kPairAhead - 1) : "memory");
+                    asm volatile("cp.async.wait_group %0;" ::"n"(2 * kRecAhead - 1) : "memory");
                     if (mine[half]) {
                         const int i = item[half] >= 0 ? item[half] : 0;
+                        __syncwarp();
                         if (t > 0)  // the partial sums of all warps, the fetched values of all gate threads
                             asm volatile("barrier.sync %0, %1;" ::"r"(1 + half), "n"(kPairFma + Y::GateWarps * 32) : "memory");
                         else
                             asm volatile("barrier.sync %0, %1;" ::"r"(3 + half), "n"(Y::GateWarps * 32) : "memory");
-                        const float* pre_t = pre_s + ((t % (kPairAhead + 1)) * 2 + half) * (Y::Items * 4) + i / Y::U * (4 * Y::U) + iu;
+                        const float* pre_t = pre_s + ((t % (kRecAhead + 1)) * 2 + half) * (Y::Items * 4) + i / Y::U * (4 * Y::U) + iu;
                         float gate[4];
 #pragma unroll
                         for (int g = 0; g < 4; ++g) gate[g] = pre_t[g * Y::U];
@@ -468,7 +520,7 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
                             cs[o] = c_state[half];
                         }
                     }
-                    fetch(t + kPairAhead, half);  // (into the place of step t - 1, which all threads have read)
+                    fetch(t + kRecAhead, half);  // (into the place of step t - 1, which all threads have read)
                 }
             }
         } else {
