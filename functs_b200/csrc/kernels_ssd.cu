@@ -118,6 +118,30 @@ struct SsdRagged {
 };
 constexpr unsigned long long kSsdWaitCycles = 2000000000ull;  // ~1 s
 
+// NMS by suppression rows, thread t = row t: of the candidates in `bits` (tame boxes), or of every box behind the row.  Out of line:
+// its code should not sit in the middle of the class kernel's instruction stream.
+__device__ __noinline__ void ssd_nms_rows(const float4* sxy, const float* sarea, int n, bool tame, const uint32_t (&bits)[kSsdWords],
+                                          float iou_thr, float thr_lo, float thr_hi, uint32_t* keep_words, uint32_t* or_words) {
+    const int t = threadIdx.x;
+    uint32_t row[kSsdWords];
+    const float4 me = t < n ? sxy[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const NmsBox bi{me.x, me.y, me.z, me.w, t < n ? sarea[t] : 0.0f};
+#pragma unroll
+    for (int w = 0; w < kSsdWords; ++w) {
+        const int first = max(t + 1 - 32 * w, 0), last = min(n - 32 * w, 32);  // the boxes behind the row: bits first .. last - 1
+        uint32_t left = t >= n || first >= last ? 0u : (0xffffffffu << first) & (0xffffffffu >> (32 - last));
+        if (tame) left &= bits[w];
+        row[w] = 0u;
+        for (; left != 0u; left &= left - 1u) {
+            const int b = __ffs(left) - 1;
+            const float4 cj = sxy[32 * w + b];
+            if (iou_exceeds(bi, NmsBox{cj.x, cj.y, cj.z, cj.w, sarea[32 * w + b]}, iou_thr, thr_lo, thr_hi)) row[w] |= 1u << b;
+        }
+    }
+    __syncthreads();
+    block_nms_resolve<kSsdNmsThreads, kSsdWords>(row, n, keep_words, or_words);
+}
+
 // dynamic smem: [SelectSmem<256>][kCandCap candidate keys]; after the selection the NMS boxes live in the selection's boundary
 // list and the pair tables in the candidate list, which are not needed any more.  The class's scores (one contiguous
 // run of the class-major array) are read from global memory once: a sampled score floor, one collection pass, and the
@@ -141,6 +165,7 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
     __shared__ uint32_t keep_words[kSsdWords];
     __shared__ int word_prefix[kSsdWords + 1];
     __shared__ uint32_t or_words[2 * kSsdWords];
+    __shared__ int pair_count[2];
 
     const int t = threadIdx.x;
     int cls = blockIdx.x, img = blockIdx.y;
@@ -170,30 +195,24 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
         sxy[t] = mybox;
         sarea[t] = myarea;
     }
-    if (t < kSsdWords) keep_words[t] = 0u;
+    if (t < 2) pair_count[t] = 0;
     const bool tame = __syncthreads_and(tame_box ? 1 : 0) != 0;  // also the barrier behind the box stores
 
-    // Suppression rows, thread t = row t.  Tame boxes only test the pairs that PairCells leaves (200 x 200 all-pairs votes
-    // took 45 % of this kernel's time); a list with a wild box tests every pair behind the row.
+    // Tame boxes only test the pairs that PairCells leaves (200 x 200 all-pairs votes took 45 % of this kernel's time); lists with
+    // a wild box, or with more pairs than fit, form suppression rows.
     const int lane = t & 31, warp = t >> 5;
-    uint32_t row[kSsdWords];
+    uint32_t bits[kSsdWords];
+    bool done = false;
     if (tame) {
-        suppression_row<kSsdWords>(sxy, sarea, mybox, myarea, n, iou_thr, thr_lo, thr_hi, *reinterpret_cast<PairCells<kSsdWords>*>(cand), row);
-    } else {
-        const NmsBox bi{mybox.x, mybox.y, mybox.z, mybox.w, myarea};
-#pragma unroll
-        for (int w = 0; w < kSsdWords; ++w) {
-            row[w] = 0u;
-            if (t >= n) continue;
-            for (int j = max(32 * w, t + 1); j < min(32 * w + 32, n); ++j) {
-                const float4 cj = sxy[j];
-                const NmsBox bj{cj.x, cj.y, cj.z, cj.w, sarea[j]};
-                if (iou_exceeds(bi, bj, iou_thr, thr_lo, thr_hi)) row[w] |= 1u << (j & 31);
-            }
-        }
+        // (the histogram of the selection and the rest of its boundary list are free)
+        static_assert(sizeof(uint16_t) * PairLists::kPairs <= sizeof(sm.hist) &&
+                          (sizeof(float4) + sizeof(float)) * kSsdSelCap + sizeof(uint16_t) * PairLists::kHits <= sizeof(sm.binlist),
+                      "the pair lists reuse the selection's memory");
+        const PairLists pl{reinterpret_cast<uint16_t*>(sm.hist), reinterpret_cast<uint16_t*>(sarea + kSsdSelCap), pair_count, or_words};
+        pair_candidates<kSsdWords>(mybox, myarea, n, iou_thr, *reinterpret_cast<PairCells<kSsdWords>*>(cand), bits);
+        done = block_nms_pairs<kSsdWords>(sxy, sarea, bits, n, iou_thr, thr_lo, thr_hi, pl, keep_words);
     }
-    __syncthreads();
-    block_nms_resolve<kSsdNmsThreads, kSsdWords>(row, n, keep_words, or_words);
+    if (!done) ssd_nms_rows(sxy, sarea, n, tame, bits, iou_thr, thr_lo, thr_hi, keep_words, or_words);
     __syncthreads();
     if (t == 0) {
         int acc = 0;

@@ -117,6 +117,27 @@ def test_ssd_nan_in_the_deltas_stays_in_the_boxes(fb):
     assert torch.equal(got[0].cpu().nan_to_num(nan=-7.0), want[0].nan_to_num(nan=-7.0))
 
 
+@pytest.mark.parametrize("spread,size", [(0.0, 40.0), (3.0, 40.0), (40.0, 40.0), (500.0, 40.0), (None, 40.0), (None, 11.0), (4e20, 1e19)])
+def test_ssd_crowded_lists(fb, spread, size):
+    """Lists from one heap of boxes (every pair suppresses) over partly and hardly overlapping ones to staircases, in which every
+    box's fate hangs on the one before it, and boxes whose areas overflow: pair lists that are empty, full and too small."""
+    g = torch.Generator().manual_seed(17)
+    p, c = 260, 3
+    if spread is None:  # neighbours overlap by nine tenths, or by a little more than the threshold, in random order of score
+        xy = torch.stack([torch.arange(p) * (4.0 if size == 40.0 else 4.05), torch.full((p,), 60.0)], dim=1)
+    else:
+        xy = 60.0 + torch.rand(p, 2, generator=g) * spread
+    pri = torch.cat([xy, torch.full((p, 2), size)], dim=1)
+    o = W.SSDPost(score_thr=0.01, topk=200)
+    mod = fb.workloads.SSDBBox(pri, score_thr=0.01, topk=200, clamp_max=3e38)
+    loc, conf = torch.randn(2, p, 4, generator=g) * 0.02, torch.randn(2, p, c + 1, generator=g)
+    boxes, dets, ids, counts = mod.forward_padded(loc, conf)
+    scores = mod._bufs[2].cpu().permute(0, 2, 1).contiguous()
+    for i, got in enumerate(mod.unpad(dets, ids, counts)):
+        for a, b in zip(got, o.post_single(boxes[i].cpu(), scores[i])):
+            assert torch.equal(a.cpu(), b)
+
+
 def test_ssd_golden_decode(fb):
     """Decode against the fixture written by the reference's delta2bbox (clamp 320)."""
     import os
