@@ -118,9 +118,9 @@ struct SsdRagged {
 };
 constexpr unsigned long long kSsdWaitCycles = 2000000000ull;  // ~1 s
 
-// NMS by suppression rows, thread t = row t: of the candidates in `bits` (tame boxes), or of every box behind the row.  Out of line:
+// NMS by suppression rows, thread t = row t: of the candidates in the tables (tame boxes), or of every box behind the row.  Out of line:
 // its code should not sit in the middle of the class kernel's instruction stream.
-__device__ __noinline__ void ssd_nms_rows(const float4* sxy, const float* sarea, int n, bool tame, const uint32_t (&bits)[kSsdWords],
+__device__ __noinline__ void ssd_nms_rows(const float4* sxy, const float* sarea, int n, const PairCells<kSsdWords>* pc, const PairWindow window,
                                           float iou_thr, float thr_lo, float thr_hi, uint32_t* keep_words, uint32_t* or_words) {
     const int t = threadIdx.x;
     uint32_t row[kSsdWords];
@@ -130,7 +130,7 @@ __device__ __noinline__ void ssd_nms_rows(const float4* sxy, const float* sarea,
     for (int w = 0; w < kSsdWords; ++w) {
         const int first = max(t + 1 - 32 * w, 0), last = min(n - 32 * w, 32);  // the boxes behind the row: bits first .. last - 1
         uint32_t left = t >= n || first >= last ? 0u : (0xffffffffu << first) & (0xffffffffu >> (32 - last));
-        if (tame) left &= bits[w];
+        if (pc != nullptr) left &= pair_word(*pc, window, w);
         row[w] = 0u;
         for (; left != 0u; left &= left - 1u) {
             const int b = __ffs(left) - 1;
@@ -201,7 +201,8 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
     // Tame boxes only test the pairs that PairCells leaves (200 x 200 all-pairs votes took 45 % of this kernel's time); lists with
     // a wild box, or with more pairs than fit, form suppression rows.
     const int lane = t & 31, warp = t >> 5;
-    uint32_t bits[kSsdWords];
+    PairCells<kSsdWords>& pc = *reinterpret_cast<PairCells<kSsdWords>*>(cand);
+    PairWindow window = {};
     bool done = false;
     if (tame) {
         // (the histogram of the selection and the rest of its boundary list are free)
@@ -209,10 +210,10 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
                           (sizeof(float4) + sizeof(float)) * kSsdSelCap + sizeof(uint16_t) * PairLists::kHits <= sizeof(sm.binlist),
                       "the pair lists reuse the selection's memory");
         const PairLists pl{reinterpret_cast<uint16_t*>(sm.hist), reinterpret_cast<uint16_t*>(sarea + kSsdSelCap), pair_count, or_words};
-        pair_candidates<kSsdWords>(mybox, myarea, n, iou_thr, *reinterpret_cast<PairCells<kSsdWords>*>(cand), bits);
-        done = block_nms_pairs<kSsdWords>(sxy, sarea, bits, n, iou_thr, thr_lo, thr_hi, pl, keep_words);
+        window = pair_tables<kSsdWords>(mybox, myarea, n, iou_thr, pc);
+        done = block_nms_pairs<kSsdWords>(sxy, sarea, pc, window, n, iou_thr, thr_lo, thr_hi, pl, keep_words);
     }
-    if (!done) ssd_nms_rows(sxy, sarea, n, tame, bits, iou_thr, thr_lo, thr_hi, keep_words, or_words);
+    if (!done) ssd_nms_rows(sxy, sarea, n, tame ? &pc : nullptr, window, iou_thr, thr_lo, thr_hi, keep_words, or_words);
     __syncthreads();
     if (t == 0) {
         int acc = 0;

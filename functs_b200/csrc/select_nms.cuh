@@ -536,6 +536,82 @@ __device__ __noinline__ int block_select_dense_outlined(const float* s, bool vec
     return block_select_topk_binned<NT, SELCAP, 8>(DenseScores{s, thr, vec4}, n, topk, hist_base, hist_shift, *sm);
 }
 
+// Same result as block_select_topk_binned for 1 <= c <= kCandCap keys in shared memory, by one counting sort: a key's bucket and its
+// place among the bucket's arrivals come from one atomic, the buckets' places from a scan, and every key counts the larger ones of
+// its own bucket (a key or two, unless many scores are nearly equal: then the general form takes over).  sm.hist is zero.
+template <int NT, int SELCAP>
+__device__ __forceinline__ int block_select_topk_list(const uint64_t* keys, int c, int topk, uint32_t hist_base, int hist_shift,
+                                                      SelectSmem<SELCAP>& sm) {
+    constexpr int kPer = kCandCap / NT, kBuckets = kHistBins / NT, kCrowd = 32;
+    static_assert(kCandCap % NT == 0 && kBuckets % 4 == 0 && kCandCap <= kBinListCap, "whole keys and buckets per thread");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint64_t k[kPer];
+    int d[kPer], arrival[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        if (u * NT >= c) break;  // uniform
+        if (u * NT + tid >= c) continue;
+        k[u] = keys[u * NT + tid];
+        d[u] = hist_digit(k[u], hist_base, hist_shift);
+        arrival[u] = atomicAdd(&sm.hist[d[u]], 1);
+    }
+    __syncthreads();
+    int4* mine = reinterpret_cast<int4*>(sm.hist) + tid * (kBuckets / 4);
+    int h[kBuckets], sum = 0;
+    bool crowd = false;
+#pragma unroll
+    for (int q = 0; q < kBuckets / 4; ++q) {
+        const int4 v = mine[q];
+        h[4 * q] = v.x; h[4 * q + 1] = v.y; h[4 * q + 2] = v.z; h[4 * q + 3] = v.w;
+    }
+#pragma unroll
+    for (int q = 0; q < kBuckets; ++q) {
+        sum += h[q];
+        crowd |= h[q] > kCrowd;
+    }
+    int incl = sum;  // from the higher buckets down
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_down_sync(kFullMask, incl, o);
+        if (lane + o < 32) incl += v;
+    }
+    if (lane == 0) sm.red_cnt[warp] = incl;
+    if (__syncthreads_or(crowd ? 1 : 0)) return block_select_topk_outlined<NT, SELCAP, 2>(ListKeys{keys}, c, topk, &sm);
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) incl += w > warp ? sm.red_cnt[w] : 0;
+    int start = incl - sum;
+#pragma unroll
+    for (int q = kBuckets - 1; q >= 0; --q) {
+        const int n = h[q];
+        h[q] = start;
+        start += n;
+    }
+#pragma unroll
+    for (int q = 0; q < kBuckets / 4; ++q) mine[q] = make_int4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+    __syncthreads();
+    uint64_t* sorted = sm.binlist;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        if (u * NT >= c) break;
+        if (u * NT + tid >= c) continue;
+        const int first = sm.hist[d[u]];
+        sorted[first + arrival[u]] = k[u];
+        arrival[u] = first;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        if (u * NT >= c) break;
+        if (u * NT + tid >= c || arrival[u] >= topk) continue;
+        const int end = d[u] > 0 ? sm.hist[d[u] - 1] : c;
+        int rank = arrival[u];
+        if (end - rank > 1)
+            for (int q = arrival[u]; q < end; ++q) rank += sorted[q] > k[u] ? 1 : 0;
+        if (rank < topk) sm.sel[rank] = k[u];
+    }
+    return c < topk ? c : topk;
+}
+
 // Same result as block_select_topk_binned for a plain fp32 score array in GLOBAL memory (key = score above thr, index),
 // reading the array once: a spread sample of the scores (one 16-byte chunk per thread) gives a score floor that should
 // leave a few hundred candidates; one pass collects every key at or above the floor into `cand` (kCandCap keys of
@@ -590,6 +666,7 @@ __device__ int block_select_topk_sampled(const float* __restrict__ s, float thr,
         if (incl >= target && incl - mine < target) sm.digit = tid * kCoarse;
     }
     if (tid == 0) sm.bin_cnt = 0;
+    for (int i = tid; i < kHistBins / 4; i += NT) reinterpret_cast<int4*>(sm.hist)[i] = make_int4(0, 0, 0, 0);  // for the selection
     __syncthreads();
     if (n > kCandCap && n4 >= NT && sm.digit > 0) {
         floor_score = __uint_as_float(hist_base + (static_cast<uint32_t>(sm.digit) << hist_shift));
@@ -630,11 +707,12 @@ __device__ int block_select_topk_sampled(const float* __restrict__ s, float thr,
     }
     __syncthreads();
     const int c = sm.bin_cnt;
-    __syncthreads();  // (the selections below reset the counter)
+    if (c == 0 && !floored) return 0;
     if (c > kCandCap || (floored && c < topk)) {
+        __syncthreads();  // (the selection resets the counter)
         return block_select_dense_outlined<NT, SELCAP>(s, head == 0, thr, n, topk, hist_base, hist_shift, &sm);
     }
-    return block_select_topk_binned<NT, SELCAP, 2>(ListKeys{cand}, c, topk, hist_base, hist_shift, sm);
+    return block_select_topk_list<NT, SELCAP>(cand, c, topk, hist_base, hist_shift, sm);
 }
 
 // ---- IoU suppression test ------------------------------------------------------------------------
@@ -695,10 +773,24 @@ __device__ __forceinline__ uint32_t ordered_bits(float v) {
 }
 __device__ __forceinline__ float from_ordered_bits(uint32_t o) { return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o); }
 
-// All 32 * WORDS threads; thread t owns box t (t < n; all boxes tame).  Fills bits[w] with the boxes 32w .. 32w + 31 behind box t
-// that box t might suppress.  Begins with a barrier; the tables are read until the caller's next one.
+// A box's cells in the six tables.  The windows along x and y are as narrow as the threshold makes them: the intersection is no wider
+// than the overlap w of the x ranges and no higher than either box, so IoU <= w / (width of box i), and a box that reaches less than
+// thr * width into box i suppresses nothing (580 -> 230 candidate pairs of 200 boxes on SSD priors).
+struct PairWindow {
+    int x1, x2, y1, y2, area_lo, area_hi;
+    bool real;
+};
+// The boxes 32w .. 32w + 31 behind box t = threadIdx.x that box t might suppress.
 template <int WORDS>
-__device__ __forceinline__ void pair_candidates(const float4 me, float area, int n, float thr, PairCells<WORDS>& pc, uint32_t (&bits)[WORDS]) {
+__device__ __forceinline__ uint32_t pair_word(const PairCells<WORDS>& pc, const PairWindow& m, int w) {
+    const int t = threadIdx.x, lane = t & 31;
+    uint32_t b = pc.t[0][w][m.x2] & pc.t[1][w][m.x1] & pc.t[2][w][m.y2] & pc.t[3][w][m.y1] & pc.t[4][w][m.area_hi] & pc.t[5][w][m.area_lo];
+    if (w == t >> 5) b &= lane == 31 ? 0u : (0xffffffffu << (lane + 1));
+    return m.real && w >= t >> 5 ? b : 0u;
+}
+// All 32 * WORDS threads; thread t owns box t (t < n; all boxes tame).  Fills the tables.
+template <int WORDS>
+__device__ __forceinline__ PairWindow pair_tables(const float4 me, float area, int n, float thr, PairCells<WORDS>& pc) {
     constexpr int NT = 32 * WORDS;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const bool real = t < n && me.z > me.x && me.w > me.y && area > 0.0f;  // others intersect nothing
@@ -760,19 +852,22 @@ __device__ __forceinline__ void pair_candidates(const float4 me, float area, int
     // the area window, a relative 1e-5 wider than the bound so that no rounding of areas or of the quotient matters
     const int a_hi = real ? area_cell(__fdividef(area, thr * (1.0f - 1.0e-5f)) * (1.0f + 1.0e-5f)) : 0;
     const int a_lo = real ? area_cell(area * (thr * (1.0f - 2.0e-5f))) : 0;
-    const int words = (n + 31) >> 5;
-#pragma unroll
-    for (int w = 0; w < WORDS; ++w) {
-        bits[w] = 0u;
-        if (w < warp || w >= words) continue;  // warp-uniform
-        bits[w] = pc.t[0][w][cx2] & pc.t[1][w][cx1] & pc.t[2][w][cy2] & pc.t[3][w][cy1] & pc.t[4][w][a_hi] & pc.t[5][w][a_lo];
-        if (w == warp) bits[w] &= lane == 31 ? 0u : (0xffffffffu << (lane + 1));
-        if (!real) bits[w] = 0u;
+    int qx1 = 0, qx2 = 0, qy1 = 0, qy2 = 0;
+    if (real) {
+        // (a relative 1e-4 of the width and 4e-7 of the coordinates wider: roundings of widths, products, sums and of the quotient)
+        const float reach = thr * (1.0f - 1.0e-4f);
+        const float dx = fmaf(me.z - me.x, reach, -4.0e-7f * fmaxf(fabsf(me.x), fabsf(me.z)));
+        const float dy = fmaf(me.w - me.y, reach, -4.0e-7f * fmaxf(fabsf(me.y), fabsf(me.w)));
+        qx1 = cell(me.x + dx);
+        qx2 = cell(me.z - dx);
+        qy1 = cell(me.y + dy);
+        qy2 = cell(me.w - dy);
     }
+    return {qx1, qx2, qy1, qy2, a_lo, a_hi, real};
 }
 
 // Greedy NMS over up to 256 boxes by a list of the candidate pairs: every thread adds its own, all threads test them in turn
-// (a thread that walks its own candidates waits for the one with the most: 12 300 cycles of 49 500 of an SSD class, of which 580
+// (a thread that walks its own candidates waits for the one with the most: 12 300 cycles of 49 500 of an SSD class, of which 230
 // candidates and 20 real pairs remain), and one warp resolves the few pairs that are left, in rounds without a block barrier.
 // A box is certainly kept once every box that could suppress it is certainly removed, and certainly removed once a certainly kept
 // box suppresses it; both sets only grow, every round settles at least the first undecided box, and the fixed point is the
@@ -785,20 +880,24 @@ struct PairLists {
     uint32_t* words;  // [2 * WORDS]
 };
 template <int WORDS>
-__device__ __forceinline__ bool block_nms_pairs(const float4* sxy, const float* sarea, const uint32_t (&bits)[WORDS], int n, float thr,
-                                                float thr_lo, float thr_hi, const PairLists& pl, uint32_t* keep_words) {
+__device__ __forceinline__ bool block_nms_pairs(const float4* sxy, const float* sarea, const PairCells<WORDS>& pc, const PairWindow& window,
+                                                int n, float thr, float thr_lo, float thr_hi, const PairLists& pl, uint32_t* keep_words) {
     constexpr int NT = 32 * WORDS;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    uint32_t bits[WORDS];
     int mine = 0;
 #pragma unroll
-    for (int w = 0; w < WORDS; ++w) mine += __popc(bits[w]);
+    for (int w = 0; w < WORDS; ++w) {
+        bits[w] = w >= warp && 32 * w < n ? pair_word(pc, window, w) : 0u;
+        mine += __popc(bits[w]);
+    }
     int upto = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int u = __shfl_up_sync(kFullMask, upto, o);
         if (lane >= o) upto += u;
     }
-    int at = 0;
+    int at = 0;  // (an atomic per lane instead of this scan takes turns for every lane: 3000 cycles more)
     if (lane == 31 && upto > 0) at = atomicAdd(pl.count, upto);
     at = __shfl_sync(kFullMask, at, 31) + upto - mine;
 #pragma unroll
@@ -811,12 +910,28 @@ __device__ __forceinline__ bool block_nms_pairs(const float4* sxy, const float* 
     __syncthreads();
     const int pairs = pl.count[0];
     if (pairs > PairLists::kPairs) return false;
-    for (int p = t; p < pairs; p += NT) {
-        const uint32_t e = pl.pairs[p], i = e >> 8, j = e & 255u;
-        const float4 a = sxy[i], b = sxy[j];
-        if (iou_exceeds(NmsBox{a.x, a.y, a.z, a.w, sarea[i]}, NmsBox{b.x, b.y, b.z, b.w, sarea[j]}, thr, thr_lo, thr_hi)) {
-            const int pos = atomicAdd(pl.count + 1, 1);
-            if (pos < PairLists::kHits) pl.hits[pos] = static_cast<uint16_t>(e);
+    constexpr int kAtOnce = 2;
+    for (int p0 = t; p0 < pairs; p0 += kAtOnce * NT) {
+        uint32_t e[kAtOnce];
+        float inter[kAtOnce], uni[kAtOnce];
+#pragma unroll
+        for (int u = 0; u < kAtOnce; ++u) {
+            const int p = p0 + u * NT;
+            e[u] = pl.pairs[p < pairs ? p : 0];
+            const float4 a = sxy[e[u] >> 8], b = sxy[e[u] & 255u];
+            const float w = fmaxf(0.0f, __fsub_rn(fminf(a.z, b.z), fmaxf(a.x, b.x)));
+            const float h = fmaxf(0.0f, __fsub_rn(fminf(a.w, b.w), fmaxf(a.y, b.y)));
+            inter[u] = __fmul_rn(w, h);
+            uni[u] = __fsub_rn(__fadd_rn(sarea[e[u] >> 8], sarea[e[u] & 255u]), inter[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kAtOnce; ++u) {
+            // iou_exceeds for tame boxes: a positive intersection implies its guards
+            if (p0 + u * NT >= pairs || !(inter[u] > 0.0f) || inter[u] < __fmul_rn(uni[u], thr_lo)) continue;
+            if (inter[u] > __fmul_rn(uni[u], thr_hi) || __fdiv_rn(inter[u], uni[u]) > thr) {
+                const int pos = atomicAdd(pl.count + 1, 1);
+                if (pos < PairLists::kHits) pl.hits[pos] = static_cast<uint16_t>(e[u]);
+            }
         }
     }
     __syncthreads();
