@@ -16,16 +16,22 @@
 namespace fb {
 
 constexpr int kSsdTile = 128;     // priors per CTA in group 1
+constexpr int kSsdTileThreads = 2 * kSsdTile;
 constexpr int kSsdMaxRow = 96;    // maximum conf columns (C + 1) supported by the register/smem layout
 
 // dynamic smem: [tile rows * ncol floats][8-byte mbarrier]
-__global__ void __launch_bounds__(kSsdTile)
+// Two threads per row, in two groups of four warps: the first columns and the last ones (fewer: the second group also decodes the box and
+// finishes the sum, which runs in column order whoever adds).  A tile takes 41 KB of shared memory, so that one thread per row left
+// five warps per scheduler.
+__global__ void __launch_bounds__(kSsdTileThreads)
 ssd_softmax_decode_kernel(const float* __restrict__ loc, const float* __restrict__ conf, const float* __restrict__ priors,
                           int num_priors, int num_classes, float clamp_max, float* __restrict__ boxes,
                           float* __restrict__ scores_cm, int use_bulk, int32_t* __restrict__ clear, int num_clear) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ float s_max[2][kSsdTile];
+    __shared__ __align__(16) float s_inv[kSsdTile];  // first the sum over the first columns
     // the words the class kernel of a ragged call counts in (none otherwise): cleared here, so that no memset runs
-    for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * kSsdTile + threadIdx.x; i < num_clear; i += gridDim.x * gridDim.y * kSsdTile)
+    for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * kSsdTileThreads + threadIdx.x; i < num_clear; i += gridDim.x * gridDim.y * kSsdTileThreads)
         clear[i] = 0;
     const int ncol = num_classes + 1;
     float* tile = reinterpret_cast<float*>(smem_raw);
@@ -33,44 +39,70 @@ ssd_softmax_decode_kernel(const float* __restrict__ loc, const float* __restrict
     const int img = blockIdx.y;
     const int p0 = blockIdx.x * kSsdTile;
     const int rows = min(kSsdTile, num_priors - p0);
-    const int t = threadIdx.x;
+    const int r = threadIdx.x % kSsdTile, part = threadIdx.x / kSsdTile;
     const float* gsrc = conf + (static_cast<int64_t>(img) * num_priors + p0) * ncol;
     const int nfl = rows * ncol;
     bool staged = false;
     if (use_bulk) {
-        if (t == 0) {
+        if (threadIdx.x == 0) {
             mbar_init(bar, 1);
             fence_barrier_init();
         }
         __syncthreads();
-        if (t == 0) {
+        if (threadIdx.x == 0) {
             mbar_arrive_expect_tx(bar, static_cast<uint32_t>(nfl) * 4u);
             bulk_copy_g2s(tile, gsrc, static_cast<uint32_t>(nfl) * 4u, bar);
         }
-        staged = mbar_wait_bounded(bar, 0, 200000u);
-        // if the wait ran out (never observed), fall through to the plain loads below after the copy engine
-        // had its chance; staged is uniform enough: every thread polls the same barrier
+        // one warp polls, the others sleep at the barrier; if the wait ran out (never observed), fall through to the plain loads
+        // below after the copy engine had its chance
+        staged = threadIdx.x >= 32 || mbar_wait_bounded(bar, 0, 200000u);
         staged = __syncthreads_and(staged ? 1 : 0) != 0;
     }
     if (!staged) {
-        for (int i = t; i < nfl; i += kSsdTile) tile[i] = __ldg(gsrc + i);
+        for (int i = threadIdx.x; i < nfl; i += kSsdTileThreads) tile[i] = __ldg(gsrc + i);
         __syncthreads();
     }
 
-    const int p = p0 + t;
-    if (t < rows) {
-        float* row = tile + t * ncol;
-        float mx = row[0];
-        for (int c = 1; c < ncol; ++c) mx = fmaxf(mx, row[c]);
-        float sum = 0.0f;
-        for (int c = 0; c < ncol; ++c) {
-            float e = expf(__fsub_rn(row[c], mx));
-            row[c] = e;
-            sum = __fadd_rn(sum, e);
+    const int p = p0 + r;
+    const int split = ncol * 3 / 5, first = part == 0 ? 0 : split, last = part == 0 ? split : ncol;  // this thread's columns
+    constexpr int kAtOnce = 8;  // columns: loads and exponentials side by side
+    const int whole = first + (last - first) / kAtOnce * kAtOnce;
+    const bool live = r < rows;
+    float* row = tile + r * ncol;
+    if (live) {
+        float mx = -INFINITY;  // (a row of nothing but NaN: exp(NaN) below)
+        for (int c = first; c < whole; c += kAtOnce) {
+            float v[kAtOnce];
+#pragma unroll
+            for (int u = 0; u < kAtOnce; ++u) v[u] = row[c + u];
+            mx = fmaxf(mx, fmaxf(fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3])), fmaxf(fmaxf(v[4], v[5]), fmaxf(v[6], v[7]))));
         }
-        const float inv = __fdiv_rn(1.0f, sum);
-        for (int c = 0; c < ncol; ++c) row[c] = __fmul_rn(row[c], inv);
-
+        for (int c = whole; c < last; ++c) mx = fmaxf(mx, row[c]);
+        s_max[part][r] = mx;
+    }
+    __syncthreads();
+    float mx = 0.0f;
+    if (live) {
+        mx = fmaxf(s_max[0][r], s_max[1][r]);
+        float sum = 0.0f;
+        for (int c = first; c < whole; c += kAtOnce) {
+            float e[kAtOnce];
+#pragma unroll
+            for (int u = 0; u < kAtOnce; ++u) e[u] = expf(__fsub_rn(row[c + u], mx));
+#pragma unroll
+            for (int u = 0; u < kAtOnce; ++u) {
+                row[c + u] = e[u];
+                if (part == 0) sum = __fadd_rn(sum, e[u]);
+            }
+        }
+        for (int c = whole; c < last; ++c) {
+            const float e = expf(__fsub_rn(row[c], mx));
+            row[c] = e;
+            if (part == 0) sum = __fadd_rn(sum, e);
+        }
+        if (part == 0) s_inv[r] = sum;
+    }
+    if (live && part == 1) {
         // decode (centre/size priors, variances 0.1 / 0.2), then clamp x to [0, max], y to [0, max]
         const float4 pr = __ldg(reinterpret_cast<const float4*>(priors) + p);
         const float4 d = __ldg(reinterpret_cast<const float4*>(loc) + static_cast<int64_t>(img) * num_priors + p);
@@ -87,11 +119,24 @@ ssd_softmax_decode_kernel(const float* __restrict__ loc, const float* __restrict
         reinterpret_cast<float4*>(boxes)[static_cast<int64_t>(img) * num_priors + p] = o;
     }
     __syncthreads();
+    if (live && part == 1) {
+        float sum = s_inv[r];
+        int c = split;
+        for (; c + 4 <= ncol; c += 4) {
+            const float e0 = row[c], e1 = row[c + 1], e2 = row[c + 2], e3 = row[c + 3];
+            sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, e0), e1), e2), e3);
+        }
+        for (; c < ncol; ++c) sum = __fadd_rn(sum, row[c]);
+        const float inv = __fdiv_rn(1.0f, sum);
+        s_inv[r] = inv;
+    }
+    __syncthreads();
     // class-major store: for a fixed class consecutive threads write consecutive priors
-    if (t < rows) {
-        const float* row = tile + t * ncol;
+    if (live) {
+        const float inv = s_inv[r];
         float* dst = scores_cm + static_cast<int64_t>(img) * num_classes * num_priors + p;
-        for (int c = 0; c < num_classes; ++c) dst[static_cast<int64_t>(c) * num_priors] = row[c];
+#pragma unroll 4
+        for (int c = part; c < num_classes; c += 2) dst[static_cast<int64_t>(c) * num_priors] = __fmul_rn(row[c], inv);
     }
 }
 
@@ -366,7 +411,7 @@ static int launch_ssd_softmax_decode(const float* loc, const float* conf, const 
                                            static_cast<int>(smem)),
                       "ssd_softmax_decode attr"));
     dim3 grid((num_priors + kSsdTile - 1) / kSsdTile, batch);
-    ssd_softmax_decode_kernel<<<grid, kSsdTile, smem, st>>>(loc, conf, priors, num_priors, num_classes, clamp_max, boxes, scores_cm,
+    ssd_softmax_decode_kernel<<<grid, kSsdTileThreads, smem, st>>>(loc, conf, priors, num_priors, num_classes, clamp_max, boxes, scores_cm,
                                                             aligned ? 1 : 0, clear, num_clear);
     count_launch();
     return check_launch("ssd_softmax_decode_kernel");
