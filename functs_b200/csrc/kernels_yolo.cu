@@ -750,6 +750,7 @@ int functs_b200_yolo_detect(const float* map0, const float* map1, const float* m
     p.fallback = f.fallback;
     p.floor = f.floor;
     p.capacity = capacity;
+    p.boxes = boxes;
     p.mask = reinterpret_cast<uint32_t*>(base + S.mask_off);
     p.thr = score_thr;
     p.iou_thr = iou_thr;

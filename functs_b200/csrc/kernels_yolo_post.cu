@@ -26,6 +26,7 @@ constexpr int kPostTop = 1024;     // largest topk
 constexpr int kPostPairs = 8192;
 constexpr int kPostCrowded = 64;   // keys of one score bucket beyond which ranks are not counted
 constexpr int kPostWords = kPostTop / 32;
+constexpr int kPostFewPairs = 512; // pairs that one warp resolves (five block barriers per round otherwise)
 
 struct RescanSlot {
     float so;  // objectness score
@@ -42,6 +43,7 @@ struct PostSmem {
             uint16_t rank[kPostTop];   // position -> place in the sorted top-k
             uint8_t label[kPostTop];
         } box;
+        float rows_out[kPostTop * 5];      // the kept rows on their way out
     };
     union {
         uint64_t sorted[kPostKeys];
@@ -191,27 +193,42 @@ __device__ __forceinline__ void post_select(const uint64_t* __restrict__ keys, i
         __syncthreads();
         return;
     }
-#pragma unroll
-    for (int q = 0; q < kPer; ++q)
-        if (k[q] != 0ull) sm.sorted[atomicAdd(&sm.hist[hist_digit(k[q], base, shift)], 1)] = k[q];
-    __syncthreads();
-    // now hist[d] is where bucket d ends and hist[d + 1] where it starts; a key counts the larger keys of its bucket
+    int start[kPer];
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
-        if (k[q] != 0ull) {
-            const int d = hist_digit(k[q], base, shift);
-            int r = d + 1 < kHistBins ? sm.hist[d + 1] : 0;
-            const int end = sm.hist[d];
-            if (r < topk) {
-                for (int j = r, j1 = end; j < j1; ++j) r += sm.sorted[j] > k[q] ? 1 : 0;
-                if (r < topk) sm.sel[r] = k[q];
-            }
-        }
+        start[q] = topk;
+        if (q * kPostThreads >= n) break;  // uniform
+        if (k[q] == 0ull) continue;
+        const int d = hist_digit(k[q], base, shift);
+        const int at = atomicAdd(&sm.hist[d], 1);
+        sm.sorted[at] = k[q];
+        start[q] = at;
+    }
+    __syncthreads();
+    // now hist[d] is where bucket d ends and hist[d + 1] where it starts; a key counts the larger keys of its bucket
+    int end[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        if (q * kPostThreads >= n) break;
+        end[q] = 0;
+        if (start[q] >= topk + kPostCrowded) continue;  // (a bucket that starts below topk holds no more)
+        const int d = hist_digit(k[q], base, shift);
+        start[q] = d + 1 < kHistBins ? sm.hist[d + 1] : 0;
+        end[q] = sm.hist[d];
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        if (q * kPostThreads >= n) break;
+        if (k[q] == 0ull || start[q] >= topk) continue;
+        int r = start[q];
+        if (end[q] - r > 1)
+            for (int j = start[q]; j < end[q]; ++j) r += sm.sorted[j] > k[q] ? 1 : 0;
+        if (r < topk) sm.sel[r] = k[q];
     }
     __syncthreads();
 }
 
-// Calls pair(i, j) for every pair of positions (this thread's p, a later q) whose boxes overlap by more than the threshold.
+// Calls pair(i, j), i < j places in the top-k, for every pair of boxes that overlap by more than the threshold, once.
 template <class F>
 __device__ __forceinline__ void post_pairs(const PostSmem& sm, int m, int reach, float thr, float thr_lo, float thr_hi, F pair) {
     const int p = threadIdx.x;
@@ -220,34 +237,59 @@ __device__ __forceinline__ void post_pairs(const PostSmem& sm, int m, int reach,
     const NmsBox bi{me.x, me.y, me.z, me.w, sm.box.area[p]};
     const int label = sm.box.label[p], rank = sm.box.rank[p];
     const uint32_t end_x = ordered_bits(me.z), end_y = ordered_bits(me.w);
-    for (int b = label; b <= min(label + reach, kYoloClasses - 1); ++b) {
-        int q = sm.cls_start[b];
+    // four tests at a time without branches: a pair can only exceed the threshold if its intersection reaches union * thr_lo (or a
+    // guard of iou_exceeds may be involved: wild values, which compare as "maybe").  (Only the overlaps in x and in y against the
+    // box's own extent: shorter, but what passes walks through the exact test lane by lane, 5300 cycles instead of 4200.)
+    auto test4 = [&](const int (&at)[4], const bool (&valid)[4]) {
+        bool maybe[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float4 c = sm.box.xy[at[u]];
+            const float w = __fsub_rn(fminf(me.z, c.z), fmaxf(me.x, c.x)), h = __fsub_rn(fminf(me.w, c.w), fmaxf(me.y, c.y));
+            const float inter = __fmul_rn(w, h), uni = __fsub_rn(__fadd_rn(bi.area, sm.box.area[at[u]]), inter);
+            maybe[u] = valid[u] && w > 0.0f && h > 0.0f && !(inter < __fmul_rn(uni, thr_lo));
+        }
+        if (!(maybe[0] || maybe[1] || maybe[2] || maybe[3])) return;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (!maybe[u]) continue;
+            const float4 c = sm.box.xy[at[u]];
+            const NmsBox bj{c.x, c.y, c.z, c.w, sm.box.area[at[u]]};
+            if (iou_exceeds(bi, bj, thr, thr_lo, thr_hi)) {
+                const int other = sm.box.rank[at[u]];
+                pair(min(rank, other), max(rank, other));
+            }
+        }
+    };
+    // the box's own class in a circle, half way round: every box has the same number of partners, and a warp does not wait for the
+    // first box of the largest class
+    {
+        const int s = sm.cls_start[label], n = sm.cls_start[label + 1] - s, i = p - s;
+        const int partners = (n - 1) / 2 + ((n & 1) == 0 && i < n / 2 ? 1 : 0);
+        for (int k = 1; k <= partners; k += 4) {
+            int at[4];
+            bool valid[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                valid[u] = k + u <= partners;
+                const int j = i + (valid[u] ? k + u : k);
+                at[u] = s + (j >= n ? j - n : j);
+            }
+            test4(at, valid);
+        }
+    }
+    for (int b = label + 1; b <= min(label + reach, kYoloClasses - 1); ++b) {
+        if (end_x <= sm.cls_min_x[b] || end_y <= sm.cls_min_y[b]) continue;
         const int q1 = sm.cls_start[b + 1];
-        if (b == label) q = p + 1;
-        else if (end_x <= sm.cls_min_x[b] || end_y <= sm.cls_min_y[b]) continue;
-        // four tests at a time without branches: a pair can only exceed the threshold if its intersection reaches
-        // union * thr_lo (or a guard of iou_exceeds may be involved: wild values, which compare as "maybe")
-        for (; q < q1; q += 4) {
-            bool maybe[4];
+        for (int q = sm.cls_start[b]; q < q1; q += 4) {
+            int at[4];
+            bool valid[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int at = min(q + u, q1 - 1);
-                const float4 c = sm.box.xy[at];
-                const float w = __fsub_rn(fminf(me.z, c.z), fmaxf(me.x, c.x)), h = __fsub_rn(fminf(me.w, c.w), fmaxf(me.y, c.y));
-                const float inter = __fmul_rn(w, h), uni = __fsub_rn(__fadd_rn(bi.area, sm.box.area[at]), inter);
-                maybe[u] = q + u < q1 && w > 0.0f && h > 0.0f && !(inter < __fmul_rn(uni, thr_lo));
+                valid[u] = q + u < q1;
+                at[u] = min(q + u, q1 - 1);
             }
-            if (!(maybe[0] || maybe[1] || maybe[2] || maybe[3])) continue;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (!maybe[u]) continue;
-                const float4 c = sm.box.xy[q + u];
-                const NmsBox bj{c.x, c.y, c.z, c.w, sm.box.area[q + u]};
-                if (iou_exceeds(bi, bj, thr, thr_lo, thr_hi)) {
-                    const int other = sm.box.rank[q + u];
-                    pair(min(rank, other), max(rank, other));
-                }
-            }
+            test4(at, valid);
         }
     }
 }
@@ -276,7 +318,6 @@ __device__ __noinline__ void post_dense(PostSmem* smp, uint32_t* mask, int m, in
     if (warp == 0) sm.words[lane] = gone;
     __syncthreads();
     sm.removed[t] = (sm.words[warp] >> lane) & 1u;
-    sm.kept[t] = t < m && sm.removed[t] == 0;
     __syncthreads();
 }
 
@@ -287,6 +328,7 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     const int img = blockIdx.x;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     sm.removed[t] = 0;
+    sm.blocked[t] = 0;
     if (t < kYoloClasses) {
         sm.cls_cursor[t] = 0;
         sm.cls_min_x[t] = 0xffffffffu;
@@ -310,6 +352,7 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     }
     const int n = static_cast<int>(n64 < 0 ? 0 : (n64 > A.capacity ? A.capacity : n64));
     const uint64_t* keys = A.keys + img * A.capacity;
+    const float4* boxes = A.boxes != nullptr ? reinterpret_cast<const float4*>(A.boxes) + static_cast<int64_t>(img) * L.num_boxes : nullptr;
     if (n <= kPostKeys) post_select(keys, n, A.topk, fmaxf(A.thr, floor), sm);
     else post_select_many(keys, n, A.topk, fmaxf(A.thr, floor), &sm);
     if (t == 0 && (short_list || n > kPostKeys)) A.fallback[img] = 1;
@@ -326,11 +369,15 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
         flat = key_index(key);
         const int box = static_cast<int>(flat / kYoloClasses);
         label = static_cast<int>(flat) - box * kYoloClasses;
-        const int lvl = box >= L.box_begin[2] ? 2 : (box >= L.box_begin[1] ? 1 : 0);
-        const int plane = L.plane[lvl], local = box - L.box_begin[lvl];
-        const int pos = local / 3, anchor = local - pos * 3;
-        const float* src = L.map[lvl] + (static_cast<int64_t>(img) * 3 + anchor) * kYoloAttrib * plane + pos;
-        bx = yolo_box(L, lvl, anchor, pos, __ldg(src), __ldg(src + plane), __ldg(src + 2 * plane), __ldg(src + 3 * plane));
+        if (boxes != nullptr) {
+            bx = __ldcg(boxes + box);
+        } else {
+            const int lvl = box >= L.box_begin[2] ? 2 : (box >= L.box_begin[1] ? 1 : 0);
+            const int plane = L.plane[lvl], local = box - L.box_begin[lvl];
+            const int pos = local / 3, anchor = local - pos * 3;
+            const float* src = L.map[lvl] + (static_cast<int64_t>(img) * 3 + anchor) * kYoloAttrib * plane + pos;
+            bx = yolo_box(L, lvl, anchor, pos, __ldg(src), __ldg(src + plane), __ldg(src + 2 * plane), __ldg(src + 3 * plane));
+        }
         top = fmaxf(top, fmaxf(fmaxf(bx.x, bx.y), fmaxf(bx.z, bx.w)));
         bottom = fminf(bottom, fminf(fminf(bx.x, bx.y), fminf(bx.z, bx.w)));
         atomicAdd(&sm.cls_cursor[label], 1);
@@ -399,7 +446,7 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     const int np = sm.npairs;
     if (np > kPostPairs) {
         post_dense(&sm, A.mask + static_cast<int64_t>(img) * kPostTop * kPostWords, m, reach, A.iou_thr, thr_lo, thr_hi);
-    } else {
+    } else if (np > kPostFewPairs) {
         for (int round = 0; round <= m; ++round) {
             sm.blocked[t] = 0;
             __syncthreads();
@@ -418,10 +465,35 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
             __syncthreads();
             if (__syncthreads_or(t < m && !kept && sm.removed[t] == 0 ? 1 : 0) == 0) break;
         }
+    } else if (np > 0) {  // the same by one warp
+        if (warp == 0) {
+            volatile uint8_t *removed = sm.removed, *blocked = sm.blocked;
+            for (int round = 0; round <= m; ++round) {
+                for (int i = lane; i < np; i += 32) {
+                    const uint32_t pr = sm.pairs[i];
+                    if (removed[pr >> 16] == 0) blocked[pr & 0xffffu] = 1;
+                }
+                __syncwarp();
+                for (int i = lane; i < np; i += 32) {  // (what this loop removes is blocked: it removes nothing)
+                    const uint32_t pr = sm.pairs[i];
+                    if (removed[pr >> 16] == 0 && blocked[pr >> 16] == 0) removed[pr & 0xffffu] = 1;
+                }
+                __syncwarp();
+                bool open = false;
+                for (int i = lane; i < np; i += 32) {
+                    const uint32_t b = sm.pairs[i] & 0xffffu;
+                    open |= blocked[b] != 0 && removed[b] == 0;
+                }
+                if (!__any_sync(kFullMask, open)) break;
+                for (int i = lane; i < np; i += 32) blocked[sm.pairs[i] & 0xffffu] = 0;
+                __syncwarp();
+            }
+        }
+        __syncthreads();
     }
 
     // ---- outputs ----
-    const bool kept = t < m && sm.kept[t] != 0;
+    const bool kept = t < m && sm.removed[t] == 0;
     const unsigned word = __ballot_sync(kFullMask, kept);
     if (lane == 0) sm.warp_sum[warp] = __popc(word);
     __syncthreads();
@@ -431,7 +503,7 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     int4* records = reinterpret_cast<int4*>(A.records);
     if (kept) {
         const int64_t row = obase + before + __popc(word & ((1u << lane) - 1u));
-        float* d = A.dets + row * 5;
+        float* d = sm.rows_out + (row - obase) * 5;  // (stored below, whole lines at a time)
         d[0] = bx.x;
         d[1] = bx.y;
         d[2] = bx.z;
@@ -446,8 +518,6 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     }
     for (int i = total + t; i < A.topk; i += kPostThreads) {  // padded rows are deterministic
         const int64_t row = obase + i;
-        float* d = A.dets + row * 5;
-        d[0] = d[1] = d[2] = d[3] = d[4] = 0.0f;
         A.labels[row] = -1;
         if (A.flat_ids != nullptr) A.flat_ids[row] = -1;
         if (records != nullptr) {
@@ -455,6 +525,8 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
             records[2 * row + 1] = make_int4(0, -1, -1, 0);
         }
     }
+    __syncthreads();
+    for (int i = t; i < 5 * A.topk; i += kPostThreads) A.dets[obase * 5 + i] = i < 5 * total ? sm.rows_out[i] : 0.0f;
     if (A.host_counts != nullptr) __syncthreads();  // a host that watches the count finds the rows complete
     if (t == 0) {
         A.out_counts[img] = total;

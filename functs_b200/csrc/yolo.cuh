@@ -63,6 +63,7 @@ struct YoloPostArgs {
     int32_t* fallback;        // [batch] 1: the image took one of the slow exact paths (observability only)
     const float* floor;       // [batch] every candidate of the image that scores at least this is in `keys` (0: all above thr)
     int64_t capacity;
+    const float* boxes;       // [batch, num_boxes, 4] decoded boxes, or null: from the logits
     uint32_t* mask;           // [batch, 1024, 32] room for the dense suppression matrix (crowded images only)
     float thr, iou_thr;
     int topk;
