@@ -17,6 +17,9 @@ bool lstm_tc_supported(int M, int K, int H);
 bool lstm_rtc_supported(int B, int H);
 int64_t lstm_rtc_scratch_bytes(int H);
 int launch_lstm_recurrent(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, int32_t* status, cudaStream_t st);  // kernels_lstm_rec.cu
+bool lstm_one_launch(int T, int B, int K, int H);
+int launch_lstm_one(const float* x, const float* w_ih, const float* b_ih, const float* b_hh, const float* w_hh, int T, int B, int K, float* hs,
+                    float* cs, int32_t* status, cudaStream_t st);
 int launch_lstm_recurrent_tc(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, void* h_tiles,
                              unsigned int* step_counter, int32_t* status, cudaStream_t st);
 
@@ -119,9 +122,14 @@ int functs_b200_lstm_forward_mode(const float* x, const float* w_ih, const float
     void* tc_scratch = base + 256 + align_up(static_cast<int64_t>(M) * 4 * hidden * 4, 256);
     void* rtc_scratch = static_cast<unsigned char*>(tc_scratch) + align_up(lstm_tc_scratch_bytes(M, input, hidden), 256);
     FB_REQUIRE(mode >= 0 && mode <= 3, "lstm_forward: mode %d unknown", mode);
-    if (mode == 0) mode = kLstmDefaultMode;
-
     record_stage_event(0, st);
+    if (mode == 0 && lstm_one_launch(seq_len, batch, input, hidden)) {
+        record_stage_event(1, st);
+        const int rc = launch_lstm_one(x, w_ih, b_ih, b_hh, w_hh, seq_len, batch, input, hs, cs, status, st);
+        record_stage_event(2, st);
+        return rc;
+    }
+    if (mode == 0) mode = kLstmDefaultMode;
     if (mode != 1 && lstm_tc_supported(M, input, hidden)) {
         FB_TRY(launch_lstm_input_proj_tc(x, w_ih, b_ih, b_hh, M, input, hidden, pre, tc_scratch, status, st));
     } else {

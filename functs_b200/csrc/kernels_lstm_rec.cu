@@ -25,6 +25,7 @@ constexpr int kRecUnitsPerWarp = 8;
 constexpr int kRecSlices = 2;  // k-slices inside a warp
 constexpr int kRecAhead = 2;   // steps that the projection's values are fetched ahead
 constexpr uint32_t kRecWaitLimit = 2000000u;
+constexpr int kOneLaunchRows = 128;  // steps times rows of a cluster up to which it forms its own projection
 
 template <int H, int R>
 struct RecLayout {
@@ -101,19 +102,106 @@ __device__ __forceinline__ uint32_t step_parity(int t) { return static_cast<uint
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
-// R rows per cluster, multiplied in one pass.
-template <int H, int R>
+// The input projection of a cluster's few rows, by the cluster itself (PQ > 0: ceil(K / 128) for H = 256): every CTA forms the columns
+// of its own units for all steps, so that nothing is launched and nothing goes through global memory in front of the first step.
+struct RecInput {
+    const float *x, *w_ih, *b_ih, *b_hh;
+    int K;
+};
+template <int H, int R, int PQ>
+struct ProjLayout {
+    static constexpr int U = H / kRecCluster;
+    static constexpr int Slices = kRecThreads / U;                  // k-slices: a thread takes four columns of a unit and 4 * PQ k
+    static constexpr int Kp = Slices * 4 * PQ;                      // the depth, zeros behind K
+    static constexpr int Rows = 16;                                 // at a time
+    static constexpr size_t x_floats = static_cast<size_t>(Rows) * Kp;
+    static constexpr size_t part_floats = static_cast<size_t>(kRecThreads / 32) * Rows * U * 4;
+    static size_t bytes(int steps) {  // in place of RecLayout's ring
+        return RecLayout<H, R>::bytes + (static_cast<size_t>(steps) * R * U * 4 + x_floats + part_floats - RecLayout<H, R>::pre_floats) * 4;
+    }
+    static_assert(U <= 16 || PQ == 0, "two slices in a warp");
+};
+// pre_all: [T][R][4][U]; x_s: [Rows][Kp]; part: [warps][Rows][U][4].  fp32 sums of 4 * PQ products per thread, 2 * warps of them added.
+template <int H, int R, int PQ>
+__device__ __forceinline__ void rec_project(const RecInput& in, int T, int B, int b0, int j0, float* pre_all, float* x_s, float* part) {
+    using P = ProjLayout<H, R, PQ>;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int unit = tid % P::U, k0 = tid / P::U * (4 * PQ);
+    unsigned long long w[PQ][4][2];
+#pragma unroll
+    for (int q = 0; q < PQ; ++q)
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int k = k0 + 4 * q + i;
+                v[i] = k < in.K ? __ldg(in.w_ih + (static_cast<int64_t>(g) * in.K + k) * H + j0 + unit) : 0.0f;
+            }
+            w[q][g][0] = pack2(v[0], v[1]);
+            w[q][g][1] = pack2(v[2], v[3]);
+        }
+    const int rows = T * R;
+    for (int r0 = 0; r0 < rows; r0 += P::Rows) {
+        const int most = min(P::Rows, rows - r0);
+        for (int e = tid; e < most * P::Kp; e += kRecThreads) {
+            const int i = e / P::Kp, k = e - i * P::Kp, t = (r0 + i) / R, row = b0 + (r0 + i) % R;
+            x_s[e] = k < in.K && row < B ? __ldg(in.x + (static_cast<int64_t>(t) * B + row) * in.K + k) : 0.0f;
+        }
+        __syncthreads();
+#pragma unroll 2
+        for (int i = 0; i < most; ++i) {
+            unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+            for (int q = 0; q < PQ; ++q) {
+                const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(x_s + i * P::Kp + k0 + 4 * q);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) acc[g] = fma2(xv.y, w[q][g][1], fma2(xv.x, w[q][g][0], acc[g]));
+            }
+            float s[4];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                s[g] = sum2(acc[g]);
+                s[g] = __fadd_rn(s[g], __shfl_xor_sync(kFullMask, s[g], 16));
+            }
+            if (lane < 16) reinterpret_cast<float4*>(part)[(warp * P::Rows + i) * P::U + unit] = make_float4(s[0], s[1], s[2], s[3]);
+        }
+        __syncthreads();
+        for (int e = tid; e < most * P::U; e += kRecThreads) {
+            const int i = e / P::U, u = e - i * P::U;
+            float4 s = reinterpret_cast<const float4*>(part)[e];
+#pragma unroll
+            for (int v = 1; v < kRecThreads / 32; ++v) {
+                const float4 m = reinterpret_cast<const float4*>(part)[v * P::Rows * P::U + e];
+                s.x = __fadd_rn(s.x, m.x);
+                s.y = __fadd_rn(s.y, m.y);
+                s.z = __fadd_rn(s.z, m.z);
+                s.w = __fadd_rn(s.w, m.w);
+            }
+            const float sums[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+                pre_all[((r0 + i) * 4 + g) * P::U + u] =
+                    __fadd_rn(sums[g], __fadd_rn(__ldg(in.b_ih + g * H + j0 + u), __ldg(in.b_hh + g * H + j0 + u)));
+        }
+        // (the next rows' barrier stands between these reads of part and its next stores)
+    }
+    __syncthreads();
+}
+
+// R rows per cluster, multiplied in one pass.  PQ: see ProjLayout; 0: the projection is in `pre`.
+template <int H, int R, int PQ>
 __global__ void __launch_bounds__(kRecThreads, 1)
 lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,
-                      float* __restrict__ cs, int32_t* status) {
+                      float* __restrict__ cs, int32_t* status, const RecInput in) {
     using Y = RecLayout<H, R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemQuads][2][kRecThreads]
     float* h_s = reinterpret_cast<float*>(smem_raw + Y::w_bytes);               // [2][16][BP]
     float* part = h_s + Y::h_floats;                                            // [KQ][R][U][4]
-    float* pre_s = part + Y::part_floats;                                       // [step % 3][R][4][U]
-    uint64_t* full = reinterpret_cast<uint64_t*>(pre_s + Y::pre_floats);        // [buffer]
+    uint64_t* full = reinterpret_cast<uint64_t*>(part + Y::part_floats);        // [buffer]
     int* late = reinterpret_cast<int*>(full + 2);                               // a wait ran out
+    float* pre_s = reinterpret_cast<float*>(full + 4);                          // [PQ > 0 ? step : step % 3][R][4][U]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = static_cast<int>(cluster_rank());
     const int b0 = static_cast<int>(blockIdx.x / kRecCluster) * R;
@@ -150,12 +238,17 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
             }
         }
     }
+    if constexpr (PQ > 0) {
+        float* x_s = pre_s + static_cast<size_t>(T) * R * Y::U * 4;
+        rec_project<H, R, PQ>(in, T, B, b0, j0, pre_s, x_s, x_s + ProjLayout<H, R, PQ>::x_floats);
+    }
     // the first warps: one thread per (row, unit) of the CTA applies the gates, keeps the cell state and writes the outputs
     const bool gating = warp < Y::GateWarps, item = tid < Y::Items;
     const int i = item ? tid : 0, iu = i % Y::U, row = b0 + i / Y::U;
     float c_state = 0.0f;
     // 16 bytes a thread: gate (tid % U) / (U / 4), four units
     auto fetch = [&](int t) {
+        if (PQ > 0) return;
         if (item && t < T) {
             const int g = iu / (Y::U / 4), u = iu % (Y::U / 4) * 4;
             const float* p = pre + (static_cast<int64_t>(t) * B + (row < B ? row : 0)) * (4 * H) + g * H + j0 + u;
@@ -173,7 +266,7 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
     const uint32_t h_off = smem_u32(h_s + rank * Y::BP + warp * 32 + quad * 4) - smem_u32(smem_raw);
     const uint32_t bar_off = smem_u32(full) - smem_u32(smem_raw);
     if (gating) {
-        pdl_wait();  // the projection; the weights are not its output
+        if (PQ == 0) pdl_wait();  // the projection; the weights are not its output
 #pragma unroll
         for (int t = 0; t < kRecAhead; ++t) fetch(t);
     }
@@ -228,10 +321,10 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
             asm volatile("barrier.arrive 1, %0;" ::"n"(kRecThreads) : "memory");
             continue;
         }
-        asm volatile("cp.async.wait_group %0;" ::"n"(kRecAhead - 1) : "memory");
+        if (PQ == 0) asm volatile("cp.async.wait_group %0;" ::"n"(kRecAhead - 1) : "memory");
         __syncwarp();
         asm volatile("barrier.sync 1, %0;" ::"n"(kRecThreads) : "memory");
-        const float* pre_t = pre_s + (t % (kRecAhead + 1)) * (Y::Items * 4) + i / Y::U * (4 * Y::U) + iu;
+        const float* pre_t = pre_s + (PQ > 0 ? t : t % (kRecAhead + 1)) * (Y::Items * 4) + i / Y::U * (4 * Y::U) + iu;
         float gate[4];
 #pragma unroll
         for (int g = 0; g < 4; ++g) gate[g] = pre_t[g * Y::U];
@@ -536,9 +629,8 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
     }
 }
 
-template <class Kernel>
-static int launch_rec(Kernel kernel, int threads, size_t smem, int rows, const float* pre, const float* w_hh, int T, int B, float* hs,
-                      float* cs, int32_t* status, cudaStream_t st) {
+template <class... KP, class... A>
+static int launch_rec(void (*kernel)(KP...), int threads, size_t smem, int rows, int B, bool after, cudaStream_t st, A... args) {
     FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "lstm_recurrent attr"));
     FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "lstm_recurrent attr"));
     cudaLaunchConfig_t cfg = {};
@@ -554,28 +646,29 @@ static int launch_rec(Kernel kernel, int threads, size_t smem, int rows, const f
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the weights are fetched while the projection ends
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    FB_TRY(check_cuda(cudaLaunchKernelEx(&cfg, kernel, pre, w_hh, T, B, hs, cs, status), "lstm_recurrent launch"));
+    cfg.numAttrs = after ? 2 : 1;
+    FB_TRY(check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<KP>(args)...), "lstm_recurrent launch"));
     count_launch();
     return FB_OK;
 }
 template <int H, int R>
 static int launch_narrow(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     static_assert(RecLayout<H, R>::bytes <= 227 * 1024, "shared memory of one CTA");
-    return launch_rec(lstm_recurrent_kernel<H, R>, kRecThreads, RecLayout<H, R>::bytes, R, pre, w_hh, T, B, hs, cs, status, st);
+    return launch_rec(lstm_recurrent_kernel<H, R, 0>, kRecThreads, RecLayout<H, R>::bytes, R, B, true, st, pre, w_hh, T, B, hs, cs, status,
+                      RecInput{});
 }
 template <int H, int R>
 static int launch_pair(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     using Y = PairLayout<H, R / 2>;
     static_assert(R % 2 == 0 && Y::bytes <= 227 * 1024, "shared memory of one CTA");
-    return launch_rec(lstm_recurrent_pair_kernel<H, R / 2>, kPairThreads, Y::bytes, R, pre, w_hh, T, B, hs, cs, status, st);
+    return launch_rec(lstm_recurrent_pair_kernel<H, R / 2>, kPairThreads, Y::bytes, R, B, true, st, pre, w_hh, T, B, hs, cs, status);
 }
 
 // Rows per cluster: the fewest that let all clusters run at once (seven clusters of sixteen whole SMs fit a B200; more clusters
 // than that run one after the other).
+constexpr int kClusters = 7;
 template <int H>
 static int launch_rec_rows(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
-    constexpr int kClusters = 7;
     if (B <= kClusters) return launch_narrow<H, 1>(pre, w_hh, T, B, hs, cs, status, st);
     if (B <= 2 * kClusters) return launch_narrow<H, 2>(pre, w_hh, T, B, hs, cs, status, st);
     if (B <= 4 * kClusters) return launch_pair<H, 4>(pre, w_hh, T, B, hs, cs, status, st);
@@ -587,6 +680,31 @@ static int launch_rec_rows(const float* pre, const float* w_hh, int T, int B, fl
 int launch_lstm_recurrent(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     FB_REQUIRE(H == 256 || H == 512, "lstm recurrence: hidden size %d not supported (256 or 512)", H);
     return H == 512 ? launch_rec_rows<512>(pre, w_hh, T, B, hs, cs, status, st) : launch_rec_rows<256>(pre, w_hh, T, B, hs, cs, status, st);
+}
+
+// ---- the whole call in one launch ----
+bool lstm_one_launch(int T, int B, int K, int H) {
+    const int rows = T * (B <= kClusters ? 1 : 2);
+    return H == 256 && B <= 2 * kClusters && K <= 512 && rows <= kOneLaunchRows;
+}
+template <int R, int PQ>
+static int launch_one(const RecInput& in, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
+    return launch_rec(lstm_recurrent_kernel<256, R, PQ>, kRecThreads, ProjLayout<256, R, PQ>::bytes(T), R, B, false, st,
+                      static_cast<const float*>(nullptr), w_hh, T, B, hs, cs, status, in);
+}
+template <int R>
+static int launch_one_depth(const RecInput& in, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
+    switch ((in.K + 127) / 128) {
+        case 1: return launch_one<R, 1>(in, w_hh, T, B, hs, cs, status, st);
+        case 2: return launch_one<R, 2>(in, w_hh, T, B, hs, cs, status, st);
+        case 3: return launch_one<R, 3>(in, w_hh, T, B, hs, cs, status, st);
+        default: return launch_one<R, 4>(in, w_hh, T, B, hs, cs, status, st);
+    }
+}
+int launch_lstm_one(const float* x, const float* w_ih, const float* b_ih, const float* b_hh, const float* w_hh, int T, int B, int K, float* hs,
+                    float* cs, int32_t* status, cudaStream_t st) {
+    const RecInput in{x, w_ih, b_ih, b_hh, K};
+    return B <= kClusters ? launch_one_depth<1>(in, w_hh, T, B, hs, cs, status, st) : launch_one_depth<2>(in, w_hh, T, B, hs, cs, status, st);
 }
 
 }  // namespace fb

@@ -155,9 +155,13 @@ class LSTM:
         self.kernels_last_call = 0
 
     @staticmethod
-    def expected_launches(seq_len: int, batch: int, hidden: int, mode: int = 0) -> int:
+    def expected_launches(seq_len: int, batch: int, hidden: int, mode: int = 0, inputs: int = 0) -> int:
         """Kernel launches of one call: the input projection of all steps and the recurrence; a projection of more 128 x 128
-        tiles than the GPU has SMs splits its operands first (not in mode 1, which does not use the tensor cores for it)."""
+        tiles than the GPU has SMs splits its operands first (not in mode 1, which does not use the tensor cores for it).  Short
+        sequences of few rows and a small cell are one launch (mode 0).  inputs: the depth of x, `hidden` unless given."""
+        rows = seq_len * (1 if batch <= 7 else 2)
+        if mode == 0 and hidden == 256 and batch <= 14 and (inputs or hidden) <= 512 and rows <= 128:
+            return 1
         tiles = -(-seq_len * batch // 128) * (4 * hidden // 128)
         return 3 if mode != 1 and tiles > 148 else 2
 
