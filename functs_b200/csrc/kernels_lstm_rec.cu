@@ -25,7 +25,9 @@ constexpr int kRecUnitsPerWarp = 8;
 constexpr int kRecSlices = 2;  // k-slices inside a warp
 constexpr int kRecAhead = 2;   // steps that the projection's values are fetched ahead
 constexpr uint32_t kRecWaitLimit = 2000000u;
-constexpr int kOneLaunchRows = 128;  // steps times rows of a cluster up to which it forms its own projection
+// Steps and rows up to which a cluster forms its own projection: 0.18 us per row instead of the 12 us of a kernel in front of it.  Two
+// launches / one, us: 25 steps of one row 48 / 42, 32 of two 59 / 56, 64 of one 72 / 73, 64 of two 88 / 94.
+constexpr int kOneLaunchSteps = 56, kOneLaunchRows = 64;
 
 template <int H, int R>
 struct RecLayout {
@@ -119,7 +121,7 @@ struct ProjLayout {
     static size_t bytes(int steps) {  // in place of RecLayout's ring
         return RecLayout<H, R>::bytes + (static_cast<size_t>(steps) * R * U * 4 + x_floats + part_floats - RecLayout<H, R>::pre_floats) * 4;
     }
-    static_assert(U <= 16 || PQ == 0, "two slices in a warp");
+    static_assert((U == 16 && Rows % 2 == 0) || PQ == 0, "two slices in a warp");
 };
 // pre_all: [T][R][4][U]; x_s: [Rows][Kp]; part: [warps][Rows][U][4].  fp32 sums of 4 * PQ products per thread, 2 * warps of them added.
 template <int H, int R, int PQ>
@@ -149,22 +151,27 @@ __device__ __forceinline__ void rec_project(const RecInput& in, int T, int B, in
             x_s[e] = k < in.K && row < B ? __ldg(in.x + (static_cast<int64_t>(t) * B + row) * in.K + k) : 0.0f;
         }
         __syncthreads();
-#pragma unroll 2
-        for (int i = 0; i < most; ++i) {
-            unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+        // two rows at a time: the lower half of a warp ends with the sums of the first one, the upper half with those of the second
+        // (an odd last row takes whatever lies behind it along)
+        const bool up = lane >= 16;
+        for (int i = 0; i < most; i += 2) {
+            unsigned long long acc[2][4] = {};
 #pragma unroll
             for (int q = 0; q < PQ; ++q) {
-                const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(x_s + i * P::Kp + k0 + 4 * q);
 #pragma unroll
-                for (int g = 0; g < 4; ++g) acc[g] = fma2(xv.y, w[q][g][1], fma2(xv.x, w[q][g][0], acc[g]));
+                for (int r = 0; r < 2; ++r) {
+                    const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(x_s + (i + r) * P::Kp + k0 + 4 * q);
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) acc[r][g] = fma2(xv.y, w[q][g][1], fma2(xv.x, w[q][g][0], acc[r][g]));
+                }
             }
             float s[4];
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-                s[g] = sum2(acc[g]);
-                s[g] = __fadd_rn(s[g], __shfl_xor_sync(kFullMask, s[g], 16));
+                const float s0 = sum2(acc[0][g]), s1 = sum2(acc[1][g]);
+                s[g] = __fadd_rn(up ? s1 : s0, __shfl_xor_sync(kFullMask, up ? s0 : s1, 16));
             }
-            if (lane < 16) reinterpret_cast<float4*>(part)[(warp * P::Rows + i) * P::U + unit] = make_float4(s[0], s[1], s[2], s[3]);
+            reinterpret_cast<float4*>(part)[(warp * P::Rows + i + (up ? 1 : 0)) * P::U + unit] = make_float4(s[0], s[1], s[2], s[3]);
         }
         __syncthreads();
         for (int e = tid; e < most * P::U; e += kRecThreads) {
@@ -321,13 +328,20 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
             asm volatile("barrier.arrive 1, %0;" ::"n"(kRecThreads) : "memory");
             continue;
         }
-        if (PQ == 0) asm volatile("cp.async.wait_group %0;" ::"n"(kRecAhead - 1) : "memory");
+        float gate[4];
+        const float* pre_t = pre_s + (PQ > 0 ? t : t % (kRecAhead + 1)) * (Y::Items * 4) + i / Y::U * (4 * Y::U) + iu;
+        if (PQ > 0) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) gate[g] = pre_t[g * Y::U];
+        } else {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kRecAhead - 1) : "memory");
+        }
         __syncwarp();
         asm volatile("barrier.sync 1, %0;" ::"n"(kRecThreads) : "memory");
-        const float* pre_t = pre_s + (PQ > 0 ? t : t % (kRecAhead + 1)) * (Y::Items * 4) + i / Y::U * (4 * Y::U) + iu;
-        float gate[4];
+        if (PQ == 0) {
 #pragma unroll
-        for (int g = 0; g < 4; ++g) gate[g] = pre_t[g * Y::U];
+            for (int g = 0; g < 4; ++g) gate[g] = pre_t[g * Y::U];
+        }
         if (t > 0) {
             const float4* p = reinterpret_cast<const float4*>(part) + i;
             float4 s = p[0];
@@ -685,7 +699,7 @@ int launch_lstm_recurrent(const float* pre, const float* w_hh, int T, int B, int
 // ---- the whole call in one launch ----
 bool lstm_one_launch(int T, int B, int K, int H) {
     const int rows = T * (B <= kClusters ? 1 : 2);
-    return H == 256 && B <= 2 * kClusters && K <= 512 && rows <= kOneLaunchRows;
+    return H == 256 && B <= 2 * kClusters && K <= 512 && T <= kOneLaunchSteps && rows <= kOneLaunchRows;
 }
 template <int R, int PQ>
 static int launch_one(const RecInput& in, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {

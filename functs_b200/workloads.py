@@ -160,7 +160,7 @@ class LSTM:
         tiles than the GPU has SMs splits its operands first (not in mode 1, which does not use the tensor cores for it).  Short
         sequences of few rows and a small cell are one launch (mode 0).  inputs: the depth of x, `hidden` unless given."""
         rows = seq_len * (1 if batch <= 7 else 2)
-        if mode == 0 and hidden == 256 and batch <= 14 and (inputs or hidden) <= 512 and rows <= 128:
+        if mode == 0 and hidden == 256 and batch <= 14 and (inputs or hidden) <= 512 and seq_len <= 56 and rows <= 64:
             return 1
         tiles = -(-seq_len * batch // 128) * (4 * hidden // 128)
         return 3 if mode != 1 and tiles > 148 else 2

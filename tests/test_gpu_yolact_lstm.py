@@ -202,6 +202,26 @@ def test_lstm_inputs_that_are_not_finite(fb, seq, batch, inputs, hidden, mode):
         assert float((got - want)[:, 3:].abs().max()) < 3e-6
 
 
+@pytest.mark.parametrize("seq,batch,inputs,hidden", [
+    (1, 1, 1, 256), (17, 1, 128, 256), (56, 7, 129, 256), (16, 7, 300, 256), (32, 14, 512, 256), (15, 9, 385, 256),  # one launch
+    (57, 1, 256, 256), (33, 14, 100, 256), (9, 1, 256, 512),          # a projection in front of the steps
+    (3, 15, 64, 256), (4, 29, 64, 512), (2, 50, 64, 256), (9, 63, 64, 512),  # halves of two to five rows, some of them empty
+])
+def test_lstm_recurrence_shapes(fb, seq, batch, inputs, hidden):
+    """Every form of the recurrence at its edges against fp64: rows and steps that fill no cluster, half or buffer.  Bound: the gates
+    are sums of K + H products of magnitudes that sum to a few units, so fp32 (or three TF32 products) leaves some 1e-6."""
+    g = torch.Generator().manual_seed(seq * 100 + batch)
+    bound = hidden ** -0.5
+    w = [(torch.rand(*s, generator=g) * 2 - 1) * bound for s in ((4, inputs, hidden), (4, hidden, hidden), (4, 1, hidden), (4, 1, hidden))]
+    x = torch.randn(seq, batch, inputs, generator=g)
+    want = W.LSTMSeq(*[t.double() for t in w])(x.double())
+    mod = fb.workloads.LSTM(*w)
+    got = mod(x)
+    assert mod.kernels_last_call == fb.workloads.LSTM.expected_launches(seq, batch, hidden, 0, inputs)
+    for a, b in zip(got, want):
+        assert float((a.cpu().double() - b).abs().max()) < 3e-6
+
+
 def test_lstm_rejects_unsupported_hidden(fb):
     x, w_ih, w_hh, b_ih, b_hh = W.make_lstm_inputs(2, 2, 64)
     with pytest.raises(fb.FunctsB200Error):
