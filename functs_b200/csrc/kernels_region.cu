@@ -108,9 +108,14 @@ __device__ __forceinline__ bool r_step(const functs_b200_ginstr I, float (&tos)[
 
 // Large form.  grid = (blocks of 256 * V elements of a region, regions), or with INTERLEAVE (blocks) and all regions per CTA.
 // Dynamic shared memory: s_out (INTERLEAVE), then V floats per thread for each load that is fetched ahead (AHEAD): all loads of
-// the CTA are on their way before the first instruction, instead of one instruction's at a time.
-template <int R, bool INTERLEAVE, bool AHEAD>
-__global__ void __launch_bounds__(kRegionThreads) region_group_kernel(const __grid_constant__ functs_b200_rprogram P) {
+// the CTA are on their way before the first instruction, instead of one instruction's at a time.  WINDOW: all loads step through
+// one tensor as the output is stepped through (an element of every pixel, whatever its place in it), so the CTA's share of it is one
+// run, fetched in 16-byte pieces; an element at a time, every line went through the load path once per region and word.
+enum RegionFetch { kEach, kAhead, kWindow };
+template <int R, bool INTERLEAVE, int FETCH>
+__global__ void __launch_bounds__(kRegionThreads) region_group_kernel(const __grid_constant__ functs_b200_rprogram P, int window) {
+    constexpr bool AHEAD = FETCH == kAhead, WINDOW = FETCH == kWindow;
+    static_assert(!WINDOW || (R == 1 && INTERLEAVE), "one run");
     constexpr int V = kRegionVec;
     extern __shared__ __align__(16) float s_region[];
     float* s_out = s_region;
@@ -139,6 +144,17 @@ __global__ void __launch_bounds__(kRegionThreads) region_group_kernel(const __gr
         }
         asm volatile("cp.async.wait_all;" ::: "memory");  // a thread reads only what it has fetched itself
     }
+    if (WINDOW) {
+        const float* p = static_cast<const float*>(P.in_ptr[P.load[0].tensor]) + i0 * P.interleave;
+        const int n = min(kRegionThreads * V * P.interleave, window - i0 * P.interleave);  // window: elements that the loads reach
+        const int n4 = (reinterpret_cast<uintptr_t>(p) & 15) == 0 ? n >> 2 : 0;
+        for (int i = t; i < n4; i += kRegionThreads)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(s_val + 4 * i)), "l"(p + 4 * i) : "memory");
+        for (int i = 4 * n4 + t; i < n; i += kRegionThreads)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(s_val + i)), "l"(p + i) : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+    }
     int slot0 = 0;  // of the region's first load
 #pragma unroll 1
     for (int r = r_begin; r < r_end; ++r) {
@@ -156,6 +172,11 @@ __global__ void __launch_bounds__(kRegionThreads) region_group_kernel(const __gr
                 return;
             }
             const functs_b200_rload& L = P.load[l];
+            if (WINDOW) {
+#pragma unroll
+                for (int v = 0; v < V; ++v) out[v] = s_val[(y[v][0] - i0) * P.interleave + L.base];
+                return;
+            }
             const void* p = P.in_ptr[L.tensor];
 #pragma unroll
             for (int v = 0; v < V; ++v) out[v] = g_fetch(p, L.dtype, r_offset<R>(L.base, L.coef, y[v]));
@@ -310,13 +331,27 @@ extern "C" int functs_b200_region_group_launch(const functs_b200_rprogram* progr
         const bool use_ahead = floats && out_bytes + ahead * kSlot <= 36 * 1024;
         const int smem = out_bytes + (use_ahead ? ahead * kSlot : 0);
         const dim3 grid(blocks, inter ? 1u : static_cast<unsigned>(P.num_regions));
-        auto run = [&](auto kernel_rank1, auto kernel_rank2, auto kernel_rank4) {
-            auto k = rank == 1 ? kernel_rank1 : rank == 2 ? kernel_rank2 : kernel_rank4;
-            k<<<grid, kRegionThreads, smem, st>>>(P);
+        // one run: rank 1, one tensor, every load at a place below the step (normalisation of 800 x 1333: 8.5 us, 10.3 with every load
+        // fetched ahead for itself; 1080 x 1440 10.3 / 12.3; 1440 x 1920, which DRAM bounds, 16.5 / 16.5)
+        int window = 0;
+        if (use_ahead && rank == 1) {
+            int last = 0;
+            bool one = P.num_loads > 0;
+            for (int l = 0; l < P.num_loads; ++l) {
+                const functs_b200_rload& L = P.load[l];
+                one = one && L.tensor == P.load[0].tensor && L.coef[0] == P.interleave && L.base >= 0 && L.base < P.interleave;
+                last = std::max(last, L.base);
+            }
+            if (one) window = P.interleave * (most - 1) + last + 1;
+        }
+        auto run = [&](auto k) { k<<<grid, kRegionThreads, window > 0 ? 2 * out_bytes : smem, st>>>(P, window); };
+        auto by_rank = [&](auto kernel_rank1, auto kernel_rank2, auto kernel_rank4) {
+            run(rank == 1 ? kernel_rank1 : rank == 2 ? kernel_rank2 : kernel_rank4);
         };
-        if (use_ahead) run(region_group_kernel<1, true, true>, region_group_kernel<2, true, true>, region_group_kernel<4, true, true>);
-        else if (inter) run(region_group_kernel<1, true, false>, region_group_kernel<2, true, false>, region_group_kernel<4, true, false>);
-        else run(region_group_kernel<1, false, false>, region_group_kernel<2, false, false>, region_group_kernel<4, false, false>);
+        if (window > 0) run(region_group_kernel<1, true, kWindow>);
+        else if (use_ahead) by_rank(region_group_kernel<1, true, kAhead>, region_group_kernel<2, true, kAhead>, region_group_kernel<4, true, kAhead>);
+        else if (inter) by_rank(region_group_kernel<1, true, kEach>, region_group_kernel<2, true, kEach>, region_group_kernel<4, true, kEach>);
+        else by_rank(region_group_kernel<1, false, kEach>, region_group_kernel<2, false, kEach>, region_group_kernel<4, false, kEach>);
     }
     count_launch();
     return check_launch("region_group_kernel");

@@ -233,6 +233,38 @@ def test_programs_cut_into_regions(env, fn, shape):
     check(env, fn, args)
 
 
+def first_of_three(x: torch.Tensor):
+    t = torch.zeros_like(x) + 1.0
+    t[:, 0] = x[:, 1] * 2.0
+    t[:, 1] = x[:, 0] + x[:, 1]
+    t[:, 2] = x[:, 0] - 1.0
+    return t
+
+
+def swapped(x: torch.Tensor):
+    t = x.clone()
+    t[:, 0] = x[:, 2] - 1.0
+    t[:, 2] = x[:, 0] * 3.0
+    return t
+
+
+@pytest.mark.parametrize("rows", [606208, 606209, 607231, 700001])
+@pytest.mark.parametrize("view", ["whole", "unaligned", "last element of the storage"])
+@pytest.mark.parametrize("fn", [swapped, first_of_three])
+def test_interleaved_regions_of_one_tensor(env, fn, rows, view):
+    """Loads that step through one tensor as the output is stepped through are fetched as one run: whole and ragged blocks, a tensor
+    off a 16-byte boundary, and one whose last word is the last that the loads reach."""
+    g = torch.Generator().manual_seed(16)
+    size = rows * 3
+    if view == "whole":
+        x = torch.randn(rows, 3, generator=g).cuda()
+    elif view == "unaligned":
+        x = torch.randn(size + 1, generator=g).cuda()[1:].view(rows, 3)
+    else:
+        x = torch.randn(size + 2, generator=g).cuda()[2:].view(rows, 3)
+    check(env, fn, (x,))
+
+
 def bounds(x: torch.Tensor, y: torch.Tensor):
     t = x.clone()
     t[:, 0] = torch.relu(t[:, 0])
