@@ -354,7 +354,7 @@ __device__ __noinline__ void yolo_collect_all(const YoloDecodeArgs* A, int lvl, 
 // holds no live slot), so what the list saves is instructions: forms in which every lane kept four neighbouring slots, dead
 // ones included, executed 17 to 22 million warp instructions for 64 images and took 42 to 53 us whatever the loads looked
 // like (registers, ten planes at a time; asynchronous copies, fifteen at a time, next tile prefetched).
-// E = 4 fills the lanes (70 live slots in 512); E = 1 makes more CTAs where there are few tiles.
+// E = 2 to 4 fill the lanes (35 to 70 live slots); E = 1 makes more CTAs where there are few tiles (launch_yolo_decode).
 // ALL: no floor, every candidate above the threshold is wanted (yolo_collect_all from the start, with a longer queue; in the other
 // form that queue would take the L1 cache its loads need: 64 images 76.0 us instead of 71.2).
 template <int E, bool BOXES, bool ALL>
@@ -630,16 +630,25 @@ static int launch_yolo_decode(const YoloDecodeArgs& a, int batch, bool pdl, cuda
         return launch_after(kernel, dim3(static_cast<unsigned>(tiles(kDecThreads))), dim3(kDecThreads), smem, st, pdl,
                             "yolo_decode_dense_kernel", a);
     }
-    // large tiles once they make four CTAs per SM
-    const int large = tiles(4 * kDecThreads);
     auto run = [&](auto kernel, int n) {
         return launch_after(kernel, dim3(static_cast<unsigned>(n)), dim3(kDecThreads), 0, st, pdl, "yolo_decode_kernel", a);
     };
-    const bool is_large = large >= 4 * kNumSMs;
-    const int n = is_large ? large : tiles(kDecThreads);
-    if (a.floor == nullptr) return is_large ? run(yolo_decode_kernel<4, true, true>, n) : run(yolo_decode_kernel<1, true, true>, n);
-    if (a.boxes != nullptr) return is_large ? run(yolo_decode_kernel<4, true, false>, n) : run(yolo_decode_kernel<1, true, false>, n);
-    return is_large ? run(yolo_decode_kernel<4, false, false>, n) : run(yolo_decode_kernel<1, false, false>, n);
+    if (a.floor == nullptr || a.boxes != nullptr) {  // large tiles once they make four CTAs per SM
+        const int large = tiles(4 * kDecThreads);
+        const bool is_large = large >= 4 * kNumSMs;
+        const int n = is_large ? large : tiles(kDecThreads);
+        if (a.floor == nullptr) return is_large ? run(yolo_decode_kernel<4, true, true>, n) : run(yolo_decode_kernel<1, true, true>, n);
+        return is_large ? run(yolo_decode_kernel<4, true, false>, n) : run(yolo_decode_kernel<1, true, false>, n);
+    }
+    // The smallest tiles that all run at once (eight CTAs per SM): small ones end together, and a few that are left for a second wave
+    // wait for the first.  Beyond that, two slots per thread.  Whole call, us, with one / two / three / four slots: 12 images of
+    // 416 x 416 25 / 25 / - / 25, 24 33 / 31.5 / - / 33, 32 42 / 42 / 41 / 43, 64 63.5 / 65 / 67 / 70, 64 with few live boxes
+    // 46.5 / 43 / 43 / 43; 8 of 608 x 608 27 / 25 / 27 / 27, 30 62 / 62 / 65 / 67.
+    constexpr int kWave = 8 * kNumSMs;
+    const int one = tiles(kDecThreads), two = tiles(2 * kDecThreads), three = tiles(3 * kDecThreads);
+    if (one <= kWave) return run(yolo_decode_kernel<1, false, false>, one);
+    if (two > kWave && three <= kWave) return run(yolo_decode_kernel<3, false, false>, three);
+    return run(yolo_decode_kernel<2, false, false>, two);
 }
 
 static inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
