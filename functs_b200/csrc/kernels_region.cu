@@ -113,7 +113,7 @@ __device__ __forceinline__ bool r_step(const functs_b200_ginstr I, float (&tos)[
 // run, fetched in 16-byte pieces; an element at a time, every line went through the load path once per region and word.
 enum RegionFetch { kEach, kAhead, kWindow };
 template <int R, bool INTERLEAVE, int FETCH>
-__global__ void __launch_bounds__(kRegionThreads) region_group_kernel(const __grid_constant__ functs_b200_rprogram P, int window) {
+__global__ void __launch_bounds__(kRegionThreads) region_group_kernel(const __grid_constant__ functs_b200_rprogram P) {
     constexpr bool AHEAD = FETCH == kAhead, WINDOW = FETCH == kWindow;
     static_assert(!WINDOW || (R == 1 && INTERLEAVE), "one run");
     constexpr int V = kRegionVec;
@@ -146,7 +146,12 @@ __global__ void __launch_bounds__(kRegionThreads) region_group_kernel(const __gr
     }
     if (WINDOW) {
         const float* p = static_cast<const float*>(P.in_ptr[P.load[0].tensor]) + i0 * P.interleave;
-        const int n = min(kRegionThreads * V * P.interleave, window - i0 * P.interleave);  // window: elements that the loads reach
+        int n = kRegionThreads * V * P.interleave;
+        if (i0 + kRegionThreads * V >= P.region[0].count) {  // the last CTA: no further than the loads reach
+            int last = 0;
+            for (int l = 0; l < P.num_loads; ++l) last = max(last, P.load[l].base);
+            n = P.interleave * (P.region[0].count - 1 - i0) + last + 1;
+        }
         const int n4 = (reinterpret_cast<uintptr_t>(p) & 15) == 0 ? n >> 2 : 0;
         for (int i = t; i < n4; i += kRegionThreads)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(s_val + 4 * i)), "l"(p + 4 * i) : "memory");
@@ -333,22 +338,16 @@ extern "C" int functs_b200_region_group_launch(const functs_b200_rprogram* progr
         const dim3 grid(blocks, inter ? 1u : static_cast<unsigned>(P.num_regions));
         // one run: rank 1, one tensor, every load at a place below the step (normalisation of 800 x 1333: 8.5 us, 10.3 with every load
         // fetched ahead for itself; 1080 x 1440 10.3 / 12.3; 1440 x 1920, which DRAM bounds, 16.5 / 16.5)
-        int window = 0;
-        if (use_ahead && rank == 1) {
-            int last = 0;
-            bool one = P.num_loads > 0;
-            for (int l = 0; l < P.num_loads; ++l) {
-                const functs_b200_rload& L = P.load[l];
-                one = one && L.tensor == P.load[0].tensor && L.coef[0] == P.interleave && L.base >= 0 && L.base < P.interleave;
-                last = std::max(last, L.base);
-            }
-            if (one) window = P.interleave * (most - 1) + last + 1;
+        bool window = use_ahead && rank == 1 && P.num_loads > 0;
+        for (int l = 0; window && l < P.num_loads; ++l) {
+            const functs_b200_rload& L = P.load[l];
+            window = L.tensor == P.load[0].tensor && L.coef[0] == P.interleave && L.base >= 0 && L.base < P.interleave;
         }
-        auto run = [&](auto k) { k<<<grid, kRegionThreads, window > 0 ? 2 * out_bytes : smem, st>>>(P, window); };
+        auto run = [&](auto k) { k<<<grid, kRegionThreads, window ? 2 * out_bytes : smem, st>>>(P); };
         auto by_rank = [&](auto kernel_rank1, auto kernel_rank2, auto kernel_rank4) {
             run(rank == 1 ? kernel_rank1 : rank == 2 ? kernel_rank2 : kernel_rank4);
         };
-        if (window > 0) run(region_group_kernel<1, true, kWindow>);
+        if (window) run(region_group_kernel<1, true, kWindow>);
         else if (use_ahead) by_rank(region_group_kernel<1, true, kAhead>, region_group_kernel<2, true, kAhead>, region_group_kernel<4, true, kAhead>);
         else if (inter) by_rank(region_group_kernel<1, true, kEach>, region_group_kernel<2, true, kEach>, region_group_kernel<4, true, kEach>);
         else by_rank(region_group_kernel<1, false, kEach>, region_group_kernel<2, false, kEach>, region_group_kernel<4, false, kEach>);
