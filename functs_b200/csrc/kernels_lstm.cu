@@ -1,4 +1,5 @@
-// C4: imperative LSTM (functs/benchmark/ai_model/lstm/lstm.py:79-98, 118-133) in two launches.
+// C4: imperative LSTM (functs/benchmark/ai_model/lstm/lstm.py:79-98, 118-133) in two launches, or in one where a cluster of
+// the recurrence has few rows (lstm_one_launch).
 //
 //   launch 1  input projection, hoisted out of the time loop because it does not depend on h:
 //             pre[t*B + b, g*H + j] = x[t, b, :] @ w_ih[g, :, j] + b_ih[g, j] + b_hh[g, j]

@@ -1,18 +1,18 @@
 // C4, the recurrence: one thread-block cluster of 16 CTAs owns a few batch rows and runs all time steps on its own.
 //
-// The rows of a batch are independent, so nothing but the 16 CTAs that share a row's hidden state has to meet between steps: a
-// cluster barrier and stores into each other's shared memory replace a device-wide counter and a round trip of h through
-// global memory.  (One bulk copy per receiver with completion on its mbarrier instead of the stores and the barrier: 1.6 us per
-// step against 1.26 at one row of H = 256, the same at ten.)  Every cluster holds all of w_hh: a CTA owns H / 16 hidden units,
+// The rows of a batch are independent, so nothing but the 16 CTAs that share a row's hidden state has to meet between steps.  h goes
+// into the others' shared memory by st.async, 16 bytes and their count on the receiver's mbarrier in one store: 0.7 us per step
+// at one row of H = 256 (plain remote stores, a fence and a cluster barrier 1.2; one bulk copy per receiver 1.6).  Every cluster holds all of w_hh: a CTA owns H / 16 hidden units,
 // four gate columns each, 64 KB (H = 256) or 256 KB (H = 512) of weights, in registers as far as they go (32 or 64 per thread),
 // the rest in shared memory.
-// What bounds it at 64 rows: seven clusters fit the chip, ten rows each; of 5.6 us per step 2.6 are fp32 multiply-adds at 128 per
-// cycle and SM, the reduction, the gates and the exchange follow one after the other (a third of the issue slots used); at one row the latency of a step: read the weights in shared memory, reduce, exchange.
+// What bounds it at 64 rows: seven clusters fit the chip, ten rows each; of 4.2 us per step (5.6 before the two halves took turns) 2.6
+// are fp32 multiply-adds at 128 per cycle and SM, the rest is what their operands' loads and the gates take of the same issue slots;
+// at one row the latency of a step: multiply 300 cycles, sum 240, gates 290, send and arrive 450.
 //
 // Thread layout: a thread multiplies two gate columns of one unit with KT consecutive k of every row, two k per packed instruction
 // (fma.rn.f32x2: one issue slot for two multiply-adds); a warp is 8 units x 2 gate pairs x 2 k-slices, the two slices are
 // summed by a shuffle that leaves one gate per lane, the warps' sums meet in shared memory, and one thread per (row, unit)
-// applies the gates, assigns hs[t] / cs[t] and stores h into the sixteen CTAs' next buffer.  (Four gate columns and half the k
+// applies the gates, assigns hs[t] / cs[t] and sends h into the sixteen CTAs' next buffer.  (Four gate columns and half the k
 // per thread needs two passes over the rows, and the weights in shared memory are then read twice: 6.5 us per step at ten
 // rows of H = 512.  A register spill here goes to L2, shared memory being full: 14 us.)
 #include "common.cuh"

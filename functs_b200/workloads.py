@@ -139,7 +139,7 @@ class SSDBBox:
 
 
 class LSTM:
-    """One-layer LSTM with per-step outputs written by slice assignment (hs[t] = h, cs[t] = c).  2 or 3 launches."""
+    """One-layer LSTM with per-step outputs written by slice assignment (hs[t] = h, cs[t] = c).  1 to 3 launches."""
 
     def __init__(self, w_ih: torch.Tensor, w_hh: torch.Tensor, b_ih: torch.Tensor, b_hh: torch.Tensor, device="cuda"):
         self.device = _dev(device)
