@@ -13,11 +13,10 @@
 #include <algorithm>
 
 #include "generic.cuh"
+#include "region_plan.h"
 
 namespace fb {
 
-constexpr int kRegionThreads = 256;
-constexpr int kRegionVec = 4;          // elements per thread and pass in the large form
 constexpr int kRegionSmall = 128;      // threads of the small form
 constexpr int kRegionMaxInterleave = 8;
 
@@ -111,7 +110,6 @@ __device__ __forceinline__ bool r_step(const functs_b200_ginstr I, float (&tos)[
 // the CTA are on their way before the first instruction, instead of one instruction's at a time.  WINDOW: all loads step through
 // one tensor as the output is stepped through (an element of every pixel, whatever its place in it), so the CTA's share of it is one
 // run, fetched in 16-byte pieces; an element at a time, every line went through the load path once per region and word.
-enum RegionFetch { kEach, kAhead, kWindow };
 template <int R, bool INTERLEAVE, int FETCH>
 __global__ void __launch_bounds__(kRegionThreads) region_group_kernel(const __grid_constant__ functs_b200_rprogram P) {
     constexpr bool AHEAD = FETCH == kAhead, WINDOW = FETCH == kWindow;
@@ -150,7 +148,7 @@ __global__ void __launch_bounds__(kRegionThreads) region_group_kernel(const __gr
         if (i0 + kRegionThreads * V >= P.region[0].count) {  // the last CTA: no further than the loads reach
             int last = 0;
             for (int l = 0; l < P.num_loads; ++l) last = max(last, P.load[l].base);
-            n = P.interleave * (P.region[0].count - 1 - i0) + last + 1;
+            n = region_run_words(P.interleave, P.region[0].count - i0, last);
         }
         const int n4 = (reinterpret_cast<uintptr_t>(p) & 15) == 0 ? n >> 2 : 0;
         for (int i = t; i < n4; i += kRegionThreads)
@@ -325,30 +323,14 @@ extern "C" int functs_b200_region_group_launch(const functs_b200_rprogram* progr
         region_group_kernel_small<<<grid, kRegionSmall, 0, st>>>(P);
     } else {
         const unsigned blocks = static_cast<unsigned>((most + kRegionThreads * kRegionVec - 1) / (kRegionThreads * kRegionVec));
-        // Fetched ahead: float loads of interleaved regions, as many as leave six CTAs on an SM (normalisation of 1440 x 1920: 20.6 us
-        // without, 18.5 with; one region per CTA gains nothing, 2500 boxes of 80 classes 16.5 us without, 19.3 with).
-        int ahead = 0;
-        bool floats = inter;
-        for (int l = 0; l < P.num_loads; ++l) floats = floats && P.load[l].dtype == 0;
-        for (int r = 0; r < P.num_regions; ++r) ahead += P.region[r].num_loads;
-        constexpr int kSlot = kRegionThreads * kRegionVec * 4;
-        const int out_bytes = inter ? P.interleave * kSlot : 0;
-        const bool use_ahead = floats && out_bytes + ahead * kSlot <= 36 * 1024;
-        const int smem = out_bytes + (use_ahead ? ahead * kSlot : 0);
+        const RegionPlan plan = region_plan(P, rank, inter);
         const dim3 grid(blocks, inter ? 1u : static_cast<unsigned>(P.num_regions));
-        // one run: rank 1, one tensor, every load at a place below the step (normalisation of 800 x 1333: 8.5 us, 10.3 with every load
-        // fetched ahead for itself; 1080 x 1440 10.3 / 12.3; 1440 x 1920, which DRAM bounds, 16.5 / 16.5)
-        bool window = use_ahead && rank == 1 && P.num_loads > 0;
-        for (int l = 0; window && l < P.num_loads; ++l) {
-            const functs_b200_rload& L = P.load[l];
-            window = L.tensor == P.load[0].tensor && L.coef[0] == P.interleave && L.base >= 0 && L.base < P.interleave;
-        }
-        auto run = [&](auto k) { k<<<grid, kRegionThreads, window ? 2 * out_bytes : smem, st>>>(P); };
+        auto run = [&](auto k) { k<<<grid, kRegionThreads, plan.shared, st>>>(P); };
         auto by_rank = [&](auto kernel_rank1, auto kernel_rank2, auto kernel_rank4) {
             run(rank == 1 ? kernel_rank1 : rank == 2 ? kernel_rank2 : kernel_rank4);
         };
-        if (window) run(region_group_kernel<1, true, kWindow>);
-        else if (use_ahead) by_rank(region_group_kernel<1, true, kAhead>, region_group_kernel<2, true, kAhead>, region_group_kernel<4, true, kAhead>);
+        if (plan.fetch == kWindow) run(region_group_kernel<1, true, kWindow>);
+        else if (plan.fetch == kAhead) by_rank(region_group_kernel<1, true, kAhead>, region_group_kernel<2, true, kAhead>, region_group_kernel<4, true, kAhead>);
         else if (inter) by_rank(region_group_kernel<1, true, kEach>, region_group_kernel<2, true, kEach>, region_group_kernel<4, true, kEach>);
         else by_rank(region_group_kernel<1, false, kEach>, region_group_kernel<2, false, kEach>, region_group_kernel<4, false, kEach>);
     }

@@ -6,6 +6,8 @@ from typing import List
 import pytest
 import torch
 
+from region_program import address, interleaved
+
 pytestmark = pytest.mark.gpu
 
 
@@ -249,20 +251,29 @@ def swapped(x: torch.Tensor):
 
 
 @pytest.mark.parametrize("rows", [606208, 606209, 607231, 700001])
-@pytest.mark.parametrize("view", ["whole", "unaligned", "last element of the storage"])
+@pytest.mark.parametrize("off", [0, 1, 2])
 @pytest.mark.parametrize("fn", [swapped, first_of_three])
-def test_interleaved_regions_of_one_tensor(env, fn, rows, view):
-    """Loads that step through one tensor as the output is stepped through are fetched as one run: whole and ragged blocks, a tensor
-    off a 16-byte boundary, and one whose last word is the last that the loads reach."""
+def test_interleaved_regions_of_one_tensor(env, fn, rows, off):
+    """Loads that step through one tensor as the output is stepped through are fetched as one run: whole and ragged blocks, and
+    tensors off a 16-byte boundary.  (Where a run ends: test_region_plan.)"""
     g = torch.Generator().manual_seed(16)
-    size = rows * 3
-    if view == "whole":
-        x = torch.randn(rows, 3, generator=g).cuda()
-    elif view == "unaligned":
-        x = torch.randn(size + 1, generator=g).cuda()[1:].view(rows, 3)
-    else:
-        x = torch.randn(size + 2, generator=g).cuda()[2:].view(rows, 3)
-    check(env, fn, (x,))
+    check(env, fn, (torch.randn(rows * 3 + off, generator=g).cuda()[off:].view(rows, 3),))
+
+
+@pytest.mark.parametrize("width,bases", [(2, [1]), (2, [0, 0]), (4, [2, 0]), (5, [4, 0, 1]), (6, [3]), (7, [6]), (7, [0, 5]), (8, [7]),
+                                         (8, [1, 2, 3])])
+@pytest.mark.parametrize("rows,off", [(606208, 0), (607231, 1)])
+def test_interleaved_regions_of_constants_and_loads(env, width, bases, rows, off):
+    """Programs as a native caller passes them: two to eight interleaved regions, few of which load, as one run or load by load."""
+    from functs_b200 import _lib
+    g = torch.Generator().manual_seed(17)
+    x = torch.randn(rows * width + off, generator=g).cuda()[off:].view(rows, width)
+    out = torch.full((rows, width), float("nan"), device="cuda")
+    p = interleaved(width, rows, bases, x.data_ptr(), out.data_ptr())
+    _lib.check(_lib.lib.functs_b200_region_group_launch(address(p), torch.cuda.current_stream().cuda_stream))
+    want = torch.arange(width, dtype=torch.float32, device="cuda").repeat(rows, 1)
+    want[:, :len(bases)] = 2.0 * x[:, bases]
+    assert torch.equal(out, want)
 
 
 def bounds(x: torch.Tensor, y: torch.Tensor):
