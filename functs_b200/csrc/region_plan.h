@@ -43,7 +43,9 @@ inline RegionPlan region_plan(const functs_b200_rprogram& P, int rank, bool inte
     bool window = rank == 1 && ahead > 0 && 2 * out_bytes <= kRegionSharedMost;
     for (int l = 0; window && l < P.num_loads; ++l) {
         const functs_b200_rload& L = P.load[l];
-        window = L.tensor == P.load[0].tensor && L.coef[0] == P.interleave && L.base >= 0 && L.base < P.interleave;
+        bool used = false;  // (the run reaches no further than a load that is made)
+        for (int r = 0; r < P.num_regions; ++r) used = used || (l >= P.region[r].first_load && l < P.region[r].first_load + P.region[r].num_loads);
+        window = used && L.tensor == P.load[0].tensor && L.coef[0] == P.interleave && L.base >= 0 && L.base < P.interleave;
     }
     return window ? RegionPlan{kWindow, 2 * out_bytes} : RegionPlan{kAhead, out_bytes + ahead * kSlot};
 }

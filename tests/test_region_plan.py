@@ -5,7 +5,7 @@ import subprocess
 
 import pytest
 
-from region_program import Program, address, interleaved
+from region_program import Load, Program, address, interleaved
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "functs_b200", "csrc")
 EACH, AHEAD, WINDOW = 0, 1, 2
@@ -65,6 +65,14 @@ def test_what_one_run_cannot_serve(rule):
     assert changed(lambda p: setattr(p.load[2], "dtype", 1)) == EACH
     p = interleaved(3, 606208, [2, 1, 0], 1 << 20, 1 << 28)
     assert rule(p, rank=2)[0] == AHEAD and rule(p, inter=False) == (EACH, 0)
+
+
+def test_a_load_that_no_region_makes_does_not_stretch_the_run(rule):
+    p = interleaved(4, 606208, [0, 1], 1 << 20, 1 << 28)
+    assert rule(p)[0] == WINDOW
+    p.load[p.num_loads] = Load(0, 0, 3, (ctypes.c_int32 * 4)(4))
+    p.num_loads += 1
+    assert rule(p)[0] == AHEAD
 
 
 def test_a_run_ends_with_the_last_word_that_is_loaded(rule):
