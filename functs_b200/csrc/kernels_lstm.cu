@@ -90,6 +90,7 @@ constexpr int kLstmDefaultMode = 3;
 
 namespace fb {
 void yolo_set_prune(int on);
+void lstm_set_drop_exchange(int on);
 }
 
 extern "C" {
@@ -155,6 +156,10 @@ int functs_b200_lstm_forward_mode(const float* x, const float* w_ih, const float
 int functs_b200_debug_set(const char* name, int32_t value) {
     if (name != nullptr && std::strcmp(name, "yolo_prune") == 0) {
         fb::yolo_set_prune(value);
+        return FB_OK;
+    }
+    if (name != nullptr && std::strcmp(name, "lstm_drop_exchange") == 0) {
+        fb::lstm_set_drop_exchange(value);
         return FB_OK;
     }
     fb::set_error("debug_set: unknown switch");

@@ -24,7 +24,10 @@ constexpr int kRecThreads = 512;
 constexpr int kRecUnitsPerWarp = 8;
 constexpr int kRecSlices = 2;  // k-slices inside a warp
 constexpr int kRecAhead = 2;   // steps that the projection's values are fetched ahead
-constexpr uint32_t kRecWaitLimit = 2000000u;
+constexpr uint32_t kRecWaitLimit = 250000u;  // about a second: a poll that fails takes 7800 cycles
+// Development switch (functs_b200_debug_set "lstm_drop_exchange"): in this thread's calls no CTA sends h, so that every wait runs out.
+static thread_local int t_rec_drop = 0;
+void lstm_set_drop_exchange(int on) { t_rec_drop = on ? 1 : 0; }
 // Steps and rows up to which a cluster forms its own projection: 0.18 us per row instead of the 12 us of a kernel in front of it.  Two
 // launches / one, us: 25 steps of one row 48 / 42, 32 of two 59 / 56, 64 of one 72 / 73, 64 of two 88 / 94.
 constexpr int kOneLaunchSteps = 56, kOneLaunchRows = 64;
@@ -83,6 +86,14 @@ __device__ __forceinline__ void store_async4(uint32_t remote, float a, float b, 
                  : "memory");
 }
 // Wait for what other CTAs of the cluster store; false when the limit runs out.
+//
+// What follows then, in both kernels.  The warp multiplies no more and goes through the named barriers of the steps that are left, in
+// step with the gate warps: barrier.arrive would let it run ahead, and a barrier that a warp meets twice in one phase loses count,
+// so that the gate warps wait for ever.  (The barrier of the step before is over by then: the other warps of its CTA have seen the same h
+// a second ago.)  The outputs then mean nothing, which the status word says.  A CTA whose gate warps, or whose thread that sets the
+// mbarriers for the next round, gave up sends no whole h any more: a gate warp that gave up sends none, and in the second
+// kernel, whose gate warps never wait, they see `late` behind the barrier.  So no mbarrier receives more than it expects, and the
+// waits of the other CTAs run out in their turn, once per warp.
 __device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity) {
     for (uint32_t i = 0; i < kRecWaitLimit; ++i) {
         uint32_t ok;
@@ -200,7 +211,7 @@ __device__ __forceinline__ void rec_project(const RecInput& in, int T, int B, in
 template <int H, int R, int PQ>
 __global__ void __launch_bounds__(kRecThreads, 1)
 lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,
-                      float* __restrict__ cs, int32_t* status, const RecInput in) {
+                      float* __restrict__ cs, int32_t* status, int drop_exchange, const RecInput in) {
     using Y = RecLayout<H, R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemQuads][2][kRecThreads]
@@ -279,13 +290,14 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
     }
     cluster_arrive();  // every CTA of the cluster runs, its barriers set, before anybody stores into another one
     cluster_wait();
-    bool waiting = true;
     for (int t = 0; t < T; ++t) {
         if (t > 0) {
-            if (waiting && !wait_cluster(smem_u32(full + (t & 1)), step_parity(t))) {
-                waiting = false;  // the rest is computed from what is there: every CTA goes through all steps
-                *late = 1;
-                if (status != nullptr) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
+            if (!__all_sync(kFullMask, wait_cluster(smem_u32(full + (t & 1)), step_parity(t)))) {
+                *late = 1;  // (see wait_cluster)
+                if (lane == 0 && status != nullptr) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
+                __syncwarp();
+                for (; t < T; ++t) asm volatile("barrier.sync 1, %0;" ::"n"(kRecThreads) : "memory");
+                break;
             }
             if (tid == 0 && t + 2 < T) mbar_arrive_expect_tx(full + (t & 1), kPhaseBytes);
             const float* h_t = h_s + ((t & 1) * kRecCluster + slice * (Y::KT / Y::U)) * Y::BP;
@@ -369,8 +381,10 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
             for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(kFullMask, hval, quad * 4 + k);
             const uint32_t to = h_off + static_cast<uint32_t>(((t + 1) & 1) * (kRecCluster * Y::BP)) * 4;
             const uint32_t bar = bar_off + static_cast<uint32_t>((t + 1) & 1) * 8;
+            if (!drop_exchange) {
 #pragma unroll
-            for (int k = 0; k < Y::Sends; ++k) store_async4(dst[k] + to, v[0], v[1], v[2], v[3], dst[k] + bar);
+                for (int k = 0; k < Y::Sends; ++k) store_async4(dst[k] + to, v[0], v[1], v[2], v[3], dst[k] + bar);
+            }
         }
         if (item && row < B) {
             const int64_t o = (static_cast<int64_t>(t) * B + row) * H + j0 + iu;
@@ -379,9 +393,10 @@ lstm_recurrent_kernel(const float* __restrict__ pre, const float* __restrict__ w
         }
         fetch(t + kRecAhead);  // (into the place of step t - 1, which all gate threads have read)
     }
+    if (PQ == 0) asm volatile("cp.async.wait_all;" ::: "memory");
     cluster_arrive();  // nobody leaves while another CTA may still store into its shared memory
     cluster_wait();
-    if (*late) {       // (after a wait that ran out, stores may be under way)
+    if (*late) {       // (stores of h that nobody waited for may be under way; they arrive within microseconds)
         const unsigned long long t0 = clock64();
         while (clock64() - t0 < 400000ull) {
         }
@@ -426,7 +441,7 @@ struct PairLayout {
 template <int H, int RH>
 __global__ void __launch_bounds__(kPairThreads, 1)
 lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restrict__ w_hh, int T, int B, float* __restrict__ hs,
-                           float* __restrict__ cs, int32_t* status) {
+                           float* __restrict__ cs, int32_t* status, int drop_exchange) {
     using Y = PairLayout<H, RH>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ulonglong2* w_s = reinterpret_cast<ulonglong2*>(smem_raw);                  // [SmemK][2][kPairFma]
@@ -434,7 +449,7 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
     float* part = h_s + Y::h_floats;                                            // [half][KQ][RH][U][4]
     float* pre_s = part + Y::part_floats;                                       // [step % 3][half][RH][4][U]
     uint64_t* full = reinterpret_cast<uint64_t*>(pre_s + Y::pre_floats);        // [half][buffer]
-    int* late = reinterpret_cast<int*>(full + 4);                               // a wait ran out
+    volatile int* late = reinterpret_cast<int*>(full + 4);                      // a wait ran out
     const int tid = threadIdx.x, lane = tid & 31;
     const int rank = static_cast<int>(cluster_rank());
     const int b0 = static_cast<int>(blockIdx.x / kRecCluster) * (2 * RH);
@@ -442,7 +457,7 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
     constexpr uint32_t kPhaseBytes = RH * H * 4;                                // one half of h
 
     if (tid == 0) {
-        *late = 0;
+        *late = drop_exchange;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             mbar_init(full + i, 1);
@@ -474,19 +489,27 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
         }
         cluster_arrive();  // every CTA of the cluster runs, its barriers set, before anybody stores into another one
         cluster_wait();
-        bool waiting = true;
+        auto give_up = [&](int u) {  // (see wait_cluster)
+            *late = 1;
+            if (lane == 0 && status != nullptr) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
+            __syncwarp();
+            for (; u < 2 * T; ++u) asm volatile("barrier.sync %0, %1;" ::"r"(1 + (u & 1)), "n"(kPairFma + Y::GateWarps * 32) : "memory");
+        };
+        // Whether all lanes' waits ended well is asked after the multiplications, where it replaces a __syncwarp; at H = 512 there is no
+        // register to keep the answer (64 steps of 64 rows, us: asked first 140.3 at H = 256, 338.6 at 512; later 139.4, 340.3).
+        constexpr bool kVoteFirst = H == 512;
         // slice s lies in the part of CTA s * KT / U
         const float* h_mine = h_s + (slice * Y::KT / Y::U) * Y::BP + slice * Y::KT % Y::U;
 #pragma unroll 1
         for (int u = 2; u < 2 * T; ++u) {                                       // (step, half)
             const int t = u >> 1, half = u & 1;
             uint64_t* bar = full + half * 2 + (t & 1);
-            if (waiting && !wait_cluster(smem_u32(bar), step_parity(t))) {
-                waiting = false;  // the rest is computed from what is there: every CTA goes through all steps
-                *late = 1;
-                if (status != nullptr) atomicOr(status, FB_STATUS_WAIT_TIMEOUT);
+            const bool ok = wait_cluster(smem_u32(bar), step_parity(t));
+            if (kVoteFirst && !__all_sync(kFullMask, ok)) {
+                give_up(u);
+                break;
             }
-            if (tid == 0 && t + 2 < T) mbar_arrive_expect_tx(bar, kPhaseBytes);
+            if (tid == 0 && ok && t + 2 < T) mbar_arrive_expect_tx(bar, kPhaseBytes);
             const float* h_t = h_mine + ((t & 1) * 2 + half) * (kRecCluster * Y::BP);
             unsigned long long acc[4][RH];
 #pragma unroll
@@ -529,7 +552,12 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
                 *reinterpret_cast<float2*>(part + (((half * Y::KQ + kq) * RH + r) * Y::U + unit + (lane >> 4)) * 4 + (odd ? 2 : 0)) =
                     make_float2(s0, s1);
             }
-            __syncwarp();
+            if (kVoteFirst) {
+                __syncwarp();
+            } else if (!__all_sync(kFullMask, ok)) {
+                give_up(u);
+                break;
+            }
             asm volatile("barrier.arrive %0, %1;" ::"r"(1 + half), "n"(kPairFma + Y::GateWarps * 32) : "memory");
         }
     } else {
@@ -604,6 +632,7 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
                             gate[2] = __fadd_rn(gate[2], s.z);
                             gate[3] = __fadd_rn(gate[3], s.w);
                         }
+                        const bool sends = item[half] >= 0 && *late == 0;
                         float sg[3] = {gate[0], gate[1], gate[3]};
                         sigmoid_f32_n(sg);
                         const float ig = sg[0], fgt = sg[1], og = sg[2], gg = tanhf(gate[2]);
@@ -615,7 +644,7 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
                             for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(kFullMask, hval, (lane & ~3) + k);
                             const uint32_t to = h_off + static_cast<uint32_t>((((t + 1) & 1) * 2 + half) * (kRecCluster * Y::BP) + (i & ~3)) * 4;
                             const uint32_t bar = bar_off + static_cast<uint32_t>(half * 2 + ((t + 1) & 1)) * 8;
-                            if (item[half] >= 0) {
+                            if (sends) {
 #pragma unroll
                                 for (int k = 0; k < 4; ++k) store_async4(dst[k] + to, v[0], v[1], v[2], v[3], dst[k] + bar);
                             }
@@ -636,7 +665,7 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
     }
     cluster_arrive();  // nobody leaves while another CTA may still store into its shared memory
     cluster_wait();
-    if (*late) {       // (after a wait that ran out, stores may be under way)
+    if (*late) {       // (stores of h that nobody waited for may be under way; they arrive within microseconds)
         const unsigned long long t0 = clock64();
         while (clock64() - t0 < 400000ull) {
         }
@@ -669,13 +698,13 @@ template <int H, int R>
 static int launch_narrow(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     static_assert(RecLayout<H, R>::bytes <= 227 * 1024, "shared memory of one CTA");
     return launch_rec(lstm_recurrent_kernel<H, R, 0>, kRecThreads, RecLayout<H, R>::bytes, R, B, true, st, pre, w_hh, T, B, hs, cs, status,
-                      RecInput{});
+                      t_rec_drop, RecInput{});
 }
 template <int H, int R>
 static int launch_pair(const float* pre, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     using Y = PairLayout<H, R / 2>;
     static_assert(R % 2 == 0 && Y::bytes <= 227 * 1024, "shared memory of one CTA");
-    return launch_rec(lstm_recurrent_pair_kernel<H, R / 2>, kPairThreads, Y::bytes, R, B, true, st, pre, w_hh, T, B, hs, cs, status);
+    return launch_rec(lstm_recurrent_pair_kernel<H, R / 2>, kPairThreads, Y::bytes, R, B, true, st, pre, w_hh, T, B, hs, cs, status, t_rec_drop);
 }
 
 // Rows per cluster: the fewest that let all clusters run at once (seven clusters of sixteen whole SMs fit a B200; more clusters
@@ -704,7 +733,7 @@ bool lstm_one_launch(int T, int B, int K, int H) {
 template <int R, int PQ>
 static int launch_one(const RecInput& in, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     return launch_rec(lstm_recurrent_kernel<256, R, PQ>, kRecThreads, ProjLayout<256, R, PQ>::bytes(T), R, B, false, st,
-                      static_cast<const float*>(nullptr), w_hh, T, B, hs, cs, status, in);
+                      static_cast<const float*>(nullptr), w_hh, T, B, hs, cs, status, t_rec_drop, in);
 }
 template <int R>
 static int launch_one_depth(const RecInput& in, const float* w_hh, int T, int B, float* hs, float* cs, int32_t* status, cudaStream_t st) {

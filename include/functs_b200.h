@@ -245,7 +245,9 @@ int functs_b200_lstm_forward_mode(const float* x, const float* w_ih, const float
 
 /* Debugging switches (name -> value); returns FB_ERR_NOT_FOUND for an unknown name.
  *   "yolo_prune": 0 makes functs_b200_yolo_postprocess keep every candidate above the score threshold instead of
- *                 those that reach the image's score floor (default 1; the outputs are the same either way). */
+ *                 those that reach the image's score floor (default 1; the outputs are the same either way).
+ *   "lstm_drop_exchange": 1 makes the CTAs of the LSTM's cluster recurrence send each other nothing, in the calls of this
+ *                 thread: every wait gives up and FB_STATUS_WAIT_TIMEOUT is set (default 0). */
 int functs_b200_debug_set(const char* name, int32_t value);
 
 /* ---- C5: YOLACT-style mask assembly ------------------------------------------------------------ */

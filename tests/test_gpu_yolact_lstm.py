@@ -222,6 +222,28 @@ def test_lstm_recurrence_shapes(fb, seq, batch, inputs, hidden):
         assert float((a.cpu().double() - b).abs().max()) < 3e-6
 
 
+@pytest.mark.parametrize("seq,batch,hidden,mode", [
+    (2, 1, 256, 0), (25, 1, 256, 0), (25, 14, 256, 0), (25, 2, 256, 3), (40, 9, 512, 3),    # warps that multiply and apply gates
+    (3, 15, 256, 0), (40, 50, 256, 0), (40, 20, 512, 0), (64, 64, 512, 0),                  # warps that only do one of the two
+])
+def test_lstm_waits_that_run_out(fb, seq, batch, hidden, mode):
+    """With the exchange between the CTAs dropped every wait runs out: the kernel goes through its steps all the same, reports it and
+    leaves the context usable.  (A warp that runs ahead of the gate warps then would leave them at a barrier for ever.)"""
+    x, w_ih, w_hh, b_ih, b_hh = W.make_lstm_inputs(seq, batch, hidden)
+    mod = fb.workloads.LSTM(w_ih, w_hh, b_ih, b_hh)
+    want = [t.clone() for t in mod(x, mode=mode)]
+    lib = fb._lib.lib
+    fb._lib.check(lib.functs_b200_debug_set(b"lstm_drop_exchange", 1), "debug_set")
+    try:
+        with pytest.raises(fb.FunctsB200Error, match="wait ran out"):
+            mod(x, mode=mode)
+    finally:
+        fb._lib.check(lib.functs_b200_debug_set(b"lstm_drop_exchange", 0), "debug_set")
+    mod._status.zero_()
+    for got, ref in zip(mod(x, mode=mode), want):
+        assert torch.equal(got, ref)
+
+
 def test_lstm_rejects_unsupported_hidden(fb):
     x, w_ih, w_hh, b_ih, b_hh = W.make_lstm_inputs(2, 2, 64)
     with pytest.raises(fb.FunctsB200Error):
