@@ -223,8 +223,7 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
     }
     const float* src = scores_cm + (static_cast<int64_t>(img) * num_classes + cls) * num_priors;
     const int n = block_select_topk_sampled<kSsdNmsThreads, kSsdSelCap>(src, score_thr, num_priors, topk, hist_base, hist_shift, sm, cand);
-    // (block_select_topk ends with a barrier when n > 1; make the hand-over explicit)
-    __syncthreads();
+    __syncthreads();  // behind the selection's last stores and reads, as it asks
 
     const float* bimg = boxes + static_cast<int64_t>(img) * num_priors * 4;
     float4 mybox = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -536,17 +536,30 @@ __device__ __noinline__ int block_select_dense_outlined(const float* s, bool vec
     return block_select_topk_binned<NT, SELCAP, 8>(DenseScores{s, thr, vec4}, n, topk, hist_base, hist_shift, *sm);
 }
 
-// Same result as block_select_topk_binned for 1 <= c <= kCandCap keys in shared memory, by one counting sort: a key's bucket and its
-// place among the bucket's arrivals come from one atomic, the buckets' places from a scan, and every key counts the larger ones of
-// its own bucket (a key or two, unless many scores are nearly equal: then the general form takes over).  sm.hist is zero.
+// The `want` largest of n keys, in order.  room: the next power of two.
+template <int NT>
+__device__ __noinline__ void block_sort_bucket(const uint64_t* keys, int n, uint64_t* room, int want, uint64_t* out) {
+    const int n2 = next_pow2(n);
+    for (int i = threadIdx.x; i < n2; i += NT) room[i] = i < n ? keys[i] : 0ull;
+    __syncthreads();
+    bitonic_sort_desc<NT>(room, n2);
+    for (int i = threadIdx.x; i < want; i += NT) out[i] = room[i];
+}
+
+// Same result as block_select_topk_binned for 1 <= c <= kCandCap keys in shared memory (whose place it uses), by one counting sort: a
+// key's bucket and its place among the bucket's arrivals come from one atomic, the buckets' places from a scan, and every key counts
+// the larger ones of its own bucket, a key or two unless many scores are nearly equal.  Buckets behind the top-k are not looked
+// at, and those that lie in it hold no more than topk keys; one that reaches beyond it is sorted where it holds many.
+// sm.hist is zero.  The caller synchronises before it reads sm.sel or uses binlist, hist or the keys' place again.
 template <int NT, int SELCAP>
-__device__ __forceinline__ int block_select_topk_list(const uint64_t* keys, int c, int topk, uint32_t hist_base, int hist_shift,
+__device__ __forceinline__ int block_select_topk_list(uint64_t* keys, int c, int topk, uint32_t hist_base, int hist_shift,
                                                       SelectSmem<SELCAP>& sm) {
-    constexpr int kPer = kCandCap / NT, kBuckets = kHistBins / NT, kCrowd = 32;
+    constexpr int kPer = kCandCap / NT, kBuckets = kHistBins / NT, kCrowd = 128;
     static_assert(kCandCap % NT == 0 && kBuckets % 4 == 0 && kCandCap <= kBinListCap, "whole keys and buckets per thread");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint64_t k[kPer];
     int d[kPer], arrival[kPer];
+    if (tid == 0) sm.inbin = 0;
 #pragma unroll
     for (int u = 0; u < kPer; ++u) {
         if (u * NT >= c) break;  // uniform
@@ -558,17 +571,13 @@ __device__ __forceinline__ int block_select_topk_list(const uint64_t* keys, int 
     __syncthreads();
     int4* mine = reinterpret_cast<int4*>(sm.hist) + tid * (kBuckets / 4);
     int h[kBuckets], sum = 0;
-    bool crowd = false;
 #pragma unroll
     for (int q = 0; q < kBuckets / 4; ++q) {
         const int4 v = mine[q];
         h[4 * q] = v.x; h[4 * q + 1] = v.y; h[4 * q + 2] = v.z; h[4 * q + 3] = v.w;
     }
 #pragma unroll
-    for (int q = 0; q < kBuckets; ++q) {
-        sum += h[q];
-        crowd |= h[q] > kCrowd;
-    }
+    for (int q = 0; q < kBuckets; ++q) sum += h[q];
     int incl = sum;  // from the higher buckets down
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -576,10 +585,21 @@ __device__ __forceinline__ int block_select_topk_list(const uint64_t* keys, int 
         if (lane + o < 32) incl += v;
     }
     if (lane == 0) sm.red_cnt[warp] = incl;
-    if (__syncthreads_or(crowd ? 1 : 0)) return block_select_topk_outlined<NT, SELCAP, 2>(ListKeys{keys}, c, topk, &sm);
+    __syncthreads();
 #pragma unroll
     for (int w = 0; w < NT / 32; ++w) incl += w > warp ? sm.red_cnt[w] : 0;
     int start = incl - sum;
+    if (sum > kCrowd && start < topk && incl > topk) {  // one thread at most
+        int above = start;
+#pragma unroll
+        for (int q = kBuckets - 1; q >= 0; --q) {
+            if (h[q] > kCrowd && above < topk && above + h[q] > topk) {
+                sm.above = above;
+                sm.inbin = h[q];
+            }
+            above += h[q];
+        }
+    }
 #pragma unroll
     for (int q = kBuckets - 1; q >= 0; --q) {
         const int n = h[q];
@@ -599,10 +619,15 @@ __device__ __forceinline__ int block_select_topk_list(const uint64_t* keys, int 
         arrival[u] = first;
     }
     __syncthreads();
+    int upto = topk;  // keys of buckets that start here or later are not ranked below
+    if (sm.inbin > 0) {
+        upto = sm.above;
+        block_sort_bucket<NT>(sorted + upto, sm.inbin, keys, topk - upto, sm.sel + upto);
+    }
 #pragma unroll
     for (int u = 0; u < kPer; ++u) {
         if (u * NT >= c) break;
-        if (u * NT + tid >= c || arrival[u] >= topk) continue;
+        if (u * NT + tid >= c || arrival[u] >= upto) continue;
         const int end = d[u] > 0 ? sm.hist[d[u] - 1] : c;
         int rank = arrival[u];
         if (end - rank > 1)

@@ -138,6 +138,31 @@ def test_ssd_crowded_lists(fb, spread, size):
             assert torch.equal(a.cpu(), b)
 
 
+@pytest.mark.parametrize("higher,crowd,priors", [(0, 33, 700), (0, 128, 700), (150, 60, 700), (0, 201, 700), (199, 129, 700), (72, 129, 700),
+                                                 (200, 300, 700), (0, 1024, 1024), (7, 1000, 1500), (250, 400, 5000), (100, 900, 9000)])
+@pytest.mark.parametrize("spread", [0.0, 1e-4])
+def test_ssd_crowded_scores(fb, higher, crowd, priors, spread):
+    """Many equal or nearly equal scores (one bucket of the selection): in the top-k, across its end, behind it, and more than the
+    candidate list holds.  Equal scores come in the order of the priors."""
+    g = torch.Generator().manual_seed(18)
+    pri = torch.cat([torch.rand(priors, 2, generator=g) * 3000, torch.full((priors, 2), 20.0)], dim=1)
+    conf = torch.full((2, priors, 4), -4.0)
+    conf[..., 3] = 4.0
+    for img in range(2):
+        for cls in range(2):
+            at = torch.randperm(priors, generator=g)
+            high, same = at[:higher], at[higher:higher + crowd]
+            conf[img, high, cls] = 8.0 + 4.0 * torch.rand(high.numel(), generator=g)
+            conf[img, same, cls] = 4.5 + spread * torch.rand(same.numel(), generator=g)
+    mod = fb.workloads.SSDBBox(pri, score_thr=0.01, topk=200, clamp_max=4000.0)
+    boxes, dets, ids, counts = mod.forward_padded(torch.zeros(2, priors, 4), conf)
+    scores = mod._bufs[2].cpu().permute(0, 2, 1).contiguous()
+    o = W.SSDPost(score_thr=0.01, topk=200)
+    for i, got in enumerate(mod.unpad(dets, ids, counts)):
+        for a, b in zip(got, o.post_single(boxes[i].cpu(), scores[i])):
+            assert torch.equal(a.cpu(), b)
+
+
 def test_ssd_golden_decode(fb):
     """Decode against the fixture written by the reference's delta2bbox (clamp 320)."""
     import os
