@@ -672,6 +672,23 @@ lstm_recurrent_pair_kernel(const float* __restrict__ pre, const float* __restric
     }
 }
 
+// A single step multiplies nothing: its gates, without a cluster that fetches weights and sets up an exchange.
+constexpr int kFirstThreads = 128;
+__global__ void __launch_bounds__(kFirstThreads)
+lstm_first_step_kernel(const float* __restrict__ pre, int B, int H, float* __restrict__ hs, float* __restrict__ cs) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * kFirstThreads + threadIdx.x;  // (row, unit)
+    const int64_t row = i / H;
+    pdl_wait();  // the projection (read with __ldcg: a __ldg could be moved up across this)
+    if (row >= B) return;
+    const float* p = pre + row * (4 * H) + (i - row * H);
+    float sg[3] = {__ldcg(p), __ldcg(p + H), __ldcg(p + 3 * H)};
+    const float gg = tanhf(__ldcg(p + 2 * H));
+    sigmoid_f32_n(sg);
+    const float c = __fadd_rn(__fmul_rn(sg[1], 0.0f), __fmul_rn(sg[0], gg));  // (a forget gate that is NaN stays one)
+    hs[i] = __fmul_rn(sg[2], tanhf(c));
+    cs[i] = c;
+}
+
 template <class... KP, class... A>
 static int launch_rec(void (*kernel)(KP...), int threads, size_t smem, int rows, int B, bool after, cudaStream_t st, A... args) {
     FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "lstm_recurrent attr"));
@@ -722,6 +739,11 @@ static int launch_rec_rows(const float* pre, const float* w_hh, int T, int B, fl
 
 int launch_lstm_recurrent(const float* pre, const float* w_hh, int T, int B, int H, float* hs, float* cs, int32_t* status, cudaStream_t st) {
     FB_REQUIRE(H == 256 || H == 512, "lstm recurrence: hidden size %d not supported (256 or 512)", H);
+    if (T == 1) {
+        const int64_t blocks = (static_cast<int64_t>(B) * H + kFirstThreads - 1) / kFirstThreads;
+        return launch_after(lstm_first_step_kernel, dim3(static_cast<unsigned>(blocks)), dim3(kFirstThreads), 0, st, true, "lstm_first_step launch",
+                            pre, B, H, hs, cs);
+    }
     return H == 512 ? launch_rec_rows<512>(pre, w_hh, T, B, hs, cs, status, st) : launch_rec_rows<256>(pre, w_hh, T, B, hs, cs, status, st);
 }
 

@@ -205,6 +205,7 @@ def test_lstm_inputs_that_are_not_finite(fb, seq, batch, inputs, hidden, mode):
 @pytest.mark.parametrize("seq,batch,inputs,hidden", [
     (1, 1, 1, 256), (17, 1, 128, 256), (56, 7, 129, 256), (16, 7, 300, 256), (32, 14, 512, 256), (15, 9, 385, 256),  # one launch
     (57, 1, 256, 256), (33, 14, 100, 256), (9, 1, 256, 512),          # a projection in front of the steps
+    (1, 15, 64, 256), (1, 3, 64, 512), (1, 71, 100, 512),             # a single step: the gates alone
     (3, 15, 64, 256), (4, 29, 64, 512), (2, 50, 64, 256), (9, 63, 64, 512),  # halves of two to five rows, some of them empty
 ])
 def test_lstm_recurrence_shapes(fb, seq, batch, inputs, hidden):
