@@ -3,7 +3,8 @@
 // Group 1 (ssd_softmax_decode_kernel): softmax over every confidence row with the background column dropped
 // (functs/benchmark/ai_model/ssd/ssd_bbox.py:268) fused with the box decode and its strided in-place clamp
 // (ssd_bbox.py:121-154).  A CTA stages a tile of conf rows in shared memory with one bulk (TMA) copy when the
-// tile is 16-byte aligned, each thread reduces one row (row stride 81 words: conflict-free), and the scores are
+// tile is 16-byte aligned; one thread reduces a row (row stride 81 words: conflict-free), or two threads a long one: the first hands
+// the sum of its columns over in s_inv, the second goes on adding in column order and leaves the reciprocal there.  The scores are
 // written class-major so that group 2 reads contiguous runs.
 //
 // Group 2 (ssd_class_nms_kernel): the loop over classes (ssd_bbox.py:163-172 + :212 per class) with every
@@ -16,22 +17,26 @@
 namespace fb {
 
 constexpr int kSsdTile = 128;     // priors per CTA in group 1
-constexpr int kSsdTileThreads = 2 * kSsdTile;
+// Conf columns from which two threads share a row.  One / two threads, us per launch: 21 columns, 48 images of 8732 priors 14.8 / 20.9,
+// of 24 564 priors 39.5 / 52; 61 columns, 48 of 8732 39.4 / 41.3; 81 columns 50.6 / 49.6, 91 58.7 / 56.8.
+constexpr int kSsdTwoParts = 70;
 constexpr int kSsdMaxRow = 96;    // maximum conf columns (C + 1) supported by the register/smem layout
 
 // dynamic smem: [tile rows * ncol floats][8-byte mbarrier]
-// Two threads per row, in two groups of four warps: the first columns and the last ones (fewer: the second group also decodes the box and
-// finishes the sum, which runs in column order whoever adds).  A tile takes 41 KB of shared memory, so that one thread per row left
-// five warps per scheduler.
-__global__ void __launch_bounds__(kSsdTileThreads)
+// PARTS = 2: two threads per row, in two groups of four warps: the first columns and the last ones (fewer: the second group also decodes
+// the box and finishes the sum, which runs in column order whoever adds).  A tile of 81 columns takes 41 KB of shared memory, so that
+// one thread per row leaves five warps per scheduler; shorter rows leave room for more CTAs (launch_ssd_softmax_decode).
+template <int PARTS>
+__global__ void __launch_bounds__(PARTS * kSsdTile)
 ssd_softmax_decode_kernel(const float* __restrict__ loc, const float* __restrict__ conf, const float* __restrict__ priors,
                           int num_priors, int num_classes, float clamp_max, float* __restrict__ boxes,
                           float* __restrict__ scores_cm, int use_bulk, int32_t* __restrict__ clear, int num_clear) {
+    constexpr int kThreads = PARTS * kSsdTile;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ float s_max[2][kSsdTile];
+    __shared__ float s_max[PARTS][kSsdTile];
     __shared__ __align__(16) float s_inv[kSsdTile];  // first the sum over the first columns
     // the words the class kernel of a ragged call counts in (none otherwise): cleared here, so that no memset runs
-    for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * kSsdTileThreads + threadIdx.x; i < num_clear; i += gridDim.x * gridDim.y * kSsdTileThreads)
+    for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x; i < num_clear; i += gridDim.x * gridDim.y * kThreads)
         clear[i] = 0;
     const int ncol = num_classes + 1;
     float* tile = reinterpret_cast<float*>(smem_raw);
@@ -59,18 +64,18 @@ ssd_softmax_decode_kernel(const float* __restrict__ loc, const float* __restrict
         staged = __syncthreads_and(staged ? 1 : 0) != 0;
     }
     if (!staged) {
-        for (int i = threadIdx.x; i < nfl; i += kSsdTileThreads) tile[i] = __ldg(gsrc + i);
+        for (int i = threadIdx.x; i < nfl; i += kThreads) tile[i] = __ldg(gsrc + i);
         __syncthreads();
     }
 
     const int p = p0 + r;
-    const int split = ncol * 3 / 5, first = part == 0 ? 0 : split, last = part == 0 ? split : ncol;  // this thread's columns
+    const int split = PARTS == 1 ? ncol : ncol * 3 / 5, first = part == 0 ? 0 : split, last = part == 0 ? split : ncol;  // this thread's columns
     constexpr int kAtOnce = 8;  // columns: loads and exponentials side by side
     const int whole = first + (last - first) / kAtOnce * kAtOnce;
     const bool live = r < rows;
     float* row = tile + r * ncol;
+    float mx = -INFINITY;  // (a row of nothing but NaN: exp(NaN) below)
     if (live) {
-        float mx = -INFINITY;  // (a row of nothing but NaN: exp(NaN) below)
         for (int c = first; c < whole; c += kAtOnce) {
             float v[kAtOnce];
 #pragma unroll
@@ -78,13 +83,12 @@ ssd_softmax_decode_kernel(const float* __restrict__ loc, const float* __restrict
             mx = fmaxf(mx, fmaxf(fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3])), fmaxf(fmaxf(v[4], v[5]), fmaxf(v[6], v[7]))));
         }
         for (int c = whole; c < last; ++c) mx = fmaxf(mx, row[c]);
-        s_max[part][r] = mx;
+        if (PARTS == 2) s_max[part][r] = mx;
     }
-    __syncthreads();
-    float mx = 0.0f;
+    if (PARTS == 2) __syncthreads();
+    float sum = 0.0f;
     if (live) {
-        mx = fmaxf(s_max[0][r], s_max[1][r]);
-        float sum = 0.0f;
+        if (PARTS == 2) mx = fmaxf(s_max[0][r], s_max[PARTS - 1][r]);
         for (int c = first; c < whole; c += kAtOnce) {
             float e[kAtOnce];
 #pragma unroll
@@ -100,9 +104,9 @@ ssd_softmax_decode_kernel(const float* __restrict__ loc, const float* __restrict
             row[c] = e;
             if (part == 0) sum = __fadd_rn(sum, e);
         }
-        if (part == 0) s_inv[r] = sum;
+        if (PARTS == 2 && part == 0) s_inv[r] = sum;
     }
-    if (live && part == 1) {
+    if (live && part == PARTS - 1) {
         // decode (centre/size priors, variances 0.1 / 0.2), then clamp x to [0, max], y to [0, max]
         const float4 pr = __ldg(reinterpret_cast<const float4*>(priors) + p);
         const float4 d = __ldg(reinterpret_cast<const float4*>(loc) + static_cast<int64_t>(img) * num_priors + p);
@@ -118,25 +122,24 @@ ssd_softmax_decode_kernel(const float* __restrict__ loc, const float* __restrict
         o.w = min_nan(max_nan(__fadd_rn(gy, hh), 0.0f), clamp_max);
         reinterpret_cast<float4*>(boxes)[static_cast<int64_t>(img) * num_priors + p] = o;
     }
-    __syncthreads();
-    if (live && part == 1) {
-        float sum = s_inv[r];
+    if (PARTS == 2) __syncthreads();
+    if (PARTS == 2 && live && part == 1) {
+        sum = s_inv[r];
         int c = split;
         for (; c + 4 <= ncol; c += 4) {
             const float e0 = row[c], e1 = row[c + 1], e2 = row[c + 2], e3 = row[c + 3];
             sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, e0), e1), e2), e3);
         }
         for (; c < ncol; ++c) sum = __fadd_rn(sum, row[c]);
-        const float inv = __fdiv_rn(1.0f, sum);
-        s_inv[r] = inv;
+        s_inv[r] = __fdiv_rn(1.0f, sum);
     }
-    __syncthreads();
+    if (PARTS == 2) __syncthreads();
     // class-major store: for a fixed class consecutive threads write consecutive priors
     if (live) {
-        const float inv = s_inv[r];
+        const float inv = PARTS == 2 ? s_inv[r] : __fdiv_rn(1.0f, sum);
         float* dst = scores_cm + static_cast<int64_t>(img) * num_classes * num_priors + p;
 #pragma unroll 4
-        for (int c = part; c < num_classes; c += 2) dst[static_cast<int64_t>(c) * num_priors] = __fmul_rn(row[c], inv);
+        for (int c = part; c < num_classes; c += PARTS) dst[static_cast<int64_t>(c) * num_priors] = __fmul_rn(row[c], inv);
     }
 }
 
@@ -406,12 +409,15 @@ static int launch_ssd_softmax_decode(const float* loc, const float* conf, const 
                          ((static_cast<int64_t>(kSsdTile) * ncol) % 4 == 0) &&
                          ((static_cast<int64_t>(num_priors % kSsdTile) * ncol) % 4 == 0);
     const size_t smem = ((static_cast<size_t>(kSsdTile) * ncol * 4 + 15) / 16) * 16 + 16;
-    FB_TRY(check_cuda(cudaFuncSetAttribute(ssd_softmax_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(smem)),
-                      "ssd_softmax_decode attr"));
-    dim3 grid((num_priors + kSsdTile - 1) / kSsdTile, batch);
-    ssd_softmax_decode_kernel<<<grid, kSsdTileThreads, smem, st>>>(loc, conf, priors, num_priors, num_classes, clamp_max, boxes, scores_cm,
-                                                            aligned ? 1 : 0, clear, num_clear);
+    auto run = [&](auto kernel, int threads) {
+        FB_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+                          "ssd_softmax_decode attr"));
+        const dim3 grid((num_priors + kSsdTile - 1) / kSsdTile, batch);
+        kernel<<<grid, threads, smem, st>>>(loc, conf, priors, num_priors, num_classes, clamp_max, boxes, scores_cm, aligned ? 1 : 0, clear,
+                                            num_clear);
+        return FB_OK;
+    };
+    FB_TRY(ncol >= kSsdTwoParts ? run(ssd_softmax_decode_kernel<2>, 2 * kSsdTile) : run(ssd_softmax_decode_kernel<1>, kSsdTile));
     count_launch();
     return check_launch("ssd_softmax_decode_kernel");
 }

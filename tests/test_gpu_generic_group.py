@@ -6,7 +6,7 @@ from typing import List
 import pytest
 import torch
 
-from region_program import address, interleaved
+from tests.region_program import address, interleaved
 
 pytestmark = pytest.mark.gpu
 

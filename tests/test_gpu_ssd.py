@@ -117,6 +117,26 @@ def test_ssd_nan_in_the_deltas_stays_in_the_boxes(fb):
     assert torch.equal(got[0].cpu().nan_to_num(nan=-7.0), want[0].nan_to_num(nan=-7.0))
 
 
+@pytest.mark.parametrize("classes", [1, 2, 6, 7, 8, 24, 68, 69, 70, 79, 90, 95])
+@pytest.mark.parametrize("priors", [1, 127, 260])
+def test_ssd_softmax_of_every_width(fb, classes, priors):
+    """Rows that one thread reduces and rows that two share, with and without a last group of columns, in tiles that the bulk copy
+    takes and in others.  A score is exp / sum in fp32: 20 * 2^-24 for an exponential (2 ulp, and its argument's rounding: 2^-20 for
+    |x - max| < 32), the same once more in the sum, `classes` additions, a reciprocal and a product."""
+    g = torch.Generator().manual_seed(classes)
+    pri = torch.cat([torch.rand(priors, 2, generator=g) * 300, torch.rand(priors, 2, generator=g) * 50 + 1], dim=1)
+    loc, conf = torch.randn(3, priors, 4, generator=g), torch.randn(3, priors, classes + 1, generator=g) * 2.0
+    conf[1, 0, -1] = float("inf")
+    conf[2, 0, 0] = float("nan")
+    boxes, scores = fb.ops.ssd_softmax_decode(loc.cuda(), conf.cuda(), pri.cuda(), 300.0)
+    want = conf.double().softmax(-1)[..., :-1].permute(0, 2, 1)
+    got = scores.cpu().double()
+    assert torch.equal(got.isnan(), want.isnan())
+    ok = ~want.isnan()
+    assert bool(((got - want).abs()[ok] <= want[ok] * (classes + 44) * 2.0 ** -24 + 1e-30).all())
+    assert torch.equal(boxes.cpu().isnan(), torch.zeros_like(loc, dtype=torch.bool)) and float(boxes.max()) <= 300.0
+
+
 @pytest.mark.parametrize("spread,size", [(0.0, 40.0), (3.0, 40.0), (40.0, 40.0), (500.0, 40.0), (None, 40.0), (None, 11.0), (4e20, 1e19)])
 def test_ssd_crowded_lists(fb, spread, size):
     """Lists from one heap of boxes (every pair suppresses) over partly and hardly overlapping ones to staircases, in which every

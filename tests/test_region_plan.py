@@ -5,7 +5,7 @@ import subprocess
 
 import pytest
 
-from region_program import Load, Program, address, interleaved
+from tests.region_program import Load, Program, address, interleaved
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "functs_b200", "csrc")
 EACH, AHEAD, WINDOW = 0, 1, 2
