@@ -251,13 +251,20 @@ def swapped(x: torch.Tensor):
 
 
 @pytest.mark.parametrize("rows", [606208, 606209, 607231, 700001])
-@pytest.mark.parametrize("off", [0, 1, 2])
+@pytest.mark.parametrize("view", ["whole", "unaligned", "last element of the storage"])
 @pytest.mark.parametrize("fn", [swapped, first_of_three])
-def test_interleaved_regions_of_one_tensor(env, fn, rows, off):
-    """Loads that step through one tensor as the output is stepped through are fetched as one run: whole and ragged blocks, and
-    tensors off a 16-byte boundary.  (Where a run ends: test_region_plan.)"""
+def test_interleaved_regions_of_one_tensor(env, fn, rows, view):
+    """Loads that step through one tensor as the output is stepped through are fetched as one run: whole and ragged blocks, a tensor
+    off a 16-byte boundary, and one whose last word is the last that the loads reach."""
     g = torch.Generator().manual_seed(16)
-    check(env, fn, (torch.randn(rows * 3 + off, generator=g).cuda()[off:].view(rows, 3),))
+    size = rows * 3
+    if view == "whole":
+        x = torch.randn(rows, 3, generator=g).cuda()
+    elif view == "unaligned":
+        x = torch.randn(size + 1, generator=g).cuda()[1:].view(rows, 3)
+    else:
+        x = torch.randn(size + 2, generator=g).cuda()[2:].view(rows, 3)
+    check(env, fn, (x,))
 
 
 @pytest.mark.parametrize("width,bases", [(2, [1]), (2, [0, 0]), (4, [2, 0]), (5, [4, 0, 1]), (6, [3]), (7, [6]), (7, [0, 5]), (8, [7]),
