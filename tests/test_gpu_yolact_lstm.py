@@ -245,6 +245,30 @@ def test_lstm_waits_that_run_out(fb, seq, batch, hidden, mode):
         assert torch.equal(got, ref)
 
 
+@pytest.mark.parametrize("seq,batch,inputs,hidden", [(3, 5, 63, 256), (2, 6, 130, 256), (3, 8, 80, 256)])
+def test_lstm_projection_of_ragged_depth_with_inputs_that_are_not_finite(fb, seq, batch, inputs, hidden):
+    """Depths that fill no k-tile in the tensor-core projection, which mode 0 leaves to the one launch at these sizes."""
+    test_lstm_inputs_that_are_not_finite(fb, seq, batch, inputs, hidden, 3)
+
+
+@pytest.mark.parametrize("seq,batch,inputs,hidden,mode", [
+    (2, 1, 256, 256, 3), (3, 8, 80, 256, 3), (5, 14, 500, 256, 3),  # one and two rows per cluster behind a projection
+    (2, 150, 64, 256, 0), (3, 90, 64, 512, 0),                      # more clusters than run at once
+])
+def test_lstm_projection_and_steps(fb, seq, batch, inputs, hidden, mode):
+    """Against fp64, bound as in test_lstm_recurrence_shapes."""
+    g = torch.Generator().manual_seed(seq * 100 + batch)
+    bound = hidden ** -0.5
+    w = [(torch.rand(*s, generator=g) * 2 - 1) * bound for s in ((4, inputs, hidden), (4, hidden, hidden), (4, 1, hidden), (4, 1, hidden))]
+    x = torch.randn(seq, batch, inputs, generator=g)
+    want = W.LSTMSeq(*[t.double() for t in w])(x.double())
+    mod = fb.workloads.LSTM(*w)
+    got = mod(x, mode=mode)
+    assert mod.kernels_last_call == 2
+    for a, b in zip(got, want):
+        assert float((a.cpu().double() - b).abs().max()) < 3e-6
+
+
 def test_lstm_rejects_unsupported_hidden(fb):
     x, w_ih, w_hh, b_ih, b_hh = W.make_lstm_inputs(2, 2, 64)
     with pytest.raises(fb.FunctsB200Error):
