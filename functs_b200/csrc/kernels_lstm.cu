@@ -83,7 +83,7 @@ lstm_input_proj_simt_kernel(const float* __restrict__ x, const float* __restrict
 
 static inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
-// what mode 0 means: the combination measured fastest at the configured shape (T = 64, B = 64, H = 512)
+// what mode 0 means beyond the one launch: the combination measured fastest at T = 64, B = 64, H = 512
 constexpr int kLstmDefaultMode = 3;
 
 }  // namespace fb

@@ -229,7 +229,8 @@ int functs_b200_ragged_split(const float* dets, const int64_t* labels, const fun
  * x [T, B, I]; w_ih [4, I, H]; w_hh [4, H, H]; b_ih, b_hh [4, H]; hs, cs [T, B, H]; gate order i, f, g, o;
  * h0 = c0 = 0.  scratch: functs_b200_lstm_scratch_bytes(T, B, I, H).
  * Two launches: the hoisted input projection (tcgen05, 3xTF32; large ones split their operands in a launch of their own first)
- * and the recurrence (clusters of 16 CTAs, a few batch rows each). */
+ * and the recurrence (clusters of 16 CTAs, a few batch rows each; a single step is a kernel of its gates alone).  Short sequences of
+ * few rows with H = 256 are one launch, whose clusters form their own projection in fp32. */
 int64_t functs_b200_lstm_scratch_bytes(int32_t seq_len, int32_t batch, int32_t input, int32_t hidden);
 int functs_b200_lstm_forward(const float* x, const float* w_ih, const float* w_hh, const float* b_ih,
                              const float* b_hh, int32_t seq_len, int32_t batch, int32_t input, int32_t hidden,
@@ -238,7 +239,8 @@ int functs_b200_lstm_forward(const float* x, const float* w_ih, const float* w_h
  * the recurrence (the on-device check of the tensor-core results); 2 = tcgen05 (3xTF32) for both — the recurrence then
  * is one persistent kernel whose CTAs keep their slice of w_hh resident in shared memory and exchange h[t] as pre-tiled
  * TF32 hi / lo operands (needs batch == 64); 3 = tensor-core projection + CUDA-core recurrence.  A shape a tensor-core
- * path does not take falls back to the CUDA-core form of that GEMM. */
+ * path does not take falls back to the CUDA-core form of that GEMM.  Mode 0 is the one launch where a call is short enough for it,
+ * and mode 3 otherwise. */
 int functs_b200_lstm_forward_mode(const float* x, const float* w_ih, const float* w_hh, const float* b_ih,
                                   const float* b_hh, int32_t seq_len, int32_t batch, int32_t input, int32_t hidden,
                                   float* hs, float* cs, int32_t* status, void* scratch, void* stream, int32_t mode);
