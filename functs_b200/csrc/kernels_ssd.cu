@@ -254,9 +254,11 @@ ssd_class_nms_kernel(const float* __restrict__ boxes, const float* __restrict__ 
     if (tame) {
         // (the histogram of the selection and the rest of its boundary list are free)
         static_assert(sizeof(uint16_t) * PairLists::kPairs <= sizeof(sm.hist) &&
-                          (sizeof(float4) + sizeof(float)) * kSsdSelCap + sizeof(uint16_t) * PairLists::kHits <= sizeof(sm.binlist),
+                          (sizeof(float4) + sizeof(float)) * kSsdSelCap + sizeof(uint16_t) * PairLists::kHits <= sizeof(sm.binlist) &&
+                          sizeof(uint32_t) * kSsdNmsThreads * kSsdWords <= sizeof(uint64_t) * kCandCap,
                       "the pair lists reuse the selection's memory");
-        const PairLists pl{reinterpret_cast<uint16_t*>(sm.hist), reinterpret_cast<uint16_t*>(sarea + kSsdSelCap), pair_count, or_words};
+        const PairLists pl{reinterpret_cast<uint16_t*>(sm.hist), reinterpret_cast<uint16_t*>(sarea + kSsdSelCap), reinterpret_cast<uint32_t*>(cand),
+                           pair_count, or_words};
         window = pair_tables<kSsdWords>(mybox, myarea, n, iou_thr, pc);
         done = block_nms_pairs<kSsdWords>(sxy, sarea, pc, window, n, iou_thr, thr_lo, thr_hi, pl, keep_words);
     }

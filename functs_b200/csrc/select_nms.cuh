@@ -893,17 +893,54 @@ __device__ __forceinline__ PairWindow pair_tables(const float4 me, float area, i
 
 // Greedy NMS over up to 256 boxes by a list of the candidate pairs: every thread adds its own, all threads test them in turn
 // (a thread that walks its own candidates waits for the one with the most: 12 300 cycles of 49 500 of an SSD class, of which 230
-// candidates and 20 real pairs remain), and one warp resolves the few pairs that are left, in rounds without a block barrier.
+// candidates and 20 real pairs remain), and one warp resolves the few pairs that are left, in rounds without a block barrier; more than
+// kHits are walked through in order (block_nms_walk).
 // A box is certainly kept once every box that could suppress it is certainly removed, and certainly removed once a certainly kept
 // box suppresses it; both sets only grow, every round settles at least the first undecided box, and the fixed point is the
 // greedy result.  Returns false, the same for all threads, where a list does not fit; keep_words is then untouched.
 struct PairLists {
-    static constexpr int kPairs = 4096, kHits = 1024;
+    static constexpr int kPairs = 4096, kHits = 64;
     uint16_t* pairs;  // [kPairs] i << 8 | j, i < j
     uint16_t* hits;   // [kHits]
+    uint32_t* rows;   // [NT * WORDS] may lie where `pc` does
     int* count;       // [2]: pairs, hits; zero, with a barrier since
     uint32_t* words;  // [2 * WORDS]
 };
+// Greedy NMS of more pairs than that: bit k of `mine` stands for the pair t + k * NT, which suppresses.  The pairs become rows of bits, and
+// one warp goes from one kept box that suppresses others to the next, some hundred cycles each.  (Rounds take the longer the more pairs
+// there are and the longer their chains.  Whole calls of 32 images x 20 classes of 200 boxes in a row, us, rounds of one warp / of the block
+// / this: scores that fall along the row, each box over the next 173 / 201 / 33, over the next five 216 / 144 / 33; random scores 47 / 39
+// / 33.  50 boxes in a row, 49 pairs: one warp's rounds 36, 45 where the block formed rows.)
+template <int WORDS>
+__device__ __noinline__ void block_nms_walk(const uint16_t* pairs, uint32_t mine, uint32_t* rows, uint32_t* suppressors, int n, uint32_t* keep_words) {
+    constexpr int NT = 32 * WORDS;
+    const int t = threadIdx.x, lane = t & 31;
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) rows[w * NT + t] = 0u;
+    if (t < WORDS) suppressors[t] = 0u;
+    __syncthreads();
+    for (; mine != 0u; mine &= mine - 1u) {
+        const uint32_t e = pairs[t + (__ffs(mine) - 1) * NT];
+        atomicOr(&rows[(e >> 8) * WORDS + ((e >> 5) & 7u)], 1u << (e & 31u));
+        atomicOr(&suppressors[e >> 13], 1u << ((e >> 8) & 31u));
+    }
+    __syncthreads();
+    if (t >= 32) return;
+    const int word = lane < WORDS ? lane : 0;
+    uint32_t next = lane < WORDS ? suppressors[lane] : 0u, gone = 0u;
+    for (int left = n; left > 0; --left) {
+        const unsigned any = __ballot_sync(kFullMask, next != 0u);
+        if (any == 0u) break;
+        const int from = __ffs(any) - 1, bit = __shfl_sync(kFullMask, __ffs(next) - 1, from);
+        gone |= rows[(32 * from + bit) * WORDS + word];
+        if (lane == from) next &= next - 1u;
+        next &= ~gone;
+    }
+    if (lane < WORDS) {
+        const uint32_t there = n >= 32 * lane + 32 ? 0xffffffffu : n > 32 * lane ? (1u << (n - 32 * lane)) - 1u : 0u;
+        keep_words[lane] = there & ~gone;
+    }
+}
 template <int WORDS>
 __device__ __forceinline__ bool block_nms_pairs(const float4* sxy, const float* sarea, const PairCells<WORDS>& pc, const PairWindow& window,
                                                 int n, float thr, float thr_lo, float thr_hi, const PairLists& pl, uint32_t* keep_words) {
@@ -936,7 +973,9 @@ __device__ __forceinline__ bool block_nms_pairs(const float4* sxy, const float* 
     const int pairs = pl.count[0];
     if (pairs > PairLists::kPairs) return false;
     constexpr int kAtOnce = 2;
-    for (int p0 = t; p0 < pairs; p0 += kAtOnce * NT) {
+    static_assert(PairLists::kPairs <= 32 * NT, "a bit for every pair of a thread");
+    uint32_t suppress = 0u;
+    for (int p0 = t, k = 0; p0 < pairs; p0 += kAtOnce * NT, k += kAtOnce) {
         uint32_t e[kAtOnce];
         float inter[kAtOnce], uni[kAtOnce];
 #pragma unroll
@@ -954,6 +993,7 @@ __device__ __forceinline__ bool block_nms_pairs(const float4* sxy, const float* 
             // iou_exceeds for tame boxes: a positive intersection implies its guards
             if (p0 + u * NT >= pairs || !(inter[u] > 0.0f) || inter[u] < __fmul_rn(uni[u], thr_lo)) continue;
             if (inter[u] > __fmul_rn(uni[u], thr_hi) || __fdiv_rn(inter[u], uni[u]) > thr) {
+                suppress |= 1u << (k + u);
                 const int pos = atomicAdd(pl.count + 1, 1);
                 if (pos < PairLists::kHits) pl.hits[pos] = static_cast<uint16_t>(e[u]);
             }
@@ -961,8 +1001,9 @@ __device__ __forceinline__ bool block_nms_pairs(const float4* sxy, const float* 
     }
     __syncthreads();
     const int hits = pl.count[1];
-    if (hits > PairLists::kHits) return false;
-    if (warp == 0) {
+    if (hits > PairLists::kHits) {
+        block_nms_walk<WORDS>(pl.pairs, suppress, pl.rows, pl.words, n, keep_words);
+    } else if (warp == 0) {
         uint32_t* maybe = pl.words;          // boxes that a not-yet-removed box suppresses
         uint32_t* gone = pl.words + WORDS;   // boxes that a kept box suppresses
         if (lane < 2 * WORDS) pl.words[lane] = 0u;

@@ -183,6 +183,26 @@ def test_ssd_crowded_scores(fb, higher, crowd, priors, spread):
             assert torch.equal(a.cpu(), b)
 
 
+@pytest.mark.parametrize("n,step,size", [(64, 8, 32), (65, 8, 32), (66, 8, 32), (200, 8, 32),  # 63 to 65 pairs, and 199
+                                         (200, 4, 60), (150, 1, 60), (200, 1, 60)])          # 985, some 3000, more than the list holds
+@pytest.mark.parametrize("order", ["falling", "random"])
+def test_ssd_boxes_in_a_row(fb, n, step, size, order):
+    """Boxes over the next one, or the next few, in the order of their scores (the fate of every box hangs on the one before it) or in none."""
+    g = torch.Generator().manual_seed(n + step)
+    pri = torch.stack([100.0 + step * torch.arange(n), torch.full((n,), 60.0), torch.full((n,), float(size)), torch.full((n,), 40.0)], dim=1)
+    conf = torch.zeros(2, n, 3)
+    for img in range(2):
+        for cls in range(2):
+            conf[img, :, cls] = torch.linspace(4.0, 2.0, n) if order == "falling" else torch.linspace(4.0, 2.0, n)[torch.randperm(n, generator=g)]
+    mod = fb.workloads.SSDBBox(pri, score_thr=0.01, topk=200, clamp_max=4000.0)
+    boxes, dets, ids, counts = mod.forward_padded(torch.zeros(2, n, 4), conf)
+    scores = mod._bufs[2].cpu().permute(0, 2, 1).contiguous()
+    o = W.SSDPost(score_thr=0.01, topk=200)
+    for i, got in enumerate(mod.unpad(dets, ids, counts)):
+        for a, b in zip(got, o.post_single(boxes[i].cpu(), scores[i])):
+            assert torch.equal(a.cpu(), b)
+
+
 def test_ssd_golden_decode(fb):
     """Decode against the fixture written by the reference's delta2bbox (clamp 320)."""
     import os
