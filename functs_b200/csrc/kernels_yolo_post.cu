@@ -26,7 +26,6 @@ constexpr int kPostTop = 1024;     // largest topk
 constexpr int kPostPairs = 8192;
 constexpr int kPostCrowded = 64;   // keys of one score bucket beyond which ranks are not counted
 constexpr int kPostWords = kPostTop / 32;
-constexpr int kPostFewPairs = 512; // pairs that one warp resolves (five block barriers per round otherwise)
 
 struct RescanSlot {
     float so;  // objectness score
@@ -328,7 +327,6 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     const int img = blockIdx.x;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     sm.removed[t] = 0;
-    sm.blocked[t] = 0;
     if (t < kYoloClasses) {
         sm.cls_cursor[t] = 0;
         sm.cls_min_x[t] = 0xffffffffu;
@@ -446,7 +444,7 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     const int np = sm.npairs;
     if (np > kPostPairs) {
         post_dense(&sm, A.mask + static_cast<int64_t>(img) * kPostTop * kPostWords, m, reach, A.iou_thr, thr_lo, thr_hi);
-    } else if (np > kPostFewPairs) {
+    } else if (np > 0) {
         for (int round = 0; round <= m; ++round) {
             sm.blocked[t] = 0;
             __syncthreads();
@@ -465,31 +463,6 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
             __syncthreads();
             if (__syncthreads_or(t < m && !kept && sm.removed[t] == 0 ? 1 : 0) == 0) break;
         }
-    } else if (np > 0) {  // the same by one warp
-        if (warp == 0) {
-            volatile uint8_t *removed = sm.removed, *blocked = sm.blocked;
-            for (int round = 0; round <= m; ++round) {
-                for (int i = lane; i < np; i += 32) {
-                    const uint32_t pr = sm.pairs[i];
-                    if (removed[pr >> 16] == 0) blocked[pr & 0xffffu] = 1;
-                }
-                __syncwarp();
-                for (int i = lane; i < np; i += 32) {  // (what this loop removes is blocked: it removes nothing)
-                    const uint32_t pr = sm.pairs[i];
-                    if (removed[pr >> 16] == 0 && blocked[pr >> 16] == 0) removed[pr & 0xffffu] = 1;
-                }
-                __syncwarp();
-                bool open = false;
-                for (int i = lane; i < np; i += 32) {
-                    const uint32_t b = sm.pairs[i] & 0xffffu;
-                    open |= blocked[b] != 0 && removed[b] == 0;
-                }
-                if (!__any_sync(kFullMask, open)) break;
-                for (int i = lane; i < np; i += 32) blocked[sm.pairs[i] & 0xffffu] = 0;
-                __syncwarp();
-            }
-        }
-        __syncthreads();
     }
 
     // ---- outputs ----

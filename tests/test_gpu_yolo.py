@@ -10,6 +10,8 @@ Parity statement checked here:
         two runs part (a score order among the selected candidates, an IoU against the threshold) is shown in fp64
         to lie inside the last-ulp band in which CPU and GPU exp() differ (tests/tieband.py); anything else fails.
 """
+import math
+
 import pytest
 import torch
 
@@ -287,6 +289,27 @@ def test_yolo_one_call_form_at_its_edges(fb, batch, sizes, kind, topk):
         m = int(cnt[b])
         assert m == wf.numel() and torch.equal(flat[b, :m], wf) and torch.equal(labels[b, :m], wl) and torch.equal(dets[b, :m], wd)
         assert torch.equal(lists[b][0].cpu(), wd) and torch.equal(lists[b][1].cpu(), wl)
+
+
+@pytest.mark.parametrize("rows,width,height", [(1, 32.0, 6.0), (9, 32.0, 6.0), (19, 32.0, 6.0), (4, 28.0, 28.0), (6, 64.0, 20.0)])
+@pytest.mark.parametrize("order", ["falling", "random"])
+def test_yolo_boxes_in_rows(fb, rows, width, height, order):
+    """Boxes of one class over their neighbours, in the order of their scores (the fate of every box hangs on the one before it) or in none."""
+    g = torch.Generator().manual_seed(rows)
+    maps = [torch.full((2, 255, s, s), -9.0) for s in (13, 26, 52)]
+    score = torch.linspace(5.0, 2.0, rows * 52)
+    v = maps[2].view(2, 3, 85, 52, 52)[:, 0, :, :rows]
+    v[:, 0:2] = 0.0
+    v[:, 2], v[:, 3], v[:, 4] = math.log(width / 10.0), math.log(height / 13.0), 5.0
+    for img in range(2):
+        v[img, 5] = (score if order == "falling" else score[torch.randperm(rows * 52, generator=g)]).view(rows, 52)
+    cmaps = [m.cuda() for m in maps]
+    boxes, obj, cls, _, _ = fb.ops.yolo_decode(cmaps, 0.5, dense=True)
+    dets, labels, flat, cnt = [t.cpu() for t in fb.workloads.YOLOV3BBox().forward_padded(cmaps)]
+    for b in range(2):
+        wd, wl, wf = W.YOLOV3Post().post_single(boxes[b].cpu(), obj[b].cpu(), cls[b].cpu())
+        m = int(cnt[b])
+        assert m == wf.numel() and torch.equal(flat[b, :m], wf) and torch.equal(labels[b, :m], wl) and torch.equal(dets[b, :m], wd)
 
 
 def test_yolo_dense_class_scores_off_a_16_byte_boundary(fb):
