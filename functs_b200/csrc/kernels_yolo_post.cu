@@ -327,6 +327,7 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     const int img = blockIdx.x;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     sm.removed[t] = 0;
+    sm.blocked[t] = 0;
     if (t < kYoloClasses) {
         sm.cls_cursor[t] = 0;
         sm.cls_min_x[t] = 0xffffffffu;
@@ -445,9 +446,7 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
     if (np > kPostPairs) {
         post_dense(&sm, A.mask + static_cast<int64_t>(img) * kPostTop * kPostWords, m, reach, A.iou_thr, thr_lo, thr_hi);
     } else if (np > 0) {
-        for (int round = 0; round <= m; ++round) {
-            sm.blocked[t] = 0;
-            __syncthreads();
+        for (int round = 0; round <= m; ++round) {  // (blocked: zero)
             for (int i = t; i < np; i += kPostThreads) {
                 const uint32_t pr = sm.pairs[i];
                 if (sm.removed[pr >> 16] == 0) sm.blocked[pr & 0xffffu] = 1;
@@ -455,6 +454,7 @@ yolo_post_kernel(const __grid_constant__ YoloLevels L, const __grid_constant__ Y
             __syncthreads();
             const bool kept = t < m && sm.removed[t] == 0 && sm.blocked[t] == 0;
             sm.kept[t] = kept ? 1 : 0;
+            sm.blocked[t] = 0;
             __syncthreads();
             for (int i = t; i < np; i += kPostThreads) {
                 const uint32_t pr = sm.pairs[i];
