@@ -901,33 +901,49 @@ __device__ __forceinline__ PairWindow pair_tables(const float4 me, float area, i
 struct PairLists {
     static constexpr int kPairs = 4096, kHits = 64;
     uint16_t* pairs;  // [kPairs] i << 8 | j, i < j
-    uint16_t* hits;   // [kHits]
+    uint16_t* hits;   // [kHits], on a 4-byte boundary
     uint32_t* rows;   // [NT * WORDS] may lie where `pc` does
     int* count;       // [2]: pairs, hits; zero, with a barrier since
     uint32_t* words;  // [2 * WORDS]
 };
-// Greedy NMS of more pairs than that: bit k of `mine` stands for the pair t + k * NT, which suppresses.  The pairs become rows of bits, and
-// one warp goes from one kept box that suppresses others to the next, some hundred cycles each.  (Rounds take the longer the more pairs
-// there are and the longer their chains.  Whole calls of 32 images x 20 classes of 200 boxes in a row, us, rounds of one warp / of the block
-// / this: scores that fall along the row, each box over the next 173 / 201 / 33, over the next five 216 / 144 / 33; random scores 47 / 39
-// / 33.  50 boxes in a row, 49 pairs: one warp's rounds 36, 45 where the block formed rows.)
+// Greedy NMS of more pairs than that: bit k of `mine` stands for the pair t + k * NT, which suppresses.  One round by all threads settles
+// heaps around a best box each; the pairs that are still open become rows of bits, and one warp goes from one kept box that suppresses
+// others to the next, some hundred cycles each.  (More rounds take the longer the more pairs there are and the longer their chains.
+// Whole calls of 16 images x 80 classes of 200 boxes, us, rounds of one warp / of the block over rows / this: in a row with scores that
+// fall along it, each box over the next 326 / 259 / 54, over the next five 412 / 128 / 58, those with random scores 77 / 73 / 58; 50 heaps of
+// four boxes 33 / 34 / 32, without the round 39.  At 49 pairs in a row one warp takes 60, rows 79.)
 template <int WORDS>
-__device__ __noinline__ void block_nms_walk(const uint16_t* pairs, uint32_t mine, uint32_t* rows, uint32_t* suppressors, int n, uint32_t* keep_words) {
+__device__ __noinline__ void block_nms_walk(const uint16_t* pairs, uint32_t mine, uint32_t* rows, uint32_t* suppressors, uint32_t* words, int n,
+                                            uint32_t* keep_words) {
     constexpr int NT = 32 * WORDS;
     const int t = threadIdx.x, lane = t & 31;
+    uint32_t *maybe = words, *settled = words + WORDS;  // boxes that others suppress, and those whose suppressor nobody suppresses
 #pragma unroll
     for (int w = 0; w < WORDS; ++w) rows[w * NT + t] = 0u;
-    if (t < WORDS) suppressors[t] = 0u;
+    if (t < 2 * WORDS) words[t] = 0u;
+    else if (t < 3 * WORDS) suppressors[t - 2 * WORDS] = 0u;
+    __syncthreads();
+    auto has = [](const uint32_t* set, uint32_t b) { return ((set[b >> 5] >> (b & 31u)) & 1u) != 0u; };
+    for (uint32_t left = mine; left != 0u; left &= left - 1u) {
+        const uint32_t e = pairs[t + (__ffs(left) - 1) * NT];
+        atomicOr(&maybe[(e >> 5) & 7u], 1u << (e & 31u));
+    }
+    __syncthreads();
+    for (uint32_t left = mine; left != 0u; left &= left - 1u) {
+        const uint32_t e = pairs[t + (__ffs(left) - 1) * NT];
+        if (!has(maybe, e >> 8)) atomicOr(&settled[(e >> 5) & 7u], 1u << (e & 31u));
+    }
     __syncthreads();
     for (; mine != 0u; mine &= mine - 1u) {
         const uint32_t e = pairs[t + (__ffs(mine) - 1) * NT];
+        if (!has(maybe, e >> 8) || has(settled, e >> 8) || has(settled, e & 255u)) continue;
         atomicOr(&rows[(e >> 8) * WORDS + ((e >> 5) & 7u)], 1u << (e & 31u));
         atomicOr(&suppressors[e >> 13], 1u << ((e >> 8) & 31u));
     }
     __syncthreads();
     if (t >= 32) return;
     const int word = lane < WORDS ? lane : 0;
-    uint32_t next = lane < WORDS ? suppressors[lane] : 0u, gone = 0u;
+    uint32_t next = lane < WORDS ? suppressors[lane] : 0u, gone = settled[word];
     for (int left = n; left > 0; --left) {
         const unsigned any = __ballot_sync(kFullMask, next != 0u);
         if (any == 0u) break;
@@ -1002,7 +1018,7 @@ __device__ __forceinline__ bool block_nms_pairs(const float4* sxy, const float* 
     __syncthreads();
     const int hits = pl.count[1];
     if (hits > PairLists::kHits) {
-        block_nms_walk<WORDS>(pl.pairs, suppress, pl.rows, pl.words, n, keep_words);
+        block_nms_walk<WORDS>(pl.pairs, suppress, pl.rows, reinterpret_cast<uint32_t*>(pl.hits), pl.words, n, keep_words);
     } else if (warp == 0) {
         uint32_t* maybe = pl.words;          // boxes that a not-yet-removed box suppresses
         uint32_t* gone = pl.words + WORDS;   // boxes that a kept box suppresses
