@@ -633,20 +633,23 @@ static int launch_yolo_decode(const YoloDecodeArgs& a, int batch, bool pdl, cuda
     auto run = [&](auto kernel, int n) {
         return launch_after(kernel, dim3(static_cast<unsigned>(n)), dim3(kDecThreads), 0, st, pdl, "yolo_decode_kernel", a);
     };
-    if (a.floor == nullptr || a.boxes != nullptr) {  // large tiles once they make four CTAs per SM
-        const int large = tiles(4 * kDecThreads);
-        const bool is_large = large >= 4 * kNumSMs;
-        const int n = is_large ? large : tiles(kDecThreads);
+    // larger tiles once tiles of four slots per thread make four CTAs per SM
+    const int large = tiles(4 * kDecThreads), one = tiles(kDecThreads);
+    const bool is_large = large >= 4 * kNumSMs;
+    if (a.floor == nullptr || a.boxes != nullptr) {
+        const int n = is_large ? large : one;
         if (a.floor == nullptr) return is_large ? run(yolo_decode_kernel<4, true, true>, n) : run(yolo_decode_kernel<1, true, true>, n);
         return is_large ? run(yolo_decode_kernel<4, true, false>, n) : run(yolo_decode_kernel<1, true, false>, n);
     }
-    // The smallest tiles that all run at once (eight CTAs per SM): small ones end together, and a few that are left for a second wave
-    // wait for the first.  Beyond that, two slots per thread.  Whole call, us, with one / two / three / four slots: 12 images of
-    // 416 x 416 25 / 25 / - / 25, 24 33 / 31.5 / - / 33, 32 42 / 42 / 41 / 43, 64 63.5 / 65 / 67 / 70, 64 with few live boxes
-    // 46.5 / 43 / 43 / 43; 8 of 608 x 608 27 / 25 / 27 / 27, 30 62 / 62 / 65 / 67.
+    // Few tiles: one slot per thread, even in a second wave: a tile of two whose slots are all live takes twice as long, and the others end
+    // before it.  Whole call, us, one / two slots: 16 images of 416 x 416 at random 28.6 / 29.5, with few live boxes 25.3 / 24.0, of live
+    // boxes only 37.7 / 41.8, with 160 live slots in one run 68 / 86; 8 of 608 x 608 30.5 / 29.2, 26.9 / 24.9, 39.7 / 41.9, 99 / 119.
+    // Otherwise two, or three if only then all run at once (eight CTAs per SM): small tiles end together, and a few that are left for a
+    // second wave wait for the first.  One / two / three / four slots: 32 images of 416 x 416 42 / 42 / 41 / 43, 64 63.5 / 65 / 67 / 70, 64
+    // with few live boxes 46.5 / 43 / 43 / 43; 30 of 608 x 608 62 / 62 / 65 / 67.
+    if (!is_large) return run(yolo_decode_kernel<1, false, false>, one);
     constexpr int kWave = 8 * kNumSMs;
-    const int one = tiles(kDecThreads), two = tiles(2 * kDecThreads), three = tiles(3 * kDecThreads);
-    if (one <= kWave) return run(yolo_decode_kernel<1, false, false>, one);
+    const int two = tiles(2 * kDecThreads), three = tiles(3 * kDecThreads);
     if (two > kWave && three <= kWave) return run(yolo_decode_kernel<3, false, false>, three);
     return run(yolo_decode_kernel<2, false, false>, two);
 }

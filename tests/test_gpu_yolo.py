@@ -246,7 +246,8 @@ def test_one_call_postprocess_replays_from_a_cuda_graph(fb):
 
 @pytest.mark.parametrize("batch,sizes,kind,topk", [
     (1, (13, 26, 52), "plain", 1000), (2, (10, 20, 40), "plain", 1),  # one slot per thread
-    (16, (13, 26, 52), "plain", 1000), (20, (11, 22, 44), "crowded tile", 1000),  # two
+    (16, (13, 26, 52), "plain", 1000), (20, (11, 22, 44), "crowded tile", 1000),  # in more than a wave
+    (40, (13, 26, 52), "plain", 1000), (41, (13, 26, 52), "crowded tile", 500),   # two
     (30, (13, 26, 52), "plain", 1000), (30, (13, 26, 52), "crowded tile", 500),   # three
     (2, (13, 26, 52), "sampled high", 1000), (2, (13, 26, 52), "sampled low", 1000),  # hits in one run of sixteen only / in all others
     (2, (13, 26, 52), "crowded tile", 1000), (3, (4, 8, 16), "equal", 1000), (2, (13, 26, 52), "equal few", 1024),
