@@ -28,8 +28,12 @@ constexpr uint32_t kRecWaitLimit = 250000u;  // about a second: a poll that fail
 // Development switch (functs_b200_debug_set "lstm_drop_exchange"): in this thread's calls no CTA sends h, so that every wait runs out.
 static thread_local int t_rec_drop = 0;
 void lstm_set_drop_exchange(int on) { t_rec_drop = on ? 1 : 0; }
-// Steps and rows up to which a cluster forms its own projection: 0.18 us per row instead of the 12 us of a kernel in front of it.  Two
-// launches / one, us: 25 steps of one row 48 / 42, 32 of two 59 / 56, 64 of one 72 / 73, 64 of two 88 / 94.
+// Steps and rows up to which a cluster forms its own projection: 0.18 us per row at an input of 256 instead of a kernel in front of it, whose
+// time grows with the depth faster than the cluster's does.  Two launches / one, us between two calls, inputs of 64, 256 and 512: 4 steps of
+// one row 12.4 / 8.4, 17.1 / 10.4, 22.7 / 10.4; 25 of one 27.6 / 26.8, 33.0 / 28.8, 39.1 / 30.9; 56 of one 50.0 / 51.4, 55.5 / 55.5,
+// 62.2 / 61.7; 56 of seven 53.5 / 51.4, 59.6 / 55.5, 69.8 / 61.9; 32 of fourteen 41.1 / 39.1, 47.3 / 43.2, 56.9 / 53.5.  Beyond (256):
+// 64 of one 72 / 73 a call, 64 of two 88 / 94.  (Inputs of 16 and 64 lose up to 4 % from 40 steps of one row on.)  H = 512 has no such form:
+// half of its weights lie in shared memory, and the partial sums of rec_project would take 128 KB beside them.
 constexpr int kOneLaunchSteps = 56, kOneLaunchRows = 64;
 
 template <int H, int R>

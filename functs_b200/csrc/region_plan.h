@@ -30,8 +30,8 @@ struct RegionPlan {
 // Fetched ahead: float loads of interleaved regions, as many as leave six CTAs on an SM (normalisation of 1440 x 1920: 20.6 us
 // without, 18.5 with; one region per CTA gains nothing, 2500 boxes of 80 classes 16.5 us without, 19.3 with).
 // One run: rank 1, one tensor, every load at a place below the step, and room for a run as long as the output's (normalisation of
-// 800 x 1333, image in L2: 8.2 us, 10.2 with every load fetched ahead for itself; 1080 x 1440 10.3 / 12.3; 1440 x 1920, which DRAM
-// bounds, 16.5 / 16.5).
+// an image that is in L2, one run / every load fetched ahead for itself: 800 x 1333 8.2 / 10.2 us, 1080 x 1440 10.7 / 12.6; of a new image
+// each call, which DRAM bounds, 10.6 / 10.6 and 12.6 / 12.7; 1440 x 1920 17.1 / 17.2 and 18.1 / 19.0).
 inline RegionPlan region_plan(const functs_b200_rprogram& P, int rank, bool inter) {
     constexpr int kSlot = kRegionThreads * kRegionVec * 4;
     const int out_bytes = inter ? P.interleave * kSlot : 0;
